@@ -210,7 +210,7 @@ struct ScanParams {
     float* heap_d;                // [nq x k] the Start's pushes, in push order
     uint32_t* heap_id;
     uint32_t* left;               // [nq] queries left to the per-query scan kernel
-    uint32_t* left_n;             // [1] (zeroed before; n_items and queue follow it)
+    uint32_t* left_n;             // [1] (zeroed before; n_items, queue and hv_alloc follow it)
     uint32_t* vl_count;           // [n1] visits per cluster (zeroed before)
     uint32_t* vl;                 // [n1 x nq] visits of each cluster: q * q_order_stride + i
     uint32_t* items;              // [2 x item bound] (cluster, chunk of 64 list entries)
@@ -218,12 +218,21 @@ struct ScanParams {
     uint32_t* queue;              // [1] work counter (zeroed before)
     uint32_t* bm;                 // [nq x q_order_stride x bm_words] candidate bitmaps
     uint32_t bm_words;            // ceil(largest cluster / 32)
+    uint32_t bm_tile;             // 1: a work item's bitmaps are kept in shared memory first
+    uint32_t* vinfo;              // [nq x q_order_stride] class of each visit: 0 no candidate, n > 0
+                                  // candidates in bm, 1 << 31 heavy (no bitmap)
+    // heavy visits: values per (vector, warmup checkpoint) and (vector, horizontal block)
+    uint32_t* hv;                 // [hv_ncp + n_hblocks][hv_cap]
+    uint32_t hv_cap;              // columns (a multiple of 32)
+    uint32_t hv_ncp;              // warmup checkpoints
+    uint32_t* hv_alloc;           // [1] columns handed out, in units of 32 (zeroed before)
     uint32_t* out_ids;            // [nq x k]
     float* out_dists;             // [nq x k]
     uint32_t* out_counts;         // [nq]
     unsigned long long* stats;    // optional, SearchParams::stats layout
     uint32_t prep_qs;             // 1: the prep kernel stages each query row in shared memory
     uint32_t prep_qs_stride;      // floats per staged row
+    uint32_t r_qpc;               // replay: queries per CTA (1..8), one warp each
     uint32_t r_surv_cap;          // replay: survivors of one cluster's first warmup step it keeps
     uint32_t r_heap_cap;          // replay shared memory per warp: heap entries,
     uint32_t r_area_bytes;        // candidate offsets / final sort area,

@@ -124,7 +124,7 @@ struct Workspace {
     uint64_t qhi_cap = 0, qlo_cap = 0;
     int* d_gemm_err = nullptr;
     // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq + 4]:
-    // first_i | lim | left | left_n, n_items, queue), Start heaps, per-cluster visit lists and
+    // first_i | lim | left | left_n, n_items, queue, hv_alloc), Start heaps, per-cluster visit lists and
     // counters, work items, candidate bitmaps
     uint32_t* d_sc_qw = nullptr;
     uint64_t sc_qw_cap = 0;
@@ -140,6 +140,11 @@ struct Workspace {
     uint64_t sc_items_cap = 0;
     uint32_t* d_sc_bm = nullptr;
     uint64_t sc_bm_cap = 0;
+    // visit classes, values of heavy visits
+    uint32_t* d_sc_vi = nullptr;
+    uint64_t sc_vi_cap = 0;
+    uint32_t* d_sc_hv = nullptr;
+    uint64_t sc_hv_cap = 0;
 };
 
 // Mutable state of a tree index once Append / Delete have been used (PDXTreeIndex,

@@ -36,7 +36,8 @@ cudaError_t launch_top_level_tiled(const TopLevelParams& tp, uint32_t vtiles, in
 cudaError_t launch_start_batched(const StartParams& sp, int grid, cudaStream_t st);
 cudaError_t launch_scan(const ScanParams& sp, int bitmap_grid, cudaStream_t st, const cudaEvent_t* ev);
 uint64_t scan_item_bound(uint32_t nq, uint32_t stride, uint32_t n1);
-int scan_bitmap_occupancy();
+int scan_bitmap_occupancy(uint32_t bm_words);
+size_t scan_bitmap_smem(uint32_t bm_words);
 uint32_t scan_queries_per_cta();
 cudaError_t launch_row_sq(const float* x, uint32_t n, uint32_t d, float* out, cudaStream_t st);
 size_t probe_select_smem(uint32_t d, uint32_t n1, uint32_t cand_cap, uint32_t sort_cap);
@@ -237,7 +238,8 @@ void free_workspace(Workspace& w) {
                     w.d_st_cl, w.d_st_q, w.d_st_items, w.d_st_dist, w.d_pq_b16, w.d_pq_r16, w.d_pq_r8,
                     w.d_pq_r8s, w.d_pq_scores,
                     w.d_req, w.d_foff, w.d_rows, w.d_qhi, w.d_qlo, w.d_gemm_err, w.d_sc_qw, w.d_sc_q,
-                    w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm};
+                    w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
+                    w.d_sc_vi, w.d_sc_hv};
     for (void* q : ptrs) cudaFree(q);
     w = Workspace();
 }
@@ -1050,6 +1052,8 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
 // (tree indexes with a separate top level). Sets L.p.start_* when it ran; a batch outside its
 // limits leaves them unset and the scan runs Start itself.
 constexpr uint32_t kStartMinQueries = 32;
+constexpr uint32_t kHeavyPerQuery = 128;          // cluster-major scan: see run_scan_cluster_major
+constexpr uint64_t kHeavyMaxValues = 64ull << 20;  // 256 MB
 
 int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st) {
     L.p.start_row = nullptr;
@@ -1120,11 +1124,24 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
                                  align_up((uint64_t)bm_words * 4, 16) + 8ull * sp.r_surv_cap);
     sp.prep_qs_stride = (lv.d + 3) & ~3u;
     sp.prep_qs = (uint64_t)scan_queries_per_cta() * sp.prep_qs_stride * 4 + 9 * 1024 <= ix->max_smem ? 1u : 0u;
-    if ((uint64_t)sp.r_warp_bytes * scan_queries_per_cta() + 1024 > ix->max_smem) return PDXG_OK;
-    const int occ = scan_bitmap_occupancy();
+    // a replay CTA of 8 warps takes as few queries as still fill the GPU at 3 CTAs per SM, so that
+    // the heavy visits of a small batch are shared by more warps
+    sp.r_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + 3 * ix->num_sms - 1) / (3 * ix->num_sms));
+    if ((uint64_t)sp.r_warp_bytes * scan_queries_per_cta() + 2048 > ix->max_smem) return PDXG_OK;
+    const int occ = scan_bitmap_occupancy(bm_words);
     if (occ <= 0) return PDXG_OK;
     const uint64_t items = scan_item_bound(nq, stride, n1);
+    // values of heavy visits: columns for kHeavyPerQuery vectors a query on average (16-70 were
+    // measured); visits past them are left to the replay
+    uint32_t cps[kMaxCheckpoints];
+    sp.hv_ncp = warmup_checkpoints(lv.dv, cps, kMaxCheckpoints);
+    const uint64_t hv_rows = (uint64_t)sp.hv_ncp + lv.n_hblocks;
+    sp.hv_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((uint64_t)nq * kHeavyPerQuery, 32768), 1u << 20);
+    sp.hv_cap = (uint32_t)std::min<uint64_t>(sp.hv_cap, kHeavyMaxValues / hv_rows) / 32 * 32;
+    if (sp.hv_ncp > (uint32_t)kMaxCheckpoints) sp.hv_cap = 0;
     int rc;
+    if ((rc = dev_grow(w.d_sc_hv, w.sc_hv_cap, hv_rows * sp.hv_cap))) return rc;
+    if ((rc = dev_grow(w.d_sc_vi, w.sc_vi_cap, (uint64_t)nq * stride))) return rc;
     if ((rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
     if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 4))) return rc;
     if ((rc = dev_grow(w.d_sc_heap, w.sc_heap_cap, 2ull * nq * k))) return rc;
@@ -1157,6 +1174,10 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.left_n = w.d_sc_q + 3ull * nq;
     sp.n_items = w.d_sc_q + 3ull * nq + 1;
     sp.queue = w.d_sc_q + 3ull * nq + 2;
+    sp.hv_alloc = w.d_sc_q + 3ull * nq + 3;
+    sp.hv = w.d_sc_hv;
+    sp.vinfo = w.d_sc_vi;
+    sp.bm_tile = scan_bitmap_smem(bm_words) ? 1u : 0u;
     sp.heap_d = reinterpret_cast<float*>(w.d_sc_heap);
     sp.heap_id = w.d_sc_heap + (uint64_t)nq * k;
     sp.vl_count = w.d_sc_cl;

@@ -27,8 +27,12 @@
 //                        64 list entries; queries this path does not take go to a list for the
 //                        per-query kernel
 //   scan_bitmap_kernel : persistent CTAs over the items: candidate bitmaps with dp4a, exact
-//                        |q - x|^2 = |q|^2 + |x|^2 - 2 q.x over the first checkpoint's dims
-//   scan_replay_kernel : warp per query -- Warmup / Prune / MergeIntoHeap / result
+//                        |q - x|^2 = |q|^2 + |x|^2 - 2 q.x over the first checkpoint's dims; each
+//                        visit is classed as empty (no candidate), light (its bitmap kept) or
+//                        heavy (so many candidates that its warmup may pass the first step)
+//   scan_replay_kernel : warp per query -- Warmup / Prune / MergeIntoHeap / result, over the
+//                        visits that are not empty; the heavy visits of a CTA's queries are
+//                        first computed by all its warps together
 #include <cfloat>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -43,6 +47,10 @@ constexpr int kBitmapThreads = 256;
 constexpr int kBitmapBPW = 4;            // 32-vector blocks a bitmap warp holds at once
 constexpr int kScanWarps = 8;            // queries per prep / replay CTA
 constexpr uint32_t kOffPath = 0xFFFFFFFFu;
+constexpr uint32_t kHeavyBit = 0x80000000u;  // visit class: 0 empty, candidates of a light visit,
+                                             // kHeavyBit a heavy one
+constexpr uint32_t kHeavyList = 64;      // heavy visits a replay CTA computes ahead
+constexpr uint32_t kBitmapTileMax = 64 * 1024;  // bytes of a work item's bitmaps in shared memory
 
 // DIMENSIONS_FETCHING_SIZES (common.hpp:47-49)
 __constant__ uint32_t c_scan_fetch[kNumFetchSizes] = {16, 16, 32, 32, 32, 32, 64, 64, 64, 64,
@@ -264,7 +272,10 @@ __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid
     // kScanCQ list entries also opens the bitmap work item of that chunk
     for (uint32_t i = fi + 1 + lane; i < cnt; i += 32) {
         const uint32_t c = __ldg(ord + i);
-        if (lv.clusters[c].n == 0) continue;  // num_embeddings == 0 (searcher.hpp:662)
+        if (lv.clusters[c].n == 0) {  // num_embeddings == 0 (searcher.hpp:662)
+            sp.vinfo[(size_t)q * sp.q_order_stride + i] = 0u;
+            continue;
+        }
         const uint32_t slot = atomicAdd(sp.vl_count + c, 1u);
         sp.vl[(size_t)c * sp.nq + slot] = q * sp.q_order_stride + i;
         if (slot % kScanCQ == 0) {
@@ -296,14 +307,19 @@ __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid
 // CTA = one work item: up to 64 visits of one cluster. Warp w holds the first-checkpoint words
 // of vector blocks w, w + 8, ... (lane = vector) in registers with |x|^2, and loops over the
 // item's queries: 4 dp4a give q.x, and the ballot of |x|^2 - 2 q.x < lim is the 32-bit word of
-// that block in the query's bitmap. Lane j keeps the word of query j mod 32 and the 32 words are
-// stored together.
+// that block in the query's bitmap. Lane j keeps the word of query j mod 32 and the 32 words go
+// to the item's bitmaps in shared memory together (sp.bm_tile; clusters too large for that write
+// all words to global memory). Once the cluster is done the CTA knows every visit's candidates:
+// most visits have none, and only the bitmaps of light visits are written out.
 __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __grid_constant__ ScanParams sp) {
     __shared__ uint4 qv[kScanCQ];
     __shared__ int32_t ql[kScanCQ];
     __shared__ uint32_t qe[kScanCQ];
+    __shared__ uint32_t qcnt[kScanCQ];
     __shared__ uint32_t item;
+    extern __shared__ uint32_t tile[];  // [kScanCQ][bm_words | 1]
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t ts = sp.bm_words | 1u;  // odd row stride: 32 rows of one column hit distinct banks
     constexpr uint32_t kWarps = kBitmapThreads / 32;
     const DevLevel& lv = sp.l1;
     const uint32_t g1 = sp.g1;
@@ -324,6 +340,7 @@ __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __gri
                                          g1 > 3 ? __ldg(w + 3) : 0u);
             ql[threadIdx.x] = sp.lim[q];
             qe[threadIdx.x] = e;
+            qcnt[threadIdx.x] = 0;
         }
         __syncthreads();
         const DevCluster cl = lv.clusters[c];
@@ -363,14 +380,37 @@ __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __gri
                 if ((j & 31) == 31 || j + 1 == nqc) {
                     const uint32_t jj = (j & ~31u) + lane;
                     if (jj <= j) {
-                        const size_t base = (size_t)qe[jj] * sp.bm_words;
+                        uint32_t* row = sp.bm_tile ? tile + jj * ts : sp.bm + (size_t)qe[jj] * sp.bm_words;
+                        uint32_t cnt = 0;
 #pragma unroll
                         for (int b = 0; b < kBitmapBPW; ++b) {
                             const uint32_t blk = b0 + b * kWarps;
-                            if (blk < nb) sp.bm[base + blk] = word[b];
+                            if (blk < nb) {
+                                row[blk] = word[b];
+                                cnt += __popc(word[b]);
+                            }
                         }
+                        if (cnt) atomicAdd(&qcnt[jj], cnt);
                     }
                 }
+            }
+        }
+        __syncthreads();
+        // class of every visit of the item; a warmup can pass its first step only when fewer than
+        // ceil(0.8 n) vectors reach the bound, and the candidates hold every vector below it
+        const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
+        if (threadIdx.x < nqc) {
+            const uint32_t cnt = qcnt[threadIdx.x];
+            const uint32_t info = (sp.cp1 < lv.dv && n - cnt < needed) ? kHeavyBit : cnt;
+            sp.vinfo[qe[threadIdx.x]] = info;
+            qcnt[threadIdx.x] = info;
+        }
+        __syncthreads();
+        if (sp.bm_tile) {
+            for (uint32_t j = warp; j < nqc; j += kWarps) {
+                const uint32_t info = qcnt[j];
+                if (info == 0 || (info & kHeavyBit)) continue;
+                for (uint32_t w = lane; w < nb; w += 32) sp.bm[(size_t)qe[j] * sp.bm_words + w] = tile[j * ts + w];
             }
         }
         __syncthreads();
@@ -402,6 +442,27 @@ __device__ __forceinline__ uint32_t sq16(const uint4& q, const uint4& x, uint32_
     return sq4(q.w, x.w, acc);
 }
 
+// The vertical dims from cur0 on in 64-dim steps for a vector below every bound up to `cur` (the
+// horizontal blocks included), tested after each step.
+__device__ __forceinline__ bool scan_follow_vertical(const ScanParams& sp, const DevCluster& c, const uint32_t* qw,
+                                                     uint32_t v, uint32_t cur0, uint32_t cur, float top, uint32_t& raw,
+                                                     unsigned long long& vbytes) {
+    const DevLevel& lv = sp.l1;
+    const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off);
+    uint32_t cur_v = cur0;
+    while (cur_v < lv.dv) {
+        const uint32_t last = (cur_v + kHDim < lv.dv) ? cur_v + kHDim : lv.dv;
+        vbytes += last - cur_v;
+        for (uint32_t g = cur_v >> 2; g < ((last + 3) >> 2); ++g)
+            raw = sq4(qw[g], __ldg(vert + (size_t)g * c.n_pad + v), raw);
+        cur = (cur + kHDim < lv.d) ? cur + kHDim : lv.d;
+        cur_v = last;
+        if (!(raw < thr_u8(top, cur, lv, sp.ratios))) return false;
+        if (cur == lv.d) break;
+    }
+    return true;
+}
+
 // One survivor of the warmup bound at checkpoint cur0: the horizontal blocks, then the
 // remaining vertical dims in 64-dim steps, tested after each against the bound of the heap top
 // `top` fixed for the whole cluster (searcher.hpp:437-540). Returns whether it is still below
@@ -427,19 +488,7 @@ __device__ __forceinline__ bool scan_follow(const ScanParams& sp, const DevClust
             if (!(raw < thr_u8(top, cur, lv, sp.ratios))) return false;
         }
     }
-    const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off);
-    uint32_t cur_v = cur0;
-    while (cur_v < lv.dv) {
-        const uint32_t last = (cur_v + kHDim < lv.dv) ? cur_v + kHDim : lv.dv;
-        vbytes += last - cur_v;
-        for (uint32_t g = cur_v >> 2; g < ((last + 3) >> 2); ++g)
-            raw = sq4(qw[g], __ldg(vert + (size_t)g * c.n_pad + v), raw);
-        cur = (cur + kHDim < lv.d) ? cur + kHDim : lv.d;
-        cur_v = last;
-        if (!(raw < thr_u8(top, cur, lv, sp.ratios))) return false;
-        if (cur == lv.d) break;
-    }
-    return true;
+    return scan_follow_vertical(sp, c, qw, v, cur0, cur, top, raw, vbytes);
 }
 
 // Positions of the set bits of one word per lane (word index w_rel of a group of 32 words),
@@ -456,13 +505,83 @@ __device__ __forceinline__ uint32_t scan_bits_to_offsets(uint32_t word, uint32_t
     return total;
 }
 
+// Values of vector v of a heavy visit into column `out` (row stride sp.hv_cap): row s < ncp is the
+// running distance at warmup checkpoint s, row ncp + b the sum of horizontal block b. They do not
+// depend on the query's heap, so the loads of 64 vertical dims, then of three blocks, are in flight
+// together (8 dims and two blocks: 152 against 108 us for the replay of a 777-query batch). Returns
+// the full distance.
+__device__ __forceinline__ uint32_t heavy_column(const ScanParams& sp, const DevCluster& c, const uint32_t* qw,
+                                                 uint32_t v, uint32_t* out) {
+    const DevLevel& lv = sp.l1;
+    const uint32_t* col = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off) + v;
+    const uint32_t groups = (lv.dv + 3) >> 2;
+    uint32_t raw = 0, s = 0, next = sp.cp1;
+    for (uint32_t g0 = 0; g0 < groups; g0 += 16) {
+        uint32_t x[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) x[t] = g0 + t < groups ? __ldg(col + (size_t)(g0 + t) * c.n_pad) : 0u;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            if (g0 + t < groups) {
+                raw = sq4(qw[g0 + t], x[t], raw);
+                if ((g0 + t + 1) * 4 >= next) {  // checkpoints are multiples of 16 dims, the last is d_v
+                    out[(size_t)s * sp.hv_cap] = raw;
+                    ++s;
+                    next += c_scan_fetch[s < kNumFetchSizes ? s : kNumFetchSizes - 1];
+                    if (next > lv.dv) next = lv.dv;
+                }
+            }
+        }
+    }
+    out += (size_t)sp.hv_ncp * sp.hv_cap;
+    const uint4* row = reinterpret_cast<const uint4*>(sp.arena + c.hor_off) + (size_t)v * 4;
+    const size_t bstride = (size_t)c.n_pad * 4;  // uint4 per block
+    for (uint32_t b0 = 0; b0 < lv.n_hblocks; b0 += 3) {
+        uint4 x[3][4];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                x[u][t] = b0 + u < lv.n_hblocks ? __ldg(row + (b0 + u) * bstride + t) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            if (b0 + u < lv.n_hblocks) {
+                const uint4* qh = reinterpret_cast<const uint4*>(qw + lv.qw_hoff + (b0 + u) * 16);
+                uint32_t sum = 0;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) sum = sq16(qh[t], x[u][t], sum);
+                out[(size_t)(b0 + u) * sp.hv_cap] = sum;
+                raw += sum;
+            }
+        }
+    }
+    return raw;
+}
+
+// A heavy visit needs the running distance of all its vectors at up to every warmup checkpoint and
+// then a long survivor path for most of them. Done by the query's own warp at the visit's turn that
+// is a chain of several hundred dependent loads: 1-2 % of the queries of a 777-query batch on the
+// 1M x 1024 SQ8 tree took about 400 us there and set the kernel's time. Here the CTA's warps first
+// share out the 32-vector blocks of its queries' heavy visits (HeavyList), and the replay reads the
+// values; a visit that finds no room in the list or in sp.hv runs its warmup in the warp.
+// A vector can only be merged when its full distance is below the bound at all d dims, at most
+// that of the heap top after the Start: those vectors are marked in the visit's bitmap, and a
+// visit without any changes nothing.
+struct HeavyList {
+    uint32_t n;
+    uint32_t warp[kHeavyList], visit[kHeavyList];
+    uint32_t base[kHeavyList];  // first column / 32 in sp.hv
+    uint32_t end[kHeavyList];   // 32-vector blocks of the list up to and with this visit
+    uint32_t thr0[kScanWarps];  // bound at all d dims of each warp's heap top after the Start
+};
+
 __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const __grid_constant__ ScanParams sp) {
     extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ HeavyList HL;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t q = blockIdx.x * kScanWarps + warp;
-    if (q >= sp.nq) return;  // whole warp
-    const uint32_t fi = sp.first_i[q];
-    if (fi == kOffPath) return;
+    // warps past r_qpc own no query (no shared-memory region either) and only share the heavy visits
+    const uint32_t q = blockIdx.x * sp.r_qpc + warp;
+    const uint32_t fi = warp < sp.r_qpc && q < sp.nq ? sp.first_i[q] : kOffPath;
     const DevLevel& lv = sp.l1;
     uint8_t* base = smem + (size_t)warp * sp.r_warp_bytes;
     ReplayWarp R;
@@ -474,37 +593,81 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
     R.sbits = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(R.cand) + sp.r_area_bytes);
     R.sv_pos = R.sbits + (sp.bm_words + 3) / 4 * 4;
     R.sv_d = R.sv_pos + sp.r_surv_cap;
-    const uint32_t kq = sp.q_k ? __ldg(sp.q_k + q) : sp.k;
     const uint32_t stride = sp.q_order_stride;
-    for (uint32_t w = lane; w < sp.nwords; w += 32) R.qw[w] = __ldg(sp.qwords + (size_t)q * sp.nwords + w);
-    for (uint32_t j = lane; j < kq; j += 32) {
-        R.hd[j] = __ldg(sp.heap_d + (size_t)q * sp.k + j);
-        R.hid[j] = __ldg(sp.heap_id + (size_t)q * sp.k + j);
+    const uint32_t* ord = sp.q_order + (size_t)q * stride;
+    const uint32_t* vis = sp.vinfo + (size_t)q * stride;
+    const uint32_t kq = fi == kOffPath ? 0u : (sp.q_k ? __ldg(sp.q_k + q) : sp.k);
+    const uint32_t cnt = fi == kOffPath ? 0u : __ldg(sp.q_order_count + q);
+    float top = 0.0f;
+    uint32_t slot = 0;
+    if (threadIdx.x == 0) HL.n = 0;
+    __syncthreads();
+    if (fi != kOffPath) {
+        for (uint32_t w = lane; w < sp.nwords; w += 32) R.qw[w] = __ldg(sp.qwords + (size_t)q * sp.nwords + w);
+        for (uint32_t j = lane; j < kq; j += 32) {
+            R.hd[j] = __ldg(sp.heap_d + (size_t)q * sp.k + j);
+            R.hid[j] = __ldg(sp.heap_id + (size_t)q * sp.k + j);
+        }
+        __syncwarp();
+        warp_heap_top(R.hd, kq, top, slot);
+        if (lane == 0) HL.thr0[warp] = thr_u8(top, lv.d, lv, sp.ratios);
+        for (uint32_t i = fi + 1 + lane; i < cnt; i += 32) {
+            if (!(__ldg(vis + i) & kHeavyBit) || HL.n >= kHeavyList) continue;
+            // columns are handed out in units of 32; none is asked for once they are used up, so the
+            // counter stays far from its range
+            if (__ldcg(sp.hv_alloc) >= sp.hv_cap / 32) continue;
+            const uint32_t nb = (lv.clusters[__ldg(ord + i)].n + 31) >> 5;
+            const uint32_t col = atomicAdd(sp.hv_alloc, nb);
+            if (col + nb > sp.hv_cap / 32) continue;
+            const uint32_t at = atomicAdd(&HL.n, 1u);
+            if (at >= kHeavyList) continue;
+            HL.warp[at] = warp;
+            HL.visit[at] = i;
+            HL.base[at] = col;
+            HL.end[at] = nb;
+        }
     }
-    __syncwarp();
+    __syncthreads();
+    const uint32_t n_heavy = HL.n < kHeavyList ? HL.n : kHeavyList;
+    if (n_heavy) {  // block-uniform
+        if (threadIdx.x == 0)
+            for (uint32_t j = 1; j < n_heavy; ++j) HL.end[j] += HL.end[j - 1];
+        __syncthreads();
+        uint32_t j = 0;
+        for (uint32_t b = warp; b < HL.end[n_heavy - 1]; b += kScanWarps) {
+            while (HL.end[j] <= b) ++j;
+            const uint32_t blk = b - (j ? HL.end[j - 1] : 0u);
+            const uint32_t hw = HL.warp[j];
+            const uint32_t hq = blockIdx.x * sp.r_qpc + hw;
+            const DevCluster c = lv.clusters[__ldg(sp.q_order + (size_t)hq * stride + HL.visit[j])];
+            const uint32_t v = blk * 32 + lane;
+            uint32_t full = 0xFFFFFFFFu;
+            if (v < c.n)
+                full = heavy_column(sp, c, reinterpret_cast<const uint32_t*>(smem + (size_t)hw * sp.r_warp_bytes), v,
+                                    sp.hv + ((size_t)(HL.base[j] + blk) << 5) + lane);
+            // statistics count the blocks of vectors that end up pruned too
+            const unsigned may = __ballot_sync(0xffffffffu, v < c.n && (sp.stats || full < HL.thr0[hw]));
+            if (lane == 0) sp.bm[((size_t)hq * stride + HL.visit[j]) * sp.bm_words + blk] = may;
+        }
+        __syncthreads();
+    }
+    if (fi == kOffPath) return;  // whole warp; no block-wide barrier follows
     uint4 q1 = make_uint4(0u, 0u, 0u, 0u);  // first checkpoint's query words (zero past g1)
     q1.x = R.qw[0];
     if (sp.g1 > 1) q1.y = R.qw[1];
     if (sp.g1 > 2) q1.z = R.qw[2];
     if (sp.g1 > 3) q1.w = R.qw[3];
-    float top;
-    uint32_t slot;
-    warp_heap_top(R.hd, kq, top, slot);
     uint32_t* scratch = sp.start_dist + (size_t)__ldg(sp.start_row + q) * sp.start_stride;
-    const uint32_t* ord = sp.q_order + (size_t)q * stride;
-    const uint32_t cnt = __ldg(sp.q_order_count + q);
     const uint32_t S = sp.r_surv_cap;
-    unsigned long long b_warm = 0, b_h = 0, b_v = 0, visits = 0, merged = 0;
+    unsigned long long b_warm = 0, b_h = 0, b_v = 0, merged = 0;
     unsigned long long n_cand = 0, n_surv = 0, n_fast = 0, n_full = 0;
+    unsigned long long b_warm_l = 0;  // per lane: the first step of every visit
+    uint32_t visits_l = 0, fast_l = 0;
 
-    // Follows the lane's survivor (alive, v, raw) through Prune with the bound at `tp`, then
-    // merges the warp's survivors in lane order (MergeIntoHeap, searcher.hpp:542-566).
-    auto prune_merge = [&](const DevCluster& c, bool alive, uint32_t v, uint32_t raw, uint32_t cur, float tp) {
-        uint32_t idv = 0;
-        if (alive) {
-            alive = scan_follow(sp, c, R.qw, v, cur, tp, raw, b_h, b_v);
-            if (alive) idv = __ldg(reinterpret_cast<const uint32_t*>(sp.arena + c.ids_off) + v);
-        }
+    // Merges the warp's vectors that stayed below every bound (alive), in lane order
+    // (MergeIntoHeap, searcher.hpp:542-566).
+    auto merge = [&](const DevCluster& c, bool alive, uint32_t v, uint32_t raw) {
+        const uint32_t idv = alive ? __ldg(reinterpret_cast<const uint32_t*>(sp.arena + c.ids_off) + v) : 0u;
         const float dd = reported_u8(raw, lv);
         unsigned bal = __ballot_sync(0xffffffffu, alive);
         merged += __popc(bal);
@@ -524,23 +687,110 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         }
     };
 
-    // the next visit's cluster record and first bitmap words, loaded one visit ahead
-    DevCluster c_nx{};
-    uint32_t bw_nx = 0;
-    auto prefetch = [&](uint32_t ii) {
-        if (ii < cnt) {
-            c_nx = lv.clusters[__ldg(ord + ii)];
-            bw_nx = lane < sp.bm_words ? __ldg(sp.bm + ((size_t)q * stride + ii) * sp.bm_words + lane) : 0u;
+    // Follows the lane's survivor (alive, v, raw) through Prune with the bound at `tp`, then merges.
+    auto prune_merge = [&](const DevCluster& c, bool alive, uint32_t v, uint32_t raw, uint32_t cur, float tp) {
+        if (alive) alive = scan_follow(sp, c, R.qw, v, cur, tp, raw, b_h, b_v);
+        merge(c, alive, v, raw);
+    };
+    // A heavy visit on its values computed ahead, hv pointing at its first vector's column.
+    // bmh: its mergeable vectors.
+    auto heavy_visit = [&](const DevCluster& c, const uint32_t* hv, const uint32_t* bmh) {
+        const uint32_t n = c.n, W = (n + 31) >> 5;
+        uint32_t any = 0;
+        for (uint32_t w = lane; w < W; w += 32) any |= bmh[w];
+        if (!__any_sync(0xffffffffu, any != 0)) return;
+        const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
+        const float tp = top;  // the bound's heap top, fixed for the whole cluster
+        uint32_t cur = 0, step = 0, n_pruned = 0;
+        while (n_pruned < needed && cur < lv.dv) {  // Warmup (searcher.hpp:374-435)
+            uint32_t last = cur + c_scan_fetch[step < kNumFetchSizes ? step : kNumFetchSizes - 1];
+            if (last > lv.dv) last = lv.dv;
+            const uint32_t thr = thr_u8(tp, last, lv, sp.ratios);
+            const uint32_t* row = hv + (size_t)step * sp.hv_cap;
+            uint32_t cntp = 0;
+            for (uint32_t v0 = 0; v0 < n; v0 += 256) {
+                uint32_t x[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const uint32_t v = v0 + 32 * u + lane;
+                    x[u] = v < n ? row[v] : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) cntp += (v0 + 32 * u + lane < n && x[u] >= thr) ? 1u : 0u;
+            }
+            n_pruned = __reduce_add_sync(0xffffffffu, cntp);
+            if (cur == 0) n_surv += n - n_pruned;
+            else b_warm += (unsigned long long)n * (last - cur);
+            cur = last;
+            ++step;
+        }
+        if (step == 1) ++n_fast;
+        else ++n_full;
+        // Prune (searcher.hpp:437-540) and merge of the mergeable vectors, 32 at a time in position
+        // order; their horizontal sums are loaded kHeavyBlocks at a time, ahead of their tests
+        constexpr int kHeavyBlocks = 6;
+        const uint32_t thr = thr_u8(tp, cur, lv, sp.ratios);
+        const uint32_t* erow = hv + (size_t)(step - 1) * sp.hv_cap;
+        const uint32_t* brow = hv + (size_t)sp.hv_ncp * sp.hv_cap;
+        for (uint32_t w0 = 0; w0 < W; w0 += 32) {
+            const uint32_t total = scan_bits_to_offsets(w0 + lane < W ? bmh[w0 + lane] : 0u, lane, R.cand);
+            for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+                bool alive = j0 + lane < total;
+                const uint32_t v = alive ? w0 * 32 + R.cand[j0 + lane] : 0u;
+                uint32_t raw = alive ? erow[v] : 0u;
+                alive = alive && raw < thr;
+                uint32_t cv = cur;
+                for (uint32_t b0 = 0; b0 < lv.n_hblocks && __any_sync(0xffffffffu, alive); b0 += kHeavyBlocks) {
+                    uint32_t x[kHeavyBlocks];
+#pragma unroll
+                    for (int u = 0; u < kHeavyBlocks; ++u)
+                        x[u] = (alive && b0 + u < lv.n_hblocks) ? brow[(size_t)(b0 + u) * sp.hv_cap + v] : 0u;
+#pragma unroll
+                    for (int u = 0; u < kHeavyBlocks; ++u) {
+                        if (alive && b0 + u < lv.n_hblocks) {
+                            raw += x[u];
+                            b_h += kHDim;
+                            cv += kHDim;
+                            alive = raw < thr_u8(tp, cv, lv, sp.ratios);
+                        }
+                    }
+                }
+                if (alive) alive = scan_follow_vertical(sp, c, R.qw, v, cur, cv, tp, raw, b_v);
+                merge(c, alive, v, raw);
+            }
+            __syncwarp();  // cand is rewritten by the next word group
         }
     };
-    prefetch(fi + 1);
-    for (uint32_t i = fi + 1; i < cnt; ++i) {
-        const DevCluster c = c_nx;
-        const uint32_t bw0 = bw_nx;
-        prefetch(i + 1);
+
+    // Visits without a candidate end their warmup at the first step with no survivor (n >= 0.8 n
+    // vectors reach the bound): only the others are walked. On the 1M x 1024 SQ8 tree a query has
+    // one or two of them in 31 visits, and walking all of them was a chain of 31 record and bitmap
+    // round trips.
+    for (uint32_t i0 = (fi + 1) & ~31u; i0 < cnt; i0 += 32) {
+      const uint32_t il = i0 + lane;
+      const bool in = il > fi && il < cnt;
+      uint32_t info_l = in ? __ldg(vis + il) : 0u;
+      if (sp.stats && in) {
+          const uint32_t n = lv.clusters[__ldg(ord + il)].n;
+          visits_l += n ? 1u : 0u;
+          b_warm_l += (unsigned long long)n * sp.cp1;
+          fast_l += (n && info_l == 0) ? 1u : 0u;
+      }
+      for (unsigned todo = __ballot_sync(0xffffffffu, info_l != 0); todo; todo &= todo - 1) {
+        const uint32_t src = __ffs(todo) - 1, i = i0 + src;
+        const uint32_t info = __shfl_sync(0xffffffffu, info_l, src);
+        const DevCluster c = lv.clusters[__ldg(ord + i)];
+        if (info & kHeavyBit) {
+            uint32_t at = 0xFFFFFFFFu;
+            for (uint32_t j = lane; j < n_heavy; j += 32)
+                if (HL.warp[j] == warp && HL.visit[j] == i) at = j;
+            at = __reduce_min_sync(0xffffffffu, at);
+            if (at != 0xFFFFFFFFu) {
+                heavy_visit(c, sp.hv + ((size_t)HL.base[at] << 5), sp.bm + ((size_t)q * stride + i) * sp.bm_words);
+                continue;
+            }
+        }
         const uint32_t n = c.n;
-        if (n == 0) continue;  // num_embeddings == 0 (searcher.hpp:662)
-        ++visits;
         const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off);
         const uint32_t W = (n + 31) >> 5;
         const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
@@ -549,10 +799,10 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         // survivors under the current bound, in position order
         const uint32_t thr1 = thr_u8(top, sp.cp1, lv, sp.ratios);
         uint32_t ns = 0;
-        for (uint32_t w0 = 0; w0 < W; w0 += 32) {
+        const bool light = !(info & kHeavyBit);  // a heavy visit keeps no bitmap
+        for (uint32_t w0 = 0; light && w0 < W; w0 += 32) {
             const uint32_t w = w0 + lane;
-            uint32_t word = w0 == 0 ? bw0 : (w < W ? __ldg(bmp + w) : 0u);
-            if (w >= W) word = 0u;
+            const uint32_t word = w < W ? __ldg(bmp + w) : 0u;
             const uint32_t total = scan_bits_to_offsets(word, lane, R.cand);
             n_cand += total;
             for (uint32_t j0 = 0; j0 < total; j0 += 32 * kCandPerLane) {
@@ -584,11 +834,10 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
             }
             __syncwarp();
         }
-        b_warm += (unsigned long long)n * sp.cp1;
         const bool exits = sp.cp1 >= lv.dv || n - ns >= needed;  // the warmup stops after step 1
         const float tp = top;  // the bound's heap top, fixed for the whole cluster
         n_surv += ns;
-        if (exits && ns <= S) {
+        if (light && exits && ns <= S) {
             ++n_fast;
             // Prune and MergeIntoHeap of the survivors, 32 at a time in position order
             for (uint32_t g0 = 0; g0 < ns; g0 += 32) {
@@ -665,6 +914,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
             }
             __syncwarp();  // cand is rewritten by the next word group
         }
+      }
     }
     // BuildResultSetFromHeap (searcher.hpp:568-585)
     const uint32_t N = next_pow2(kq);
@@ -690,6 +940,11 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
     if (sp.stats) {
         const unsigned long long h = __reduce_add_sync(0xffffffffu, (uint32_t)b_h);
         const unsigned long long vv = __reduce_add_sync(0xffffffffu, (uint32_t)b_v);
+        const uint32_t visits = __reduce_add_sync(0xffffffffu, visits_l);
+        n_fast += __reduce_add_sync(0xffffffffu, fast_l);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) b_warm_l += __shfl_xor_sync(0xffffffffu, b_warm_l, o);
+        b_warm += b_warm_l;
         if (lane == 0) {
             add_stat(sp, 0, b_warm + h + vv);
             add_stat(sp, 3 + kWarmup, b_warm);
@@ -710,9 +965,18 @@ uint64_t scan_item_bound(uint32_t nq, uint32_t stride, uint32_t n1) {
     return (uint64_t)nq * stride / kScanCQ + n1 + 1;
 }
 
-int scan_bitmap_occupancy() {
+// Shared memory of a bitmap work item's tile; 0: the bitmaps of clusters this large go straight
+// to global memory.
+size_t scan_bitmap_smem(uint32_t bm_words) {
+    const size_t b = (size_t)kScanCQ * (bm_words | 1u) * 4;
+    return b <= kBitmapTileMax ? b : 0;
+}
+
+int scan_bitmap_occupancy(uint32_t bm_words) {
     int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, scan_bitmap_kernel, kBitmapThreads, 0);
+    const size_t tile = scan_bitmap_smem(bm_words);
+    if (tile) cudaFuncSetAttribute(scan_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, scan_bitmap_kernel, kBitmapThreads, tile);
     return blocks;
 }
 
@@ -722,8 +986,8 @@ uint32_t scan_queries_per_cta() { return kScanWarps; }
 cudaError_t launch_scan(const ScanParams& sp, int bitmap_grid, cudaStream_t st, const cudaEvent_t* ev) {
     cudaError_t e = cudaMemsetAsync(sp.vl_count, 0, sizeof(uint32_t) * sp.l1.nclusters, st);
     if (e != cudaSuccess) return e;
-    // left_n, n_items and queue are consecutive
-    if ((e = cudaMemsetAsync(sp.left_n, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    // left_n, n_items, queue and hv_alloc are consecutive
+    if ((e = cudaMemsetAsync(sp.left_n, 0, 4 * sizeof(uint32_t), st)) != cudaSuccess) return e;
     const uint32_t ctas = (sp.nq + kScanWarps - 1) / kScanWarps;
     const size_t prep_smem = sp.prep_qs ? (size_t)kScanWarps * sp.prep_qs_stride * 4 : 0;
     if (prep_smem) {
@@ -733,13 +997,18 @@ cudaError_t launch_scan(const ScanParams& sp, int bitmap_grid, cudaStream_t st, 
     scan_prep_kernel<<<ctas, kScanWarps * 32, prep_smem, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
-    scan_bitmap_kernel<<<bitmap_grid, kBitmapThreads, 0, st>>>(sp);
+    const size_t tile = scan_bitmap_smem(sp.bm_words);
+    if (tile) {
+        e = cudaFuncSetAttribute(scan_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile);
+        if (e != cudaSuccess) return e;
+    }
+    scan_bitmap_kernel<<<bitmap_grid, kBitmapThreads, tile, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[1], st)) != cudaSuccess) return e;
-    const size_t smem = (size_t)kScanWarps * sp.r_warp_bytes;
+    const size_t smem = (size_t)sp.r_qpc * sp.r_warp_bytes;
     e = cudaFuncSetAttribute(scan_replay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    scan_replay_kernel<<<ctas, kScanWarps * 32, smem, st>>>(sp);
+    scan_replay_kernel<<<(sp.nq + sp.r_qpc - 1) / sp.r_qpc, kScanWarps * 32, smem, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[2], st)) != cudaSuccess) return e;
     return cudaSuccess;
