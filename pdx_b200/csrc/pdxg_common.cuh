@@ -89,6 +89,7 @@ struct SearchParams {
     const uint32_t* q_order;        // [nq x q_order_stride]
     const uint32_t* q_order_count;  // [nq]
     uint32_t q_order_stride;
+    uint32_t q_order_filtered;      // 1: the filtered queries have a row too (exact probe ahead)
     // batched Start (pdxg_start.cu): exact U8 distances to every vector of each query's first
     // visited cluster, computed ahead with reuse across queries
     const int32_t* start_row;       // optional [nq]: row in start_dist, -1 = none
@@ -137,11 +138,12 @@ struct TopLevelParams {
     unsigned long long* stats;   // optional, SearchParams::stats layout
     // replay shared memory (bytes per warp and carve-up)
     uint32_t r_heap_cap, r_work_cap, r_sort_cap, r_pre_floats, r_warp_bytes, r_smem;
-    uint32_t probe_smem;         // meso probe CTA: queries + sort keys
-    uint32_t probe_q;            // queries per meso probe CTA (1..8)
+    uint32_t* probe_keys;        // [nq x nL0] meso centroid distances (float bits)
+    uint32_t probe_smem;         // meso list CTA: sort keys, list counters
+    uint32_t probe_q;            // queries per meso list CTA (1..16), one warp each
 };
 
-// Reduced-precision centroid probe (pdxg_probe.cu).
+// Centroid probes ahead of the scan (pdxg_probe.cu): reduced-precision and exact.
 struct ProbeParams {
     const float* queries;        // prepared queries [nq x d] (FP32)
     const float* centroids;      // [nclusters x d] FP32
@@ -155,6 +157,11 @@ struct ProbeParams {
     uint32_t* count;             // [nq]
     uint32_t cand_cap, sort_cap; // shared-memory capacities (candidates, sort keys)
     uint32_t score_bytes;        // bytes per centroid element read by the approximate scores
+    // exact probe: distances of the probed queries to every centroid (float bits), and optionally
+    // the list of those queries (all of them without it)
+    uint32_t* keys;              // [keys_rows x nclusters]
+    uint32_t keys_rows;
+    const uint32_t* q_list;      // [nq], or null
     unsigned long long* stats;   // optional, SearchParams::stats layout
 };
 

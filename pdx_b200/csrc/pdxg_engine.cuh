@@ -111,8 +111,13 @@ struct Workspace {
     uint64_t pq_r8s_cap = 0;
     float* d_pq_scores = nullptr;
     uint64_t pq_scores_cap = 0;
+    // exact probe: centroid distances, list of the filtered queries
+    uint32_t* d_pr_keys = nullptr;
+    uint64_t pr_keys_cap = 0;
+    uint32_t* d_pr_list = nullptr;
+    uint64_t pr_list_cap = 0;
     // per-query request parameters (pdxg_search_requests)
-    uint32_t* d_req = nullptr;  // q_k | q_nprobe | q_top | filter_of, nq each
+    uint32_t* d_req = nullptr;  // q_k | q_nprobe | q_top | filter_of | filtered queries, nq each
     uint64_t req_cap = 0;
     unsigned long long* d_foff = nullptr;
     uint64_t foff_cap = 0;

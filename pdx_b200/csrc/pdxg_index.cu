@@ -236,7 +236,7 @@ void free_workspace(Workspace& w) {
                     w.d_sel, w.d_pass, w.d_filter_of, w.d_stats, w.d_top_order, w.d_top_off,
                     w.d_top_lists, w.d_top_count, w.d_top_vals, w.d_l1_order, w.d_l1_count,
                     w.d_st_cl, w.d_st_q, w.d_st_items, w.d_st_dist, w.d_pq_b16, w.d_pq_r16, w.d_pq_r8,
-                    w.d_pq_r8s, w.d_pq_scores,
+                    w.d_pq_r8s, w.d_pq_scores, w.d_pr_keys, w.d_pr_list,
                     w.d_req, w.d_foff, w.d_rows, w.d_qhi, w.d_qlo, w.d_gemm_err, w.d_sc_qw, w.d_sc_q,
                     w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
                     w.d_sc_vi, w.d_sc_hv};
@@ -744,10 +744,8 @@ int run_top_level_tiled(pdxg_index* ix, Workspace& w, const float* qp, uint32_t 
     if (vals_bytes + (uint64_t)nL0 * nq * 4 > (8ull << 30)) return PDXG_OK;
     const uint32_t max_n0 = std::max(l0.max_n, 1u);
     if (max_n0 > (1u << 20)) return PDXG_OK;
-    tp.probe_q = 8;
-    auto probe_bytes = [&](uint32_t qn) {
-        return align_up((uint64_t)qn * l0.d * 4, 16) + (uint64_t)qn * next_pow2(nL0) * 8;
-    };
+    tp.probe_q = 16;
+    auto probe_bytes = [&](uint32_t qn) { return (uint64_t)qn * next_pow2(nL0) * 8 + (uint64_t)nL0 * 4; };
     while (tp.probe_q > 1 && probe_bytes(tp.probe_q) + 1024 > ix->max_smem) tp.probe_q >>= 1;
     if (probe_bytes(tp.probe_q) + 1024 > ix->max_smem) return PDXG_OK;
     tp.probe_smem = (uint32_t)probe_bytes(tp.probe_q);
@@ -772,6 +770,8 @@ int run_top_level_tiled(pdxg_index* ix, Workspace& w, const float* qp, uint32_t 
     if ((rc = dev_grow(w.d_top_vals, w.top_vals_cap, std::max<uint64_t>((uint64_t)nq * per_query, 4)))) return rc;
     if ((rc = dev_grow(w.d_l1_order, w.l1_order_cap, (uint64_t)(q_offset + nq) * k1))) return rc;
     if ((rc = dev_grow(w.d_l1_count, w.l1_count_cap, q_offset + nq))) return rc;
+    if ((rc = dev_grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)nq * nL0))) return rc;
+    tp.probe_keys = w.d_pr_keys;
     tp.arena = ix->arena;
     tp.l0 = l0;
     tp.ratios = L.p.ratios;
@@ -796,7 +796,7 @@ int run_top_level_tiled(pdxg_index* ix, Workspace& w, const float* qp, uint32_t 
     tp.r_smem = (uint32_t)(ratio_bytes + (uint64_t)warps * wb);
     PDXG_CUDA(launch_top_level_tiled(tp, vtiles, warps, st, timed ? ix->tev + 8 : nullptr));
     ix->tev_tiled = timed;
-    L.top_launches = 3;
+    L.top_launches = 4;
     L.p.q_order = w.d_l1_order;
     L.p.q_order_count = w.d_l1_count;
     L.p.q_order_stride = k1;
@@ -1012,24 +1012,35 @@ int run_probe_gemm(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq, bo
     return PDXG_OK;
 }
 
-// Exact probe of a flat index ahead of the scan (probe_exact_kernel): same order as the scan
-// kernel's own probe; lets the scan keep per-vector arrays only.
-constexpr uint32_t kProbeAheadMinQueries = 32;
+// Exact probe ahead of the scan (centroid_dist_kernel, probe_pick_kernel): the order of the scan
+// kernel's own probe; lets the scan keep per-vector arrays only, and shares every centroid read
+// among 32 queries. Few queries gain too: 16 filtered queries x 1,000 centroids x 1024 dims spent 580 us
+// in the scan kernel with its own probe and 337 us after a probe of 30 us.
+constexpr uint32_t kProbeAheadMinQueries = 32;  // smaller batches report no visit orders
+constexpr uint64_t kProbeKeysMax = 64ull << 20;
 
 bool probe_exact_ok(const pdxg_index* ix) {
     const uint32_t n1 = (uint32_t)ix->l1.fc.size();
-    return !ix->tree && probe_select_smem(ix->d, n1, (n1 + 3) & ~3u, next_pow2(n1)) + 2048 <= ix->max_smem;
+    return n1 > 0 && probe_select_smem(ix->d, n1, (n1 + 3) & ~3u, next_pow2(n1)) + 2048 <= ix->max_smem;
 }
 
-int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st) {
+// The probe of all nq queries, or of the n_list queries of d_list only: their rows of the visit
+// orders (the others' rows are left as they are).
+int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st,
+                    const uint32_t* d_list = nullptr, uint32_t n_list = 0) {
     const uint32_t n1 = L.p.l1.nclusters, k1 = L.p.nprobe;
+    const uint32_t rows = d_list ? n_list : nq;
     int rc;
     if ((rc = dev_grow(w.d_l1_order, w.l1_order_cap, (uint64_t)nq * k1))) return rc;
     if ((rc = dev_grow(w.d_l1_count, w.l1_count_cap, nq))) return rc;
     ProbeParams pp{};
+    pp.keys_rows = (uint32_t)std::min<uint64_t>(rows, std::max<uint64_t>(kProbeKeysMax / n1, 32));
+    if ((rc = dev_grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)pp.keys_rows * n1))) return rc;
+    pp.keys = w.d_pr_keys;
+    pp.q_list = d_list;
     pp.queries = qp;
     pp.centroids = ix->d_cent1;
-    pp.nq = nq;
+    pp.nq = rows;
     pp.d = ix->d;
     pp.nclusters = n1;
     pp.nprobe = k1;
@@ -1038,13 +1049,14 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
     pp.stride = k1;
     pp.count = w.d_l1_count;
     pp.cand_cap = (n1 + 3) & ~3u;
-    pp.sort_cap = next_pow2(n1);
+    pp.sort_cap = next_pow2(std::min(k1, n1));
     pp.stats = L.p.stats;
     PDXG_CUDA(launch_probe_exact(pp, st));
-    L.probe_launches += 1;
+    L.probe_launches += 2 * ((rows + pp.keys_rows - 1) / pp.keys_rows);
     L.p.q_order = w.d_l1_order;
     L.p.q_order_count = w.d_l1_count;
     L.p.q_order_stride = k1;
+    L.p.q_order_filtered = 1;
     return PDXG_OK;
 }
 
@@ -1199,11 +1211,13 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
 
 namespace {
 
-// Core device-side search: queries/ids/dists/counts are device pointers.
+// Core device-side search: queries/ids/dists/counts are device pointers. d_filtered: the
+// n_filtered queries with a filter.
 int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq, uint32_t k, uint32_t flags,
                        const uint32_t* d_order, uint32_t n_order, const uint32_t* d_sel,
-                       const uint32_t* d_pass, const int32_t* d_filter_of, bool any_filter,
-                       uint32_t* ids, float* dists, uint32_t* counts, cudaStream_t st) {
+                       const uint32_t* d_pass, const int32_t* d_filter_of, const uint32_t* d_filtered,
+                       uint32_t n_filtered, uint32_t* ids, float* dists, uint32_t* counts, cudaStream_t st) {
+    const bool any_filter = n_filtered != 0, any_plain = n_filtered < nq;
     if (nq == 0) return PDXG_OK;
     if (k == 0) {
         PDXG_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * nq, st));
@@ -1231,8 +1245,7 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
     }
     if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[1], st));
     Launch L;
-    const bool probe_ahead = !gemm_probe && !ix->tree && !any_filter && !d_order && nq >= kProbeAheadMinQueries &&
-                             probe_exact_ok(ix);
+    const bool probe_ahead = !gemm_probe && !ix->tree && !d_order && probe_exact_ok(ix);
     rc = plan_search(ix, nq, k, n_order, any_filter, L, 0xFFFFFFFFu, 0xFFFFFFFFu, probe_ahead, st);
     if (rc) return rc;
     L.p.queries = qp;
@@ -1256,20 +1269,29 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
         if (rc) return rc;
         qp = L.p.queries;
         launches += L.probe_launches;
-    } else if (ix->tree && !any_filter && !d_order) {
-        rc = run_top_level(ix, w, qp, nq, L, st, 0, timed);
-        if (rc) return rc;
-        launches += L.top_launches;
+    } else if (ix->tree && !d_order) {
+        if (any_plain) {
+            rc = run_top_level(ix, w, qp, nq, L, st, 0, timed);
+            if (rc) return rc;
+            launches += L.top_launches;
+        }
+        // filtered queries probe the L1 centroids directly; their orders go beside the others'
+        if (any_filter && (L.p.q_order || !any_plain) && probe_exact_ok(ix)) {
+            rc = run_probe_exact(ix, w, qp, nq, L, st, d_filtered, n_filtered);
+            if (rc) return rc;
+            launches += L.probe_launches;
+        }
     } else if (probe_ahead) {
         rc = run_probe_exact(ix, w, qp, nq, L, st);
         if (rc) return rc;
         launches += L.probe_launches;
     }
     ix->tev_top = L.p.q_order != nullptr;
-    ix->last_order_stride = L.p.q_order ? L.p.q_order_stride : 0;
+    ix->last_order_stride =
+        L.p.q_order && !any_filter && (!probe_ahead || nq >= kProbeAheadMinQueries) ? L.p.q_order_stride : 0;
     // the batched Start belongs to the scan's time
     if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[2], st));
-    if ((rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
+    if (any_plain && (rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
     launches += L.start_launches;
     if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
     if ((rc = run_scan_cluster_major(ix, w, nq, L, st, timed))) return rc;
@@ -1376,7 +1398,8 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
     auto chunk_off = [&](uint32_t c) { return c == 0 ? 0u : std::min(first, nq); };
     auto chunk_len = [&](uint32_t c) { return c == 0 ? std::min(first, nq) : nq - std::min(first, nq); };
     Launch L;
-    if ((rc = plan_search(ix, nq, k, 0, false, L))) return rc;
+    const bool probe_ahead = !ix->tree && probe_exact_ok(ix);
+    if ((rc = plan_search(ix, nq, k, 0, false, L, 0xFFFFFFFFu, 0xFFFFFFFFu, probe_ahead))) return rc;
     L.p.out_ids = w.d_ids;
     L.p.out_dists = w.d_dists;
     L.p.out_counts = w.d_counts;
@@ -1415,12 +1438,16 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
         L.p.q_order_count = w.d_l1_count;
         L.p.q_order_stride = k1;
     }
+    if (probe_ahead) {
+        if ((rc = run_probe_exact(ix, w, L.p.queries, nq, L, st))) return rc;
+        launches += L.probe_launches;
+    }
     if ((rc = run_start_batched(ix, w, L.p.queries, nq, L, st))) return rc;
     launches += L.start_launches;
     if ((rc = run_scan_cluster_major(ix, w, nq, L, st))) return rc;
     launches += L.scan_launches;
     ix->last_launches = launches;
-    ix->last_order_stride = L.p.q_order ? k1 : 0;
+    ix->last_order_stride = L.p.q_order && !probe_ahead ? k1 : 0;
     PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
     PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, sizeof(uint32_t) * nq * k, cudaMemcpyDeviceToHost, st));
@@ -1457,9 +1484,12 @@ int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t
     const uint32_t* d_sel = nullptr;
     const uint32_t* d_pass = nullptr;
     const int32_t* d_fo = nullptr;
-    bool any_filter = false;
+    std::vector<uint32_t> filtered;  // queries with a filter
     if (sel && !sel->empty()) {
-        any_filter = true;
+        for (uint32_t q = 0; q < nq; ++q)
+            if ((*filter_of)[q] != -1) filtered.push_back(q);
+        if ((rc = dev_grow(w.d_pr_list, w.pr_list_cap, filtered.size()))) return rc;
+        PDXG_CUDA(cudaMemcpyAsync(w.d_pr_list, filtered.data(), filtered.size() * 4, cudaMemcpyHostToDevice, st));
         if ((rc = dev_grow(w.d_sel, w.sel_cap, sel->size()))) return rc;
         if ((rc = dev_grow(w.d_pass, w.pass_cap, pass->size()))) return rc;
         uint64_t cap = w.fo_cap;
@@ -1474,7 +1504,7 @@ int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t
         d_fo = w.d_filter_of;
     }
     rc = search_device_impl(ix, w, w.d_q, nq, k, flags, d_order, n_order, d_sel, d_pass, d_fo,
-                            any_filter, w.d_ids, w.d_dists, w.d_counts, st);
+                            w.d_pr_list, (uint32_t)filtered.size(), w.d_ids, w.d_dists, w.d_counts, st);
     if (rc) return rc;
     PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, sizeof(uint32_t) * nq * k, cudaMemcpyDeviceToHost, st));
     PDXG_CUDA(cudaMemcpyAsync(dists, w.d_dists, sizeof(float) * nq * k, cudaMemcpyDeviceToHost, st));
@@ -1626,7 +1656,7 @@ int pdxg_search_device(pdxg_index* ix, const float* queries, uint32_t nq, uint32
     PDXG_CUDA(cudaSetDevice(ix->device));
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ix->stream;
     return search_device_impl(ix, ix->ws, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr,
-                              false, ids, distances, counts, st);
+                              nullptr, 0, ids, distances, counts, st);
 }
 
 }  // extern "C"
@@ -1650,7 +1680,7 @@ int pdxg_graph_create(pdxg_index* ix, const float* queries, uint32_t nq, uint32_
     std::lock_guard<std::mutex> lock(ix->mu);
     PDXG_CUDA(cudaSetDevice(ix->device));
     // a direct run sizes every workspace buffer for this batch, so the capture allocates nothing
-    int rc = search_device_impl(ix, ix->ws, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr, false,
+    int rc = search_device_impl(ix, ix->ws, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0,
                                 ids, distances, counts, ix->stream);
     if (rc) return rc;
     PDXG_CUDA(cudaStreamSynchronize(ix->stream));
@@ -1661,7 +1691,7 @@ int pdxg_graph_create(pdxg_index* ix, const float* queries, uint32_t nq, uint32_
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        rc = search_device_impl(ix, ix->ws, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr, false,
+        rc = search_device_impl(ix, ix->ws, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0,
                                 ids, distances, counts, cs);
         e = cudaStreamEndCapture(cs, &graph);
     }
@@ -1741,7 +1771,7 @@ int pdxg_autotune(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k,
                     if (cudaEventRecord(e0, ix->stream) != cudaSuccess) rc = fail(PDXG_ERR_CUDA, "event");
                     if (rc == PDXG_OK)
                         rc = search_device_impl(ix, ix->ws, queries, nq, k, flags, nullptr, 0, nullptr, nullptr,
-                                                nullptr, false, ids, dists, counts, ix->stream);
+                                                nullptr, nullptr, 0, ids, dists, counts, ix->stream);
                     if (rc == PDXG_OK && (cudaEventRecord(e1, ix->stream) != cudaSuccess ||
                                           cudaEventSynchronize(e1) != cudaSuccess))
                         rc = fail(PDXG_ERR_CUDA, "event");
@@ -2169,18 +2199,20 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
             any_plain = true;
         }
     }
-    // pinned staging: q_k, q_np, q_top, filter_of (nq each), filter offsets (nf + 1), rows
-    const size_t req_bytes = (size_t)nq * 16, foff_bytes = ((size_t)nf + 1) * 8, row_bytes = nrows * 4;
+    // pinned staging: q_k, q_np, q_top, filter_of, filtered queries (nq each), filter offsets
+    // (nf + 1), rows
+    const size_t req_bytes = align_up((size_t)nq * 20, 8), foff_bytes = ((size_t)nf + 1) * 8, row_bytes = nrows * 4;
     if (ctx->staged_pending) PDXG_CUDA(cudaEventSynchronize(ctx->staged));
     int rc = stage_grow(ctx, req_bytes + foff_bytes + row_bytes + 64);
     if (rc) return rc;
     uint32_t* h_req = reinterpret_cast<uint32_t*>(ctx->h_stage);
     unsigned long long* h_foff = reinterpret_cast<unsigned long long*>(ctx->h_stage + req_bytes);
     uint32_t* h_rows = reinterpret_cast<uint32_t*>(ctx->h_stage + req_bytes + foff_bytes);
-    uint32_t f = 0;
+    uint32_t f = 0, n_filtered = 0;
     unsigned long long pos = 0;
     for (uint32_t q = 0; q < nq; ++q) {
         const pdxg_request& r = requests[q];
+        if (r.filter_id >= 0 || r.filter_begin != UINT64_MAX) h_req[4 * nq + n_filtered++] = q;
         const uint32_t npf = (r.nprobe == 0 || r.nprobe > n1) ? n1 : r.nprobe;
         uint32_t top = 0;
         if (ix->tree) {
@@ -2209,7 +2241,7 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
     h_foff[nf] = pos;
     Workspace& w = ctx->ws;
     if ((rc = ensure_ws(ix, w, nq, k_max))) return rc;
-    if ((rc = dev_grow(w.d_req, w.req_cap, (uint64_t)nq * 4))) return rc;
+    if ((rc = dev_grow(w.d_req, w.req_cap, (uint64_t)nq * 5 + 1))) return rc;
     if ((rc = dev_grow(w.d_foff, w.foff_cap, (uint64_t)nf + 1))) return rc;
     if ((rc = dev_grow(w.d_rows, w.rows_cap, std::max<uint64_t>(nrows, 1)))) return rc;
     PDXG_CUDA(cudaMemcpyAsync(w.d_req, h_req, req_bytes, cudaMemcpyHostToDevice, st));
@@ -2240,7 +2272,8 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
         qp = w.d_rq;
     }
     Launch L;
-    if ((rc = plan_search(ix, nq, k_max, 0, any_filter, L, np_max, top_max, false, st))) return rc;
+    const bool probe_ahead = !gemm_probe && !ix->tree && probe_exact_ok(ix);
+    if ((rc = plan_search(ix, nq, k_max, 0, any_filter, L, np_max, top_max, probe_ahead, st))) return rc;
     L.p.queries = qp;
     L.p.q_k = w.d_req;
     L.p.q_nprobe = w.d_req + nq;
@@ -2260,9 +2293,17 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
         if ((rc = run_probe_gemm(ix, w, queries, nq, (flags & PDXG_QUERY_TRANSFORMED) != 0, L, st))) return rc;
         qp = L.p.queries;
         if ((rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
-    } else if (ix->tree && any_plain) {
-        if ((rc = run_top_level(ix, w, qp, nq, L, st))) return rc;
-        if ((rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
+    } else if (ix->tree) {
+        if (any_plain) {
+            if ((rc = run_top_level(ix, w, qp, nq, L, st))) return rc;
+            if ((rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
+        }
+        if (any_filter && (L.p.q_order || !any_plain) && probe_exact_ok(ix) &&
+            (rc = run_probe_exact(ix, w, qp, nq, L, st, w.d_req + 4 * (uint64_t)nq, n_filtered)))
+            return rc;
+    } else if (probe_ahead) {
+        if ((rc = run_probe_exact(ix, w, qp, nq, L, st))) return rc;
+        if (any_plain && (rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
     }
     if ((rc = run_scan_cluster_major(ix, w, nq, L, st))) return rc;
     PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));

@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(T) search_kernel(const __grid_constant__ Searc
             nvisit = npq < p.n_order ? npq : p.n_order;
             for (uint32_t i = threadIdx.x; i < nvisit; i += T) sh.order[i] = __ldg(p.order + i);
             __syncthreads();
-        } else if (filter == -1 && p.q_order) {
+        } else if (p.q_order && (filter == -1 || p.q_order_filtered)) {
             // the tree top level (pdxg_toplevel.cu) or a probe ahead of the scan (pdxg_probe.cu)
             // already produced this query's L1 order: read in place
             nvisit = __ldg(p.q_order_count + q);

@@ -8,9 +8,9 @@
 // its load pipe. This form computes the exact per-pair quantities once, with reuse across
 // queries, and then replays the reference's decisions on them:
 //
-//   1. meso_probe_kernel: exact centroid distances in the AVX2 order of Horizontal
-//      (searcher.hpp:181-215), the `top` nearest meso clusters per query sorted by (distance,
-//      id), and per meso cluster the list of queries that probe it.
+//   1. centroid_dist_kernel (pdxg_probe.cu): exact centroid distances in the AVX2 order of
+//      Horizontal (searcher.hpp:181-215); meso_list_kernel: the `top` nearest meso clusters per
+//      query sorted by (distance, id), and per meso cluster the list of queries that probe it.
 //   2. meso_partials_kernel: one CTA per (meso cluster, 128 of its queries, 32 of its
 //      vectors). Query rows and cluster blocks are staged in shared memory with cp.async;
 //      each thread keeps 4 queries x 4 vectors of FP32 chains in registers, so a staged
@@ -37,97 +37,63 @@
 
 namespace pdxg {
 
-// -------------------------------------------------------------------------------- probe
-// CTA = up to kProbeQ queries; thread (centroid c of a group of 32, lane sub of 8) runs lane
-// `sub` of Horizontal (avx2_computers.hpp:47-98: dims sub, sub + 8, ... with FMA) for every
-// query of the CTA, so each centroid element is loaded once per CTA. The 8 lanes then combine
-// in double exactly as horiz_f32_group8 does; the d % 8 tail is added by lane 0 in double.
-constexpr int kProbeThreads = 256;
-constexpr int kProbeQ = 8;
+cudaError_t launch_centroid_dist(const float* queries, const uint32_t* q_list, uint32_t nq, uint32_t d,
+                                 const float* centroids, uint32_t n, uint32_t* keys, cudaStream_t st);
 
-__global__ void __launch_bounds__(kProbeThreads) meso_probe_kernel(const __grid_constant__ TopLevelParams tp) {
+// -------------------------------------------------------------------------------- probe
+// Warp per query, on the distances of centroid_dist_kernel (pdxg_probe.cu): the `m` smallest
+// (distance, id) pairs, ascending (the list of LevelOps::probe), the offsets of their partials,
+// and the query's entry in the list of each. The entries of a CTA's queries are counted in shared
+// memory first, so a meso cluster's counter takes one atomic per CTA: at 10,000 queries x 16 of 32
+// clusters one atomic per entry queues 5,000 deep on each counter. Distances and lists were one
+// kernel (8 queries x 32 centroids a CTA, one load in flight per thread): 95.6 us for 10,000
+// queries x 32 centroids x 1024 dims and 34 us for 512, against 42.7 + 14.8 and 17.8 + 6.1 us.
+__global__ void __launch_bounds__(512) meso_list_kernel(const __grid_constant__ TopLevelParams tp) {
     extern __shared__ __align__(16) uint8_t smem[];
     const DevLevel& l0 = tp.l0;
-    const uint32_t d = l0.d, nc = l0.nclusters, qp = tp.probe_q;
-    const uint32_t q0 = blockIdx.x * qp;
-    const uint32_t nqc = (tp.nq - q0) < qp ? (tp.nq - q0) : qp;  // queries of this CTA
+    const uint32_t nc = l0.nclusters, qp = tp.probe_q;
     const uint32_t N = next_pow2(nc);
-    float* qs = reinterpret_cast<float*>(smem);                              // [qp][d]
-    uint64_t* keys = reinterpret_cast<uint64_t*>(smem + ((size_t)qp * d * 4 + 15) / 16 * 16);  // [qp][N]
-    for (uint32_t i = threadIdx.x; i < nqc * d; i += kProbeThreads) qs[i] = __ldg(tp.queries + (size_t)q0 * d + i);
+    uint64_t* keys = reinterpret_cast<uint64_t*>(smem);            // [qp][N]
+    uint32_t* count = reinterpret_cast<uint32_t*>(keys + (size_t)qp * N);  // [nc]
+    for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) count[c] = 0;
     __syncthreads();
-    const uint32_t sub = threadIdx.x & 7;
-    const uint32_t full = d & ~7u;
-    for (uint32_t c0 = 0; c0 < nc; c0 += kProbeThreads / 8) {
-        const uint32_t c = c0 + (threadIdx.x >> 3);
-        const bool active = c < nc;
-        const float* x = l0.centroids + (size_t)(active ? c : 0) * d;
-        float acc[kProbeQ];
-#pragma unroll
-        for (int j = 0; j < kProbeQ; ++j) acc[j] = 0.0f;
-        if (active) {
-            for (uint32_t i = 0; i < full; i += 8) {
-                const float xv = __ldg(x + i + sub);
-#pragma unroll
-                for (int j = 0; j < kProbeQ; ++j) {
-                    if (j < (int)nqc) {
-                        const float t = __fsub_rn(qs[j * d + i + sub], xv);
-                        acc[j] = __fmaf_rn(t, t, acc[j]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kProbeQ; ++j) {
-            double sm = (double)acc[j] + (double)__shfl_down_sync(0xffffffffu, acc[j], 4, 8);
-            sm = sm + __shfl_down_sync(0xffffffffu, sm, 2, 8);
-            sm = sm + __shfl_down_sync(0xffffffffu, sm, 1, 8);
-            if (active && sub == 0 && j < (int)nqc) {
-                for (uint32_t i = full; i < d; ++i) {
-                    const float t = __fsub_rn(qs[j * d + i], __ldg(x + i));
-                    sm += (double)__fmul_rn(t, t);
-                }
-                keys[(size_t)j * N + c] = ((uint64_t)__float_as_uint((float)sm) << 32) | c;
-            }
-        }
-    }
-    for (uint32_t i = threadIdx.x; i < nqc * N; i += kProbeThreads)
-        if (i % N >= nc) keys[i] = ~0ull;
-    __syncthreads();
-    // warp j: query q0 + j -- the `m` smallest (distance, id) pairs, ascending (the list of
-    // LevelOps::probe)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (uint32_t j = warp; j < nqc; j += kProbeThreads / 32) {
-        const uint32_t q = q0 + j;
-        if (tp.filter_of && __ldg(tp.filter_of + q) != -1) {
-            if (lane == 0) tp.ntop[q] = 0;
-            continue;
-        }
-        uint64_t* kq = keys + (size_t)j * N;
+    const uint32_t q = blockIdx.x * qp + warp;
+    const bool mine = q < tp.nq && !(tp.filter_of && __ldg(tp.filter_of + q) != -1);  // warp-uniform
+    uint64_t* kq = keys + (size_t)warp * N;
+    uint32_t m = 0;
+    if (mine) {
+        const uint32_t* src = tp.probe_keys + (size_t)q * nc;
+        for (uint32_t c = lane; c < N; c += 32) kq[c] = c < nc ? (((uint64_t)__ldg(src + c) << 32) | c) : ~0ull;
+        __syncwarp();
         warp_sort_u64(kq, N);
         const uint32_t topq = tp.q_top ? __ldg(tp.q_top + q) : tp.top;
-        const uint32_t m = topq < nc ? topq : nc;
-        // offsets: exclusive prefix of nvals * stride over the probe list
+        m = topq < nc ? topq : nc;
+        // offsets: exclusive prefix of nvals * stride over the probe list; the sort key's distance
+        // half makes room for the entry's slot among the CTA's entries of that cluster
         uint32_t carry = 0;
         for (uint32_t r0 = 0; r0 < m; r0 += 32) {
             const uint32_t r = r0 + lane;
             const uint32_t c = r < m ? (uint32_t)kq[r] : 0u;
             const uint32_t sz = r < m ? tp.nvals * ((l0.clusters[c].n + 3u) & ~3u) : 0u;
-            uint32_t incl = sz;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= (uint32_t)o) incl += t;
-            }
+            uint32_t total;
+            const uint32_t at = carry + warp_exclusive_scan(sz, total);
             if (r < m) {
                 tp.order[(size_t)q * tp.top + r] = c;
-                tp.off[(size_t)q * tp.top + r] = carry + incl - sz;
-                const uint32_t slot = atomicAdd(tp.list_count + c, 1u);
-                tp.lists[(size_t)c * tp.nq + slot] = q * tp.top + r;
+                tp.off[(size_t)q * tp.top + r] = at;
+                kq[r] = ((uint64_t)atomicAdd(count + c, 1u) << 32) | c;
             }
-            carry += __shfl_sync(0xffffffffu, incl, 31);
+            carry += total;
         }
-        if (lane == 0) tp.ntop[q] = m;
+    }
+    if (q < tp.nq && lane == 0) tp.ntop[q] = m;
+    __syncthreads();
+    for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x)
+        if (count[c]) count[c] = atomicAdd(tp.list_count + c, count[c]);
+    __syncthreads();
+    for (uint32_t r = lane; r < m; r += 32) {
+        const uint32_t c = (uint32_t)kq[r];
+        tp.lists[(size_t)c * tp.nq + count[c] + (uint32_t)(kq[r] >> 32)] = q * tp.top + r;
     }
 }
 
@@ -145,27 +111,6 @@ struct PartialsSmem {
     uint32_t qrow[kTQ];           // query index of each slot
     uint32_t cp[kMaxCheckpoints]; // warmup checkpoints
 };
-
-// Packed FP32 pairs (sm_100): each half rounds exactly as the scalar sub.rn / fma.rn.
-__device__ __forceinline__ uint64_t f32x2_dup(float a) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
-    return r;
-}
-__device__ __forceinline__ uint64_t f32x2_sub(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ void f32x2_unpack(uint64_t v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 
 __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(const __grid_constant__ TopLevelParams tp) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -618,9 +563,11 @@ cudaError_t launch_top_level_tiled(const TopLevelParams& tp, uint32_t vtiles, in
                                    cudaStream_t st, const cudaEvent_t* ev) {
     cudaError_t e = cudaMemsetAsync(tp.list_count, 0, sizeof(uint32_t) * tp.l0.nclusters, st);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(meso_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp.probe_smem);
+    e = launch_centroid_dist(tp.queries, nullptr, tp.nq, tp.l0.d, tp.l0.centroids, tp.l0.nclusters, tp.probe_keys, st);
     if (e != cudaSuccess) return e;
-    meso_probe_kernel<<<(tp.nq + tp.probe_q - 1) / tp.probe_q, kProbeThreads, tp.probe_smem, st>>>(tp);
+    e = cudaFuncSetAttribute(meso_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp.probe_smem);
+    if (e != cudaSuccess) return e;
+    meso_list_kernel<<<(tp.nq + tp.probe_q - 1) / tp.probe_q, 32 * tp.probe_q, tp.probe_smem, st>>>(tp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
     const int psmem = (int)sizeof(PartialsSmem);
