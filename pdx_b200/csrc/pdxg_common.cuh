@@ -139,6 +139,7 @@ struct TopLevelParams {
     // replay shared memory (bytes per warp and carve-up)
     uint32_t r_heap_cap, r_work_cap, r_sort_cap, r_pre_floats, r_warp_bytes, r_smem;
     uint32_t* probe_keys;        // [nq x nL0] meso centroid distances (float bits)
+    uint32_t parts;              // CTAs that share the stages of a partials tile (1: one runs all)
     uint32_t probe_smem;         // meso list CTA: sort keys, list counters
     uint32_t probe_q;            // queries per meso list CTA (1..16), one warp each
 };

@@ -112,6 +112,10 @@ struct PartialsSmem {
     uint32_t cp[kMaxCheckpoints]; // warmup checkpoints
 };
 
+// blockIdx.z: vector tile and part. With one part (large batches) a CTA runs all stages. A small
+// batch has too few (cluster, query, vector) tiles to fill the GPU, and the stages are a chain of
+// round trips there (about 5 us each): its horizontal blocks, which do not depend on each other or
+// on the vertical chains, go to tp.parts - 1 CTAs beside the one that runs the vertical dims.
 __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(const __grid_constant__ TopLevelParams tp) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     PartialsSmem& S = *reinterpret_cast<PartialsSmem*>(smem_raw);
@@ -121,7 +125,8 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
     if (first >= cnt) return;
     const DevLevel& l0 = tp.l0;
     const DevCluster c = l0.clusters[m];
-    const uint32_t v0 = blockIdx.z * kTV;
+    const uint32_t part = blockIdx.z % tp.parts;
+    const uint32_t v0 = blockIdx.z / tp.parts * kTV;
     if (v0 >= c.n) return;
     const uint32_t n_pad = c.n_pad, stride = (c.n + 3u) & ~3u;
     const uint32_t d = l0.d, dv = l0.dv, nb = l0.n_hblocks, ncp = tp.ncp;
@@ -145,6 +150,10 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
     const float* hor = reinterpret_cast<const float*>(tp.arena + c.hor_off);
     const uint32_t nvc = (dv + kTD - 1) / kTD;  // vertical stages
     const uint32_t nst = nvc + nb;
+    // this CTA's stages: all; part 0 the vertical ones, parts 1 .. a share of the horizontal blocks each
+    const uint32_t s_begin = part == 0 ? 0u : nvc + (part - 1) * nb / (tp.parts - 1);
+    const uint32_t s_end = tp.parts == 1 ? nst : (part == 0 ? nvc : nvc + part * nb / (tp.parts - 1));
+    if (s_begin == s_end) return;
 
     // stage s: query dims and the cluster block it covers, into buffer s & 1
     auto issue = [&](uint32_t st) {
@@ -194,11 +203,11 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
     auto slot_ok = [&](int i) { return slot0 + 4 * i < ntile; };
     auto out_row = [&](int i, uint32_t row) { return tp.vals + S.qoff[slot0 + 4 * i] + (size_t)row * stride; };
 
-    issue(0);
+    issue(s_begin);
     cp_async_commit();
     // Stage st is in buffer st & 1 once this returns; st + 1 is in flight.
     auto begin_stage = [&](uint32_t st) {
-        if (st + 1 < nst) issue(st + 1);
+        if (st + 1 < s_end) issue(st + 1);
         cp_async_commit();
         cp_async_wait1();
         __syncthreads();
@@ -253,7 +262,9 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
         }
     };
     const bool tail = c.n - v0 <= 16u;
-    if (tail) vertical(std::integral_constant<int, 1>());
+    if (part != 0) {
+        // another CTA's
+    } else if (tail) vertical(std::integral_constant<int, 1>());
     else vertical(std::integral_constant<int, 2>());
 
     // horizontal blocks: per (query, vector) the AVX2 Horizontal sum of each block. Lanes
@@ -263,7 +274,7 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
     // per thread; it stores nothing from the rest.
     auto horizontal = [&](auto nb_tag, int passes) {
         constexpr int NB = decltype(nb_tag)::value;
-        for (uint32_t st = nvc; st < nst; ++st) {
+        for (uint32_t st = s_begin > nvc ? s_begin : nvc; st < s_end; ++st) {
             begin_stage(st);
             const float* qs = S.q[st & 1];
             const float* xs = S.x[st & 1];
@@ -334,11 +345,88 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
 }
 
 // -------------------------------------------------------------------------------- replay
+// Bound by the latency of one warp's chain of visits, merge by merge. So the heap is kept in
+// registers once it is full (HR per lane: k <= 32 HR; HR = 0 keeps it in shared memory), a visit's
+// cluster record, ids and partials are requested a visit ahead, four warmup steps and four
+// horizontal blocks are read together, and a candidate that a merge has ruled out costs nothing:
+// 292 us for 10,000 queries (16 of 32 meso clusters of 31 vectors each, k 32) and 81 us for 777,
+// against 344 and 94 with the heap in shared memory and each of these read at its use.
+
+// The full heap: slot j's distance bits and id in lane j % 32, register j / 32.
+template <int HR>
+struct TopHeap {
+    uint32_t d[HR ? HR : 1], id[HR ? HR : 1];
+    float* hd;
+    uint32_t* hid;
+    __device__ __forceinline__ void load(uint32_t k) {
+        const uint32_t lane = threadIdx.x & 31;
+        if constexpr (HR > 0) {
+#pragma unroll
+            for (int r = 0; r < HR; ++r) {
+                const uint32_t j = 32 * r + lane;
+                // an unused slot is never the lowest slot of the largest key
+                d[r] = j < k ? __float_as_uint(hd[j]) : 0u;
+                id[r] = j < k ? hid[j] : 0u;
+            }
+        }
+    }
+    // largest distance and its lowest slot, on every lane
+    __device__ __forceinline__ void top(uint32_t k, float& t, uint32_t& slot) const {
+        if constexpr (HR == 0) {
+            warp_heap_top(hd, k, t, slot);
+        } else {
+            const uint32_t lane = threadIdx.x & 31;
+            uint32_t best = d[0], bs = lane;
+#pragma unroll
+            for (int r = 1; r < HR; ++r)
+                if (d[r] > best) {
+                    best = d[r];
+                    bs = 32 * r + lane;
+                }
+            const uint32_t gmax = __reduce_max_sync(0xffffffffu, best);
+            if constexpr (HR == 1) slot = __ffs(__ballot_sync(0xffffffffu, best == gmax)) - 1;
+            else slot = __reduce_min_sync(0xffffffffu, best == gmax ? bs : 0xFFFFFFFFu);
+            t = __uint_as_float(gmax);
+        }
+    }
+    __device__ __forceinline__ void set(uint32_t slot, float dist, uint32_t row) {
+        const uint32_t lane = threadIdx.x & 31;
+        if constexpr (HR == 0) {
+            if (lane == 0) {
+                hd[slot] = dist;
+                hid[slot] = row;
+            }
+            __syncwarp();
+        } else {
+#pragma unroll
+            for (int r = 0; r < HR; ++r)
+                if (slot == 32 * r + lane) {
+                    d[r] = __float_as_uint(dist);
+                    id[r] = row;
+                }
+        }
+    }
+    __device__ __forceinline__ void store(uint32_t k) const {
+        if constexpr (HR > 0) {
+            const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+            for (int r = 0; r < HR; ++r) {
+                const uint32_t j = 32 * r + lane;
+                if (j < k) {
+                    hd[j] = __uint_as_float(d[r]);
+                    hid[j] = id[r];
+                }
+            }
+            __syncwarp();
+        }
+    }
+};
 
 // Shared memory of the replay: the ratio table (d floats) for the CTA, then per warp
-//   sortbuf [r_sort_cap] u64 | pre [2][r_pre_floats] | hd, hid [r_heap_cap] | dist, pos [r_work_cap]
-//   | meta [top] x {cluster, partials offset}
-__global__ void top_replay_kernel(const __grid_constant__ TopLevelParams tp) {
+//   sortbuf [r_sort_cap] u64 | pre [2][r_pre_floats] | hd, hid [r_heap_cap] | dist [r_work_cap]
+//   | meta [top] x {cluster, partials offset, vectors}
+template <int HR>
+__global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__ TopLevelParams tp) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const DevLevel& l0 = tp.l0;
@@ -358,9 +446,9 @@ __global__ void top_replay_kernel(const __grid_constant__ TopLevelParams tp) {
     float* hd = prebuf + 2 * tp.r_pre_floats;
     uint32_t* hid = reinterpret_cast<uint32_t*>(hd + tp.r_heap_cap);
     float* dist = reinterpret_cast<float*>(hid + tp.r_heap_cap);
-    uint32_t* pos = reinterpret_cast<uint32_t*>(dist + tp.r_work_cap);
-    uint32_t* meta_c = pos + tp.r_work_cap;   // [top] probed meso cluster
+    uint32_t* meta_c = reinterpret_cast<uint32_t*>(dist + tp.r_work_cap);  // [top] probed meso cluster
     uint32_t* meta_o = meta_c + tp.top;       // [top] offset of its partials
+    uint32_t* meta_n = meta_o + tp.top;       // [top] its vectors
 
     const uint32_t k = tp.q_nprobe ? __ldg(tp.q_nprobe + q) : tp.k1;
     const uint32_t m_top = tp.ntop[q];
@@ -373,47 +461,60 @@ __global__ void top_replay_kernel(const __grid_constant__ TopLevelParams tp) {
         return __fmul_rn(top, r);
     };
     for (uint32_t r = lane; r < m_top; r += 32) {
-        meta_c[r] = tp.order[(size_t)q * tp.top + r];
+        const uint32_t c = tp.order[(size_t)q * tp.top + r];
+        meta_c[r] = c;
         meta_o[r] = tp.off[(size_t)q * tp.top + r];
+        meta_n[r] = l0.clusters[c].n;
     }
     __syncwarp();
     // next probed cluster with vectors at or after r (m_top if none)
     auto next_nonempty = [&](uint32_t r) {
-        while (r < m_top && l0.clusters[meta_c[r]].n == 0) ++r;
+        while (r < m_top && meta_n[r] == 0) ++r;
         return r;
     };
     // all partial rows of probed cluster r into buffer `buf`, asynchronously
     auto fetch = [&](uint32_t r, int buf) {
-        const uint32_t n = l0.clusters[meta_c[r]].n;
-        const uint32_t n4 = tp.nvals * ((n + 3u) & ~3u) / 4;
+        const uint32_t n4 = tp.nvals * ((meta_n[r] + 3u) & ~3u) / 4;
         const float4* src = reinterpret_cast<const float4*>(qvals + meta_o[r]);
         float* dst = prebuf + (size_t)buf * tp.r_pre_floats;
         for (uint32_t i = lane; i < n4; i += 32) cp_async16(dst + 4 * i, src + i);
         cp_async_commit();
     };
+    // cluster record and the ids of its first 32 vectors
+    auto first_ids = [&](const DevCluster& c) {
+        return lane < c.n ? __ldg(reinterpret_cast<const uint32_t*>(tp.arena + c.ids_off) + lane) : 0u;
+    };
 
     uint32_t hsize = 0, slot = 0;
     float top = 0.0f;
+    TopHeap<HR> heap;
+    heap.hd = hd;
+    heap.hid = hid;
     uint32_t r = next_nonempty(0);
     int buf = 0;
-    if (r < m_top) fetch(r, 0);
+    DevCluster c{}, cn{};
+    uint32_t id0 = 0;
+    if (r < m_top) {
+        fetch(r, 0);
+        c = l0.clusters[meta_c[r]];
+        id0 = first_ids(c);
+    }
     while (r < m_top) {
         const uint32_t rn = next_nonempty(r + 1);
         if (rn < m_top) {
             fetch(rn, buf ^ 1);
+            cn = l0.clusters[meta_c[rn]];
             cp_async_wait1();
         } else {
             cp_async_wait0();
         }
         __syncwarp();
         const float* pre = prebuf + (size_t)buf * tp.r_pre_floats;
-        const DevCluster c = l0.clusters[meta_c[r]];
         const uint32_t n = c.n;
         ++visits;
         const uint32_t stride = (n + 3u) & ~3u;
-        // the loop body runs once per non-empty probed cluster; `continue` is not used below
-        do {
         const uint32_t* ids = reinterpret_cast<const uint32_t*>(tp.arena + c.ids_off);
+        uint32_t id0n = 0;
         if (hsize < k) {
             // Start (searcher.hpp:217-281): full distances, push the best k - |heap| in the
             // order LevelOps::push_smallest uses (below the m-th key by position, then ties)
@@ -443,98 +544,111 @@ __global__ void top_replay_kernel(const __grid_constant__ TopLevelParams tp) {
                     const uint32_t at = cntp + __popc(bal & ((1u << lane) - 1u));
                     if (sel && at < mm) {
                         hd[hsize + at] = dist[v];
-                        hid[hsize + at] = __ldg(ids + v);
+                        hid[hsize + at] = b0 ? __ldg(ids + v) : id0;
                     }
                     cntp += __popc(bal);
                 }
             }
             hsize += mm;
             __syncwarp();
-            warp_heap_top(hd, hsize, top, slot);
-            break;
-        }
-        // Warmup (searcher.hpp:374-435): vertical checkpoints until >= ceil(0.8 n) fail the bound
-        const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
-        uint32_t cur = 0, step = 0, n_pruned = 0;
-        while (n_pruned < needed && cur < dv) {
-            const uint32_t last = tp.cp[step];
-            const float thr = thr_at(last, top);
-            bytes += (unsigned long long)n * (last - cur) * 4u;
-            uint32_t cntp = 0;
-            const float* row = pre + (size_t)step * stride;
-            for (uint32_t v = lane; v < n; v += 32) cntp += row[v] >= thr ? 1u : 0u;
-            n_pruned = __reduce_add_sync(0xffffffffu, cntp);
-            cur = last;
-            ++step;
-        }
-        // Prune (searcher.hpp:437-540). The bound's heap top is fixed until the merge, so each
-        // vector's way through the horizontal blocks and the remaining vertical dims depends on
-        // that vector alone: each lane follows its own vectors, and the survivors of every
-        // step are the same, in the same order, as with the step-by-step compaction.
-        const float* erow = pre + (size_t)(step - 1) * stride;
-        const float* vert = reinterpret_cast<const float*>(tp.arena + c.vert_off);
-        unsigned long long lane_bytes = 0;
-        for (uint32_t c0 = 0; c0 < n; c0 += 32) {
-            const uint32_t v = c0 + lane;
-            bool alive = v < n;
-            float dd = alive ? erow[v] : 0.0f;
-            uint32_t cv = cur;
-            alive = alive && dd < thr_at(cv, top);
-            for (uint32_t b = 0; alive && b < nb; ++b) {
-                lane_bytes += kHDim * 4u;
-                dd = __fadd_rn(dd, pre[(size_t)(ncp + b) * stride + v]);
-                cv += kHDim;
-                alive = dd < thr_at(cv, top);
+            if (hsize >= k) {  // full: from here on only merges change it
+                heap.load(k);
+                heap.top(k, top, slot);
             }
-            uint32_t cur_v = cur;
-            while (alive && cur_v < dv) {
-                const uint32_t last = (cur_v + kHDim < dv) ? cur_v + kHDim : dv;
-                lane_bytes += (unsigned long long)(last - cur_v) * 4u;
-                for (uint32_t j = cur_v; j < last; ++j) {
-                    const float t = __fsub_rn(__ldg(qf + j), __ldg(vert + (size_t)j * c.n_pad + v));
-                    dd = __fmaf_rn(t, t, dd);
-                }
-                cv = (cv + kHDim < d) ? cv + kHDim : d;
-                cur_v = last;
-                alive = dd < thr_at(cv, top);
-                if (cv == d) break;
-            }
-            if (v < n) {
-                dist[v] = dd;
-                pos[v] = alive ? 1u : 0u;
-            }
-        }
-        bytes += __reduce_add_sync(0xffffffffu, (uint32_t)lane_bytes);
-        __syncwarp();
-        // MergeIntoHeap (searcher.hpp:542-566): sequential, strict-<, in position order
-        for (uint32_t c0 = 0; c0 < n; c0 += 32) {
-            const uint32_t v = c0 + lane;
-            const bool alive = v < n && pos[v] != 0u;
-            const float dd = alive ? dist[v] : 0.0f;
-            const uint32_t idv = alive ? __ldg(ids + v) : 0u;
-            unsigned bal = __ballot_sync(0xffffffffu, alive);
-            while (bal) {
-                const int i = __ffs(bal) - 1;
-                bal &= bal - 1;
-                const float ddi = __shfl_sync(0xffffffffu, dd, i);
-                const uint32_t idi = __shfl_sync(0xffffffffu, idv, i);
-                if (hsize < k || ddi < top) {
-                    if (lane == 0) {
-                        const uint32_t at = (hsize >= k) ? slot : hsize;
-                        hd[at] = ddi;
-                        hid[at] = idi;
+            if (rn < m_top) id0n = first_ids(cn);
+        } else {
+            // Warmup (searcher.hpp:374-435): vertical checkpoints until >= ceil(0.8 n) fail the bound
+            const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
+            uint32_t step = 0;
+            for (uint32_t s0 = 0, n_pruned = 0; n_pruned < needed && s0 < ncp; s0 += 4) {
+                uint32_t cnt[4] = {0, 0, 0, 0};
+                for (uint32_t c0 = 0; c0 < n; c0 += 32) {
+                    const uint32_t v = c0 + lane;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const bool on = v < n && s0 + u < ncp;
+                        const float x = on ? pre[(size_t)(s0 + u) * stride + v] : 0.0f;
+                        const float thr = s0 + u < ncp ? thr_at(tp.cp[s0 + u], top) : 0.0f;
+                        cnt[u] += __popc(__ballot_sync(0xffffffffu, on && x >= thr));
                     }
-                    if (hsize < k) ++hsize;
-                    __syncwarp();
-                    warp_heap_top(hd, hsize, top, slot);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (n_pruned < needed && s0 + u < ncp) {
+                        n_pruned = cnt[u];
+                        step = s0 + u + 1;
+                    }
+            }
+            const uint32_t cur = tp.cp[step - 1];
+            bytes += (unsigned long long)n * cur * 4u;
+            if (rn < m_top) id0n = first_ids(cn);
+            // Prune (searcher.hpp:437-540) and MergeIntoHeap (searcher.hpp:542-566). The bound's heap
+            // top is the one before the cluster's merges, so each vector's way through the
+            // horizontal blocks and the remaining vertical dims depends on that vector alone: each
+            // lane follows its own vectors, and the survivors of every step are the same, in the
+            // same order, as with the step-by-step compaction.
+            const float tc = top;
+            const float* erow = pre + (size_t)(step - 1) * stride;
+            const float* vert = reinterpret_cast<const float*>(tp.arena + c.vert_off);
+            uint32_t lane_bytes = 0;
+            for (uint32_t c0 = 0; c0 < n; c0 += 32) {
+                const uint32_t v = c0 + lane;
+                const bool in = v < n;
+                float dd = in ? erow[v] : 0.0f;
+                uint32_t cv = cur;
+                bool alive = in && dd < thr_at(cv, tc);
+                for (uint32_t b0 = 0; b0 < nb && __any_sync(0xffffffffu, alive); b0 += 4) {
+                    float x[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) x[u] = in && b0 + u < nb ? pre[(size_t)(ncp + b0 + u) * stride + v] : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (alive && b0 + u < nb) {
+                            lane_bytes += kHDim * 4u;
+                            dd = __fadd_rn(dd, x[u]);
+                            cv += kHDim;
+                            alive = dd < thr_at(cv, tc);
+                        }
+                    }
+                }
+                uint32_t cur_v = cur;
+                while (alive && cur_v < dv) {
+                    const uint32_t last = (cur_v + kHDim < dv) ? cur_v + kHDim : dv;
+                    lane_bytes += (last - cur_v) * 4u;
+                    for (uint32_t j = cur_v; j < last; ++j) {
+                        const float t = __fsub_rn(__ldg(qf + j), __ldg(vert + (size_t)j * c.n_pad + v));
+                        dd = __fmaf_rn(t, t, dd);
+                    }
+                    cv = (cv + kHDim < d) ? cv + kHDim : d;
+                    cur_v = last;
+                    alive = dd < thr_at(cv, tc);
+                    if (cv == d) break;
+                }
+                // sequential, strict-<, in position order; the top only falls, so a vector that is
+                // not below it once never is
+                unsigned bal = __ballot_sync(0xffffffffu, alive && dd < top);
+                if (bal) {
+                    const uint32_t idv = c0 ? (alive ? __ldg(ids + v) : 0u) : id0;
+                    while (bal) {
+                        const int i = __ffs(bal) - 1;
+                        const float ddi = __shfl_sync(0xffffffffu, dd, i);
+                        const uint32_t idi = __shfl_sync(0xffffffffu, idv, i);
+                        heap.set(slot, ddi, idi);
+                        heap.top(k, top, slot);
+                        bal &= bal - 1;
+                        bal &= __ballot_sync(0xffffffffu, dd < top);
+                    }
                 }
             }
+            if (tp.stats) bytes += __reduce_add_sync(0xffffffffu, lane_bytes);
         }
-        } while (false);
         __syncwarp();  // every lane is done with `pre` before the next fetch overwrites it
         r = rn;
         buf ^= 1;
+        c = cn;
+        id0 = id0n;
     }
+    if (hsize >= k) heap.store(k);
     // BuildResultSetFromHeap (searcher.hpp:568-585): the L1 clusters, nearest first
     const uint32_t N = next_pow2(hsize ? hsize : 1);
     for (uint32_t i = lane; i < N; i += 32)
@@ -573,14 +687,16 @@ cudaError_t launch_top_level_tiled(const TopLevelParams& tp, uint32_t vtiles, in
     const int psmem = (int)sizeof(PartialsSmem);
     e = cudaFuncSetAttribute(meso_partials_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem);
     if (e != cudaSuccess) return e;
-    dim3 grid((tp.nq + kTQ - 1) / kTQ, tp.l0.nclusters, vtiles);
+    dim3 grid((tp.nq + kTQ - 1) / kTQ, tp.l0.nclusters, vtiles * tp.parts);
     meso_partials_kernel<<<grid, kPartialsThreads, psmem, st>>>(tp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[1], st)) != cudaSuccess) return e;
     const size_t rsmem = tp.r_smem;
-    e = cudaFuncSetAttribute(top_replay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem);
+    // heap registers a lane: k1 (the largest k of the batch) up to 32 or 128
+    auto replay = tp.k1 <= 32 ? top_replay_kernel<1> : tp.k1 <= 128 ? top_replay_kernel<4> : top_replay_kernel<0>;
+    e = cudaFuncSetAttribute(replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem);
     if (e != cudaSuccess) return e;
-    top_replay_kernel<<<(tp.nq + replay_warps - 1) / replay_warps, 32 * replay_warps, rsmem, st>>>(tp);
+    replay<<<(tp.nq + replay_warps - 1) / replay_warps, 32 * replay_warps, rsmem, st>>>(tp);
     return cudaGetLastError();
 }
 
