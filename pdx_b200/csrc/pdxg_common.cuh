@@ -92,10 +92,11 @@ struct SearchParams {
     uint32_t q_order_filtered;      // 1: the filtered queries have a row too (exact probe ahead)
     // batched Start (pdxg_start.cu): exact U8 distances to every vector of each query's first
     // visited cluster, computed ahead with reuse across queries
-    const int32_t* start_row;       // optional [nq]: row in start_dist, -1 = none
-    const uint32_t* start_first;    // [nq] the cluster of that row
+    const int32_t* start_row;       // optional [nq x start_visits]: row in start_dist, -1 = none
+    const uint32_t* start_first;    // [nq x start_visits] the cluster of that row
     const uint32_t* start_dist;     // [rows x start_stride]
     uint32_t start_stride;
+    uint32_t start_visits;
     // optional: only the queries q_list[0 .. *q_list_n) are searched (the rest of a batch went
     // through the cluster-major scan, pdxg_scan.cu)
     const uint32_t* q_list;
@@ -176,21 +177,26 @@ struct StartParams {
     const uint32_t* q_order_count;
     uint32_t q_order_stride;
     const int32_t* filter_of;     // optional: queries with filter_of != -1 are left out
-    uint32_t* cl_count;           // [n1] queries per first cluster (zeroed before)
+    uint32_t k;
+    const uint32_t* q_k;          // optional per-query k (<= k)
+    uint32_t visits;              // Starts computed for a query at most
+    uint32_t* cl_count;           // [n1] Starts per cluster (zeroed before)
     uint32_t* cl_off;             // [n1] first row of each cluster
     uint32_t* cl_items;           // [n1] first work item of each cluster
-    uint32_t* first_cl;           // [nq] first non-empty visited cluster (~0u: none)
-    uint32_t* slot_of;            // [nq] position among that cluster's queries
-    int32_t* row_of;              // [nq] row in dist (-1: none)
-    uint32_t* sorted_q;           // [nq] queries grouped by first cluster (row order)
+    uint32_t* first_cl;           // [nq x visits] non-empty visited clusters that fill the heap (~0u: none)
+    uint32_t* slot_of;            // [nq x visits] position among that cluster's Starts
+    int32_t* row_of;              // [nq x visits] row in dist (-1: none)
+    uint32_t* sorted_q;           // [nq x visits] Starts q * visits + s grouped by cluster (row order)
+    uint32_t* full_at;            // [nq] position in the order of the Start that fills the heap (~0u: the
+                                  // query needs more than `visits` Starts, or has none)
     uint32_t* items;              // [2 x item bound] (cluster, query chunk << 16 | vector chunk)
     uint32_t* n_items;            // [1]
     uint32_t* queue;              // [1] work counter
-    uint32_t* dist;               // [nq x stride] exact U8 distances
+    uint32_t* dist;               // [nq x visits rows x stride] distances (U8 integers / float bits)
     uint32_t stride;              // >= largest L1 cluster
 };
 
-// Cluster-major scan of U8 levels (pdxg_scan.cu): the first warmup step of every (query,
+// Cluster-major scan (pdxg_scan.cu): the first warmup step of every (query,
 // visited cluster) pair computed per cluster for all its queries, then one warp per query
 // replaying PDXearch on those results.
 struct ScanParams {
@@ -205,25 +211,29 @@ struct ScanParams {
     const uint32_t* q_order;      // [nq x q_order_stride] L1 visit orders
     const uint32_t* q_order_count;
     uint32_t q_order_stride;
-    const int32_t* start_row;     // batched Start (pdxg_start.cu): row of each query, -1 none
-    const uint32_t* start_first;  // [nq] the cluster of that row
+    const int32_t* start_row;     // batched Start (pdxg_start.cu): [nq x start_visits] rows, -1 none
+    const uint32_t* start_first;  // [nq x start_visits] the clusters of those rows
+    uint32_t start_visits;
+    const uint32_t* full_at;      // [nq] position in the order of the Start that fills the heap, ~0u none
     uint32_t* start_dist;         // [rows x start_stride]; a query's row is its scratch afterwards
     uint32_t start_stride;
     uint32_t cp1;                 // first warmup checkpoint: min(16, d_v)
-    uint32_t g1;                  // vertical words it covers: ceil(cp1 / 4) (<= 4)
-    uint32_t nwords;              // packed query words: qw_hoff + 16 n_hblocks
-    uint32_t* qwords;             // [nq x nwords] quantized queries, packed as the scan packs them
-    uint32_t* first_i;            // [nq] position of the Start cluster in the order; ~0u: not here
-    int32_t* lim;                 // [nq] a vector is a candidate when |x|^2 - 2 q.x < lim
+    uint32_t g1;                  // vertical words it covers: ceil(cp1 / 4) (<= 4), F32 cp1
+    uint32_t nwords;              // query words: U8 qw_hoff + 16 n_hblocks, F32 d
+    uint32_t* qwords;             // [nq x nwords] U8: quantized queries, packed as the scan packs
+                                  // them (written by the prep kernel); F32: the queries themselves
+    uint32_t* first_i;            // [nq] position of the last Start in the order; ~0u: not here
+    int32_t* lim;                 // [nq] a vector is a candidate when |x|^2 - 2 q.x < lim (F32: lim is a
+                                  // float, with the margin of scan_bitmap_kernel)
     float* heap_d;                // [nq x k] the Start's pushes, in push order
     uint32_t* heap_id;
     uint32_t* left;               // [nq] queries left to the per-query scan kernel
-    uint32_t* left_n;             // [1] (zeroed before; n_items, queue and hv_alloc follow it)
+    uint32_t* left_n;             // [1] (zeroed before; n_items and hv_alloc follow it)
     uint32_t* vl_count;           // [n1] visits per cluster (zeroed before)
     uint32_t* vl;                 // [n1 x nq] visits of each cluster: q * q_order_stride + i
-    uint32_t* items;              // [2 x item bound] (cluster, chunk of 64 list entries)
+    uint32_t* items;              // [2 x item bound] (cluster, first list entry of a chunk)
     uint32_t* n_items;            // [1] (zeroed before)
-    uint32_t* queue;              // [1] work counter (zeroed before)
+    uint32_t item_bound;          // n_items at most
     uint32_t* bm;                 // [nq x q_order_stride x bm_words] candidate bitmaps
     uint32_t bm_words;            // ceil(largest cluster / 32)
     uint32_t bm_tile;             // 1: a work item's bitmaps are kept in shared memory first
@@ -240,6 +250,7 @@ struct ScanParams {
     unsigned long long* stats;    // optional, SearchParams::stats layout
     uint32_t prep_qs;             // 1: the prep kernel stages each query row in shared memory
     uint32_t prep_qs_stride;      // floats per staged row
+    uint32_t p_qpc;               // prep: queries per CTA (1..8), one warp each
     uint32_t r_qpc;               // replay: queries per CTA (1..8), one warp each
     uint32_t r_surv_cap;          // replay: survivors of one cluster's first warmup step it keeps
     uint32_t r_heap_cap;          // replay shared memory per warp: heap entries,

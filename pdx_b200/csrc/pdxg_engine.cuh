@@ -90,8 +90,8 @@ struct Workspace {
     uint64_t l1_order_cap = 0;
     uint32_t* d_l1_count = nullptr;
     uint64_t l1_count_cap = 0;
-    // batched Start: per-cluster counters ([3 x n1]), per-query arrays ([4 x nq]), work items,
-    // counters, distances
+    // batched Start: per-cluster counters ([3 x n1]), per-query arrays (4 per Start, 1 per query) and
+    // two counters, work items, distances
     uint32_t* d_st_cl = nullptr;
     uint64_t st_cl_cap = 0;
     uint32_t* d_st_q = nullptr;
@@ -128,8 +128,8 @@ struct Workspace {
     float* d_qlo = nullptr;
     uint64_t qhi_cap = 0, qlo_cap = 0;
     int* d_gemm_err = nullptr;
-    // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq + 4]:
-    // first_i | lim | left | left_n, n_items, queue, hv_alloc), Start heaps, per-cluster visit lists and
+    // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq + 3]:
+    // first_i | lim | left | left_n, n_items, hv_alloc), Start heaps, per-cluster visit lists and
     // counters, work items, candidate bitmaps
     uint32_t* d_sc_qw = nullptr;
     uint64_t sc_qw_cap = 0;
@@ -198,6 +198,7 @@ struct Launch {
     int grid = 1;
     uint32_t top_launches = 0;  // kernels of a separate tree top level
     uint32_t scan_launches = 0;  // kernels of the cluster-major scan ahead of the per-query kernel
+    const uint32_t* start_full_at = nullptr;  // batched Start: where each query's heap is full
     uint32_t start_launches = 0;  // kernels of the batched Start
     uint32_t probe_launches = 0;  // kernels of the reduced-precision probe (rotation included)
 };

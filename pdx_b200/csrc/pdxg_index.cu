@@ -34,18 +34,17 @@ int top_level_occupancy(size_t smem, int threads);
 cudaError_t launch_top_level_tiled(const TopLevelParams& tp, uint32_t vtiles, int replay_warps,
                                    cudaStream_t st, const cudaEvent_t* ev);
 cudaError_t launch_start_batched(const StartParams& sp, int grid, cudaStream_t st);
-cudaError_t launch_scan(const ScanParams& sp, int bitmap_grid, cudaStream_t st, const cudaEvent_t* ev);
-uint64_t scan_item_bound(uint32_t nq, uint32_t stride, uint32_t n1);
-int scan_bitmap_occupancy(uint32_t bm_words);
+cudaError_t launch_scan(const ScanParams& sp, cudaStream_t st, const cudaEvent_t* ev);
+uint64_t scan_item_bound(uint32_t nq, uint32_t stride, uint32_t n1, uint32_t max_n);
 size_t scan_bitmap_smem(uint32_t bm_words);
 uint32_t scan_queries_per_cta();
 cudaError_t launch_row_sq(const float* x, uint32_t n, uint32_t d, float* out, cudaStream_t st);
 size_t probe_select_smem(uint32_t d, uint32_t n1, uint32_t cand_cap, uint32_t sort_cap);
 cudaError_t launch_probe_select(const ProbeParams& pp, cudaStream_t st);
 cudaError_t launch_probe_exact(const ProbeParams& pp, cudaStream_t st);
-int start_dist_occupancy(size_t smem);
+int start_dist_occupancy(bool u8, size_t smem);
 size_t start_dist_smem(const DevLevel& lv);
-uint64_t start_item_bound(uint32_t nq, uint32_t n1, uint32_t max_n);
+uint64_t start_item_bound(bool u8, uint32_t nq, uint32_t n1, uint32_t max_n);
 }  // namespace pdxg
 
 using namespace pdxg;
@@ -1065,29 +1064,47 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
     return PDXG_OK;
 }
 
-// Batched Start (pdxg_start.cu) for U8 levels whose visit orders are known before the scan
+// Batched Start (pdxg_start.cu) for levels whose visit orders are known before the scan
 // (tree indexes with a separate top level). Sets L.p.start_* when it ran; a batch outside its
 // limits leaves them unset and the scan runs Start itself.
 constexpr uint32_t kStartMinQueries = 32;
+constexpr uint32_t kStartMaxVisits = 4;
+
+// Starts a query needs to fill a heap of k, at most kStartMaxVisits: the smallest clusters' turn.
+uint32_t start_visits(const HostLevel& lv, uint32_t k) {
+    std::vector<uint32_t> n;
+    for (uint32_t x : lv.n)
+        if (x && x < k) n.push_back(x);
+    if (n.empty()) return 1;
+    const size_t m = std::min<size_t>(n.size(), kStartMaxVisits - 1);
+    std::partial_sort(n.begin(), n.begin() + m, n.end());
+    uint64_t have = 0;
+    uint32_t s = 0;
+    while (s < m && have < k) have += n[s++];
+    return have < k ? s + 1 : s;
+}
 constexpr uint32_t kHeavyPerQuery = 128;          // cluster-major scan: see run_scan_cluster_major
 constexpr uint64_t kHeavyMaxValues = 64ull << 20;  // 256 MB
 
 int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st) {
     L.p.start_row = nullptr;
-    if (!ix->u8 || !L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return PDXG_OK;
+    if (!L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return PDXG_OK;
     const uint32_t n1 = L.p.l1.nclusters;
     const uint32_t stride = (std::max(L.p.l1.max_n, 1u) + 3) & ~3u;
-    const uint64_t items = start_item_bound(nq, n1, std::max(L.p.l1.max_n, 1u));
-    if ((uint64_t)nq * stride * 4 > (4ull << 30) || items > 0xFFFFFFFFull || nq > (1u << 20)) return PDXG_OK;
+    uint32_t visits = start_visits(ix->l1, L.p.k);
+    while (visits > 1 && (uint64_t)nq * visits * stride * 4 > (4ull << 30)) --visits;
+    const uint64_t ne = (uint64_t)nq * visits;
+    const uint64_t items = start_item_bound(ix->u8, (uint32_t)ne, n1, std::max(L.p.l1.max_n, 1u));
+    if (items == 0 || (uint64_t)nq * stride * 4 > (4ull << 30) || items > 0xFFFFFFFFull || nq > (1u << 20)) return PDXG_OK;
     const size_t smem = start_dist_smem(L.p.l1);
     if (smem + 1024 > ix->max_smem) return PDXG_OK;
-    const int occ = start_dist_occupancy(smem);
+    const int occ = start_dist_occupancy(ix->u8, smem);
     if (occ <= 0) return PDXG_OK;
     int rc;
     if ((rc = dev_grow(w.d_st_cl, w.st_cl_cap, (uint64_t)3 * n1))) return rc;
-    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, (uint64_t)4 * nq + 2))) return rc;
+    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + nq + 2))) return rc;
     if ((rc = dev_grow(w.d_st_items, w.st_items_cap, 2 * items))) return rc;
-    if ((rc = dev_grow(w.d_st_dist, w.st_dist_cap, (uint64_t)nq * stride))) return rc;
+    if ((rc = dev_grow(w.d_st_dist, w.st_dist_cap, ne * stride))) return rc;
     StartParams sp{};
     sp.arena = ix->arena;
     sp.l1 = L.p.l1;
@@ -1100,12 +1117,16 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     sp.cl_count = w.d_st_cl;
     sp.cl_off = w.d_st_cl + n1;
     sp.cl_items = w.d_st_cl + 2 * (uint64_t)n1;
+    sp.k = L.p.k;
+    sp.q_k = L.p.q_k;
+    sp.visits = visits;
     sp.first_cl = w.d_st_q;
-    sp.slot_of = w.d_st_q + nq;
-    sp.row_of = reinterpret_cast<int32_t*>(w.d_st_q + 2 * (uint64_t)nq);
-    sp.sorted_q = w.d_st_q + 3 * (uint64_t)nq;
-    sp.n_items = w.d_st_q + 4 * (uint64_t)nq;
-    sp.queue = w.d_st_q + 4 * (uint64_t)nq + 1;
+    sp.slot_of = w.d_st_q + ne;
+    sp.row_of = reinterpret_cast<int32_t*>(w.d_st_q + 2 * ne);
+    sp.sorted_q = w.d_st_q + 3 * ne;
+    sp.full_at = w.d_st_q + 4 * ne;
+    sp.n_items = w.d_st_q + 4 * ne + nq;
+    sp.queue = w.d_st_q + 4 * ne + nq + 1;
     sp.items = w.d_st_items;
     sp.dist = w.d_st_dist;
     sp.stride = stride;
@@ -1114,6 +1135,8 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     L.p.start_first = sp.first_cl;
     L.p.start_dist = sp.dist;
     L.p.start_stride = stride;
+    L.p.start_visits = visits;
+    L.start_full_at = sp.full_at;
     L.start_launches = 3;
     return PDXG_OK;
 }
@@ -1126,12 +1149,14 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     L.p.q_list_n = nullptr;
     L.scan_launches = 0;
     ix->tev_scan = false;
-    if (ix->scan_mode != 0 || !L.u8 || !L.p.start_row || !L.p.q_order || L.p.order || L.p.l1.tomb) return PDXG_OK;
+    if (ix->scan_mode != 0 || !L.p.start_row || !L.p.q_order || L.p.order || L.p.l1.tomb) return PDXG_OK;
     const DevLevel& lv = L.p.l1;
     const uint32_t n1 = lv.nclusters, stride = L.p.q_order_stride, k = L.p.k;
-    const uint32_t nwords = lv.qw_hoff + lv.n_hblocks * 16;
+    const uint32_t nwords = L.u8 ? lv.qw_hoff + lv.n_hblocks * 16 : lv.d;
     const uint32_t bm_words = (std::max(lv.max_n, 1u) + 31) / 32;
-    if ((uint64_t)nq * stride >= 0xFFFFFFFFull || (uint64_t)n1 * nq > (256ull << 20) || stride == 0) return PDXG_OK;
+    if ((uint64_t)nq * stride >= 0xFFFFFFFFull || (uint64_t)n1 * nq > (256ull << 20) || stride == 0 ||
+        (uint64_t)nq * stride * bm_words > (2ull << 30))  // 8 GB of bitmaps
+        return PDXG_OK;
     ScanParams sp{};
     sp.r_heap_cap = (k + 3) & ~3u;
     sp.r_area_bytes = (uint32_t)align_up(std::max<uint64_t>(2048, 8ull * next_pow2(k)), 16);
@@ -1140,14 +1165,14 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.r_warp_bytes = (uint32_t)(align_up((uint64_t)nwords * 4, 16) + 8ull * sp.r_heap_cap + sp.r_area_bytes +
                                  align_up((uint64_t)bm_words * 4, 16) + 8ull * sp.r_surv_cap);
     sp.prep_qs_stride = (lv.d + 3) & ~3u;
-    sp.prep_qs = (uint64_t)scan_queries_per_cta() * sp.prep_qs_stride * 4 + 9 * 1024 <= ix->max_smem ? 1u : 0u;
+    sp.prep_qs = (uint64_t)scan_queries_per_cta() * sp.prep_qs_stride * 4 + 1024 <= ix->max_smem ? 1u : 0u;
+    sp.p_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + ix->num_sms - 1) / ix->num_sms);
     // a replay CTA of 8 warps takes as few queries as still fill the GPU at 3 CTAs per SM, so that
     // the heavy visits of a small batch are shared by more warps
     sp.r_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + 3 * ix->num_sms - 1) / (3 * ix->num_sms));
     if ((uint64_t)sp.r_warp_bytes * scan_queries_per_cta() + 2048 > ix->max_smem) return PDXG_OK;
-    const int occ = scan_bitmap_occupancy(bm_words);
-    if (occ <= 0) return PDXG_OK;
-    const uint64_t items = scan_item_bound(nq, stride, n1);
+    const uint64_t items = scan_item_bound(nq, stride, n1, std::max(lv.max_n, 1u));
+    if (items > 0x7FFFFFFFull) return PDXG_OK;
     // values of heavy visits: columns for kHeavyPerQuery vectors a query on average (16-70 were
     // measured); visits past them are left to the replay
     uint32_t cps[kMaxCheckpoints];
@@ -1159,8 +1184,8 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     int rc;
     if ((rc = dev_grow(w.d_sc_hv, w.sc_hv_cap, hv_rows * sp.hv_cap))) return rc;
     if ((rc = dev_grow(w.d_sc_vi, w.sc_vi_cap, (uint64_t)nq * stride))) return rc;
-    if ((rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
-    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 4))) return rc;
+    if (L.u8 && (rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
+    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 3))) return rc;
     if ((rc = dev_grow(w.d_sc_heap, w.sc_heap_cap, 2ull * nq * k))) return rc;
     if ((rc = dev_grow(w.d_sc_cl, w.sc_cl_cap, (uint64_t)n1))) return rc;
     if ((rc = dev_grow(w.d_sc_vl, w.sc_vl_cap, (uint64_t)n1 * nq))) return rc;
@@ -1179,19 +1204,21 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.q_order_stride = stride;
     sp.start_row = L.p.start_row;
     sp.start_first = L.p.start_first;
+    sp.start_visits = L.p.start_visits;
+    sp.full_at = L.start_full_at;
     sp.start_dist = const_cast<uint32_t*>(L.p.start_dist);
     sp.start_stride = L.p.start_stride;
     sp.cp1 = std::min(16u, lv.dv);
-    sp.g1 = (sp.cp1 + 3) / 4;
+    sp.g1 = L.u8 ? (sp.cp1 + 3) / 4 : sp.cp1;
     sp.nwords = nwords;
-    sp.qwords = w.d_sc_qw;
+    sp.qwords = L.u8 ? w.d_sc_qw : reinterpret_cast<uint32_t*>(const_cast<float*>(L.p.queries));
     sp.first_i = w.d_sc_q;
     sp.lim = reinterpret_cast<int32_t*>(w.d_sc_q + nq);
     sp.left = w.d_sc_q + 2ull * nq;
     sp.left_n = w.d_sc_q + 3ull * nq;
     sp.n_items = w.d_sc_q + 3ull * nq + 1;
-    sp.queue = w.d_sc_q + 3ull * nq + 2;
-    sp.hv_alloc = w.d_sc_q + 3ull * nq + 3;
+    sp.hv_alloc = w.d_sc_q + 3ull * nq + 2;
+    sp.item_bound = (uint32_t)items;
     sp.hv = w.d_sc_hv;
     sp.vinfo = w.d_sc_vi;
     sp.bm_tile = scan_bitmap_smem(bm_words) ? 1u : 0u;
@@ -1206,7 +1233,7 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.out_dists = L.p.out_dists;
     sp.out_counts = L.p.out_counts;
     sp.stats = L.p.stats;
-    PDXG_CUDA(launch_scan(sp, occ * ix->num_sms, st, timed ? ix->tev + 5 : nullptr));
+    PDXG_CUDA(launch_scan(sp, st, timed ? ix->tev + 5 : nullptr));
     ix->tev_scan = timed;
     L.p.q_list = sp.left;
     L.p.q_list_n = sp.left_n;

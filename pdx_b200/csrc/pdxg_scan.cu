@@ -1,17 +1,18 @@
-// Cluster-major scan of U8 levels: PDXearch (searcher.hpp:217-566) for a whole batch, with the
-// first warmup step computed once per cluster for all the queries that visit it.
+// Cluster-major scan: PDXearch (searcher.hpp:217-566) for a whole batch, with the first warmup
+// step computed once per cluster for all the queries that visit it. Instantiated for U8 and F32
+// levels; "raw" distances are u32 integers or float bits.
 //
-// Per query, PDXearch visits its clusters in order. The first non-empty one is a Start (full
-// distances, the best k pushed); every later one runs Warmup: partial distances over the
+// Per query, PDXearch visits its clusters in order. The first non-empty ones are Starts (full
+// distances, the best pushed) until the heap holds k; every later one runs Warmup: partial distances over the
 // vertical dims in steps of 16, 16, 32, ... (DIMENSIONS_FETCHING_SIZES), testing after each step
-// how many vectors reach the ADSampling bound thr(top) = top * ratio[dims] (as U8 raw distances)
+// how many vectors reach the ADSampling bound thr(top) = top * ratio[dims] (as raw distances)
 // and stopping once ceil(0.8 n) do. On the IVF2 SQ8 workloads that exit comes after the first
 // step almost always, so most of the scan is the first 16 dims of every vector of every visited
 // cluster, one query at a time, each query re-reading the same clusters.
 //
 // The heap top only falls once the heap is full (MergeIntoHeap replaces the top with a smaller
 // distance), and the bound is monotone in it. So the bound a query applies at any later cluster
-// is at most tau0, its heap top right after the Start, and a vector below that later bound at
+// is at most tau0, its heap top right after the last Start, and a vector below that later bound at
 // the first checkpoint is below the bound at tau0. That set -- the candidates -- is computed
 // cluster-major: every cluster's first-checkpoint rows are read once per group of 64 queries and
 // each (query, cluster) pair gets a bitmap of its candidates. Then one warp per query replays
@@ -21,14 +22,15 @@
 // whole warmup itself. Survivors then follow Prune (searcher.hpp:437-540) one per lane and are
 // merged in position order (searcher.hpp:542-566), as in the per-query kernel.
 //
-//   scan_prep_kernel   : warp per query -- quantized query words, the Start's pushes (the m
+//   scan_prep_kernel   : warp per query -- quantized query words, the Starts' pushes (the m
 //                        smallest batched-Start distances, ties by position) and tau0's bound;
 //                        every later visit appended to its cluster's list, with a work item per
-//                        64 list entries; queries this path does not take go to a list for the
+//                        8 to 64 list entries; queries this path does not take go to a list for the
 //                        per-query kernel
-//   scan_bitmap_kernel : persistent CTAs over the items: candidate bitmaps with dp4a, exact
-//                        |q - x|^2 = |q|^2 + |x|^2 - 2 q.x over the first checkpoint's dims; each
-//                        visit is classed as empty (no candidate), light (its bitmap kept) or
+//   scan_bitmap_kernel : a CTA per item: candidate bitmaps over the first checkpoint's dims, with
+//                        |q - x|^2 = |q|^2 + |x|^2 - 2 q.x and q.x on the tensor cores (U8 exact;
+//                        F32 in TF32 with a margin for its error, so the candidates are a superset
+//                        of that set); each visit is classed as empty (no candidate), light (its bitmap kept) or
 //                        heavy (so many candidates that its warmup may pass the first step)
 //   scan_replay_kernel : warp per query -- Warmup / Prune / MergeIntoHeap / result, over the
 //                        visits that are not empty; the heavy visits of a CTA's queries are
@@ -42,9 +44,10 @@
 
 namespace pdxg {
 
-constexpr uint32_t kScanCQ = 64;         // visits per bitmap work item
-constexpr int kBitmapThreads = 256;
-constexpr int kBitmapBPW = 4;            // 32-vector blocks a bitmap warp holds at once
+constexpr uint32_t kScanCQ = 64;         // visits per bitmap work item at most
+constexpr uint32_t kScanCQMin = 8;
+constexpr uint32_t kScanDims = 16;       // dims of the first warmup step at most
+constexpr int kBitmapThreads = 128;
 constexpr int kScanWarps = 8;            // queries per prep / replay CTA
 constexpr uint32_t kOffPath = 0xFFFFFFFFu;
 constexpr uint32_t kHeavyBit = 0x80000000u;  // visit class: 0 empty, candidates of a light visit,
@@ -55,6 +58,15 @@ constexpr uint32_t kBitmapTileMax = 64 * 1024;  // bytes of a work item's bitmap
 // DIMENSIONS_FETCHING_SIZES (common.hpp:47-49)
 __constant__ uint32_t c_scan_fetch[kNumFetchSizes] = {16, 16, 32, 32, 32, 32, 64, 64, 64, 64,
                                                      128, 128, 128, 128, 256, 256, 512, 1024, 2048, 16384};
+
+// Visits per bitmap work item of a cluster of n vectors: cluster sizes differ by a factor of ten and
+// the largest are visited most, so an item is at most about this many pairs, for its time not to
+// stand out at the end of the kernel.
+__host__ __device__ __forceinline__ uint32_t scan_chunk(uint32_t n) {
+    uint32_t cq = kScanCQ;
+    while (cq > kScanCQMin && cq * n > 65536u) cq >>= 1;
+    return cq;
+}
 
 __device__ __forceinline__ uint32_t sq4(uint32_t a, uint32_t b, uint32_t acc) {
     const uint32_t d = __vabsdiffu4(a, b);
@@ -69,56 +81,123 @@ __device__ __forceinline__ uint32_t thr_u8(float top, uint32_t cur, const DevLev
     return scaled >= 4294967296.0f ? 0xFFFFFFFFu : __float2uint_rz(scaled);
 }
 
-__device__ __forceinline__ float reported_u8(uint32_t raw, const DevLevel& lv) {
-    return __fmul_rn(__uint2float_rn(raw), lv.inv_scale_sq);
+// Raw distances of a level: their bound, comparisons and reported form. `below` is the pruning
+// test, `reached` the warmup's count; a float distance that is not a number is neither.
+template <bool U8>
+struct Raw {
+    static constexpr uint32_t kElem = U8 ? 1u : 4u;  // bytes per dimension
+    static __device__ __forceinline__ uint32_t thr(float top, uint32_t cur, const DevLevel& lv, const float* ratios) {
+        if constexpr (U8) return thr_u8(top, cur, lv, ratios);
+        return __float_as_uint(__fmul_rn(top, (cur == lv.d) ? 1.0f : __ldg(ratios + cur)));
+    }
+    static __device__ __forceinline__ bool below(uint32_t raw, uint32_t t) {
+        return U8 ? raw < t : __uint_as_float(raw) < __uint_as_float(t);
+    }
+    static __device__ __forceinline__ bool reached(uint32_t raw, uint32_t t) {
+        return U8 ? raw >= t : __uint_as_float(raw) >= __uint_as_float(t);
+    }
+    static __device__ __forceinline__ float reported(uint32_t raw, const DevLevel& lv) {
+        return U8 ? __fmul_rn(__uint2float_rn(raw), lv.inv_scale_sq) : __uint_as_float(raw);
+    }
+    static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
+        return U8 ? a + b : __float_as_uint(__fadd_rn(__uint_as_float(a), __uint_as_float(b)));
+    }
+    // one more vertical word: 4 U8 dims or one F32 dim
+    static __device__ __forceinline__ uint32_t step(uint32_t q, uint32_t x, uint32_t raw) {
+        if constexpr (U8) return sq4(q, x, raw);
+        const float t = __fsub_rn(__uint_as_float(q), __uint_as_float(x));
+        return __float_as_uint(__fmaf_rn(t, t, __uint_as_float(raw)));
+    }
+    // first word past vertical dim `dim` (U8: the d_v % 4 tail is a zero-padded word)
+    static __device__ __forceinline__ uint32_t word(uint32_t dim) { return U8 ? (dim + 3) >> 2 : dim; }
+    // words of a horizontal block's vector, and the first of block b in the query's words
+    static constexpr uint32_t kHWords = U8 ? 16u : 64u;
+    static __device__ __forceinline__ uint32_t hword(const DevLevel& lv, uint32_t b) {
+        return (U8 ? lv.qw_hoff : lv.dv) + b * kHWords;
+    }
+};
+
+// Sum of one horizontal block: `row` its 16-byte pieces, q the query's words of the block (F32: in
+// the AVX2 order of avx2_computers.hpp:47-98).
+template <bool U8>
+__device__ __forceinline__ uint32_t hblock_sum(const uint32_t* q, const uint4* row);
+
+__device__ __forceinline__ uint32_t sq16(const uint4& q, const uint4& x, uint32_t acc) {
+    acc = sq4(q.x, x.x, acc);
+    acc = sq4(q.y, x.y, acc);
+    acc = sq4(q.z, x.z, acc);
+    return sq4(q.w, x.w, acc);
+}
+
+template <>
+__device__ __forceinline__ uint32_t hblock_sum<true>(const uint32_t* q, const uint4* row) {
+    uint4 x[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) x[t] = __ldg(row + t);
+    const uint4* qh = reinterpret_cast<const uint4*>(q);
+    uint32_t sum = 0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) sum = sq16(qh[t], x[t], sum);
+    return sum;
+}
+
+template <>
+__device__ __forceinline__ uint32_t hblock_sum<false>(const uint32_t* q, const uint4* row) {
+    float a[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    uint4 x[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) x[t] = __ldg(row + t);
+    const float* qf = reinterpret_cast<const float*>(q);
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        const uint32_t xw[4] = {x[t].x, x[t].y, x[t].z, x[t].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float df = __fsub_rn(qf[4 * t + j], __uint_as_float(xw[j]));
+            a[(4 * t + j) & 7] = __fmaf_rn(df, df, a[(4 * t + j) & 7]);
+        }
+    }
+    const double s0 = (double)a[0] + (double)a[4], s1 = (double)a[1] + (double)a[5];
+    const double s2 = (double)a[2] + (double)a[6], s3 = (double)a[3] + (double)a[7];
+    return __float_as_uint((float)((s0 + s2) + (s1 + s3)));
 }
 
 __device__ __forceinline__ void add_stat(const ScanParams& sp, int idx, unsigned long long v) {
     if (v) atomicAdd(sp.stats + idx, v);
 }
 
+constexpr float kTf32Keep = 1.0f - 0.001953125f;  // 1 - 2^-9
+constexpr float kTf32Tiny = 1e-36f;               // products below the normal range
+__device__ __forceinline__ float nan_unless_finite(float x) {
+    return fabsf(x) <= FLT_MAX ? x : __int_as_float(0x7fffffff);
+}
+
 // ------------------------------------------------------------------------------------ prep
 constexpr int kRegKeys = 32;  // Start distances a prep lane keeps in registers (clusters <= 1024)
 
-// The m-th smallest of the n keys key(v) (exact radix select, 8 bits a pass; hist: 256 words of
-// this warp's shared memory).
+// The m-th smallest of the n keys (1 <= m <= n): the smallest key with at least m keys not above
+// it, found bit by bit between the keys' common prefix and their lowest bit with one count of the
+// keys below a trial value per bit. All keys of a cluster share their high bits, so a radix
+// histogram's first passes queue most of their shared-memory atomics on one bin (with it: 187 us
+// for the prep kernel on 10,000 queries and clusters of 1,000 vectors, 54 us on 777).
 template <class Key>
-__device__ __forceinline__ uint32_t warp_radix_select(uint32_t n, uint32_t m, uint32_t* hist, Key key) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t prefix = 0, mask = 0, rem = m;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) hist[lane * 8 + j] = 0;
-        __syncwarp();
-        key.for_each(n, [&](uint32_t, uint32_t k) {
-            if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & 255u], 1u);
-        });
-        __syncwarp();
-        uint32_t loc[8], sum = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            loc[j] = hist[lane * 8 + j];
-            sum += loc[j];
-        }
-        uint32_t tot;
-        const uint32_t excl = warp_exclusive_scan(sum, tot);
-        const unsigned own = __ballot_sync(0xffffffffu, excl < rem && rem <= excl + sum);
-        const uint32_t owner = __ffs(own) - 1;
-        uint32_t bin = 0, cum = excl;
-        if (lane == owner) {
-            int b = 0;
-            for (; b < 7; ++b) {
-                if (cum + loc[b] >= rem) break;
-                cum += loc[b];
-            }
-            bin = lane * 8 + b;
-        }
-        bin = __shfl_sync(0xffffffffu, bin, owner);
-        cum = __shfl_sync(0xffffffffu, cum, owner);
-        prefix |= bin << shift;
-        mask |= 0xFFu << shift;
-        rem -= cum;
-        __syncwarp();
+__device__ __forceinline__ uint32_t warp_select(uint32_t n, uint32_t m, const Key& key) {
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+    key.for_each(n, [&](uint32_t, uint32_t k) {
+        lo = k < lo ? k : lo;
+        hi = k > hi ? k : hi;
+    });
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lo == hi) return lo;
+    const int top = 31 - __clz(lo ^ hi);
+    // every key agrees above bit `top`; the answer's bits from there down, high to low
+    uint32_t prefix = top == 31 ? 0u : (hi >> (top + 1)) << (top + 1);
+    for (int b = top; b >= 0; --b) {
+        const uint32_t trial = prefix | (1u << b);
+        uint32_t below = 0;
+        key.for_each(n, [&](uint32_t, uint32_t k) { below += k < trial ? 1u : 0u; });
+        if (__reduce_add_sync(0xffffffffu, below) < m) prefix = trial;
     }
     return prefix;
 }
@@ -170,11 +249,11 @@ struct MemKeys {
 // Start (searcher.hpp:256-280): the m smallest keys pushed in the order of
 // LevelOps::push_smallest -- the keys below the m-th in position order, then the ties at it.
 // Returns the m-th key.
-template <class Key>
-__device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint32_t m, uint32_t* hist,
+template <bool U8, class Key>
+__device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint32_t m,
                                                const uint32_t* ids, const DevLevel& lv, float* hd, uint32_t* hid) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t kth = warp_radix_select(n, m, hist, key);
+    const uint32_t kth = warp_select(n, m, key);
     uint32_t pushed = 0;
     for (int pass = 0; pass < 2 && pushed < m; ++pass) {
         key.for_chunks(n, [&](uint32_t v0, uint32_t kv) {
@@ -183,7 +262,7 @@ __device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint3
             const unsigned b = __ballot_sync(0xffffffffu, sel);
             const uint32_t at = pushed + __popc(b & ((1u << lane) - 1u));
             if (sel && at < m) {
-                hd[at] = reported_u8(kv, lv);
+                hd[at] = Raw<U8>::reported(kv, lv);
                 hid[at] = __ldg(ids + v);
             }
             pushed += __popc(b);
@@ -194,55 +273,37 @@ __device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint3
 
 // Dynamic shared memory: the warps' query rows (prep_qs set: kScanWarps x d floats), staged
 // with one coalesced pass; without it the query is read from global memory.
+template <bool U8>
 __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid_constant__ ScanParams sp) {
-    __shared__ uint32_t hist_all[kScanWarps][256];
     extern __shared__ __align__(16) float qs_all[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t q = blockIdx.x * kScanWarps + warp;
+    const uint32_t q = blockIdx.x * sp.p_qpc + warp;
     if (q >= sp.nq) return;  // whole warp
-    uint32_t* hist = hist_all[warp];
     const DevLevel& lv = sp.l1;
     const bool plain = !sp.filter_of || __ldg(sp.filter_of + q) == -1;
-    const int32_t row = plain ? __ldg(sp.start_row + q) : -1;
+    // position of the Start that fills the heap
+    const uint32_t fi = plain ? __ldg(sp.full_at + q) : kOffPath;
     const uint32_t kq = sp.q_k ? __ldg(sp.q_k + q) : sp.k;
-    auto leave = [&]() {
+    if (fi == kOffPath) {
         if (lane == 0) {
             sp.first_i[q] = kOffPath;
             sp.left[atomicAdd(sp.left_n, 1u)] = q;
         }
-    };
-    if (row < 0) {
-        leave();
         return;
     }
-    const uint32_t first = __ldg(sp.start_first + q);
-    const DevCluster cl = lv.clusters[first];
-    const uint32_t n = cl.n;
-    const uint32_t m = kq < n ? kq : n;
-    if (m < kq) {  // the heap is not full after the Start: the next cluster is a Start too
-        leave();
-        return;
-    }
-    // position of the Start cluster in the visit order
+    const int32_t* rows = sp.start_row + (size_t)q * sp.start_visits;
+    const uint32_t* starts = sp.start_first + (size_t)q * sp.start_visits;
+    DevCluster cl = lv.clusters[__ldg(starts)];
     const uint32_t* ord = sp.q_order + (size_t)q * sp.q_order_stride;
     const uint32_t cnt = __ldg(sp.q_order_count + q);
-    uint32_t fi = kOffPath;
-    for (uint32_t i0 = 0; i0 < cnt && fi == kOffPath; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        const unsigned b = __ballot_sync(0xffffffffu, i < cnt && __ldg(ord + i) == first);
-        if (b) fi = i0 + __ffs(b) - 1;
-    }
-    if (fi == kOffPath) {
-        leave();
-        return;
-    }
-    const uint32_t* src = sp.start_dist + (size_t)row * sp.start_stride;
+    const uint32_t* src = sp.start_dist + (size_t)__ldg(rows) * sp.start_stride;
     RegKeys rk;
-    if (n <= 32u * kRegKeys) rk.load(src, n);  // in flight while the query is quantized
+    if (cl.n <= 32u * kRegKeys) rk.load(src, cl.n);  // in flight while the query is quantized
     // QuantizeEmbedding (scalar.hpp:76-94) in the scan's packed word layout; |q|^2 over the
     // first checkpoint's words
     const float* qf = sp.queries + (size_t)q * lv.d;
-    if (sp.prep_qs) {
+    uint32_t qn = 0;
+    if (U8 && sp.prep_qs) {
         float* qs = qs_all + (size_t)warp * sp.prep_qs_stride;
         for (uint32_t i0 = 0; i0 < lv.d; i0 += 128) {
             float t[4];
@@ -260,138 +321,244 @@ __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid
         __syncwarp();
         qf = qs;
     }
-    uint32_t* qw = sp.qwords + (size_t)q * sp.nwords;
-    uint32_t qn = 0;
-    for (uint32_t w = lane; w < sp.nwords; w += 32) {
-        const uint32_t word = quantize_word(qf, lv, w);
-        qw[w] = word;
-        if (w < sp.g1) qn = __dp4a(word, word, qn);
+    if constexpr (U8) {
+        uint32_t* qw = sp.qwords + (size_t)q * sp.nwords;
+        for (uint32_t w = lane; w < sp.nwords; w += 32) {
+            const uint32_t word = quantize_word(qf, lv, w);
+            qw[w] = word;
+            if (w < sp.g1) qn = __dp4a(word, word, qn);
+        }
+        qn = __reduce_add_sync(0xffffffffu, qn);
     }
-    qn = __reduce_add_sync(0xffffffffu, qn);
+    if constexpr (!U8) {  // |q|^2 over the first checkpoint's dims
+        const float x = lane < sp.cp1 ? __ldg(qf + lane) : 0.0f;
+        float sq = x * x;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        qn = __float_as_uint(sq);
+    }
     // every later non-empty visit into its cluster's list; the visit that opens a chunk of
-    // kScanCQ list entries also opens the bitmap work item of that chunk
-    for (uint32_t i = fi + 1 + lane; i < cnt; i += 32) {
-        const uint32_t c = __ldg(ord + i);
-        if (lv.clusters[c].n == 0) {  // num_embeddings == 0 (searcher.hpp:662)
-            sp.vinfo[(size_t)q * sp.q_order_stride + i] = 0u;
-            continue;
+    // scan_chunk list entries also opens the bitmap work item of that chunk. Four visits a lane at a
+    // time: each is a chain of three round trips (cluster, size, list slot).
+    for (uint32_t i0 = fi + 1 + lane; i0 < cnt; i0 += 128) {
+        uint32_t c[4], slot[4], n[4];
+        bool on[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = i0 + 32 * u < cnt ? __ldg(ord + i0 + 32 * u) : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            n[u] = i0 + 32 * u < cnt ? lv.clusters[c[u]].n : 0u;
+            on[u] = n[u] != 0;
         }
-        const uint32_t slot = atomicAdd(sp.vl_count + c, 1u);
-        sp.vl[(size_t)c * sp.nq + slot] = q * sp.q_order_stride + i;
-        if (slot % kScanCQ == 0) {
-            const uint32_t it = atomicAdd(sp.n_items, 1u);
-            sp.items[2 * it] = c;
-            sp.items[2 * it + 1] = slot / kScanCQ;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) slot[u] = on[u] ? atomicAdd(sp.vl_count + c[u], 1u) : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t i = i0 + 32 * u;
+            if (i >= cnt) continue;
+            if (!on[u]) {  // num_embeddings == 0 (searcher.hpp:662)
+                sp.vinfo[(size_t)q * sp.q_order_stride + i] = 0u;
+                continue;
+            }
+            sp.vl[(size_t)c[u] * sp.nq + slot[u]] = q * sp.q_order_stride + i;
+            if (slot[u] % scan_chunk(n[u]) == 0) {
+                const uint32_t it = atomicAdd(sp.n_items, 1u);
+                sp.items[2 * it] = c[u];
+                sp.items[2 * it + 1] = slot[u];
+            }
         }
     }
-    const uint32_t* ids = reinterpret_cast<const uint32_t*>(sp.arena + cl.ids_off);
     float* hd = sp.heap_d + (size_t)q * sp.k;
     uint32_t* hid = sp.heap_id + (size_t)q * sp.k;
-    const uint32_t kth = n <= 32u * kRegKeys ? start_push(rk, n, m, hist, ids, lv, hd, hid)
-                                             : start_push(MemKeys{src}, n, m, hist, ids, lv, hd, hid);
-    if (lane == 0) {
-        // heap top after the pushes: the m-th key; the first checkpoint's bound at it
-        const float tau0 = reported_u8(kth, lv);
-        const long long lim = (long long)thr_u8(tau0, sp.cp1, lv, sp.ratios) - (long long)qn;
-        sp.lim[q] = lim > 0x7FFFFFFFll ? 0x7FFFFFFF : (int32_t)lim;
-        sp.first_i[q] = fi;
-        if (sp.stats) {
-            add_stat(sp, 0, (unsigned long long)n * lv.d);
-            add_stat(sp, 3 + kStart, (unsigned long long)n * lv.d);
+    uint32_t have = 0, top = 0;
+    for (uint32_t s = 0;;) {  // the Starts up to the one that fills the heap
+        const uint32_t n = cl.n;
+        const uint32_t m = kq - have < n ? kq - have : n;
+        const uint32_t* ids = reinterpret_cast<const uint32_t*>(sp.arena + cl.ids_off);
+        const uint32_t kth = n <= 32u * kRegKeys ? start_push<U8>(rk, n, m, ids, lv, hd + have, hid + have)
+                                                 : start_push<U8>(MemKeys{src}, n, m, ids, lv, hd + have, hid + have);
+        top = kth > top ? kth : top;
+        have += m;
+        if (sp.stats && lane == 0) {
+            add_stat(sp, 0, (unsigned long long)n * lv.d * Raw<U8>::kElem);
+            add_stat(sp, 3 + kStart, (unsigned long long)n * lv.d * Raw<U8>::kElem);
             add_stat(sp, 1, 1ull);
         }
+        if (have >= kq) break;
+        ++s;
+        cl = lv.clusters[__ldg(starts + s)];
+        src = sp.start_dist + (size_t)__ldg(rows + s) * sp.start_stride;
+        if (cl.n <= 32u * kRegKeys) rk.load(src, cl.n);
+    }
+    if (lane == 0) {
+        // heap top after the pushes: the largest of their last keys; the first checkpoint's bound at it
+        const float tau0 = Raw<U8>::reported(top, lv);
+        const uint32_t thr = Raw<U8>::thr(tau0, sp.cp1, lv, sp.ratios);
+        const long long lim = (long long)thr - (long long)qn;
+        if constexpr (U8)
+            sp.lim[q] = lim > 0x7FFFFFFFll ? 0x7FFFFFFF : (int32_t)lim;
+        else  // scan_bitmap_kernel's margin for the TF32 products
+            sp.lim[q] = __float_as_int(nan_unless_finite(__uint_as_float(thr) - __uint_as_float(qn) * kTf32Keep + kTf32Tiny));
+        sp.first_i[q] = fi;
     }
 }
 
 // ------------------------------------------------------------------------------------ bitmaps
-// CTA = one work item: up to 64 visits of one cluster. Warp w holds the first-checkpoint words
-// of vector blocks w, w + 8, ... (lane = vector) in registers with |x|^2, and loops over the
-// item's queries: 4 dp4a give q.x, and the ballot of |x|^2 - 2 q.x < lim is the 32-bit word of
-// that block in the query's bitmap. Lane j keeps the word of query j mod 32 and the 32 words go
-// to the item's bitmaps in shared memory together (sp.bm_tile; clusters too large for that write
-// all words to global memory). Once the cluster is done the CTA knows every visit's candidates:
-// most visits have none, and only the bitmaps of light visits are written out.
+// CTA = one work item: up to 64 visits of one cluster. A warp takes every fourth 32-vector block and
+// loops over the item's queries, 16 at a time, with one mma per 8 vectors (U8, m16n8k16) or two
+// (TF32, m16n8k8). Column n of tile t is vector 4 n + t of the block, so a lane loads four vectors'
+// words with one 16-byte read, and its eight results of a query are the bits 8 gk .. 8 gk + 7 of that
+// query's 32-bit word. The words go to the item's bitmaps in shared memory (sp.bm_tile; clusters too
+// large for that write all words to global memory). Once the cluster is done the CTA knows every
+// visit's candidates: most visits have none, and only the bitmaps of light visits are written out.
+//
+// An F32 vector is left out only when it surely reaches the bound. The TF32 operands are off by
+// 2^-11 of each factor, so q.x by at most 2^-10 |q||x| <= 2^-11 (|q|^2 + |x|^2), which counts twice;
+// the test allows 2^-9 (|q|^2 + |x|^2) for that and for the sums' own rounding, and what is not
+// finite is a candidate. The replay computes the reference's exact first-step distance of every candidate.
+//
+// Pairs were computed one query at a time before, with dp4a (U8: 186 us for 310,000 visits of
+// 1,000-vector clusters) or the chains in packed FP32 (2 x 16 operations a pair: 171 us for 300
+// queries x 895 clusters of 223 vectors, 63 us for 1,000 x 16 of 316): both bound by issue slots.
+__device__ __forceinline__ void mma_first(int (&c)[4], const uint32_t (&a)[2], uint32_t b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(b));
+}
+__device__ __forceinline__ void mma_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t to_tf32(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return r;
+}
+template <bool U8>
 __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __grid_constant__ ScanParams sp) {
-    __shared__ uint4 qv[kScanCQ];
+    constexpr uint32_t QS = U8 ? 4 : kScanDims + 4;  // words per staged query: fragment rows hit distinct banks
+    constexpr uint32_t kWarps = kBitmapThreads / 32;
+    __shared__ __align__(16) uint32_t qd[kScanCQ * QS];
     __shared__ int32_t ql[kScanCQ];
     __shared__ uint32_t qe[kScanCQ];
     __shared__ uint32_t qcnt[kScanCQ];
-    __shared__ uint32_t item;
     extern __shared__ uint32_t tile[];  // [kScanCQ][bm_words | 1]
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t ts = sp.bm_words | 1u;  // odd row stride: 32 rows of one column hit distinct banks
-    constexpr uint32_t kWarps = kBitmapThreads / 32;
+    const uint32_t gq = lane >> 2, gk = lane & 3;  // fragment row / k-group of this lane
+    const uint32_t ts = sp.bm_words | 1u;
     const DevLevel& lv = sp.l1;
     const uint32_t g1 = sp.g1;
-    for (;;) {
-        if (threadIdx.x == 0) item = atomicAdd(sp.queue, 1u);
-        __syncthreads();
-        const uint32_t it = item;
-        __syncthreads();
-        if (it >= sp.n_items[0]) break;
-        const uint32_t c = sp.items[2 * it], a = sp.items[2 * it + 1];
-        const uint32_t L = sp.vl_count[c];
-        const uint32_t nqc = (L - a * kScanCQ) < kScanCQ ? (L - a * kScanCQ) : kScanCQ;
+    for (uint32_t it = blockIdx.x; it < sp.n_items[0]; it += gridDim.x) {
+        const uint32_t c = sp.items[2 * it], first = sp.items[2 * it + 1];
+        const uint32_t left = sp.vl_count[c] - first;
+        const DevCluster cl = lv.clusters[c];
+        const uint32_t n = cl.n, nb = (n + 31) >> 5;
+        const uint32_t cq = scan_chunk(n), nqc = left < cq ? left : cq;
         if (threadIdx.x < nqc) {
-            const uint32_t e = sp.vl[(size_t)c * sp.nq + a * kScanCQ + threadIdx.x];
-            const uint32_t q = e / sp.q_order_stride;
-            const uint32_t* w = sp.qwords + (size_t)q * sp.nwords;
-            qv[threadIdx.x] = make_uint4(__ldg(w), g1 > 1 ? __ldg(w + 1) : 0u, g1 > 2 ? __ldg(w + 2) : 0u,
-                                         g1 > 3 ? __ldg(w + 3) : 0u);
-            ql[threadIdx.x] = sp.lim[q];
+            const uint32_t e = sp.vl[(size_t)c * sp.nq + first + threadIdx.x];
             qe[threadIdx.x] = e;
-            qcnt[threadIdx.x] = 0;
+            ql[threadIdx.x] = sp.lim[e / sp.q_order_stride];
+        }
+        if (threadIdx.x < kScanCQ) qcnt[threadIdx.x] = 0;
+        __syncthreads();
+        for (uint32_t e = threadIdx.x; e < kScanCQ * (U8 ? 4 : kScanDims); e += kBitmapThreads) {
+            const uint32_t j = e / (U8 ? 4 : kScanDims), g = e % (U8 ? 4 : kScanDims);
+            uint32_t w = 0;
+            if (j < nqc && g < g1) w = __ldg(sp.qwords + (size_t)(qe[j] / sp.q_order_stride) * sp.nwords + g);
+            qd[j * QS + g] = U8 ? w : to_tf32(__uint_as_float(w));
         }
         __syncthreads();
-        const DevCluster cl = lv.clusters[c];
-        const uint32_t n = cl.n;
-        const uint32_t nb = (n + 31) >> 5;
         const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + cl.vert_off);
-        for (uint32_t b0 = warp; b0 < nb; b0 += kWarps * kBitmapBPW) {
-            uint32_t x[kBitmapBPW][4], xn[kBitmapBPW], word[kBitmapBPW];
-            bool valid[kBitmapBPW];
+        for (uint32_t blk = warp; blk < nb; blk += kWarps) {
+            // words g = gk, gk + 4, ... of vectors 4 gq .. 4 gq + 3 of the block (inside n_pad; what
+            // lies past n is masked), and |x|^2 of the vectors of this lane's results
+            constexpr int G = U8 ? 1 : 4;
+            uint4 x[G];
 #pragma unroll
-            for (int b = 0; b < kBitmapBPW; ++b) {
-                const uint32_t blk = b0 + b * kWarps;
-                const uint32_t v = blk * 32 + lane;
-                valid[b] = blk < nb && v < n;
-                xn[b] = 0;
-                word[b] = 0;
+            for (int g = 0; g < G; ++g)
+                x[g] = gk + 4 * g < g1
+                           ? __ldg(reinterpret_cast<const uint4*>(vert + (size_t)(gk + 4 * g) * cl.n_pad + blk * 32) + gq)
+                           : make_uint4(0u, 0u, 0u, 0u);
+            uint32_t b[G][4];
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    // rows past the cluster's vectors but inside n_pad hold padding: never read
-                    x[b][g] = (valid[b] && (uint32_t)g < g1) ? __ldg(vert + (size_t)g * cl.n_pad + v) : 0u;
-                    xn[b] = __dp4a(x[b][g], x[b][g], xn[b]);
-                }
+            for (int g = 0; g < G; ++g) {
+                b[g][0] = x[g].x;
+                b[g][1] = x[g].y;
+                b[g][2] = x[g].z;
+                b[g][3] = x[g].w;
             }
-            for (uint32_t j = 0; j < nqc; ++j) {
-                const uint4 qq = qv[j];
-                const int32_t lj = ql[j];
+            uint32_t xn[2][4];  // [e][t]: vector 4 (2 gk + e) + t
 #pragma unroll
-                for (int b = 0; b < kBitmapBPW; ++b) {
-                    uint32_t dot = __dp4a(qq.x, x[b][0], 0u);
-                    dot = __dp4a(qq.y, x[b][1], dot);
-                    dot = __dp4a(qq.z, x[b][2], dot);
-                    dot = __dp4a(qq.w, x[b][3], dot);
-                    const int32_t val = (int32_t)xn[b] - 2 * (int32_t)dot;  // |q - x|^2 - |q|^2
-                    const unsigned bal = __ballot_sync(0xffffffffu, valid[b] && val < lj);
-                    if (lane == (j & 31)) word[b] = bal;
-                }
-                if ((j & 31) == 31 || j + 1 == nqc) {
-                    const uint32_t jj = (j & ~31u) + lane;
-                    if (jj <= j) {
-                        uint32_t* row = sp.bm_tile ? tile + jj * ts : sp.bm + (size_t)qe[jj] * sp.bm_words;
-                        uint32_t cnt = 0;
+            for (int t = 0; t < 4; ++t) {
+                uint32_t s;
+                if constexpr (U8) {
+                    s = __dp4a(b[0][t], b[0][t], 0u);
+                    s += __shfl_xor_sync(0xffffffffu, s, 1);
+                    s += __shfl_xor_sync(0xffffffffu, s, 2);
+                } else {
+                    float sf = 0.0f;
 #pragma unroll
-                        for (int b = 0; b < kBitmapBPW; ++b) {
-                            const uint32_t blk = b0 + b * kWarps;
-                            if (blk < nb) {
-                                row[blk] = word[b];
-                                cnt += __popc(word[b]);
-                            }
-                        }
-                        if (cnt) atomicAdd(&qcnt[jj], cnt);
+                    for (int g = 0; g < G; ++g) {
+                        const float xf = __uint_as_float(b[g][t]);
+                        sf = fmaf(xf, xf, sf);
+                        b[g][t] = to_tf32(xf);
                     }
+                    sf += __shfl_xor_sync(0xffffffffu, sf, 1);
+                    sf += __shfl_xor_sync(0xffffffffu, sf, 2);
+                    s = __float_as_uint(nan_unless_finite(sf * kTf32Keep));
+                }
+                xn[0][t] = __shfl_sync(0xffffffffu, s, gk * 8);
+                xn[1][t] = __shfl_sync(0xffffffffu, s, gk * 8 + 4);
+            }
+            const uint32_t valid = n - blk * 32 >= 32 ? 0xFFFFFFFFu : (1u << (n - blk * 32)) - 1u;
+            for (uint32_t j0 = 0; j0 < nqc; j0 += 16) {
+                const uint32_t* q0 = qd + (j0 + gq) * QS + gk;
+                const uint32_t* q1 = q0 + 8 * QS;
+                uint32_t w0 = 0, w1 = 0;  // this lane's bits of queries j0 + gq and j0 + gq + 8
+                if constexpr (U8) {
+                    const uint32_t a[2] = {q0[0], q1[0]};
+                    const int32_t l0 = ql[j0 + gq], l1 = ql[j0 + gq + 8];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        int d[4] = {0, 0, 0, 0};
+                        mma_first(d, a, b[0][t]);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {  // |q - x|^2 - |q|^2 against lim
+                            if ((int32_t)xn[e][t] - 2 * d[e] < l0) w0 |= 1u << (4 * e + t);
+                            if ((int32_t)xn[e][t] - 2 * d[2 + e] < l1) w1 |= 1u << (4 * e + t);
+                        }
+                    }
+                } else {
+                    const uint32_t a0[4] = {q0[0], q1[0], q0[4], q1[4]}, a1[4] = {q0[8], q1[8], q0[12], q1[12]};
+                    const float l0 = __int_as_float(ql[j0 + gq]), l1 = __int_as_float(ql[j0 + gq + 8]);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                        mma_first(d, a0, b[0][t], b[1][t]);
+                        mma_first(d, a1, b[2][t], b[3][t]);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (!(fmaf(-2.0f, d[e], __uint_as_float(xn[e][t])) >= l0)) w0 |= 1u << (4 * e + t);
+                            if (!(fmaf(-2.0f, d[2 + e], __uint_as_float(xn[e][t])) >= l1)) w1 |= 1u << (4 * e + t);
+                        }
+                    }
+                }
+                w0 <<= 8 * gk;
+                w1 <<= 8 * gk;
+                w0 |= __shfl_xor_sync(0xffffffffu, w0, 1);
+                w1 |= __shfl_xor_sync(0xffffffffu, w1, 1);
+                w0 |= __shfl_xor_sync(0xffffffffu, w0, 2);
+                w1 |= __shfl_xor_sync(0xffffffffu, w1, 2);
+                const uint32_t j = j0 + gq + 8 * gk;
+                if (gk < 2 && j < nqc) {
+                    const uint32_t word = (gk ? w1 : w0) & valid;
+                    uint32_t* row = sp.bm_tile ? tile + j * ts : sp.bm + (size_t)qe[j] * sp.bm_words;
+                    row[blk] = word;
+                    if (word) atomicAdd(&qcnt[j], (uint32_t)__popc(word));
                 }
             }
         }
@@ -413,7 +580,7 @@ __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __gri
                 for (uint32_t w = lane; w < nb; w += 32) sp.bm[(size_t)qe[j] * sp.bm_words + w] = tile[j * ts + w];
             }
         }
-        __syncthreads();
+        __syncthreads();  // the next item overwrites the arrays
     }
 }
 
@@ -432,18 +599,14 @@ struct ReplayWarp {
     uint32_t* sv_d;
 };
 
-constexpr int kCandPerLane = 4;  // candidates a replay lane tests per memory round trip
+// candidates a replay lane tests per memory round trip
+template <bool U8>
+constexpr int kCandPerLane = U8 ? 4 : 2;
 constexpr int kFallPerLane = 4;  // vectors a replay lane carries through a full warmup step
-
-__device__ __forceinline__ uint32_t sq16(const uint4& q, const uint4& x, uint32_t acc) {
-    acc = sq4(q.x, x.x, acc);
-    acc = sq4(q.y, x.y, acc);
-    acc = sq4(q.z, x.z, acc);
-    return sq4(q.w, x.w, acc);
-}
 
 // The vertical dims from cur0 on in 64-dim steps for a vector below every bound up to `cur` (the
 // horizontal blocks included), tested after each step.
+template <bool U8>
 __device__ __forceinline__ bool scan_follow_vertical(const ScanParams& sp, const DevCluster& c, const uint32_t* qw,
                                                      uint32_t v, uint32_t cur0, uint32_t cur, float top, uint32_t& raw,
                                                      unsigned long long& vbytes) {
@@ -452,43 +615,47 @@ __device__ __forceinline__ bool scan_follow_vertical(const ScanParams& sp, const
     uint32_t cur_v = cur0;
     while (cur_v < lv.dv) {
         const uint32_t last = (cur_v + kHDim < lv.dv) ? cur_v + kHDim : lv.dv;
-        vbytes += last - cur_v;
-        for (uint32_t g = cur_v >> 2; g < ((last + 3) >> 2); ++g)
-            raw = sq4(qw[g], __ldg(vert + (size_t)g * c.n_pad + v), raw);
+        vbytes += (last - cur_v) * Raw<U8>::kElem;
+        const uint32_t g_end = Raw<U8>::word(last);
+        for (uint32_t g0 = U8 ? cur_v >> 2 : cur_v; g0 < g_end; g0 += 8) {
+            uint32_t x[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) x[t] = g0 + t < g_end ? __ldg(vert + (size_t)(g0 + t) * c.n_pad + v) : 0u;
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (g0 + t < g_end) raw = Raw<U8>::step(qw[g0 + t], x[t], raw);
+        }
         cur = (cur + kHDim < lv.d) ? cur + kHDim : lv.d;
         cur_v = last;
-        if (!(raw < thr_u8(top, cur, lv, sp.ratios))) return false;
+        if (!Raw<U8>::below(raw, Raw<U8>::thr(top, cur, lv, sp.ratios))) return false;
         if (cur == lv.d) break;
     }
     return true;
+}
+
+// 16-byte pieces of vector v's row in horizontal block b.
+template <bool U8>
+__device__ __forceinline__ const uint4* hblock_row(const ScanParams& sp, const DevCluster& c, uint32_t b, uint32_t v) {
+    return reinterpret_cast<const uint4*>(sp.arena + c.hor_off) + ((size_t)b * c.n_pad + v) * (Raw<U8>::kHWords / 4);
 }
 
 // One survivor of the warmup bound at checkpoint cur0: the horizontal blocks, then the
 // remaining vertical dims in 64-dim steps, tested after each against the bound of the heap top
 // `top` fixed for the whole cluster (searcher.hpp:437-540). Returns whether it is still below
 // the bound at the end; raw is its running distance.
+template <bool U8>
 __device__ __forceinline__ bool scan_follow(const ScanParams& sp, const DevCluster& c, const uint32_t* qw,
                                             uint32_t v, uint32_t cur0, float top, uint32_t& raw,
                                             unsigned long long& hbytes, unsigned long long& vbytes) {
     const DevLevel& lv = sp.l1;
-    const uint32_t nhb = lv.n_hblocks;
     uint32_t cur = cur0;
-    if (nhb) {
-        const uint4* row = reinterpret_cast<const uint4*>(sp.arena + c.hor_off) + (size_t)v * 4;
-        const size_t bstride = (size_t)c.n_pad * 4;  // uint4 per block
-        for (uint32_t b = 0; b < nhb; ++b) {
-            uint4 x[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) x[t] = __ldg(row + b * bstride + t);
-            const uint4* qh = reinterpret_cast<const uint4*>(qw + lv.qw_hoff + b * 16);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) raw = sq16(qh[t], x[t], raw);
-            hbytes += kHDim;
-            cur += kHDim;
-            if (!(raw < thr_u8(top, cur, lv, sp.ratios))) return false;
-        }
+    for (uint32_t b = 0; b < lv.n_hblocks; ++b) {
+        raw = Raw<U8>::add(raw, hblock_sum<U8>(qw + Raw<U8>::hword(lv, b), hblock_row<U8>(sp, c, b, v)));
+        hbytes += kHDim * Raw<U8>::kElem;
+        cur += kHDim;
+        if (!Raw<U8>::below(raw, Raw<U8>::thr(top, cur, lv, sp.ratios))) return false;
     }
-    return scan_follow_vertical(sp, c, qw, v, cur0, cur, top, raw, vbytes);
+    return scan_follow_vertical<U8>(sp, c, qw, v, cur0, cur, top, raw, vbytes);
 }
 
 // Positions of the set bits of one word per lane (word index w_rel of a group of 32 words),
@@ -507,14 +674,16 @@ __device__ __forceinline__ uint32_t scan_bits_to_offsets(uint32_t word, uint32_t
 
 // Values of vector v of a heavy visit into column `out` (row stride sp.hv_cap): row s < ncp is the
 // running distance at warmup checkpoint s, row ncp + b the sum of horizontal block b. They do not
-// depend on the query's heap, so the loads of 64 vertical dims, then of three blocks, are in flight
-// together (8 dims and two blocks: 152 against 108 us for the replay of a 777-query batch). Returns
-// the full distance.
+// depend on the query's heap, so the loads of 16 vertical words, then of three blocks (F32: one), are
+// in flight together (U8, 2 words and two blocks: 152 against 108 us for the replay of a 777-query
+// batch). Returns the full distance: for F32 that of a warmup over all vertical dims (an earlier exit
+// adds the same terms in another order).
+template <bool U8>
 __device__ __forceinline__ uint32_t heavy_column(const ScanParams& sp, const DevCluster& c, const uint32_t* qw,
                                                  uint32_t v, uint32_t* out) {
     const DevLevel& lv = sp.l1;
     const uint32_t* col = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off) + v;
-    const uint32_t groups = (lv.dv + 3) >> 2;
+    const uint32_t groups = Raw<U8>::word(lv.dv);
     uint32_t raw = 0, s = 0, next = sp.cp1;
     for (uint32_t g0 = 0; g0 < groups; g0 += 16) {
         uint32_t x[16];
@@ -523,8 +692,8 @@ __device__ __forceinline__ uint32_t heavy_column(const ScanParams& sp, const Dev
 #pragma unroll
         for (int t = 0; t < 16; ++t) {
             if (g0 + t < groups) {
-                raw = sq4(qw[g0 + t], x[t], raw);
-                if ((g0 + t + 1) * 4 >= next) {  // checkpoints are multiples of 16 dims, the last is d_v
+                raw = Raw<U8>::step(qw[g0 + t], x[t], raw);
+                if ((g0 + t + 1) * (U8 ? 4 : 1) >= next) {  // checkpoints are multiples of 16 dims, the last is d_v
                     out[(size_t)s * sp.hv_cap] = raw;
                     ++s;
                     next += c_scan_fetch[s < kNumFetchSizes ? s : kNumFetchSizes - 1];
@@ -534,15 +703,21 @@ __device__ __forceinline__ uint32_t heavy_column(const ScanParams& sp, const Dev
         }
     }
     out += (size_t)sp.hv_ncp * sp.hv_cap;
-    const uint4* row = reinterpret_cast<const uint4*>(sp.arena + c.hor_off) + (size_t)v * 4;
-    const size_t bstride = (size_t)c.n_pad * 4;  // uint4 per block
+    if constexpr (!U8) {
+        for (uint32_t b = 0; b < lv.n_hblocks; ++b) {
+            const uint32_t sum = hblock_sum<false>(qw + Raw<U8>::hword(lv, b), hblock_row<U8>(sp, c, b, v));
+            out[(size_t)b * sp.hv_cap] = sum;
+            raw = Raw<U8>::add(raw, sum);
+        }
+        return raw;
+    }
     for (uint32_t b0 = 0; b0 < lv.n_hblocks; b0 += 3) {
         uint4 x[3][4];
 #pragma unroll
         for (int u = 0; u < 3; ++u)
 #pragma unroll
             for (int t = 0; t < 4; ++t)
-                x[u][t] = b0 + u < lv.n_hblocks ? __ldg(row + (b0 + u) * bstride + t) : make_uint4(0u, 0u, 0u, 0u);
+                x[u][t] = b0 + u < lv.n_hblocks ? __ldg(hblock_row<U8>(sp, c, b0 + u, v) + t) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
             if (b0 + u < lv.n_hblocks) {
@@ -556,6 +731,16 @@ __device__ __forceinline__ uint32_t heavy_column(const ScanParams& sp, const Dev
         }
     }
     return raw;
+}
+
+// Whether a vector with full distance `full` may stay below bound `thr` at all d dims. F32 leaves
+// room for another order of the sum: its d + 1 non-negative terms are each rounded at most d + 2
+// times by 2^-24 in either order (2^-22 d is twice the difference that allows).
+template <bool U8>
+__device__ __forceinline__ bool may_stay_below(uint32_t full, uint32_t thr, uint32_t d) {
+    if constexpr (U8) return full < thr;
+    const float t = __uint_as_float(thr);
+    return !(__uint_as_float(full) > t + t * ((float)(d + 16) * 2.384185791015625e-7f));
 }
 
 // A heavy visit needs the running distance of all its vectors at up to every warmup checkpoint and
@@ -575,7 +760,8 @@ struct HeavyList {
     uint32_t thr0[kScanWarps];  // bound at all d dims of each warp's heap top after the Start
 };
 
-__global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const __grid_constant__ ScanParams sp) {
+template <bool U8>
+__global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kernel(const __grid_constant__ ScanParams sp) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ HeavyList HL;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -610,7 +796,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         }
         __syncwarp();
         warp_heap_top(R.hd, kq, top, slot);
-        if (lane == 0) HL.thr0[warp] = thr_u8(top, lv.d, lv, sp.ratios);
+        if (lane == 0) HL.thr0[warp] = Raw<U8>::thr(top, lv.d, lv, sp.ratios);
         for (uint32_t i = fi + 1 + lane; i < cnt; i += 32) {
             if (!(__ldg(vis + i) & kHeavyBit) || HL.n >= kHeavyList) continue;
             // columns are handed out in units of 32; none is asked for once they are used up, so the
@@ -643,21 +829,16 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
             const uint32_t v = blk * 32 + lane;
             uint32_t full = 0xFFFFFFFFu;
             if (v < c.n)
-                full = heavy_column(sp, c, reinterpret_cast<const uint32_t*>(smem + (size_t)hw * sp.r_warp_bytes), v,
+                full = heavy_column<U8>(sp, c, reinterpret_cast<const uint32_t*>(smem + (size_t)hw * sp.r_warp_bytes), v,
                                     sp.hv + ((size_t)(HL.base[j] + blk) << 5) + lane);
             // statistics count the blocks of vectors that end up pruned too
-            const unsigned may = __ballot_sync(0xffffffffu, v < c.n && (sp.stats || full < HL.thr0[hw]));
+            const unsigned may = __ballot_sync(0xffffffffu, v < c.n && (sp.stats || may_stay_below<U8>(full, HL.thr0[hw], lv.d)));
             if (lane == 0) sp.bm[((size_t)hq * stride + HL.visit[j]) * sp.bm_words + blk] = may;
         }
         __syncthreads();
     }
     if (fi == kOffPath) return;  // whole warp; no block-wide barrier follows
-    uint4 q1 = make_uint4(0u, 0u, 0u, 0u);  // first checkpoint's query words (zero past g1)
-    q1.x = R.qw[0];
-    if (sp.g1 > 1) q1.y = R.qw[1];
-    if (sp.g1 > 2) q1.z = R.qw[2];
-    if (sp.g1 > 3) q1.w = R.qw[3];
-    uint32_t* scratch = sp.start_dist + (size_t)__ldg(sp.start_row + q) * sp.start_stride;
+    uint32_t* scratch = sp.start_dist + (size_t)__ldg(sp.start_row + (size_t)q * sp.start_visits) * sp.start_stride;
     const uint32_t S = sp.r_surv_cap;
     unsigned long long b_warm = 0, b_h = 0, b_v = 0, merged = 0;
     unsigned long long n_cand = 0, n_surv = 0, n_fast = 0, n_full = 0;
@@ -668,7 +849,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
     // (MergeIntoHeap, searcher.hpp:542-566).
     auto merge = [&](const DevCluster& c, bool alive, uint32_t v, uint32_t raw) {
         const uint32_t idv = alive ? __ldg(reinterpret_cast<const uint32_t*>(sp.arena + c.ids_off) + v) : 0u;
-        const float dd = reported_u8(raw, lv);
+        const float dd = Raw<U8>::reported(raw, lv);
         unsigned bal = __ballot_sync(0xffffffffu, alive);
         merged += __popc(bal);
         while (bal) {
@@ -689,7 +870,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
 
     // Follows the lane's survivor (alive, v, raw) through Prune with the bound at `tp`, then merges.
     auto prune_merge = [&](const DevCluster& c, bool alive, uint32_t v, uint32_t raw, uint32_t cur, float tp) {
-        if (alive) alive = scan_follow(sp, c, R.qw, v, cur, tp, raw, b_h, b_v);
+        if (alive) alive = scan_follow<U8>(sp, c, R.qw, v, cur, tp, raw, b_h, b_v);
         merge(c, alive, v, raw);
     };
     // A heavy visit on its values computed ahead, hv pointing at its first vector's column.
@@ -705,7 +886,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         while (n_pruned < needed && cur < lv.dv) {  // Warmup (searcher.hpp:374-435)
             uint32_t last = cur + c_scan_fetch[step < kNumFetchSizes ? step : kNumFetchSizes - 1];
             if (last > lv.dv) last = lv.dv;
-            const uint32_t thr = thr_u8(tp, last, lv, sp.ratios);
+            const uint32_t thr = Raw<U8>::thr(tp, last, lv, sp.ratios);
             const uint32_t* row = hv + (size_t)step * sp.hv_cap;
             uint32_t cntp = 0;
             for (uint32_t v0 = 0; v0 < n; v0 += 256) {
@@ -716,11 +897,11 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
                     x[u] = v < n ? row[v] : 0u;
                 }
 #pragma unroll
-                for (int u = 0; u < 8; ++u) cntp += (v0 + 32 * u + lane < n && x[u] >= thr) ? 1u : 0u;
+                for (int u = 0; u < 8; ++u) cntp += (v0 + 32 * u + lane < n && Raw<U8>::reached(x[u], thr)) ? 1u : 0u;
             }
             n_pruned = __reduce_add_sync(0xffffffffu, cntp);
             if (cur == 0) n_surv += n - n_pruned;
-            else b_warm += (unsigned long long)n * (last - cur);
+            else b_warm += (unsigned long long)n * (last - cur) * Raw<U8>::kElem;
             cur = last;
             ++step;
         }
@@ -729,7 +910,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         // Prune (searcher.hpp:437-540) and merge of the mergeable vectors, 32 at a time in position
         // order; their horizontal sums are loaded kHeavyBlocks at a time, ahead of their tests
         constexpr int kHeavyBlocks = 6;
-        const uint32_t thr = thr_u8(tp, cur, lv, sp.ratios);
+        const uint32_t thr = Raw<U8>::thr(tp, cur, lv, sp.ratios);
         const uint32_t* erow = hv + (size_t)(step - 1) * sp.hv_cap;
         const uint32_t* brow = hv + (size_t)sp.hv_ncp * sp.hv_cap;
         for (uint32_t w0 = 0; w0 < W; w0 += 32) {
@@ -738,7 +919,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
                 bool alive = j0 + lane < total;
                 const uint32_t v = alive ? w0 * 32 + R.cand[j0 + lane] : 0u;
                 uint32_t raw = alive ? erow[v] : 0u;
-                alive = alive && raw < thr;
+                alive = alive && Raw<U8>::below(raw, thr);
                 uint32_t cv = cur;
                 for (uint32_t b0 = 0; b0 < lv.n_hblocks && __any_sync(0xffffffffu, alive); b0 += kHeavyBlocks) {
                     uint32_t x[kHeavyBlocks];
@@ -748,14 +929,14 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
 #pragma unroll
                     for (int u = 0; u < kHeavyBlocks; ++u) {
                         if (alive && b0 + u < lv.n_hblocks) {
-                            raw += x[u];
-                            b_h += kHDim;
+                            raw = Raw<U8>::add(raw, x[u]);
+                            b_h += kHDim * Raw<U8>::kElem;
                             cv += kHDim;
-                            alive = raw < thr_u8(tp, cv, lv, sp.ratios);
+                            alive = Raw<U8>::below(raw, Raw<U8>::thr(tp, cv, lv, sp.ratios));
                         }
                     }
                 }
-                if (alive) alive = scan_follow_vertical(sp, c, R.qw, v, cur, cv, tp, raw, b_v);
+                if (alive) alive = scan_follow_vertical<U8>(sp, c, R.qw, v, cur, cv, tp, raw, b_v);
                 merge(c, alive, v, raw);
             }
             __syncwarp();  // cand is rewritten by the next word group
@@ -773,7 +954,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
       if (sp.stats && in) {
           const uint32_t n = lv.clusters[__ldg(ord + il)].n;
           visits_l += n ? 1u : 0u;
-          b_warm_l += (unsigned long long)n * sp.cp1;
+          b_warm_l += (unsigned long long)n * sp.cp1 * Raw<U8>::kElem;
           fast_l += (n && info_l == 0) ? 1u : 0u;
       }
       for (unsigned todo = __ballot_sync(0xffffffffu, info_l != 0); todo; todo &= todo - 1) {
@@ -797,32 +978,36 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         const uint32_t* bmp = sp.bm + ((size_t)q * stride + i) * sp.bm_words;
         // Warmup step 1 from the candidates: the exact first-checkpoint distance of each, and the
         // survivors under the current bound, in position order
-        const uint32_t thr1 = thr_u8(top, sp.cp1, lv, sp.ratios);
-        uint32_t ns = 0;
+        const uint32_t thr1 = Raw<U8>::thr(top, sp.cp1, lv, sp.ratios);
+        uint32_t ns = 0, open = 0;  // below the bound; not reaching it (F32: not a number, too)
         const bool light = !(info & kHeavyBit);  // a heavy visit keeps no bitmap
         for (uint32_t w0 = 0; light && w0 < W; w0 += 32) {
             const uint32_t w = w0 + lane;
             const uint32_t word = w < W ? __ldg(bmp + w) : 0u;
             const uint32_t total = scan_bits_to_offsets(word, lane, R.cand);
             n_cand += total;
-            for (uint32_t j0 = 0; j0 < total; j0 += 32 * kCandPerLane) {
-                uint32_t v[kCandPerLane];
-                uint4 x[kCandPerLane];
+            constexpr int CP = kCandPerLane<U8>;
+            constexpr int GW = U8 ? 4 : (int)kScanDims;  // words of the first step at most
+            for (uint32_t j0 = 0; j0 < total; j0 += 32 * CP) {
+                uint32_t v[CP], x[CP][GW];
 #pragma unroll
-                for (int u = 0; u < kCandPerLane; ++u) {
+                for (int u = 0; u < CP; ++u) {
                     const uint32_t j = j0 + 32 * u + lane;
                     v[u] = j < total ? w0 * 32 + R.cand[j] : 0xFFFFFFFFu;
                     const bool in = v[u] != 0xFFFFFFFFu;
                     const uint32_t* col = vert + (in ? v[u] : 0u);
-                    x[u].x = in ? __ldg(col) : 0u;
-                    x[u].y = (in && sp.g1 > 1) ? __ldg(col + (size_t)c.n_pad) : 0u;
-                    x[u].z = (in && sp.g1 > 2) ? __ldg(col + 2 * (size_t)c.n_pad) : 0u;
-                    x[u].w = (in && sp.g1 > 3) ? __ldg(col + 3 * (size_t)c.n_pad) : 0u;
+#pragma unroll
+                    for (int g = 0; g < GW; ++g)
+                        x[u][g] = (in && (uint32_t)g < sp.g1) ? __ldg(col + (size_t)g * c.n_pad) : 0u;
                 }
 #pragma unroll
-                for (int u = 0; u < kCandPerLane; ++u) {
-                    const uint32_t d1 = sq16(q1, x[u], 0u);
-                    const bool s = v[u] != 0xFFFFFFFFu && d1 < thr1;
+                for (int u = 0; u < CP; ++u) {
+                    uint32_t d1 = 0;
+#pragma unroll
+                    for (int g = 0; g < GW; ++g)
+                        if ((uint32_t)g < sp.g1) d1 = Raw<U8>::step(R.qw[g], x[u][g], d1);
+                    const bool in = v[u] != 0xFFFFFFFFu;
+                    const bool s = in && Raw<U8>::below(d1, thr1);
                     const unsigned bal = __ballot_sync(0xffffffffu, s);
                     const uint32_t r = ns + __popc(bal & ((1u << lane) - 1u));
                     if (s && r < S) {
@@ -830,11 +1015,13 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
                         R.sv_d[r] = d1;
                     }
                     ns += __popc(bal);
+                    if constexpr (U8) open = ns;
+                    else open += __popc(__ballot_sync(0xffffffffu, in && !Raw<U8>::reached(d1, thr1)));
                 }
             }
             __syncwarp();
         }
-        const bool exits = sp.cp1 >= lv.dv || n - ns >= needed;  // the warmup stops after step 1
+        const bool exits = sp.cp1 >= lv.dv || n - open >= needed;  // the warmup stops after step 1
         const float tp = top;  // the bound's heap top, fixed for the whole cluster
         n_surv += ns;
         if (light && exits && ns <= S) {
@@ -855,8 +1042,8 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
         while (n_pruned < needed && cur < lv.dv) {
             uint32_t last = cur + c_scan_fetch[step < kNumFetchSizes ? step : kNumFetchSizes - 1];
             if (last > lv.dv) last = lv.dv;
-            const uint32_t thr = thr_u8(top, last, lv, sp.ratios);
-            const uint32_t g0 = cur >> 2, g_end = (last + 3) >> 2;
+            const uint32_t thr = Raw<U8>::thr(top, last, lv, sp.ratios);
+            const uint32_t g0 = U8 ? cur >> 2 : cur, g_end = Raw<U8>::word(last);
             uint32_t cntp = 0;
             for (uint32_t v0 = 0; v0 < n; v0 += 32 * kFallPerLane) {
                 uint32_t acc[kFallPerLane];
@@ -876,9 +1063,9 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
                         }
 #pragma unroll
                     for (int gg = 0; gg < 4; ++gg) {
-                        const uint32_t qv = g + gg < g_end ? R.qw[g + gg] : 0u;
+                        const uint32_t qv = g + gg < g_end ? R.qw[g + gg] : 0u;  // past the end: adds 0
 #pragma unroll
-                        for (int u = 0; u < kFallPerLane; ++u) acc[u] = sq4(qv, xs[gg][u], acc[u]);
+                        for (int u = 0; u < kFallPerLane; ++u) acc[u] = Raw<U8>::step(qv, xs[gg][u], acc[u]);
                     }
                 }
 #pragma unroll
@@ -886,20 +1073,20 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
                     const uint32_t v = v0 + 32 * u + lane;
                     if (v < n) {
                         scratch[v] = acc[u];
-                        cntp += acc[u] >= thr ? 1u : 0u;
+                        cntp += Raw<U8>::reached(acc[u], thr) ? 1u : 0u;
                     }
                 }
             }
             n_pruned = __reduce_add_sync(0xffffffffu, cntp);
-            if (cur > 0) b_warm += (unsigned long long)n * (last - cur);
+            if (cur > 0) b_warm += (unsigned long long)n * (last - cur) * Raw<U8>::kElem;
             cur = last;
             ++step;
         }
         // Prune: the vectors below the bound at the warmup's last checkpoint, in position order
-        const uint32_t thr = thr_u8(top, cur, lv, sp.ratios);
+        const uint32_t thr = Raw<U8>::thr(top, cur, lv, sp.ratios);
         for (uint32_t v0 = 0; v0 < n; v0 += 32) {
             const uint32_t v = v0 + lane;
-            const unsigned bal = __ballot_sync(0xffffffffu, v < n && scratch[v] < thr);
+            const unsigned bal = __ballot_sync(0xffffffffu, v < n && Raw<U8>::below(scratch[v], thr));
             if (lane == 0) R.sbits[v0 >> 5] = bal;
         }
         __syncwarp();
@@ -961,8 +1148,8 @@ __global__ void __launch_bounds__(kScanWarps * 32, 3) scan_replay_kernel(const _
 }
 
 // ------------------------------------------------------------------------------------ launch
-uint64_t scan_item_bound(uint32_t nq, uint32_t stride, uint32_t n1) {
-    return (uint64_t)nq * stride / kScanCQ + n1 + 1;
+uint64_t scan_item_bound(uint32_t nq, uint32_t stride, uint32_t n1, uint32_t max_n) {
+    return (uint64_t)nq * stride / scan_chunk(max_n) + n1 + 1;
 }
 
 // Shared memory of a bitmap work item's tile; 0: the bitmaps of clusters this large go straight
@@ -972,46 +1159,43 @@ size_t scan_bitmap_smem(uint32_t bm_words) {
     return b <= kBitmapTileMax ? b : 0;
 }
 
-int scan_bitmap_occupancy(uint32_t bm_words) {
-    int blocks = 0;
-    const size_t tile = scan_bitmap_smem(bm_words);
-    if (tile) cudaFuncSetAttribute(scan_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, scan_bitmap_kernel, kBitmapThreads, tile);
-    return blocks;
-}
-
 uint32_t scan_queries_per_cta() { return kScanWarps; }
 
-// ev (optional, 3 events): recorded after the prep kernel, the bitmaps and the replay.
-cudaError_t launch_scan(const ScanParams& sp, int bitmap_grid, cudaStream_t st, const cudaEvent_t* ev) {
+template <bool U8>
+static cudaError_t launch_scan_t(const ScanParams& sp, cudaStream_t st, const cudaEvent_t* ev) {
     cudaError_t e = cudaMemsetAsync(sp.vl_count, 0, sizeof(uint32_t) * sp.l1.nclusters, st);
     if (e != cudaSuccess) return e;
-    // left_n, n_items, queue and hv_alloc are consecutive
-    if ((e = cudaMemsetAsync(sp.left_n, 0, 4 * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    const uint32_t ctas = (sp.nq + kScanWarps - 1) / kScanWarps;
-    const size_t prep_smem = sp.prep_qs ? (size_t)kScanWarps * sp.prep_qs_stride * 4 : 0;
+    // left_n, n_items and hv_alloc are consecutive
+    if ((e = cudaMemsetAsync(sp.left_n, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    const uint32_t ctas = (sp.nq + sp.p_qpc - 1) / sp.p_qpc;
+    const size_t prep_smem = U8 && sp.prep_qs ? (size_t)sp.p_qpc * sp.prep_qs_stride * 4 : 0;
     if (prep_smem) {
-        e = cudaFuncSetAttribute(scan_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem);
+        e = cudaFuncSetAttribute(scan_prep_kernel<U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem);
         if (e != cudaSuccess) return e;
     }
-    scan_prep_kernel<<<ctas, kScanWarps * 32, prep_smem, st>>>(sp);
+    scan_prep_kernel<U8><<<ctas, sp.p_qpc * 32, prep_smem, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
     const size_t tile = scan_bitmap_smem(sp.bm_words);
     if (tile) {
-        e = cudaFuncSetAttribute(scan_bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile);
+        e = cudaFuncSetAttribute(scan_bitmap_kernel<U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile);
         if (e != cudaSuccess) return e;
     }
-    scan_bitmap_kernel<<<bitmap_grid, kBitmapThreads, tile, st>>>(sp);
+    scan_bitmap_kernel<U8><<<sp.item_bound < 8192 ? sp.item_bound : 8192, kBitmapThreads, tile, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[1], st)) != cudaSuccess) return e;
     const size_t smem = (size_t)sp.r_qpc * sp.r_warp_bytes;
-    e = cudaFuncSetAttribute(scan_replay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(scan_replay_kernel<U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    scan_replay_kernel<<<(sp.nq + sp.r_qpc - 1) / sp.r_qpc, kScanWarps * 32, smem, st>>>(sp);
+    scan_replay_kernel<U8><<<(sp.nq + sp.r_qpc - 1) / sp.r_qpc, kScanWarps * 32, smem, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[2], st)) != cudaSuccess) return e;
     return cudaSuccess;
+}
+
+// ev (optional, 3 events): recorded after the prep kernel, the bitmaps and the replay.
+cudaError_t launch_scan(const ScanParams& sp, cudaStream_t st, const cudaEvent_t* ev) {
+    return sp.l1.is_u8 ? launch_scan_t<true>(sp, st, ev) : launch_scan_t<false>(sp, st, ev);
 }
 
 }  // namespace pdxg

@@ -75,7 +75,7 @@ struct LevelOps {
     const uint32_t* fsel;   // this query's selection bitmap over the level (null = unfiltered)
     const uint32_t* fpass;  // this query's passing count per cluster
     bool top_level;         // the tree's meso-cluster search
-    int32_t pre_row = -1;   // row of this query's batched first-cluster distances (U8), or -1
+    int32_t pre_row = -1;   // row of this query's batched first-cluster distances, or -1
     uint32_t pre_cluster = 0xFFFFFFFFu;  // the cluster they belong to
 
     __device__ LevelOps(const SearchParams& p_, const DevLevel& lv_, Shared& sh_, Scalars& s_,
@@ -464,7 +464,7 @@ struct LevelOps {
     }
 
     // searcher.hpp:217-281 on distances computed ahead by the batched Start (pdxg_start.cu):
-    // the same exact U8 sums, read instead of recomputed.
+    // the same values, read instead of recomputed.
     __device__ void start_pre(const DevCluster& c, uint32_t k) {
         count_bytes((unsigned long long)c.n * lv.d * kElem, kStart);
         const uint32_t* src = p.start_dist + (size_t)pre_row * p.start_stride;
@@ -874,9 +874,9 @@ __global__ void __launch_bounds__(T) search_kernel(const __grid_constant__ Searc
             t_q0 = now;
         }
         LevelOps<T, U8, TOMB> ops(p, p.l1, sh, s, filter);
-        if (U8 && p.start_row && filter == -1) {
-            ops.pre_row = __ldg(p.start_row + q);
-            ops.pre_cluster = __ldg(p.start_first + q);
+        if (p.start_row && filter == -1) {
+            ops.pre_row = __ldg(p.start_row + (size_t)q * p.start_visits);
+            ops.pre_cluster = __ldg(p.start_first + (size_t)q * p.start_visits);
         }
         ops.run(kq, nvisit, visit);
         const uint32_t cnt = ops.sort_heap(kq);

@@ -1,18 +1,22 @@
-// Batched Start for U8 levels (PDXearch::Start, searcher.hpp:217-281), ahead of the scan.
+// Batched Start (PDXearch::Start, searcher.hpp:217-281), ahead of the scan.
 //
 // A query's first Start computes the full distance from the query to every vector of the first
-// cluster it visits, then keeps the best k. In a batch many queries start in the same cluster,
+// cluster it visits, then keeps the best k; while the heap is not full, the next clusters are
+// Starts too (k 100 on clusters of 70 vectors takes two or more). In a batch many queries start in the same cluster,
 // and the reference reads that whole cluster once per query. Here the queries of a batch are
-// grouped by their first visited cluster and each cluster is read once per group of up to
-// kStartQ queries, with the query-vector dot products on the integer tensor cores. U8
+// grouped by their first visited cluster and each cluster is read once per group of queries.
+// U8 (groups of up to 16): the query-vector dot products run on the integer tensor cores; the
 // distances are exact integer sums (no rounding): |q - x|^2 = |q|^2 + |x|^2 - 2 q.x holds
-// exactly, so the values equal those of the per-query Start. The search kernel then runs
-// push_smallest on them (searcher.hpp:256-280) instead of recomputing.
+// exactly, so the values equal those of the per-query Start. F32 (groups of up to 8): the
+// per-query Start's own chains, in its order. The search kernel then runs push_smallest on them
+// (searcher.hpp:256-280) instead of recomputing.
 //
-//   start_count_kernel : first non-empty cluster of each unfiltered query, counted per cluster
+//   start_count_kernel : the clusters that fill each unfiltered query's heap (up to sp.visits of
+//                        them), counted per cluster
 //   start_plan_kernel  : one CTA -- per-cluster offsets, each query's row, work items
 //   start_dist_kernel  : persistent CTAs over (cluster, <= kStartQ queries, 256 vectors) items,
 //                        mma.sync m16n8k32 u8 x u8 -> s32 (a 16 x 8 x 32 tile per instruction)
+//   start_f32_kernel   : the same over (cluster, <= kStartQF queries, 64 vectors) items
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -23,22 +27,35 @@ namespace pdxg {
 
 constexpr int kStartQ = 16;        // queries per work item
 constexpr int kStartV = 256;       // vectors per work item (one per thread)
+constexpr int kStartQF = 8;        // the same for F32 levels
+constexpr int kStartVF = 64;
 constexpr int kPlanThreads = 1024;
 
 __global__ void start_count_kernel(const __grid_constant__ StartParams sp) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= sp.nq) return;
-    sp.row_of[q] = -1;
-    sp.first_cl[q] = 0xFFFFFFFFu;
+    const size_t e0 = (size_t)q * sp.visits;
+    for (uint32_t s = 0; s < sp.visits; ++s) {
+        sp.row_of[e0 + s] = -1;
+        sp.first_cl[e0 + s] = 0xFFFFFFFFu;
+    }
+    sp.full_at[q] = 0xFFFFFFFFu;
     if (sp.filter_of && sp.filter_of[q] != -1) return;
-    const uint32_t cnt = sp.q_order_count[q];
+    const uint32_t cnt = sp.q_order_count[q], k = sp.q_k ? __ldg(sp.q_k + q) : sp.k;
     const uint32_t* ord = sp.q_order + (size_t)q * sp.q_order_stride;
-    for (uint32_t i = 0; i < cnt; ++i) {
+    uint32_t s = 0, have = 0;
+    for (uint32_t i = 0; i < cnt && s < sp.visits; ++i) {
         const uint32_t c = ord[i];
-        if (sp.l1.clusters[c].live == 0) continue;  // num_embeddings == 0 (searcher.hpp:662)
-        sp.first_cl[q] = c;
-        sp.slot_of[q] = atomicAdd(sp.cl_count + c, 1u);
-        return;
+        const DevCluster& cl = sp.l1.clusters[c];
+        if (cl.live == 0) continue;  // num_embeddings == 0 (searcher.hpp:662)
+        sp.first_cl[e0 + s] = c;
+        sp.slot_of[e0 + s] = atomicAdd(sp.cl_count + c, 1u);
+        ++s;
+        have += cl.n;
+        if (have >= k) {
+            sp.full_at[q] = i;
+            return;
+        }
     }
 }
 
@@ -79,28 +96,29 @@ __device__ uint32_t cta_exclusive_scan(uint32_t* a, uint32_t n, uint32_t* warp_t
 __global__ void __launch_bounds__(kPlanThreads) start_plan_kernel(const __grid_constant__ StartParams sp) {
     __shared__ uint32_t warp_tot[33];
     const uint32_t n1 = sp.l1.nclusters;
+    const uint32_t iq = sp.l1.is_u8 ? kStartQ : kStartQF, iv = sp.l1.is_u8 ? kStartV : kStartVF;
     // cl_off[c] = first row of cluster c; cl_items[c] = first work item of cluster c
     for (uint32_t c = threadIdx.x; c < n1; c += kPlanThreads) {
         const uint32_t L = sp.cl_count[c];
         sp.cl_off[c] = L;
         const uint32_t nv = sp.l1.clusters[c].n;
-        sp.cl_items[c] = L ? ((L + kStartQ - 1) / kStartQ) * ((nv + kStartV - 1) / kStartV) : 0u;
+        sp.cl_items[c] = L ? ((L + iq - 1) / iq) * ((nv + iv - 1) / iv) : 0u;
     }
     __syncthreads();
     cta_exclusive_scan(sp.cl_off, n1, warp_tot);
     const uint32_t total_items = cta_exclusive_scan(sp.cl_items, n1, warp_tot);
-    for (uint32_t q = threadIdx.x; q < sp.nq; q += kPlanThreads) {
-        const uint32_t c = sp.first_cl[q];
+    for (uint32_t e = threadIdx.x; e < sp.nq * sp.visits; e += kPlanThreads) {
+        const uint32_t c = sp.first_cl[e];
         if (c == 0xFFFFFFFFu) continue;
-        const uint32_t row = sp.cl_off[c] + sp.slot_of[q];
-        sp.row_of[q] = (int32_t)row;
-        sp.sorted_q[row] = q;
+        const uint32_t row = sp.cl_off[c] + sp.slot_of[e];
+        sp.row_of[e] = (int32_t)row;
+        sp.sorted_q[row] = e;
     }
     for (uint32_t c = threadIdx.x; c < n1; c += kPlanThreads) {
         const uint32_t L = sp.cl_count[c];
         if (!L) continue;
         const uint32_t nv = sp.l1.clusters[c].n;
-        const uint32_t nqc = (L + kStartQ - 1) / kStartQ, nvc = (nv + kStartV - 1) / kStartV;
+        const uint32_t nqc = (L + iq - 1) / iq, nvc = (nv + iv - 1) / iv;
         uint32_t it = sp.cl_items[c];
         for (uint32_t a = 0; a < nqc; ++a)
             for (uint32_t b = 0; b < nvc; ++b, ++it) {
@@ -153,7 +171,7 @@ __global__ void __launch_bounds__(kStartV) start_dist_kernel(const __grid_consta
         // rows past nqc are zero
         for (uint32_t e = threadIdx.x; e < kStartQ * nwords; e += kStartV) {
             const uint32_t j = e / nwords, w = e % nwords;
-            qw[j * qs + w] = j < nqc ? quantize_word(sp.queries + (size_t)sp.sorted_q[r0 + j] * lv.d, lv, w) : 0u;
+            qw[j * qs + w] = j < nqc ? quantize_word(sp.queries + (size_t)(sp.sorted_q[r0 + j] / sp.visits) * lv.d, lv, w) : 0u;
         }
         __syncthreads();
         if (warp < kStartQ / 2) {
@@ -258,7 +276,164 @@ __global__ void __launch_bounds__(kStartV) start_dist_kernel(const __grid_consta
     }
 }
 
+// ------------------------------------------------------------------------------------ F32
+constexpr int kStartFD = 64;           // dims per stage
+constexpr int kStartFRow = kStartFD + 4;  // floats per staged row: 16-byte reads of 8 rows hit distinct banks
+constexpr int kStartFThreads = 128;
+
+struct StartF32Smem {
+    float x[2][kStartVF * kStartFRow];  // vertical: [dim][64 vectors]; horizontal: [vector][dim]
+    float q[2][kStartQF * kStartFRow];  // [slot][dim]
+    uint32_t qrow[kStartQF];
+    uint32_t item;
+};
+
+// One stage for NQ query slots of a thread (vector v, slots slot0 .. slot0 + NQ - 1): vertical dims
+// (one fused multiply-add per dimension, in dimension order) or one horizontal block
+// (avx2_computers.hpp:47-98, lanes j and j + 1 as one packed chain), added to acc.
+template <int NQ>
+__device__ __forceinline__ void start_f32_stage(const float* xs, const float* qs, uint32_t v, uint32_t slot0,
+                                                bool vertical, uint32_t len, float (&acc)[4]) {
+    if (vertical) {
+        for (uint32_t j = 0; j < len; ++j) {
+            const float x = xs[j * kStartVF + v];
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) {
+                const float t = __fsub_rn(qs[(slot0 + i) * kStartFRow + j], x);
+                acc[i] = __fmaf_rn(t, t, acc[i]);
+            }
+        }
+        return;
+    }
+    uint64_t a[NQ][4];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[i][j] = 0ull;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const ulonglong2 x0 = *reinterpret_cast<const ulonglong2*>(xs + v * kStartFRow + 8 * t);
+        const ulonglong2 x1 = *reinterpret_cast<const ulonglong2*>(xs + v * kStartFRow + 8 * t + 4);
+        const uint64_t x[4] = {x0.x, x0.y, x1.x, x1.y};
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(qs + (slot0 + i) * kStartFRow + 8 * t);
+            const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(qs + (slot0 + i) * kStartFRow + 8 * t + 4);
+            const uint64_t q[4] = {q0.x, q0.y, q1.x, q1.y};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint64_t df = f32x2_sub(q[j], x[j]);
+                a[i][j] = f32x2_fma(df, df, a[i][j]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        float l[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f32x2_unpack(a[i][j], l[2 * j], l[2 * j + 1]);
+        const double s0 = (double)l[0] + (double)l[4], s1 = (double)l[1] + (double)l[5];
+        const double s2 = (double)l[2] + (double)l[6], s3 = (double)l[3] + (double)l[7];
+        acc[i] = __fadd_rn(acc[i], (float)((s0 + s2) + (s1 + s3)));
+    }
+}
+
+// CTA = one work item: up to 8 queries x 64 vectors of one cluster; thread (vector tid & 63, half of
+// the queries). A cluster's first visit by a batch reads it from HBM, and with a few queries per
+// cluster that is what bounds the kernel, so the 64-dim stages are copied asynchronously, two deep,
+// and small enough (39 KB) for five CTAs on an SM to keep 80 KB of copies in flight.
+// 138 us for 2,000 queries on 200,000 x 768 (895 clusters, 614 MB: 94 us at the copy rate); the scan
+// that begins with it takes 962 us in the per-query kernel, which reads a cluster once per query.
+// VEC: d and d_v multiples of 4 and 16-byte aligned queries.
+template <bool VEC>
+__global__ void __launch_bounds__(kStartFThreads, 5) start_f32_kernel(const __grid_constant__ StartParams sp) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    StartF32Smem& S = *reinterpret_cast<StartF32Smem*>(smem_raw);
+    const DevLevel& lv = sp.l1;
+    const uint32_t tid = threadIdx.x, v = tid & (kStartVF - 1);
+    const uint32_t d = lv.d, dv = lv.dv;
+    const uint32_t nvc = (dv + kStartFD - 1) / kStartFD, nst = nvc + lv.n_hblocks;
+    for (;;) {
+        if (tid == 0) S.item = atomicAdd(sp.queue, 1u);
+        __syncthreads();
+        const uint32_t it = S.item;
+        if (it >= sp.n_items[0]) break;
+        const uint32_t c = sp.items[2 * it];
+        const uint32_t ab = sp.items[2 * it + 1];
+        const uint32_t qa = ab >> 16, v0 = (ab & 0xFFFFu) * kStartVF;
+        const uint32_t L = sp.cl_count[c];
+        const uint32_t r0 = sp.cl_off[c] + qa * kStartQF;
+        const uint32_t nqc = (L - qa * kStartQF) < (uint32_t)kStartQF ? (L - qa * kStartQF) : (uint32_t)kStartQF;
+        if (tid < kStartQF) S.qrow[tid] = sp.sorted_q[r0 + (tid < nqc ? tid : 0)] / sp.visits;
+        __syncthreads();
+        const DevCluster cl = lv.clusters[c];
+        const float* vert = reinterpret_cast<const float*>(sp.arena + cl.vert_off);
+        const float* hor = reinterpret_cast<const float*>(sp.arena + cl.hor_off);
+        auto issue = [&](uint32_t st) {
+            float* xb = S.x[st & 1];
+            float* qb = S.q[st & 1];
+            const bool vs = st < nvc;
+            const uint32_t j0 = vs ? st * kStartFD : dv + (st - nvc) * kStartFD;
+            const uint32_t len = vs && dv - j0 < (uint32_t)kStartFD ? dv - j0 : (uint32_t)kStartFD;
+#pragma unroll
+            for (int t = 0; t < kStartVF * kStartFD / 4 / kStartFThreads; ++t) {
+                const uint32_t e = tid + t * kStartFThreads, r = e >> 4, c4 = (e & 15) * 4;
+                if (vs) {  // dim j0 + r, vectors v0 + c4 ..: rows are n_pad long
+                    const bool in = r < len && v0 + c4 < cl.n_pad;
+                    cp_async16_zfill(xb + r * kStartVF + c4, vert + (in ? (size_t)(j0 + r) * cl.n_pad + v0 + c4 : 0), in);
+                } else {   // vector v0 + r, dims c4 .. of the block
+                    const bool in = v0 + r < cl.n_pad;
+                    cp_async16_zfill(xb + r * kStartFRow + c4,
+                                     hor + (in ? ((size_t)(st - nvc) * cl.n_pad + v0 + r) * kHDim + c4 : 0), in);
+                }
+            }
+            if constexpr (VEC) {
+                const uint32_t r = tid >> 4, c4 = (tid & 15) * 4;
+                static_assert(kStartQF * kStartFD / 4 == kStartFThreads, "one piece per thread");
+                const bool in = r < nqc && c4 < len;
+                cp_async16_zfill(qb + r * kStartFRow + c4, sp.queries + (size_t)S.qrow[r] * d + (in ? j0 + c4 : 0), in);
+            } else {
+                for (uint32_t e = tid; e < kStartQF * kStartFD; e += kStartFThreads) {
+                    const uint32_t r = e >> 6, j = e & 63;
+                    qb[r * kStartFRow + j] = r < nqc && j < len ? __ldg(sp.queries + (size_t)S.qrow[r] * d + j0 + j) : 0.0f;
+                }
+            }
+        };
+        // the two thread halves split the queries: nq2 slots each
+        const uint32_t nq2 = (nqc + 1) / 2, slot0 = (tid >> 6) * nq2;
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        issue(0);
+        cp_async_commit();
+        for (uint32_t st = 0; st < nst; ++st) {
+            if (st + 1 < nst) issue(st + 1);
+            cp_async_commit();
+            cp_async_wait1();
+            __syncthreads();
+            const bool vs = st < nvc;
+            const uint32_t len = vs && dv - st * kStartFD < (uint32_t)kStartFD ? dv - st * kStartFD : (uint32_t)kStartFD;
+            const float* xs = S.x[st & 1];
+            const float* qs = S.q[st & 1];
+            if (nq2 == 1) start_f32_stage<1>(xs, qs, v, slot0, vs, len, acc);
+            else if (nq2 == 2) start_f32_stage<2>(xs, qs, v, slot0, vs, len, acc);
+            else if (nq2 == 3) start_f32_stage<3>(xs, qs, v, slot0, vs, len, acc);
+            else start_f32_stage<4>(xs, qs, v, slot0, vs, len, acc);
+            __syncthreads();
+        }
+        if (v0 + v < cl.n) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if ((uint32_t)i < nq2 && slot0 + i < nqc)
+                    sp.dist[(size_t)(r0 + slot0 + i) * sp.stride + v0 + v] = __float_as_uint(acc[i]);
+        }
+    }
+}
+
+static bool start_f32_vec(const StartParams& sp) {
+    return sp.l1.d % 4 == 0 && sp.l1.dv % 4 == 0 && ((uintptr_t)sp.queries & 15) == 0;
+}
+
 size_t start_dist_smem(const DevLevel& lv) {
+    if (!lv.is_u8) return sizeof(StartF32Smem);
     return (size_t)kStartQ * (lv.qw_hoff + lv.n_hblocks * 16 + 4) * 4;
 }
 
@@ -270,21 +445,37 @@ cudaError_t launch_start_batched(const StartParams& sp, int grid, cudaStream_t s
     start_plan_kernel<<<1, kPlanThreads, 0, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t smem = start_dist_smem(sp.l1);
+    if (!sp.l1.is_u8) {
+        auto kern = start_f32_vec(sp) ? start_f32_kernel<true> : start_f32_kernel<false>;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, kStartFThreads, smem, st>>>(sp);
+        return cudaGetLastError();
+    }
     e = cudaFuncSetAttribute(start_dist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     start_dist_kernel<<<grid, kStartV, smem, st>>>(sp);
     return cudaGetLastError();
 }
 
-int start_dist_occupancy(size_t smem) {
+int start_dist_occupancy(bool u8, size_t smem) {
     int blocks = 0;
+    if (!u8) {
+        cudaFuncSetAttribute(start_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, start_f32_kernel<true>, kStartFThreads, smem);
+        return blocks;
+    }
     cudaFuncSetAttribute(start_dist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, start_dist_kernel, kStartV, smem);
     return blocks;
 }
 
-uint64_t start_item_bound(uint32_t nq, uint32_t n1, uint32_t max_n) {
-    return ((uint64_t)(nq + kStartQ - 1) / kStartQ + n1) * ((max_n + kStartV - 1) / kStartV);
+// Work items of nq Starts at most; 0 when the items' 16-bit chunk numbers cannot hold them.
+uint64_t start_item_bound(bool u8, uint32_t nq, uint32_t n1, uint32_t max_n) {
+    const uint32_t iq = u8 ? kStartQ : kStartQF, iv = u8 ? kStartV : kStartVF;
+    const uint64_t nqc = ((uint64_t)nq + iq - 1) / iq, nvc = ((uint64_t)max_n + iv - 1) / iv;
+    if (nqc > 65536 || nvc > 65536) return 0;
+    return (nqc + n1) * nvc;
 }
 
 }  // namespace pdxg
