@@ -180,6 +180,9 @@ struct StartParams {
     uint32_t k;
     const uint32_t* q_k;          // optional per-query k (<= k)
     uint32_t visits;              // Starts computed for a query at most
+    uint32_t nwords;              // U8: query words, qw_hoff + 16 n_hblocks
+    uint32_t* qwords;             // U8: [nq x nwords] quantized queries, packed as the scan packs them
+    uint32_t* qsq;                // U8: [nq] their |q|^2
     uint32_t* cl_count;           // [n1] Starts per cluster (zeroed before)
     uint32_t* cl_off;             // [n1] first row of each cluster
     uint32_t* cl_items;           // [n1] first work item of each cluster
@@ -220,8 +223,8 @@ struct ScanParams {
     uint32_t cp1;                 // first warmup checkpoint: min(16, d_v)
     uint32_t g1;                  // vertical words it covers: ceil(cp1 / 4) (<= 4), F32 cp1
     uint32_t nwords;              // query words: U8 qw_hoff + 16 n_hblocks, F32 d
-    uint32_t* qwords;             // [nq x nwords] U8: quantized queries, packed as the scan packs
-                                  // them (written by the prep kernel); F32: the queries themselves
+    const uint32_t* qwords;       // [nq x nwords] U8: the quantized queries of the batched Start; F32: the
+                                  // queries themselves
     uint32_t* first_i;            // [nq] position of the last Start in the order; ~0u: not here
     int32_t* lim;                 // [nq] a vector is a candidate when |x|^2 - 2 q.x < lim (F32: lim is a
                                   // float, with the margin of scan_bitmap_kernel)
@@ -248,8 +251,6 @@ struct ScanParams {
     float* out_dists;             // [nq x k]
     uint32_t* out_counts;         // [nq]
     unsigned long long* stats;    // optional, SearchParams::stats layout
-    uint32_t prep_qs;             // 1: the prep kernel stages each query row in shared memory
-    uint32_t prep_qs_stride;      // floats per staged row
     uint32_t p_qpc;               // prep: queries per CTA (1..8), one warp each
     uint32_t r_qpc;               // replay: queries per CTA (1..8), one warp each
     uint32_t r_surv_cap;          // replay: survivors of one cluster's first warmup step it keeps

@@ -90,7 +90,7 @@ struct Workspace {
     uint64_t l1_order_cap = 0;
     uint32_t* d_l1_count = nullptr;
     uint64_t l1_count_cap = 0;
-    // batched Start: per-cluster counters ([3 x n1]), per-query arrays (4 per Start, 1 per query) and
+    // batched Start: per-cluster counters ([3 x n1]), per-query arrays (4 per Start, 2 per query) and
     // two counters, work items, distances
     uint32_t* d_st_cl = nullptr;
     uint64_t st_cl_cap = 0;

@@ -1102,7 +1102,9 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     if (occ <= 0) return PDXG_OK;
     int rc;
     if ((rc = dev_grow(w.d_st_cl, w.st_cl_cap, (uint64_t)3 * n1))) return rc;
-    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + nq + 2))) return rc;
+    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + 2ull * nq + 2))) return rc;
+    const uint32_t nwords = L.p.l1.qw_hoff + L.p.l1.n_hblocks * 16;
+    if (ix->u8 && (rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
     if ((rc = dev_grow(w.d_st_items, w.st_items_cap, 2 * items))) return rc;
     if ((rc = dev_grow(w.d_st_dist, w.st_dist_cap, ne * stride))) return rc;
     StartParams sp{};
@@ -1127,6 +1129,9 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     sp.full_at = w.d_st_q + 4 * ne;
     sp.n_items = w.d_st_q + 4 * ne + nq;
     sp.queue = w.d_st_q + 4 * ne + nq + 1;
+    sp.qsq = w.d_st_q + 4 * ne + nq + 2;
+    sp.nwords = nwords;
+    sp.qwords = w.d_sc_qw;
     sp.items = w.d_st_items;
     sp.dist = w.d_st_dist;
     sp.stride = stride;
@@ -1137,7 +1142,7 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     L.p.start_stride = stride;
     L.p.start_visits = visits;
     L.start_full_at = sp.full_at;
-    L.start_launches = 3;
+    L.start_launches = ne > 1024 ? 4 : 3;
     return PDXG_OK;
 }
 
@@ -1164,8 +1169,6 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.r_surv_cap = (std::max(lv.max_n, 1u) / 5 + 33 + 31) / 32 * 32;
     sp.r_warp_bytes = (uint32_t)(align_up((uint64_t)nwords * 4, 16) + 8ull * sp.r_heap_cap + sp.r_area_bytes +
                                  align_up((uint64_t)bm_words * 4, 16) + 8ull * sp.r_surv_cap);
-    sp.prep_qs_stride = (lv.d + 3) & ~3u;
-    sp.prep_qs = (uint64_t)scan_queries_per_cta() * sp.prep_qs_stride * 4 + 1024 <= ix->max_smem ? 1u : 0u;
     sp.p_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + ix->num_sms - 1) / ix->num_sms);
     // a replay CTA of 8 warps takes as few queries as still fill the GPU at 3 CTAs per SM, so that
     // the heavy visits of a small batch are shared by more warps
@@ -1184,7 +1187,6 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     int rc;
     if ((rc = dev_grow(w.d_sc_hv, w.sc_hv_cap, hv_rows * sp.hv_cap))) return rc;
     if ((rc = dev_grow(w.d_sc_vi, w.sc_vi_cap, (uint64_t)nq * stride))) return rc;
-    if (L.u8 && (rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
     if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 3))) return rc;
     if ((rc = dev_grow(w.d_sc_heap, w.sc_heap_cap, 2ull * nq * k))) return rc;
     if ((rc = dev_grow(w.d_sc_cl, w.sc_cl_cap, (uint64_t)n1))) return rc;
@@ -1211,7 +1213,7 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.cp1 = std::min(16u, lv.dv);
     sp.g1 = L.u8 ? (sp.cp1 + 3) / 4 : sp.cp1;
     sp.nwords = nwords;
-    sp.qwords = L.u8 ? w.d_sc_qw : reinterpret_cast<uint32_t*>(const_cast<float*>(L.p.queries));
+    sp.qwords = L.u8 ? w.d_sc_qw : reinterpret_cast<const uint32_t*>(L.p.queries);
     sp.first_i = w.d_sc_q;
     sp.lim = reinterpret_cast<int32_t*>(w.d_sc_q + nq);
     sp.left = w.d_sc_q + 2ull * nq;

@@ -22,7 +22,7 @@
 // whole warmup itself. Survivors then follow Prune (searcher.hpp:437-540) one per lane and are
 // merged in position order (searcher.hpp:542-566), as in the per-query kernel.
 //
-//   scan_prep_kernel   : warp per query -- quantized query words, the Starts' pushes (the m
+//   scan_prep_kernel   : warp per query -- the Starts' pushes (the m
 //                        smallest batched-Start distances, ties by position) and tau0's bound;
 //                        every later visit appended to its cluster's list, with a work item per
 //                        8 to 64 list entries; queries this path does not take go to a list for the
@@ -177,9 +177,7 @@ constexpr int kRegKeys = 32;  // Start distances a prep lane keeps in registers 
 
 // The m-th smallest of the n keys (1 <= m <= n): the smallest key with at least m keys not above
 // it, found bit by bit between the keys' common prefix and their lowest bit with one count of the
-// keys below a trial value per bit. All keys of a cluster share their high bits, so a radix
-// histogram's first passes queue most of their shared-memory atomics on one bin (with it: 187 us
-// for the prep kernel on 10,000 queries and clusters of 1,000 vectors, 54 us on 777).
+// keys below a trial value per bit.
 template <class Key>
 __device__ __forceinline__ uint32_t warp_select(uint32_t n, uint32_t m, const Key& key) {
     uint32_t lo = 0xFFFFFFFFu, hi = 0;
@@ -248,10 +246,10 @@ struct MemKeys {
 
 // Start (searcher.hpp:256-280): the m smallest keys pushed in the order of
 // LevelOps::push_smallest -- the keys below the m-th in position order, then the ties at it.
-// Returns the m-th key.
-template <bool U8, class Key>
-__device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint32_t m,
-                                               const uint32_t* ids, const DevLevel& lv, float* hd, uint32_t* hid) {
+// Returns the m-th key. This form walks all keys; start_push below needs it for long selections.
+template <bool U8>
+__device__ __noinline__ uint32_t start_push_all(MemKeys key, uint32_t n, uint32_t m, const uint32_t* ids,
+                                                const DevLevel& lv, float* hd, uint32_t* hid) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t kth = warp_select(n, m, key);
     uint32_t pushed = 0;
@@ -271,11 +269,100 @@ __device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint3
     return kth;
 }
 
-// Dynamic shared memory: the warps' query rows (prep_qs set: kScanWarps x d floats), staged
-// with one coalesced pass; without it the query is read from global memory.
+// A few counts bring a bound above at least m keys and at most kSelectList of them; those, in
+// position order, are all that the selection and the pushes then look at. Selecting over all keys,
+// bit by bit and with two passes of ballots, and quantizing the query here, took the warp about
+// 9,000 instructions on 1,000 vectors: 200 us for the prep kernel on 10,000 queries, 58 us on 777,
+// against 102 and 26.
+constexpr uint32_t kSelectList = 128;
+
+template <bool U8, class Key>
+__device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint32_t m, const uint32_t* ids,
+                                               const DevLevel& lv, float* hd, uint32_t* hid, uint64_t* list,
+                                               const uint32_t* src) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (m > kSelectList) return start_push_all<U8>(MemKeys{src}, n, m, ids, lv, hd, hid);
+    // bound T with m <= #(keys <= T) <= kSelectList, by bisection between the smallest and largest key
+    uint32_t T = 0xFFFFFFFFu, cnt = n;
+    if (n > kSelectList) {
+        uint32_t lo = 0xFFFFFFFFu, hi = 0;
+        key.for_each(n, [&](uint32_t, uint32_t k) {
+            lo = k < lo ? k : lo;
+            hi = k > hi ? k : hi;
+        });
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        T = hi = __reduce_max_sync(0xffffffffu, hi);
+        while (cnt > kSelectList && lo < T) {
+            const uint32_t mid = lo + (T - lo) / 2;
+            uint32_t c = 0;
+            key.for_each(n, [&](uint32_t, uint32_t k) { c += k <= mid ? 1u : 0u; });
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (c >= m) {
+                T = mid;
+                cnt = c;
+            } else {
+                lo = mid + 1;
+            }
+        }
+        // more ties at the m-th key than the list holds
+        if (cnt > kSelectList) return start_push_all<U8>(MemKeys{src}, n, m, ids, lv, hd, hid);
+    }
+    uint32_t len = 0;
+    key.for_chunks(n, [&](uint32_t v0, uint32_t kv) {
+        const bool in = v0 + lane < n && kv <= T;
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) list[len + __popc(b & ((1u << lane) - 1u))] = ((uint64_t)kv << 32) | (v0 + lane);
+        len += __popc(b);
+    });
+    __syncwarp();
+    // the list in registers, entry 32 u + lane in register u; rows of the pushes requested already
+    constexpr int R = kSelectList / 32;
+    uint32_t k[R], id[R];
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const bool in = 32u * u + lane < len;
+        const uint64_t e = in ? list[32 * u + lane] : 0ull;
+        k[u] = (uint32_t)(e >> 32);
+        id[u] = in ? __ldg(ids + (uint32_t)e) : 0u;
+        if (in) {
+            lo = k[u] < lo ? k[u] : lo;
+            hi = k[u] > hi ? k[u] : hi;
+        }
+    }
+    __syncwarp();  // the list may be rewritten by the next Start
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    while (lo < hi) {  // kth in [lo, hi]
+        const uint32_t mid = lo + (hi - lo) / 2;
+        uint32_t c = 0;
+#pragma unroll
+        for (int u = 0; u < R; ++u) c += (32u * u + lane < len && k[u] <= mid) ? 1u : 0u;
+        if (__reduce_add_sync(0xffffffffu, c) >= m) hi = mid;
+        else lo = mid + 1;
+    }
+    const uint32_t kth = lo;
+    uint32_t pushed = 0;
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const bool sel = 32u * u + lane < len && (pass == 0 ? k[u] < kth : k[u] == kth);
+            const unsigned b = __ballot_sync(0xffffffffu, sel);
+            const uint32_t at = pushed + __popc(b & ((1u << lane) - 1u));
+            if (sel && at < m) {
+                hd[at] = Raw<U8>::reported(k[u], lv);
+                hid[at] = id[u];
+            }
+            pushed += __popc(b);
+        }
+    }
+    return kth;
+}
+
 template <bool U8>
 __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid_constant__ ScanParams sp) {
-    extern __shared__ __align__(16) float qs_all[];
+    __shared__ uint64_t list_all[kScanWarps][kSelectList];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t q = blockIdx.x * sp.p_qpc + warp;
     if (q >= sp.nq) return;  // whole warp
@@ -299,39 +386,13 @@ __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid
     const uint32_t* src = sp.start_dist + (size_t)__ldg(rows) * sp.start_stride;
     RegKeys rk;
     if (cl.n <= 32u * kRegKeys) rk.load(src, cl.n);  // in flight while the query is quantized
-    // QuantizeEmbedding (scalar.hpp:76-94) in the scan's packed word layout; |q|^2 over the
-    // first checkpoint's words
-    const float* qf = sp.queries + (size_t)q * lv.d;
+    // |q|^2 over the first checkpoint's dims
     uint32_t qn = 0;
-    if (U8 && sp.prep_qs) {
-        float* qs = qs_all + (size_t)warp * sp.prep_qs_stride;
-        for (uint32_t i0 = 0; i0 < lv.d; i0 += 128) {
-            float t[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t i = i0 + 32 * u + lane;
-                t[u] = i < lv.d ? __ldg(qf + i) : 0.0f;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t i = i0 + 32 * u + lane;
-                if (i < lv.d) qs[i] = t[u];
-            }
-        }
-        __syncwarp();
-        qf = qs;
-    }
     if constexpr (U8) {
-        uint32_t* qw = sp.qwords + (size_t)q * sp.nwords;
-        for (uint32_t w = lane; w < sp.nwords; w += 32) {
-            const uint32_t word = quantize_word(qf, lv, w);
-            qw[w] = word;
-            if (w < sp.g1) qn = __dp4a(word, word, qn);
-        }
-        qn = __reduce_add_sync(0xffffffffu, qn);
-    }
-    if constexpr (!U8) {  // |q|^2 over the first checkpoint's dims
-        const float x = lane < sp.cp1 ? __ldg(qf + lane) : 0.0f;
+        const uint32_t word = lane < sp.g1 ? __ldg(sp.qwords + (size_t)q * sp.nwords + lane) : 0u;
+        qn = __reduce_add_sync(0xffffffffu, __dp4a(word, word, 0u));
+    } else {
+        const float x = lane < sp.cp1 ? __ldg(sp.queries + (size_t)q * lv.d + lane) : 0.0f;
         float sq = x * x;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
@@ -375,8 +436,8 @@ __global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid
         const uint32_t n = cl.n;
         const uint32_t m = kq - have < n ? kq - have : n;
         const uint32_t* ids = reinterpret_cast<const uint32_t*>(sp.arena + cl.ids_off);
-        const uint32_t kth = n <= 32u * kRegKeys ? start_push<U8>(rk, n, m, ids, lv, hd + have, hid + have)
-                                                 : start_push<U8>(MemKeys{src}, n, m, ids, lv, hd + have, hid + have);
+        const uint32_t kth = n <= 32u * kRegKeys ? start_push<U8>(rk, n, m, ids, lv, hd + have, hid + have, list_all[warp], src)
+                                                 : start_push<U8>(MemKeys{src}, n, m, ids, lv, hd + have, hid + have, list_all[warp], src);
         top = kth > top ? kth : top;
         have += m;
         if (sp.stats && lane == 0) {
@@ -1168,12 +1229,7 @@ static cudaError_t launch_scan_t(const ScanParams& sp, cudaStream_t st, const cu
     // left_n, n_items and hv_alloc are consecutive
     if ((e = cudaMemsetAsync(sp.left_n, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
     const uint32_t ctas = (sp.nq + sp.p_qpc - 1) / sp.p_qpc;
-    const size_t prep_smem = U8 && sp.prep_qs ? (size_t)sp.p_qpc * sp.prep_qs_stride * 4 : 0;
-    if (prep_smem) {
-        e = cudaFuncSetAttribute(scan_prep_kernel<U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem);
-        if (e != cudaSuccess) return e;
-    }
-    scan_prep_kernel<U8><<<ctas, sp.p_qpc * 32, prep_smem, st>>>(sp);
+    scan_prep_kernel<U8><<<ctas, sp.p_qpc * 32, 0, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ev && (e = cudaEventRecord(ev[0], st)) != cudaSuccess) return e;
     const size_t tile = scan_bitmap_smem(sp.bm_words);

@@ -12,7 +12,8 @@
 // (searcher.hpp:256-280) instead of recomputing.
 //
 //   start_count_kernel : the clusters that fill each unfiltered query's heap (up to sp.visits of
-//                        them), counted per cluster
+//                        them), counted per cluster; U8: the quantized query, once for the Start
+//                        and the scan
 //   start_plan_kernel  : one CTA -- per-cluster offsets, each query's row, work items
 //   start_dist_kernel  : persistent CTAs over (cluster, <= kStartQ queries, 256 vectors) items,
 //                        mma.sync m16n8k32 u8 x u8 -> s32 (a 16 x 8 x 32 tile per instruction)
@@ -31,9 +32,24 @@ constexpr int kStartQF = 8;        // the same for F32 levels
 constexpr int kStartVF = 64;
 constexpr int kPlanThreads = 1024;
 
-__global__ void start_count_kernel(const __grid_constant__ StartParams sp) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int kCountThreads = 256;
+
+// Warp per query: lane 0 walks the first visits, all lanes quantize (U8).
+__global__ void __launch_bounds__(kCountThreads) start_count_kernel(const __grid_constant__ StartParams sp) {
+    const uint32_t q = (blockIdx.x * kCountThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (q >= sp.nq) return;
+    if (sp.l1.is_u8) {
+        const float* qf = sp.queries + (size_t)q * sp.l1.d;
+        uint32_t sq = 0;
+        for (uint32_t w = lane; w < sp.nwords; w += 32) {
+            const uint32_t word = quantize_word(qf, sp.l1, w);
+            sp.qwords[(size_t)q * sp.nwords + w] = word;
+            sq = __dp4a(word, word, sq);
+        }
+        sq = __reduce_add_sync(0xffffffffu, sq);
+        if (lane == 0) sp.qsq[q] = sq;
+    }
+    if (lane) return;
     const size_t e0 = (size_t)q * sp.visits;
     for (uint32_t s = 0; s < sp.visits; ++s) {
         sp.row_of[e0 + s] = -1;
@@ -93,6 +109,23 @@ __device__ uint32_t cta_exclusive_scan(uint32_t* a, uint32_t n, uint32_t* warp_t
     return carry;
 }
 
+// Row of Start e. More than kPlanRows of them take their own launch: as a loop of the one planning
+// CTA (two dependent reads a turn) 10,000 took 34 of its 37 us, 2,000 8 of 13.
+constexpr uint32_t kPlanRows = 1024;
+
+__device__ __forceinline__ void start_row(const StartParams& sp, uint32_t e) {
+    const uint32_t c = sp.first_cl[e];
+    if (c == 0xFFFFFFFFu) return;
+    const uint32_t row = sp.cl_off[c] + sp.slot_of[e];
+    sp.row_of[e] = (int32_t)row;
+    sp.sorted_q[row] = e;
+}
+
+__global__ void __launch_bounds__(256) start_rows_kernel(const __grid_constant__ StartParams sp) {
+    const uint32_t e = blockIdx.x * 256 + threadIdx.x;
+    if (e < sp.nq * sp.visits) start_row(sp, e);
+}
+
 __global__ void __launch_bounds__(kPlanThreads) start_plan_kernel(const __grid_constant__ StartParams sp) {
     __shared__ uint32_t warp_tot[33];
     const uint32_t n1 = sp.l1.nclusters;
@@ -107,13 +140,8 @@ __global__ void __launch_bounds__(kPlanThreads) start_plan_kernel(const __grid_c
     __syncthreads();
     cta_exclusive_scan(sp.cl_off, n1, warp_tot);
     const uint32_t total_items = cta_exclusive_scan(sp.cl_items, n1, warp_tot);
-    for (uint32_t e = threadIdx.x; e < sp.nq * sp.visits; e += kPlanThreads) {
-        const uint32_t c = sp.first_cl[e];
-        if (c == 0xFFFFFFFFu) continue;
-        const uint32_t row = sp.cl_off[c] + sp.slot_of[e];
-        sp.row_of[e] = (int32_t)row;
-        sp.sorted_q[row] = e;
-    }
+    if (sp.nq * sp.visits <= kPlanRows)
+        for (uint32_t e = threadIdx.x; e < sp.nq * sp.visits; e += kPlanThreads) start_row(sp, e);
     for (uint32_t c = threadIdx.x; c < n1; c += kPlanThreads) {
         const uint32_t L = sp.cl_count[c];
         if (!L) continue;
@@ -143,23 +171,50 @@ __device__ __forceinline__ void mma_u8_16x8x32(int (&c)[4], const uint32_t (&a)[
 }
 
 // CTA = one work item: up to 16 queries x 256 vectors of one cluster. Warp w takes vectors
-// [32 w, 32 w + 32) in four 8-vector tiles. The squared distance of an integer query q and
-// vector x is |q|^2 + |x|^2 - 2 q.x exactly; q.x runs on the tensor cores, |x|^2 with dp4a on
-// the same loaded words, |q|^2 once per query.
-__global__ void __launch_bounds__(kStartV) start_dist_kernel(const __grid_constant__ StartParams sp) {
+// [32 w, 32 w + 32) as four 8-vector tiles: column n of tile t is vector 4 n + t. The squared
+// distance of an integer query q and vector x is |q|^2 + |x|^2 - 2 q.x exactly; q.x runs on the
+// tensor cores, |x|^2 with dp4a on the same loaded words.
+//
+// The kernel reads every started cluster once from HBM and is bound by how that read is asked for.
+// A dot product may take its dims in any order, so the k-groups are assigned for 16-byte loads: per
+// 64 dims a lane (row gq, k-group gk) takes words 4 gk .. 4 gk + 3 of the query and of the four
+// vectors 4 gq .. 4 gq + 3 -- four loads, which for a horizontal block cover 2 KB of contiguous
+// memory per warp (word order as the fragments number it took 16 4-byte loads that used half of
+// each sector) -- and the next 64 dims are loaded while these are computed. 10,000 queries on 1.02 GB
+// of clusters (157 us at the copy rate): 248 us; 288 without the loads ahead, 333 with the 4-byte
+// loads and each CTA quantizing its queries; 777 queries 134, 152 and 156.
+__device__ __forceinline__ void start_mma_64(int (&acc)[4][4], uint32_t (&xsq)[4], const uint4& a0, const uint4& a1,
+                                             const uint4 (&x)[4]) {
+    const uint32_t lo[4] = {a0.x, a1.x, a0.y, a1.y}, hi[4] = {a0.z, a1.z, a0.w, a1.w};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        xsq[t] = __dp4a(x[t].x, x[t].x, xsq[t]);
+        xsq[t] = __dp4a(x[t].y, x[t].y, xsq[t]);
+        xsq[t] = __dp4a(x[t].z, x[t].z, xsq[t]);
+        xsq[t] = __dp4a(x[t].w, x[t].w, xsq[t]);
+        mma_u8_16x8x32(acc[t], lo, x[t].x, x[t].y);
+        mma_u8_16x8x32(acc[t], hi, x[t].z, x[t].w);
+    }
+}
+
+__host__ __device__ inline uint32_t start_row_words(uint32_t nwords) {
+    return (nwords + 31) / 32 * 32 + 16;  // two rows of a 16-byte fragment load hit distinct banks
+}
+
+__global__ void __launch_bounds__(kStartV, 3) start_dist_kernel(const __grid_constant__ StartParams sp) {
     extern __shared__ __align__(16) uint32_t qw[];  // [kStartQ][qs] packed query words
     __shared__ uint32_t item;
     __shared__ uint32_t qsq[kStartQ];
     const DevLevel& lv = sp.l1;
-    const uint32_t nwords = lv.qw_hoff + lv.n_hblocks * 16;
-    const uint32_t qs = nwords + 4;  // row stride: fragment loads of 8 rows hit distinct banks
+    const uint32_t nwords = sp.nwords, qs = start_row_words(nwords);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t gq = lane >> 2, gk = lane & 3;  // fragment row / k-group of this lane
+    const uint32_t* qa0 = qw + gq * qs + 4 * gk;
+    const uint32_t* qa1 = qa0 + 8 * qs;
     for (;;) {
         if (threadIdx.x == 0) item = atomicAdd(sp.queue, 1u);
         __syncthreads();
         const uint32_t it = item;
-        __syncthreads();
         if (it >= sp.n_items[0]) break;
         const uint32_t c = sp.items[2 * it];
         const uint32_t ab = sp.items[2 * it + 1];
@@ -167,31 +222,16 @@ __global__ void __launch_bounds__(kStartV) start_dist_kernel(const __grid_consta
         const uint32_t L = sp.cl_count[c];
         const uint32_t r0 = sp.cl_off[c] + qa * kStartQ;
         const uint32_t nqc = (L - qa * kStartQ) < (uint32_t)kStartQ ? (L - qa * kStartQ) : (uint32_t)kStartQ;
-        // QuantizeEmbedding of the item's queries, packed as the search kernel packs them;
-        // rows past nqc are zero
-        for (uint32_t e = threadIdx.x; e < kStartQ * nwords; e += kStartV) {
-            const uint32_t j = e / nwords, w = e % nwords;
-            qw[j * qs + w] = j < nqc ? quantize_word(sp.queries + (size_t)(sp.sorted_q[r0 + j] / sp.visits) * lv.d, lv, w) : 0u;
-        }
-        __syncthreads();
-        if (warp < kStartQ / 2) {
-            // |q|^2: warp w sums queries 2 w and 2 w + 1
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t j = 2 * warp + h;
-                uint32_t acc = 0;
-                for (uint32_t w = lane; w < nwords; w += 32) acc = __dp4a(qw[j * qs + w], qw[j * qs + w], acc);
-                acc = __reduce_add_sync(0xffffffffu, acc);
-                if (lane == 0) qsq[j] = acc;
-            }
+        // the item's query words; rows past nqc and words past the last are zero
+        for (uint32_t j = warp; j < kStartQ; j += kStartV / 32) {
+            const uint32_t q = j < nqc ? sp.sorted_q[r0 + j] / sp.visits : 0u;
+            const uint32_t* src = sp.qwords + (size_t)q * nwords;
+            for (uint32_t w = lane; w < qs; w += 32) qw[j * qs + w] = j < nqc && w < nwords ? __ldg(src + w) : 0u;
+            if (lane == 0) qsq[j] = j < nqc ? sp.qsq[q] : 0u;
         }
         __syncthreads();
         const DevCluster cl = lv.clusters[c];
-        const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + cl.vert_off);
-        const uint8_t* hor = sp.arena + cl.hor_off;
-        // four 8-vector tiles per warp, all in flight at once; tiles past the cluster load
-        // in-bounds padding (n_pad) and are not stored
-        const uint32_t vw = vb * kStartV + warp * 32;  // first vector of this warp
+        const uint32_t vw = vb * kStartV + warp * 32;  // first vector of this warp; its 32 are inside n_pad
         if (vw < cl.n) {
             int acc[4][4];
             uint32_t xsq[4];
@@ -201,74 +241,68 @@ __global__ void __launch_bounds__(kStartV) start_dist_kernel(const __grid_consta
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[t][e] = 0;
             }
-            const bool tile_in[4] = {true, vw + 8 < cl.n_pad, vw + 16 < cl.n_pad, vw + 24 < cl.n_pad};
-            // vertical words: k step of 8 words (32 dims); lane holds words gk and gk + 4
-#pragma unroll 2
-            for (uint32_t g = 0; g < lv.qw_hoff; g += 8) {
-                const uint32_t w0 = g + gk, w1 = g + 4 + gk;
-                uint32_t b0[4], b1[4];
+            const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + cl.vert_off) + vw + 4 * gq;
+            const uint4* hor = reinterpret_cast<const uint4*>(sp.arena + cl.hor_off) + (size_t)(vw + 4 * gq) * 4 + gk;
+            const size_t bstride = (size_t)cl.n_pad * 4;  // 16-byte pieces per block
+            // steps of 64 dims: the vertical words, then the horizontal blocks; the next step's loads
+            // are in flight while one is computed
+            const uint32_t nvs = (lv.n_vwords + 15) >> 4, steps = nvs + lv.n_hblocks;
+            auto fetch = [&](uint32_t st, uint4 (&r)[4]) {
+                if (st < nvs) {
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const uint32_t v = vw + 8 * t + gq;
-                    b0[t] = (tile_in[t] && w0 < lv.n_vwords) ? __ldg(vert + (size_t)w0 * cl.n_pad + v) : 0u;
-                    b1[t] = (tile_in[t] && w1 < lv.n_vwords) ? __ldg(vert + (size_t)w1 * cl.n_pad + v) : 0u;
-                }
-                uint32_t a[4];
-                a[0] = w0 < lv.qw_hoff ? qw[gq * qs + w0] : 0u;
-                a[1] = w0 < lv.qw_hoff ? qw[(gq + 8) * qs + w0] : 0u;
-                a[2] = w1 < lv.qw_hoff ? qw[gq * qs + w1] : 0u;
-                a[3] = w1 < lv.qw_hoff ? qw[(gq + 8) * qs + w1] : 0u;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    xsq[t] = __dp4a(b0[t], b0[t], xsq[t]);
-                    xsq[t] = __dp4a(b1[t], b1[t], xsq[t]);
-                    mma_u8_16x8x32(acc[t], a, b0[t], b1[t]);
-                }
-            }
-            // horizontal blocks: 16 words per vector row, two k steps per block
-            for (uint32_t b = 0; b < lv.n_hblocks; ++b) {
-                uint4 x[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const uint32_t v = vw + 8 * t + gq;
-                    const uint32_t* row = reinterpret_cast<const uint32_t*>(hor + ((size_t)b * cl.n_pad + v) * kHDim);
-                    // words gk, 4 + gk, 8 + gk, 12 + gk of the row
-                    x[t] = tile_in[t] ? make_uint4(__ldg(row + gk), __ldg(row + 4 + gk), __ldg(row + 8 + gk),
-                                                   __ldg(row + 12 + gk))
-                                      : make_uint4(0u, 0u, 0u, 0u);
-                }
-                const uint32_t qo = lv.qw_hoff + b * 16;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t a[4];
-                    a[0] = qw[gq * qs + qo + 8 * h + gk];
-                    a[1] = qw[(gq + 8) * qs + qo + 8 * h + gk];
-                    a[2] = qw[gq * qs + qo + 8 * h + 4 + gk];
-                    a[3] = qw[(gq + 8) * qs + qo + 8 * h + 4 + gk];
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const uint32_t b0 = h ? x[t].z : x[t].x, b1 = h ? x[t].w : x[t].y;
-                        xsq[t] = __dp4a(b0, b0, xsq[t]);
-                        xsq[t] = __dp4a(b1, b1, xsq[t]);
-                        mma_u8_16x8x32(acc[t], a, b0, b1);
+                    for (int i = 0; i < 4; ++i) {  // word 16 st + 4 gk + i of the four vectors
+                        const uint32_t w = st * 16 + 4 * gk + i;
+                        r[i] = w < lv.n_vwords ? __ldg(reinterpret_cast<const uint4*>(vert + (size_t)w * cl.n_pad))
+                                               : make_uint4(0u, 0u, 0u, 0u);
                     }
+                } else {
+                    const uint4* src = hor + (st - nvs) * bstride;
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) r[t] = __ldg(src + 4 * t);
+                }
+            };
+            auto compute = [&](uint32_t st, const uint4 (&r)[4]) {
+                const uint32_t qo = st < nvs ? st * 16 : lv.qw_hoff + (st - nvs) * 16;
+                const uint4 a0 = *reinterpret_cast<const uint4*>(qa0 + qo), a1 = *reinterpret_cast<const uint4*>(qa1 + qo);
+                if (st < nvs) {
+                    const uint4 x[4] = {make_uint4(r[0].x, r[1].x, r[2].x, r[3].x), make_uint4(r[0].y, r[1].y, r[2].y, r[3].y),
+                                        make_uint4(r[0].z, r[1].z, r[2].z, r[3].z), make_uint4(r[0].w, r[1].w, r[2].w, r[3].w)};
+                    start_mma_64(acc, xsq, a0, a1, x);
+                } else {
+                    start_mma_64(acc, xsq, a0, a1, r);
+                }
+            };
+            uint4 ra[4], rb[4];
+            fetch(0, ra);
+            for (uint32_t st = 0; st < steps; st += 2) {
+                if (st + 1 < steps) fetch(st + 1, rb);
+                compute(st, ra);
+                if (st + 1 < steps) {
+                    if (st + 2 < steps) fetch(st + 2, ra);
+                    compute(st + 1, rb);
                 }
             }
+            // |x|^2: the four lanes of a row's k-groups hold a quarter each
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                // |x|^2 of vector vw + 8 t + gq: the four lanes of its k-groups hold a quarter each
-                uint32_t xs4 = xsq[t];
-                xs4 += __shfl_xor_sync(0xffffffffu, xs4, 1);
-                xs4 += __shfl_xor_sync(0xffffffffu, xs4, 2);
-                // accumulator layout: acc[0..1] = (row gq, cols 2 gk, 2 gk + 1), acc[2..3] = row gq + 8
+                xsq[t] += __shfl_xor_sync(0xffffffffu, xsq[t], 1);
+                xsq[t] += __shfl_xor_sync(0xffffffffu, xsq[t], 2);
+            }
+            // accumulator layout: acc[t][0..1] = (row gq, columns 2 gk, 2 gk + 1), acc[t][2..3] = row
+            // gq + 8: over the tiles, four adjacent vectors per column
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint32_t j = gq + (e >> 1) * 8;
-                    const uint32_t col = 2 * gk + (e & 1);
-                    const uint32_t vx = vw + 8 * t + col;
-                    const uint32_t xs = __shfl_sync(0xffffffffu, xs4, col * 4);  // lane of vector col
-                    if (j < nqc && vx < cl.n)
-                        sp.dist[(size_t)(r0 + j) * sp.stride + vx] = qsq[j] + xs - 2u * (uint32_t)acc[t][e];
+            for (int e = 0; e < 2; ++e) {
+                uint32_t xs[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) xs[t] = __shfl_sync(0xffffffffu, xsq[t], (2 * gk + e) * 4);
+                const uint32_t vx = vw + 4 * (2 * gk + e);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t j = gq + 8 * h, qq = qsq[j];
+                    if (j < nqc && vx < cl.n)  // rows are a multiple of four long
+                        *reinterpret_cast<uint4*>(sp.dist + (size_t)(r0 + j) * sp.stride + vx) =
+                            make_uint4(qq + xs[0] - 2u * (uint32_t)acc[0][2 * h + e], qq + xs[1] - 2u * (uint32_t)acc[1][2 * h + e],
+                                       qq + xs[2] - 2u * (uint32_t)acc[2][2 * h + e], qq + xs[3] - 2u * (uint32_t)acc[3][2 * h + e]);
                 }
             }
         }
@@ -434,16 +468,20 @@ static bool start_f32_vec(const StartParams& sp) {
 
 size_t start_dist_smem(const DevLevel& lv) {
     if (!lv.is_u8) return sizeof(StartF32Smem);
-    return (size_t)kStartQ * (lv.qw_hoff + lv.n_hblocks * 16 + 4) * 4;
+    return (size_t)kStartQ * start_row_words(lv.qw_hoff + lv.n_hblocks * 16) * 4;
 }
 
 cudaError_t launch_start_batched(const StartParams& sp, int grid, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(sp.cl_count, 0, sizeof(uint32_t) * sp.l1.nclusters, st);
     if (e != cudaSuccess) return e;
-    start_count_kernel<<<(sp.nq + 255) / 256, 256, 0, st>>>(sp);
+    start_count_kernel<<<(sp.nq + kCountThreads / 32 - 1) / (kCountThreads / 32), kCountThreads, 0, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     start_plan_kernel<<<1, kPlanThreads, 0, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (sp.nq * sp.visits > kPlanRows) {
+        start_rows_kernel<<<(sp.nq * sp.visits + 255) / 256, 256, 0, st>>>(sp);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     const size_t smem = start_dist_smem(sp.l1);
     if (!sp.l1.is_u8) {
         auto kern = start_f32_vec(sp) ? start_f32_kernel<true> : start_f32_kernel<false>;
