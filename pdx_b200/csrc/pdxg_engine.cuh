@@ -123,6 +123,8 @@ struct Workspace {
     uint64_t foff_cap = 0;
     uint32_t* d_rows = nullptr;
     uint64_t rows_cap = 0;
+    uint64_t* d_rows64 = nullptr;  // row ids of a filtered host batch
+    uint64_t rows64_cap = 0;
     // tensor-core rotation: TF32 hi / lo planes of the (normalized) queries, GEMM error flag
     float* d_qhi = nullptr;
     float* d_qlo = nullptr;

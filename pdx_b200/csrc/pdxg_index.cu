@@ -236,7 +236,7 @@ void free_workspace(Workspace& w) {
                     w.d_top_lists, w.d_top_count, w.d_top_vals, w.d_l1_order, w.d_l1_count,
                     w.d_st_cl, w.d_st_q, w.d_st_items, w.d_st_dist, w.d_pq_b16, w.d_pq_r16, w.d_pq_r8,
                     w.d_pq_r8s, w.d_pq_scores, w.d_pr_keys, w.d_pr_list,
-                    w.d_req, w.d_foff, w.d_rows, w.d_qhi, w.d_qlo, w.d_gemm_err, w.d_sc_qw, w.d_sc_q,
+                    w.d_req, w.d_foff, w.d_rows, w.d_rows64, w.d_qhi, w.d_qlo, w.d_gemm_err, w.d_sc_qw, w.d_sc_q,
                     w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
                     w.d_sc_vi, w.d_sc_hv};
     for (void* q : ptrs) cudaFree(q);
@@ -532,6 +532,14 @@ int load_from_bytes(const uint8_t* buf, uint64_t size, int device, pdxg_index** 
 namespace pdxg {
 namespace host {
 
+static int set_search_threads(pdxg_index* ix, uint32_t nq, int threads, Launch& L) {
+    const int occ = search_occupancy(L.u8, threads, L.p.smem_total);
+    if (occ <= 0) return fail(PDXG_ERR_CAPACITY, "search kernel cannot be resident with this configuration");
+    L.threads = threads;
+    L.grid = (int)std::min<uint64_t>(nq, (uint64_t)occ * ix->num_sms);
+    return PDXG_OK;
+}
+
 int plan_search(pdxg_index* ix, uint32_t nq, uint32_t k, uint32_t n_order, bool any_filter,
                 Launch& L, uint32_t np_flat_max, uint32_t top_max, bool probe_ahead, cudaStream_t st) {
     if (int rc = flush_maintenance(ix, st)) return rc;
@@ -596,11 +604,19 @@ int plan_search(pdxg_index* ix, uint32_t nq, uint32_t k, uint32_t n_order, bool 
     L.u8 = ix->u8;
     int threads = (int)ix->threads;
     if (threads == 0) threads = 128;  // measured fastest on B200 (IVF2 SQ8 1M x 1024)
-    L.threads = threads;
-    const int occ = search_occupancy(L.u8, threads, off);
-    if (occ <= 0) return fail(PDXG_ERR_CAPACITY, "search kernel cannot be resident with this configuration");
-    L.grid = (int)std::min<uint64_t>(nq, (uint64_t)occ * ix->num_sms);
-    return PDXG_OK;
+    return set_search_threads(ix, nq, threads, L);
+}
+
+// Threads per query of the per-query scan when it only runs `n` queries of a batch (the filtered
+// ones, or a batch too small for the cluster-major scan): with at most one or two per SM the
+// visits' latency counts, not the throughput of many CTAs. 16 filtered queries, 32 clusters of 1,000
+// vectors each: 337 us with 128 threads and every slot of a cluster masked and selected from, 235 us
+// with 512 on the selected slots alone; 255 of a serving batch 1356 and 1040 us (256 threads).
+int widen_search(pdxg_index* ix, uint32_t nq, uint32_t n, Launch& L) {
+    if (ix->threads != 0 || n > 2u * (uint32_t)ix->num_sms) return PDXG_OK;
+    const int threads = n <= (uint32_t)ix->num_sms ? 512 : 256;
+    if (search_occupancy(L.u8, threads, L.p.smem_total) <= 0) return PDXG_OK;
+    return set_search_threads(ix, nq, threads, L);
 }
 
 
@@ -1331,6 +1347,7 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
     if ((rc = run_scan_cluster_major(ix, w, nq, L, st, timed))) return rc;
     launches += L.scan_launches;
     ix->last_launches = launches;
+    if ((rc = widen_search(ix, nq, L.p.q_list ? n_filtered : nq, L))) return rc;
     PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
     PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     if (timed) {
@@ -1406,7 +1423,72 @@ int check_index(const pdxg_index* ix) {
 
 namespace {
 
-// Host-buffer search shared by pdxg_search / _with_order / filtered variants.
+// One bit per cluster slot: filter f selects row r when bit pos(r) of cluster(r) is set;
+// passing[f][c] counts distinct selected rows (CreatePredicateEvaluator, index.hpp:436-446). rows
+// holds the row ids numbered r0 .. r1 - 1; filter f's are foff[f] .. foff[f + 1] - 1.
+template <class Row>
+__global__ void build_filters_kernel(const Row* __restrict__ rows, unsigned long long r0, unsigned long long r1,
+                                     const unsigned long long* __restrict__ foff, uint32_t nf,
+                                     const uint32_t* __restrict__ rid_cluster,
+                                     const uint32_t* __restrict__ rid_pos, uint64_t n_rows,
+                                     const DevCluster* __restrict__ clusters, uint32_t words,
+                                     uint32_t ncl, uint32_t* sel, uint32_t* passing) {
+    const uint32_t f = blockIdx.y;
+    if (f >= nf) return;
+    const unsigned long long a = foff[f] > r0 ? foff[f] : r0, b = foff[f + 1] < r1 ? foff[f + 1] : r1;
+    for (unsigned long long i = a + blockIdx.x * blockDim.x + threadIdx.x; i < b;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        const Row r = rows[i - r0];
+        if (r >= n_rows) continue;
+        const uint32_t c = rid_cluster[r];
+        if (c == 0xFFFFFFFFu) continue;
+        const uint32_t pos = rid_pos[r];
+        const uint32_t bit = 1u << (pos & 31);
+        const uint32_t old = atomicOr(sel + (size_t)f * words + clusters[c].sel_word + (pos >> 5), bit);
+        if (!(old & bit)) atomicAdd(passing + (size_t)f * ncl + c, 1u);
+    }
+}
+
+// Row-id lists of a filtered host batch: list f is rows[foff[f] .. foff[f + 1]).
+struct FilterLists {
+    std::vector<int32_t> filter_of;        // [nq] list of each query, -1 none
+    std::vector<unsigned long long> foff;  // [lists + 1]
+    const uint64_t* rows = nullptr;
+};
+
+// Selection bitmaps and passing counts of the lists, built on the GPU from the uploaded row ids,
+// 32 M of them at a time. On the host each id is a random access into the row maps and the bitmap:
+// 1.6 M ids in 16 lists over 1 M rows, 5.5 ms for the search and 2.0 with the upload (0.59 ms) and this.
+int build_filters_device(pdxg_index* ix, Workspace& w, const FilterLists& fl, cudaStream_t st) {
+    if (int rc = flush_maintenance(ix, st)) return rc;  // the device row maps
+    const uint32_t nf = (uint32_t)fl.foff.size() - 1, words = ix->l1.sel_words, n1 = (uint32_t)ix->l1.fc.size();
+    constexpr unsigned long long kChunk = 32ull << 20;
+    const unsigned long long first = fl.foff[0], last = fl.foff[nf];
+    int rc;
+    if ((rc = dev_grow(w.d_foff, w.foff_cap, (uint64_t)nf + 1))) return rc;
+    if ((rc = dev_grow(w.d_rows64, w.rows64_cap, std::max<uint64_t>(std::min(last - first, kChunk), 1)))) return rc;
+    if ((rc = dev_grow(w.d_sel, w.sel_cap, (uint64_t)nf * words))) return rc;
+    if ((rc = dev_grow(w.d_pass, w.pass_cap, (uint64_t)nf * n1))) return rc;
+    PDXG_CUDA(cudaMemcpyAsync(w.d_foff, fl.foff.data(), (size_t)(nf + 1) * 8, cudaMemcpyHostToDevice, st));
+    PDXG_CUDA(cudaMemsetAsync(w.d_sel, 0, (size_t)nf * words * 4, st));
+    PDXG_CUDA(cudaMemsetAsync(w.d_pass, 0, (size_t)nf * n1 * 4, st));
+    unsigned long long max_len = 0;
+    for (uint32_t f = 0; f < nf; ++f) max_len = std::max(max_len, fl.foff[f + 1] - fl.foff[f]);
+    for (unsigned long long r0 = first; r0 < last; r0 += kChunk) {
+        const unsigned long long r1 = std::min(last, r0 + kChunk);
+        PDXG_CUDA(cudaMemcpyAsync(w.d_rows64, fl.rows + r0, (size_t)(r1 - r0) * 8, cudaMemcpyHostToDevice, st));
+        for (uint32_t f0 = 0; f0 < nf; f0 += 65535) {
+            const uint32_t m = std::min(nf - f0, 65535u);
+            const dim3 grid((uint32_t)std::min<unsigned long long>((max_len + 255) / 256, 256), m);
+            build_filters_kernel<<<grid, 256, 0, st>>>(w.d_rows64, r0, r1, w.d_foff + f0, m, ix->d_rid_cluster,
+                                                       ix->d_rid_pos, ix->rid_cluster.size(), ix->d_cl1, words, n1,
+                                                       w.d_sel + (uint64_t)f0 * words, w.d_pass + (uint64_t)f0 * n1);
+            PDXG_CUDA(cudaGetLastError());
+        }
+    }
+    return PDXG_OK;
+}
+
 // Host-buffer search of a plain batch (no order, no filter) with the query upload pipelined:
 // the batch goes up in chunks on a copy stream, each chunk is rotated and runs its tree top
 // level on the compute stream while the next chunk uploads; the batched Start and the scan then
@@ -1491,10 +1573,9 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
     return check_gemm_error(w);
 }
 
+// Host-buffer search shared by pdxg_search / _with_order / filtered variants.
 int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k, uint32_t flags,
-                     const uint32_t* order, uint32_t n_order,
-                     const std::vector<uint32_t>* sel, const std::vector<uint32_t>* pass,
-                     const std::vector<int32_t>* filter_of, uint32_t* ids, float* dists,
+                     const uint32_t* order, uint32_t n_order, const FilterLists* fl, uint32_t* ids, float* dists,
                      uint32_t* counts) {
     if (!queries || !ids || !dists || !counts)
         return fail(PDXG_ERR_INVALID_ARGUMENT, "NULL buffer");
@@ -1503,7 +1584,7 @@ int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t
     if (rc) return rc;
     Workspace& w = ix->ws;
     cudaStream_t st = ix->stream;
-    if (nq >= kPipelineMinQueries && k > 0 && !(order && n_order) && !(sel && !sel->empty()) &&
+    if (nq >= kPipelineMinQueries && k > 0 && !(order && n_order) && !fl &&
         ix->probe_mode == 0 && !(flags & PDXG_COLLECT_STATS) && !(flags & PDXG_TIME_KERNELS))
         return search_host_pipelined(ix, queries, nq, k, flags, ids, dists, counts);
     PDXG_CUDA(cudaMemcpyAsync(w.d_q, queries, sizeof(float) * nq * ix->d, cudaMemcpyHostToDevice, st));
@@ -1519,20 +1600,16 @@ int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t
     const uint32_t* d_pass = nullptr;
     const int32_t* d_fo = nullptr;
     std::vector<uint32_t> filtered;  // queries with a filter
-    if (sel && !sel->empty()) {
+    if (fl) {
         for (uint32_t q = 0; q < nq; ++q)
-            if ((*filter_of)[q] != -1) filtered.push_back(q);
+            if (fl->filter_of[q] != -1) filtered.push_back(q);
         if ((rc = dev_grow(w.d_pr_list, w.pr_list_cap, filtered.size()))) return rc;
         PDXG_CUDA(cudaMemcpyAsync(w.d_pr_list, filtered.data(), filtered.size() * 4, cudaMemcpyHostToDevice, st));
-        if ((rc = dev_grow(w.d_sel, w.sel_cap, sel->size()))) return rc;
-        if ((rc = dev_grow(w.d_pass, w.pass_cap, pass->size()))) return rc;
         uint64_t cap = w.fo_cap;
-        if ((rc = dev_grow(w.d_filter_of, cap, filter_of->size()))) return rc;
+        if ((rc = dev_grow(w.d_filter_of, cap, nq))) return rc;
         w.fo_cap = (uint32_t)cap;
-        PDXG_CUDA(cudaMemcpyAsync(w.d_sel, sel->data(), sel->size() * 4, cudaMemcpyHostToDevice, st));
-        PDXG_CUDA(cudaMemcpyAsync(w.d_pass, pass->data(), pass->size() * 4, cudaMemcpyHostToDevice, st));
-        PDXG_CUDA(cudaMemcpyAsync(w.d_filter_of, filter_of->data(), filter_of->size() * 4,
-                                  cudaMemcpyHostToDevice, st));
+        PDXG_CUDA(cudaMemcpyAsync(w.d_filter_of, fl->filter_of.data(), (size_t)nq * 4, cudaMemcpyHostToDevice, st));
+        if ((rc = build_filters_device(ix, w, *fl, st))) return rc;
         d_sel = w.d_sel;
         d_pass = w.d_pass;
         d_fo = w.d_filter_of;
@@ -1676,8 +1753,7 @@ int pdxg_search(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k, u
                 uint32_t* ids, float* distances, uint32_t* counts) {
     if (int rc = check_index(ix)) return rc;
     std::lock_guard<std::mutex> lock(ix->mu);
-    return search_host_impl(ix, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr, ids,
-                            distances, counts);
+    return search_host_impl(ix, queries, nq, k, flags, nullptr, 0, nullptr, ids, distances, counts);
 }
 
 int pdxg_search_device(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k,
@@ -1846,8 +1922,8 @@ int pdxg_search_with_order(pdxg_index* ix, const float* queries, uint32_t nq, ui
     std::lock_guard<std::mutex> lock(ix->mu);
     const uint32_t saved = ix->nprobe;
     if (ix->tree && ix->nprobe == 0) ix->nprobe = n1;
-    int rc = search_host_impl(ix, queries, nq, k, flags, order, n_order ? n_order : 0, nullptr,
-                              nullptr, nullptr, ids, distances, counts);
+    int rc = search_host_impl(ix, queries, nq, k, flags, order, n_order ? n_order : 0, nullptr, ids, distances,
+                              counts);
     ix->nprobe = saved;
     return rc;
 }
@@ -1858,15 +1934,11 @@ int pdxg_filtered_search_batch(pdxg_index* ix, const float* queries, uint32_t nq
     if (int rc = check_index(ix)) return rc;
     if (!offsets) return fail(PDXG_ERR_INVALID_ARGUMENT, "offsets is NULL");
     std::lock_guard<std::mutex> lock(ix->mu);
-    const uint32_t words = ix->l1.sel_words;
-    const uint32_t ncl = (uint32_t)ix->l1.fc.size();
-    std::vector<int32_t> filter_of(nq, -1);
-    uint32_t nf = 0;
-    for (uint32_t q = 0; q < nq; ++q)
-        if (offsets[q] != UINT64_MAX) filter_of[q] = (int32_t)nf++;
-    std::vector<uint32_t> sel((uint64_t)nf * words, 0), pass((uint64_t)nf * ncl, 0);
+    FilterLists fl;
+    fl.filter_of.assign(nq, -1);
+    fl.rows = row_ids;
     for (uint32_t q = 0; q < nq; ++q) {
-        if (filter_of[q] < 0) continue;
+        if (offsets[q] == UINT64_MAX) continue;
         uint64_t a = offsets[q], b = offsets[q + 1];
         if (b == UINT64_MAX) {
             // next query unfiltered: find the next valid end offset
@@ -1876,15 +1948,13 @@ int pdxg_filtered_search_batch(pdxg_index* ix, const float* queries, uint32_t nq
         }
         if (b < a) return fail(PDXG_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing");
         if (!row_ids && b > a) return fail(PDXG_ERR_INVALID_ARGUMENT, "row_ids is NULL");
-        const uint32_t f = (uint32_t)filter_of[q];
-        build_filter(ix, row_ids + a, b - a, sel.data() + (uint64_t)f * words,
-                     pass.data() + (uint64_t)f * ncl);
+        // lists follow one another: this one's end is the next one's start
+        if (fl.foff.empty()) fl.foff.push_back(a);
+        fl.filter_of[q] = (int32_t)fl.foff.size() - 1;
+        fl.foff.push_back(b);
     }
-    if (nf == 0)
-        return search_host_impl(ix, queries, nq, k, flags, nullptr, 0, nullptr, nullptr, nullptr,
-                                ids, distances, counts);
-    return search_host_impl(ix, queries, nq, k, flags, nullptr, 0, &sel, &pass, &filter_of, ids,
-                            distances, counts);
+    return search_host_impl(ix, queries, nq, k, flags, nullptr, 0, fl.foff.empty() ? nullptr : &fl, ids, distances,
+                            counts);
 }
 
 int pdxg_filtered_search(pdxg_index* ix, const float* query, uint32_t k, const uint64_t* row_ids,
@@ -2125,30 +2195,6 @@ struct pdxg_context {
 
 namespace {
 
-// One bit per cluster slot: filter f selects row r when bit pos(r) of cluster(r) is set;
-// passing[f][c] counts distinct selected rows (CreatePredicateEvaluator, index.hpp:436-446).
-__global__ void build_filters_kernel(const uint32_t* __restrict__ rows,
-                                     const unsigned long long* __restrict__ foff, uint32_t nf,
-                                     const uint32_t* __restrict__ rid_cluster,
-                                     const uint32_t* __restrict__ rid_pos, uint64_t n_rows,
-                                     const DevCluster* __restrict__ clusters, uint32_t words,
-                                     uint32_t ncl, uint32_t* sel, uint32_t* passing) {
-    const uint32_t f = blockIdx.y;
-    if (f >= nf) return;
-    const unsigned long long a = foff[f], b = foff[f + 1];
-    for (unsigned long long i = a + blockIdx.x * blockDim.x + threadIdx.x; i < b;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t r = rows[i];
-        if (r >= n_rows) continue;
-        const uint32_t c = rid_cluster[r];
-        if (c == 0xFFFFFFFFu) continue;
-        const uint32_t pos = rid_pos[r];
-        const uint32_t bit = 1u << (pos & 31);
-        const uint32_t old = atomicOr(sel + (size_t)f * words + clusters[c].sel_word + (pos >> 5), bit);
-        if (!(old & bit)) atomicAdd(passing + (size_t)f * ncl + c, 1u);
-    }
-}
-
 int stage_grow(pdxg_context* ctx, size_t need) {
     if (need <= ctx->h_cap) return PDXG_OK;
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -2294,7 +2340,7 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
         uint64_t max_len = 0;
         for (uint32_t i = 0; i < nf; ++i) max_len = std::max<uint64_t>(max_len, h_foff[i + 1] - h_foff[i]);
         dim3 grid((uint32_t)std::min<uint64_t>((max_len + 255) / 256 + 1, 64), nf);
-        build_filters_kernel<<<grid, 256, 0, st>>>(w.d_rows, w.d_foff, nf, ix->d_rid_cluster, ix->d_rid_pos,
+        build_filters_kernel<<<grid, 256, 0, st>>>(w.d_rows, 0ull, h_foff[nf], w.d_foff, nf, ix->d_rid_cluster, ix->d_rid_pos,
                                                    ix->rid_cluster.size(), ix->d_cl1, words, n1, w.d_sel,
                                                    w.d_pass);
         PDXG_CUDA(cudaGetLastError());
@@ -2340,6 +2386,7 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
         if (any_plain && (rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
     }
     if ((rc = run_scan_cluster_major(ix, w, nq, L, st))) return rc;
+    if ((rc = widen_search(ix, nq, L.p.q_list ? n_filtered : nq, L))) return rc;
     PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
     PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     return PDXG_OK;

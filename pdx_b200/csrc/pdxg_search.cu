@@ -476,15 +476,12 @@ struct LevelOps {
         push_smallest(c, m);
     }
 
-    // searcher.hpp:283-372
-    __device__ void filtered_start(const DevCluster& c, uint32_t k, uint32_t passing) {
+    // searcher.hpp:283-372, over masked distances of every slot.
+    __device__ void filtered_start_masked(const DevCluster& c, uint32_t k, uint32_t passing) {
         zero_dist(c.n);
         const uint32_t nsel = block_compact<T>(
             c.n, [&](uint32_t i, uint32_t) { return selected(c, i); }, [](uint32_t i) { return i; },
             sh.pos, s);
-        count_bytes((unsigned long long)nsel * lv.dh * kElem +
-                    (unsigned long long)((__fdiv_rn((float)passing, (float)c.n) > (1.0f - kSelectivity)) ? c.n : nsel) *
-                        lv.dv * kElem, kStart);
         for (uint32_t b = 0; b < lv.n_hblocks; ++b) horizontal(c, b, nsel, false);
         const float pct = __fdiv_rn((float)passing, (float)c.n);
         if (pct > (1.0f - kSelectivity)) {
@@ -502,19 +499,185 @@ struct LevelOps {
         push_smallest(c, m);
     }
 
+    // The selected positions of the cluster, ascending, into sh.pos; returns their number.
+    __device__ uint32_t select_positions(const DevCluster& c) {
+        const uint32_t words = (c.n + 31) >> 5;
+        for (uint32_t w = threadIdx.x; w < words; w += T) sh.bits[w] = __ldg(fsel + c.sel_word + w);
+        __syncthreads();
+        return compact_bits(c.n);
+    }
+
+    // Full distances of the listed positions into sh.dist, by list index: horizontal blocks first,
+    // then the vertical dims (the order of filtered_start_masked), without a barrier per block and
+    // with several loads of a vector in flight.
+    __device__ void listed_distances(const DevCluster& c, uint32_t npos) {
+        const uint32_t np = c.n_pad, nhb = lv.n_hblocks;
+        const uint32_t lane = lane_id();
+        if constexpr (U8) {
+            const uint32_t sub = lane & 3;
+            for (uint32_t base = 0; base < npos; base += T / 4) {
+                const uint32_t i = base + (threadIdx.x >> 2);
+                const bool active = i < npos;
+                const uint4* row = reinterpret_cast<const uint4*>(p.arena + c.hor_off) + (size_t)(active ? sh.pos[i] : 0u) * 4 + sub;
+                const uint4* qh = reinterpret_cast<const uint4*>(sh.qw + lv.qw_hoff) + sub;
+                uint32_t acc = 0;
+                for (uint32_t b0 = 0; b0 < nhb; b0 += 4) {
+                    uint4 x[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        x[u] = active && b0 + u < nhb ? __ldg(row + (size_t)(b0 + u) * np * 4) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (b0 + u < nhb) {
+                            const uint4 q4 = qh[(b0 + u) * 4];
+                            acc = sqdiff4(q4.x, x[u].x, acc);
+                            acc = sqdiff4(q4.y, x[u].y, acc);
+                            acc = sqdiff4(q4.z, x[u].z, acc);
+                            acc = sqdiff4(q4.w, x[u].w, acc);
+                        }
+                    }
+                }
+                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                if (active && sub == 0) sh.dist[i] = acc;
+            }
+        } else {
+            const uint32_t sub = lane & 7;
+            for (uint32_t base = 0; base < npos; base += T / 8) {
+                const uint32_t i = base + (threadIdx.x >> 3);
+                const bool active = i < npos;
+                const float* row = reinterpret_cast<const float*>(p.arena + c.hor_off) + (size_t)(active ? sh.pos[i] : 0u) * kHDim + sub;
+                const float* qh = sh.qf + lv.dv + sub;
+                float dist = 0.0f;
+                for (uint32_t b0 = 0; b0 < nhb; b0 += 2) {
+                    float x[2][8];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int t = 0; t < 8; ++t)
+                            x[u][t] = active && b0 + u < nhb ? __ldg(row + (size_t)(b0 + u) * np * kHDim + 8 * t) : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        if (b0 + u < nhb) {  // avx2_computers.hpp:47-98, as in horizontal()
+                            float acc = 0.0f;
+#pragma unroll
+                            for (int t = 0; t < 8; ++t) {
+                                const float dd = __fsub_rn(qh[(b0 + u) * kHDim + 8 * t], x[u][t]);
+                                acc = __fmaf_rn(dd, dd, acc);
+                            }
+                            double sm = (double)acc + (double)__shfl_down_sync(0xffffffffu, acc, 4, 8);
+                            sm = sm + __shfl_down_sync(0xffffffffu, sm, 2, 8);
+                            sm = sm + __shfl_down_sync(0xffffffffu, sm, 1, 8);
+                            dist = __fadd_rn(dist, (float)sm);
+                        }
+                    }
+                }
+                if (active && sub == 0) sh.dist[i] = __float_as_uint(dist);
+            }
+        }
+        __syncthreads();
+        const uint32_t* base = vert(c);
+        const uint32_t words = U8 ? (lv.dv + 3) >> 2 : lv.dv;
+        for (uint32_t i = threadIdx.x; i < npos; i += T) {
+            const uint32_t v = sh.pos[i];
+            uint32_t acc = sh.dist[i];
+            for (uint32_t g0 = 0; g0 < words; g0 += 16) {
+                uint32_t x[16];
+#pragma unroll
+                for (int t = 0; t < 16; ++t) x[t] = g0 + t < words ? __ldg(base + (size_t)(g0 + t) * np + v) : 0u;
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    if (g0 + t < words) {
+                        if constexpr (U8) {
+                            acc = sqdiff4(sh.qw[g0 + t], x[t], acc);
+                        } else {
+                            const float dd = __fsub_rn(sh.qf[g0 + t], __uint_as_float(x[t]));
+                            acc = __float_as_uint(__fmaf_rn(dd, dd, __uint_as_float(acc)));
+                        }
+                    }
+                }
+            }
+            sh.dist[i] = acc;
+        }
+        __syncthreads();
+    }
+
+    // searcher.hpp:283-372. Only the selected vectors are touched: positions from the selection
+    // bitmap, their distances, and the best of that list pushed in push_smallest's order. A masked
+    // slot is never among them (U8 sums stay below the mask; a float one at or above it takes the
+    // masked form). Masking, selecting from and pushing over every slot of the cluster, with a
+    // barrier per horizontal block, cost a visit the same whatever the filter passed.
+    __device__ void filtered_start(const DevCluster& c, uint32_t k, uint32_t passing) {
+        const uint32_t nsel = select_positions(c);
+        count_bytes((unsigned long long)nsel * lv.dh * kElem +
+                    (unsigned long long)((__fdiv_rn((float)passing, (float)c.n) > (1.0f - kSelectivity)) ? c.n : nsel) *
+                        lv.dv * kElem, kStart);
+        const uint32_t hs = s.hsize;
+        const uint32_t m = k - hs < nsel ? k - hs : nsel;
+        if (m == 0) return;
+        listed_distances(c, nsel);
+        uint32_t kth;
+        if (m < nsel) {
+            uint32_t less;
+            block_radix_select<T>(sh.dist, nsel, m, s, kth, less);
+        } else {
+            uint32_t best = 0;
+            for (uint32_t i = threadIdx.x; i < nsel; i += T) best = sh.dist[i] > best ? sh.dist[i] : best;
+            best = __reduce_max_sync(0xffffffffu, best);
+            if (lane_id() == 0) s.warp[warp_id()] = best;
+            __syncthreads();
+            kth = 0;
+#pragma unroll
+            for (int w = 0; w < T / 32; ++w) kth = s.warp[w] > kth ? s.warp[w] : kth;
+            __syncthreads();
+        }
+        if (!U8 && kth >= mask_raw()) {  // block-uniform
+            filtered_start_masked(c, k, passing);
+            return;
+        }
+        const uint32_t* idp = ids(c);
+        const uint32_t lane = lane_id(), warp = warp_id();
+        uint32_t pushed = 0;
+        for (int pass = 0; pass < 2 && pushed < m; ++pass) {
+            for (uint32_t i0 = 0; i0 < nsel; i0 += T) {
+                const uint32_t i = i0 + threadIdx.x;
+                const uint32_t key = i < nsel ? sh.dist[i] : 0u;
+                const bool sel = i < nsel && (pass == 0 ? key < kth : key == kth);
+                const unsigned b = __ballot_sync(0xffffffffu, sel);
+                if (lane == 0) s.warp[warp] = __popc(b);
+                __syncthreads();
+                uint32_t at = pushed + __popc(b & ((1u << lane) - 1u));
+#pragma unroll
+                for (int w = 0; w < T / 32; ++w) {
+                    const uint32_t x = s.warp[w];
+                    at += w < (int)warp ? x : 0u;
+                    pushed += x;
+                }
+                if (sel && at < m) {
+                    sh.hd[hs + at] = reported(key);
+                    sh.hid[hs + at] = __ldg(idp + sh.pos[i]);
+                }
+                __syncthreads();
+            }
+        }
+        if (threadIdx.x == 0) s.hsize = hs + m;
+        __syncthreads();
+        recompute_top();
+    }
+
     // Warmup + Prune + MergeIntoHeap for one cluster with a full heap.
     __device__ void prune_cluster(const DevCluster& c, uint32_t k, uint32_t passing) {
         const uint32_t n = c.n;
         uint32_t cur = 0;
         bool skip_warmup = false;
         if (fsel) {
-            zero_dist(n);
-            const uint32_t mask = mask_raw();
-            for (uint32_t v = threadIdx.x; v < n; v += T)
-                if (!selected(c, v)) sh.dist[v] = mask;
-            __syncthreads();
             const float pct = __fdiv_rn((float)passing, (float)n);
             skip_warmup = pct < (1.0f - kSelectivity);
+            if (!skip_warmup) {  // without a warmup only the selected slots are looked at
+                const uint32_t mask = mask_raw();
+                for (uint32_t v = threadIdx.x; v < n; v += T) sh.dist[v] = selected(c, v) ? 0u : mask;
+                __syncthreads();
+            }
         }
         bool bits_ready = false;  // sh.bits holds the vectors below the bound at `cur`
         // tombstoned slots (unfiltered; a filter never selects them) start the warmup at the
@@ -545,7 +708,8 @@ struct LevelOps {
         uint32_t* dist = sh.dist;
         const LevelOps* self = this;  // captured by the predicate
         const uint32_t nsurv =
-            bits_ready ? compact_bits(n)
+            skip_warmup ? (below(0u, thr) ? select_positions(c) : 0u)
+            : bits_ready ? compact_bits(n)
                        : block_compact<T>(
                              n,
                              [&](uint32_t i, uint32_t) { return self->below(dist[i], thr) && self->selected(c, i); },
@@ -557,7 +721,7 @@ struct LevelOps {
         uint32_t hbytes = 0, vbytes = 0;
         for (uint32_t i = threadIdx.x; i < nsurv; i += T) {
             const uint32_t v = sh.pos[i];
-            uint32_t raw = sh.dist[v];
+            uint32_t raw = skip_warmup ? 0u : sh.dist[v];
             if (follow_survivor(c, v, cur, raw, hbytes, vbytes)) sh.dist[v] = raw;
             else sh.pos[i] = 0xFFFFFFFFu;
         }
