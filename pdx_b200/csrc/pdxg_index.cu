@@ -1291,7 +1291,7 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
         if ((rc = prepare_dev(ix, w, q, nq, w.d_rq, st))) return rc;
         qp = w.d_rq;
         // TF32 split + tensor-core GEMM, or [norms +] SIMT GEMM
-        launches += (ix->rot_tc && ix->rot_mode == 0 && nq > 8) ? 2 : (ix->normalized ? 2 : 1);
+        launches += (ix->rot_tc && ix->rot_mode == 0 && nq > 8) ? 2 : (ix->normalized && nq > 8 ? 2 : 1);
     }
     if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[1], st));
     Launch L;
@@ -1539,7 +1539,7 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
         if (!transformed) {
             if ((rc = prepare_dev(ix, w, qc, n, w.d_rq + (uint64_t)off * d, st))) return rc;
             qc = w.d_rq + (uint64_t)off * d;
-            launches += (ix->rot_tc && ix->rot_mode == 0 && n > 8) ? 2 : (ix->normalized ? 2 : 1);
+            launches += (ix->rot_tc && ix->rot_mode == 0 && n > 8) ? 2 : (ix->normalized && n > 8 ? 2 : 1);
         }
         if (top) {
             Launch Lc = L;
