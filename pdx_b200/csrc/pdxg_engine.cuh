@@ -125,6 +125,10 @@ struct Workspace {
     uint64_t rows_cap = 0;
     uint64_t* d_rows64 = nullptr;  // row ids of a filtered host batch
     uint64_t rows64_cap = 0;
+    // pinned staging of small host batches: queries in, results and GEMM status out
+    uint8_t* h_io = nullptr;
+    uint64_t io_cap = 0;
+    bool io_pending = false;  // copies from or to it may be in flight
     // tensor-core rotation: TF32 hi / lo planes of the (normalized) queries, GEMM error flag
     float* d_qhi = nullptr;
     float* d_qlo = nullptr;

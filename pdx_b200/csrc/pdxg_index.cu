@@ -240,6 +240,7 @@ void free_workspace(Workspace& w) {
                     w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
                     w.d_sc_vi, w.d_sc_hv};
     for (void* q : ptrs) cudaFree(q);
+    if (w.h_io) cudaFreeHost(w.h_io);
     w = Workspace();
 }
 
@@ -1573,6 +1574,65 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
     return check_gemm_error(w);
 }
 
+// Small host batches go through pinned staging: a copy to or from pageable memory waits for the
+// device by itself, so the three results and the GEMM status of one query cost four waits (about
+// 70 of 340 us), the staged ones one. Larger copies gain nothing from the extra pass over them.
+constexpr uint64_t kStageInBytes = 64 << 10, kStageOutBytes = 512 << 10;
+
+int stage_io(Workspace& w, cudaStream_t st) {
+    if (!w.h_io) {
+        PDXG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&w.h_io), kStageInBytes + kStageOutBytes, cudaHostAllocDefault));
+        w.io_cap = kStageInBytes + kStageOutBytes;
+    }
+    // a call that failed midway may have left copies behind
+    if (w.io_pending) PDXG_CUDA(cudaStreamSynchronize(st));
+    w.io_pending = true;
+    return PDXG_OK;
+}
+
+// Queries to the device, results from it (with the wait and the GEMM status).
+int upload_queries(pdxg_index* ix, Workspace& w, const float* queries, uint32_t nq, cudaStream_t st) {
+    const size_t bytes = sizeof(float) * (size_t)nq * ix->d;
+    const void* src = queries;
+    if (bytes <= kStageInBytes) {
+        if (int rc = stage_io(w, st)) return rc;
+        std::memcpy(w.h_io, queries, bytes);
+        src = w.h_io;
+    }
+    PDXG_CUDA(cudaMemcpyAsync(w.d_q, src, bytes, cudaMemcpyHostToDevice, st));
+    return PDXG_OK;
+}
+
+int download_results(Workspace& w, uint32_t nq, uint32_t k, uint32_t* ids, float* dists, uint32_t* counts,
+                     cudaStream_t st) {
+    const size_t nk = (size_t)nq * k * 4, nc = (size_t)nq * 4;
+    if (2 * nk + nc + 4 <= kStageOutBytes) {
+        if (!w.h_io || !w.io_pending)
+            if (int rc = stage_io(w, st)) return rc;
+        uint8_t* h = w.h_io + kStageInBytes;
+        uint8_t *h_d = h + nk, *h_c = h_d + nk, *h_e = h_c + nc;
+        PDXG_CUDA(cudaMemcpyAsync(h, w.d_ids, nk, cudaMemcpyDeviceToHost, st));
+        PDXG_CUDA(cudaMemcpyAsync(h_d, w.d_dists, nk, cudaMemcpyDeviceToHost, st));
+        PDXG_CUDA(cudaMemcpyAsync(h_c, w.d_counts, nc, cudaMemcpyDeviceToHost, st));
+        int err = 0;
+        std::memcpy(h_e, &err, 4);
+        if (w.d_gemm_err) PDXG_CUDA(cudaMemcpyAsync(h_e, w.d_gemm_err, 4, cudaMemcpyDeviceToHost, st));
+        PDXG_CUDA(cudaStreamSynchronize(st));
+        w.io_pending = false;
+        std::memcpy(ids, h, nk);
+        std::memcpy(dists, h_d, nk);
+        std::memcpy(counts, h_c, nc);
+        std::memcpy(&err, h_e, 4);
+        return err ? check_gemm_error(w) : PDXG_OK;
+    }
+    PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, nk, cudaMemcpyDeviceToHost, st));
+    PDXG_CUDA(cudaMemcpyAsync(dists, w.d_dists, nk, cudaMemcpyDeviceToHost, st));
+    PDXG_CUDA(cudaMemcpyAsync(counts, w.d_counts, nc, cudaMemcpyDeviceToHost, st));
+    PDXG_CUDA(cudaStreamSynchronize(st));
+    w.io_pending = false;
+    return check_gemm_error(w);
+}
+
 // Host-buffer search shared by pdxg_search / _with_order / filtered variants.
 int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k, uint32_t flags,
                      const uint32_t* order, uint32_t n_order, const FilterLists* fl, uint32_t* ids, float* dists,
@@ -1587,7 +1647,7 @@ int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t
     if (nq >= kPipelineMinQueries && k > 0 && !(order && n_order) && !fl &&
         ix->probe_mode == 0 && !(flags & PDXG_COLLECT_STATS) && !(flags & PDXG_TIME_KERNELS))
         return search_host_pipelined(ix, queries, nq, k, flags, ids, dists, counts);
-    PDXG_CUDA(cudaMemcpyAsync(w.d_q, queries, sizeof(float) * nq * ix->d, cudaMemcpyHostToDevice, st));
+    if ((rc = upload_queries(ix, w, queries, nq, st))) return rc;
     const uint32_t* d_order = nullptr;
     if (order && n_order) {
         uint64_t cap = w.order_cap;
@@ -1617,11 +1677,7 @@ int search_host_impl(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t
     rc = search_device_impl(ix, w, w.d_q, nq, k, flags, d_order, n_order, d_sel, d_pass, d_fo,
                             w.d_pr_list, (uint32_t)filtered.size(), w.d_ids, w.d_dists, w.d_counts, st);
     if (rc) return rc;
-    PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, sizeof(uint32_t) * nq * k, cudaMemcpyDeviceToHost, st));
-    PDXG_CUDA(cudaMemcpyAsync(dists, w.d_dists, sizeof(float) * nq * k, cudaMemcpyDeviceToHost, st));
-    PDXG_CUDA(cudaMemcpyAsync(counts, w.d_counts, sizeof(uint32_t) * nq, cudaMemcpyDeviceToHost, st));
-    PDXG_CUDA(cudaStreamSynchronize(st));
-    return check_gemm_error(w);
+    return download_results(w, nq, k, ids, dists, counts, st);
 }
 
 }  // namespace
