@@ -195,6 +195,7 @@ struct StartParams {
     uint32_t* items;              // [2 x item bound] (cluster, query chunk << 16 | vector chunk)
     uint32_t* n_items;            // [1]
     uint32_t* queue;              // [1] work counter
+    uint32_t* n_rows;             // [1] Starts planned
     uint32_t* dist;               // [nq x visits rows x stride] distances (U8 integers / float bits)
     uint32_t stride;              // >= largest L1 cluster
 };
@@ -218,6 +219,8 @@ struct ScanParams {
     const uint32_t* start_first;  // [nq x start_visits] the clusters of those rows
     uint32_t start_visits;
     const uint32_t* full_at;      // [nq] position in the order of the Start that fills the heap, ~0u none
+    const uint32_t* by_start;     // optional: the queries with a Start, grouped by its cluster (the replay's
+    const uint32_t* n_by_start;   // order), and their number
     uint32_t* start_dist;         // [rows x start_stride]; a query's row is its scratch afterwards
     uint32_t start_stride;
     uint32_t cp1;                 // first warmup checkpoint: min(16, d_v)
@@ -231,7 +234,7 @@ struct ScanParams {
     float* heap_d;                // [nq x k] the Start's pushes, in push order
     uint32_t* heap_id;
     uint32_t* left;               // [nq] queries left to the per-query scan kernel
-    uint32_t* left_n;             // [1] (zeroed before; n_items and hv_alloc follow it)
+    uint32_t* left_n;             // [1] (zeroed before; n_items, hv_alloc, hv_next, hv_done, hv_full follow)
     uint32_t* vl_count;           // [n1] visits per cluster (zeroed before)
     uint32_t* vl;                 // [n1 x nq] visits of each cluster: q * q_order_stride + i
     uint32_t* items;              // [2 x item bound] (cluster, first list entry of a chunk)
@@ -241,12 +244,17 @@ struct ScanParams {
     uint32_t bm_words;            // ceil(largest cluster / 32)
     uint32_t bm_tile;             // 1: a work item's bitmaps are kept in shared memory first
     uint32_t* vinfo;              // [nq x q_order_stride] class of each visit: 0 no candidate, n > 0
-                                  // candidates in bm, 1 << 31 heavy (no bitmap)
+                                  // candidates in bm, 1 << 31 | x heavy (x: 1 + first column / 32, 0
+                                  // none; no bitmap)
     // heavy visits: values per (vector, warmup checkpoint) and (vector, horizontal block)
     uint32_t* hv;                 // [hv_ncp + n_hblocks][hv_cap]
     uint32_t hv_cap;              // columns (a multiple of 32)
     uint32_t hv_ncp;              // warmup checkpoints
     uint32_t* hv_alloc;           // [1] columns handed out, in units of 32 (zeroed before)
+    uint32_t* hv_full;            // [hv_cap] full distances (zeroed before)
+    uint32_t* hv_blk;             // [2 x hv_cap / 32] visit (~0u none) and 32-vector block of each
+    uint32_t* hv_next;            // [1] work units claimed, and
+    uint32_t* hv_done;            // [1] completed (zeroed before)
     uint32_t* out_ids;            // [nq x k]
     float* out_dists;             // [nq x k]
     uint32_t* out_counts;         // [nq]

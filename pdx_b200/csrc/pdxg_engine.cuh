@@ -134,8 +134,8 @@ struct Workspace {
     float* d_qlo = nullptr;
     uint64_t qhi_cap = 0, qlo_cap = 0;
     int* d_gemm_err = nullptr;
-    // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq + 3]:
-    // first_i | lim | left | left_n, n_items, hv_alloc), Start heaps, per-cluster visit lists and
+    // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq + 5
+    // + hv_cap]: first_i | lim | left | left_n, n_items, hv_alloc, hv_next, hv_done | hv_full), Start heaps, per-cluster visit lists and
     // counters, work items, candidate bitmaps
     uint32_t* d_sc_qw = nullptr;
     uint64_t sc_qw_cap = 0;
@@ -156,6 +156,8 @@ struct Workspace {
     uint64_t sc_vi_cap = 0;
     uint32_t* d_sc_hv = nullptr;
     uint64_t sc_hv_cap = 0;
+    uint32_t* d_sc_hb = nullptr;
+    uint64_t sc_hb_cap = 0;
 };
 
 // Mutable state of a tree index once Append / Delete have been used (PDXTreeIndex,
@@ -205,6 +207,8 @@ struct Launch {
     uint32_t top_launches = 0;  // kernels of a separate tree top level
     uint32_t scan_launches = 0;  // kernels of the cluster-major scan ahead of the per-query kernel
     const uint32_t* start_full_at = nullptr;  // batched Start: where each query's heap is full
+    const uint32_t* start_by_cluster = nullptr;  // batched Start: its queries grouped by cluster, their
+    const uint32_t* start_n_rows = nullptr;      // number (one Start per query only)
     uint32_t start_launches = 0;  // kernels of the batched Start
     uint32_t probe_launches = 0;  // kernels of the reduced-precision probe (rotation included)
 };

@@ -238,7 +238,7 @@ void free_workspace(Workspace& w) {
                     w.d_pq_r8s, w.d_pq_scores, w.d_pr_keys, w.d_pr_list,
                     w.d_req, w.d_foff, w.d_rows, w.d_rows64, w.d_qhi, w.d_qlo, w.d_gemm_err, w.d_sc_qw, w.d_sc_q,
                     w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
-                    w.d_sc_vi, w.d_sc_hv};
+                    w.d_sc_vi, w.d_sc_hv, w.d_sc_hb};
     for (void* q : ptrs) cudaFree(q);
     if (w.h_io) cudaFreeHost(w.h_io);
     w = Workspace();
@@ -1119,7 +1119,7 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     if (occ <= 0) return PDXG_OK;
     int rc;
     if ((rc = dev_grow(w.d_st_cl, w.st_cl_cap, (uint64_t)3 * n1))) return rc;
-    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + 2ull * nq + 2))) return rc;
+    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + 2ull * nq + 3))) return rc;
     const uint32_t nwords = L.p.l1.qw_hoff + L.p.l1.n_hblocks * 16;
     if (ix->u8 && (rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
     if ((rc = dev_grow(w.d_st_items, w.st_items_cap, 2 * items))) return rc;
@@ -1146,7 +1146,8 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     sp.full_at = w.d_st_q + 4 * ne;
     sp.n_items = w.d_st_q + 4 * ne + nq;
     sp.queue = w.d_st_q + 4 * ne + nq + 1;
-    sp.qsq = w.d_st_q + 4 * ne + nq + 2;
+    sp.n_rows = w.d_st_q + 4 * ne + nq + 2;
+    sp.qsq = w.d_st_q + 4 * ne + nq + 3;
     sp.nwords = nwords;
     sp.qwords = w.d_sc_qw;
     sp.items = w.d_st_items;
@@ -1159,6 +1160,8 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     L.p.start_stride = stride;
     L.p.start_visits = visits;
     L.start_full_at = sp.full_at;
+    L.start_by_cluster = visits == 1 ? sp.sorted_q : nullptr;
+    L.start_n_rows = sp.n_rows;
     L.start_launches = ne > 1024 ? 4 : 3;
     return PDXG_OK;
 }
@@ -1187,9 +1190,9 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.r_warp_bytes = (uint32_t)(align_up((uint64_t)nwords * 4, 16) + 8ull * sp.r_heap_cap + sp.r_area_bytes +
                                  align_up((uint64_t)bm_words * 4, 16) + 8ull * sp.r_surv_cap);
     sp.p_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + ix->num_sms - 1) / ix->num_sms);
-    // a replay CTA of 8 warps takes as few queries as still fill the GPU at 3 CTAs per SM, so that
-    // the heavy visits of a small batch are shared by more warps
-    sp.r_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + 3 * ix->num_sms - 1) / (3 * ix->num_sms));
+    // a replay CTA of 8 warps takes as few queries as still fill the GPU at 2 CTAs per SM: all its
+    // warps share the heavy visits
+    sp.r_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + 2 * ix->num_sms - 1) / (2 * ix->num_sms));
     if ((uint64_t)sp.r_warp_bytes * scan_queries_per_cta() + 2048 > ix->max_smem) return PDXG_OK;
     const uint64_t items = scan_item_bound(nq, stride, n1, std::max(lv.max_n, 1u));
     if (items > 0x7FFFFFFFull) return PDXG_OK;
@@ -1204,7 +1207,8 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     int rc;
     if ((rc = dev_grow(w.d_sc_hv, w.sc_hv_cap, hv_rows * sp.hv_cap))) return rc;
     if ((rc = dev_grow(w.d_sc_vi, w.sc_vi_cap, (uint64_t)nq * stride))) return rc;
-    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 3))) return rc;
+    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 5 + sp.hv_cap))) return rc;
+    if ((rc = dev_grow(w.d_sc_hb, w.sc_hb_cap, std::max<uint64_t>(sp.hv_cap / 16, 1)))) return rc;
     if ((rc = dev_grow(w.d_sc_heap, w.sc_heap_cap, 2ull * nq * k))) return rc;
     if ((rc = dev_grow(w.d_sc_cl, w.sc_cl_cap, (uint64_t)n1))) return rc;
     if ((rc = dev_grow(w.d_sc_vl, w.sc_vl_cap, (uint64_t)n1 * nq))) return rc;
@@ -1225,6 +1229,8 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.start_first = L.p.start_first;
     sp.start_visits = L.p.start_visits;
     sp.full_at = L.start_full_at;
+    sp.by_start = L.start_by_cluster;
+    sp.n_by_start = L.start_n_rows;
     sp.start_dist = const_cast<uint32_t*>(L.p.start_dist);
     sp.start_stride = L.p.start_stride;
     sp.cp1 = std::min(16u, lv.dv);
@@ -1239,6 +1245,10 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.hv_alloc = w.d_sc_q + 3ull * nq + 2;
     sp.item_bound = (uint32_t)items;
     sp.hv = w.d_sc_hv;
+    sp.hv_next = w.d_sc_q + 3ull * nq + 3;
+    sp.hv_done = w.d_sc_q + 3ull * nq + 4;
+    sp.hv_full = w.d_sc_q + 3ull * nq + 5;
+    sp.hv_blk = w.d_sc_hb;
     sp.vinfo = w.d_sc_vi;
     sp.bm_tile = scan_bitmap_smem(bm_words) ? 1u : 0u;
     sp.heap_d = reinterpret_cast<float*>(w.d_sc_heap);

@@ -32,9 +32,9 @@
 //                        F32 in TF32 with a margin for its error, so the candidates are a superset
 //                        of that set); each visit is classed as empty (no candidate), light (its bitmap kept) or
 //                        heavy (so many candidates that its warmup may pass the first step)
-//   scan_replay_kernel : warp per query -- Warmup / Prune / MergeIntoHeap / result, over the
-//                        visits that are not empty; the heavy visits of a CTA's queries are
-//                        first computed by all its warps together
+//   scan_replay_kernel : the values of all heavy visits, shared out over the GPU's warps; then warp
+//                        per query -- Warmup / Prune / MergeIntoHeap / result, over the visits that
+//                        are not empty
 #include <cfloat>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -51,8 +51,11 @@ constexpr int kBitmapThreads = 128;
 constexpr int kScanWarps = 8;            // queries per prep / replay CTA
 constexpr uint32_t kOffPath = 0xFFFFFFFFu;
 constexpr uint32_t kHeavyBit = 0x80000000u;  // visit class: 0 empty, candidates of a light visit,
-                                             // kHeavyBit a heavy one
-constexpr uint32_t kHeavyList = 64;      // heavy visits a replay CTA computes ahead
+                                             // kHeavyBit | 1 + its first column / 32 in hv (0: no
+                                             // room) a heavy one
+constexpr uint32_t kHeavyPolls = 1u << 20;  // bound of the wait for the heavy values
+template <bool U8>
+constexpr uint32_t kHeavyBlocks = 2;  // horizontal blocks of a heavy work unit
 constexpr uint32_t kBitmapTileMax = 64 * 1024;  // bytes of a work item's bitmaps in shared memory
 
 // DIMENSIONS_FETCHING_SIZES (common.hpp:47-49)
@@ -629,7 +632,22 @@ __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __gri
         const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
         if (threadIdx.x < nqc) {
             const uint32_t cnt = qcnt[threadIdx.x];
-            const uint32_t info = (sp.cp1 < lv.dv && n - cnt < needed) ? kHeavyBit : cnt;
+            uint32_t info = cnt;
+            if (sp.cp1 < lv.dv && n - cnt < needed) {
+                // columns are handed out in units of 32; none is asked for once they are used up, so
+                // the counter stays far from its range
+                info = kHeavyBit;
+                const uint32_t cap = sp.hv_cap / 32;
+                if (__ldcg(sp.hv_alloc) < cap) {
+                    const uint32_t col = atomicAdd(sp.hv_alloc, nb);
+                    const bool fits = col + nb <= cap;
+                    if (fits) info |= col + 1;
+                    for (uint32_t b = 0; b < nb && col + b < cap; ++b) {
+                        sp.hv_blk[2 * (col + b)] = fits ? qe[threadIdx.x] : 0xFFFFFFFFu;
+                        sp.hv_blk[2 * (col + b) + 1] = b;
+                    }
+                }
+            }
             sp.vinfo[qe[threadIdx.x]] = info;
             qcnt[threadIdx.x] = info;
         }
@@ -733,67 +751,6 @@ __device__ __forceinline__ uint32_t scan_bits_to_offsets(uint32_t word, uint32_t
     return total;
 }
 
-// Values of vector v of a heavy visit into column `out` (row stride sp.hv_cap): row s < ncp is the
-// running distance at warmup checkpoint s, row ncp + b the sum of horizontal block b. They do not
-// depend on the query's heap, so the loads of 16 vertical words, then of three blocks (F32: one), are
-// in flight together (U8, 2 words and two blocks: 152 against 108 us for the replay of a 777-query
-// batch). Returns the full distance: for F32 that of a warmup over all vertical dims (an earlier exit
-// adds the same terms in another order).
-template <bool U8>
-__device__ __forceinline__ uint32_t heavy_column(const ScanParams& sp, const DevCluster& c, const uint32_t* qw,
-                                                 uint32_t v, uint32_t* out) {
-    const DevLevel& lv = sp.l1;
-    const uint32_t* col = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off) + v;
-    const uint32_t groups = Raw<U8>::word(lv.dv);
-    uint32_t raw = 0, s = 0, next = sp.cp1;
-    for (uint32_t g0 = 0; g0 < groups; g0 += 16) {
-        uint32_t x[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) x[t] = g0 + t < groups ? __ldg(col + (size_t)(g0 + t) * c.n_pad) : 0u;
-#pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            if (g0 + t < groups) {
-                raw = Raw<U8>::step(qw[g0 + t], x[t], raw);
-                if ((g0 + t + 1) * (U8 ? 4 : 1) >= next) {  // checkpoints are multiples of 16 dims, the last is d_v
-                    out[(size_t)s * sp.hv_cap] = raw;
-                    ++s;
-                    next += c_scan_fetch[s < kNumFetchSizes ? s : kNumFetchSizes - 1];
-                    if (next > lv.dv) next = lv.dv;
-                }
-            }
-        }
-    }
-    out += (size_t)sp.hv_ncp * sp.hv_cap;
-    if constexpr (!U8) {
-        for (uint32_t b = 0; b < lv.n_hblocks; ++b) {
-            const uint32_t sum = hblock_sum<false>(qw + Raw<U8>::hword(lv, b), hblock_row<U8>(sp, c, b, v));
-            out[(size_t)b * sp.hv_cap] = sum;
-            raw = Raw<U8>::add(raw, sum);
-        }
-        return raw;
-    }
-    for (uint32_t b0 = 0; b0 < lv.n_hblocks; b0 += 3) {
-        uint4 x[3][4];
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                x[u][t] = b0 + u < lv.n_hblocks ? __ldg(hblock_row<U8>(sp, c, b0 + u, v) + t) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-            if (b0 + u < lv.n_hblocks) {
-                const uint4* qh = reinterpret_cast<const uint4*>(qw + lv.qw_hoff + (b0 + u) * 16);
-                uint32_t sum = 0;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) sum = sq16(qh[t], x[u][t], sum);
-                out[(size_t)(b0 + u) * sp.hv_cap] = sum;
-                raw += sum;
-            }
-        }
-    }
-    return raw;
-}
-
 // Whether a vector with full distance `full` may stay below bound `thr` at all d dims. F32 leaves
 // room for another order of the sum: its d + 1 non-negative terms are each rounded at most d + 2
 // times by 2^-24 in either order (2^-22 d is twice the difference that allows).
@@ -805,30 +762,131 @@ __device__ __forceinline__ bool may_stay_below(uint32_t full, uint32_t thr, uint
 }
 
 // A heavy visit needs the running distance of all its vectors at up to every warmup checkpoint and
-// then a long survivor path for most of them. Done by the query's own warp at the visit's turn that
-// is a chain of several hundred dependent loads: 1-2 % of the queries of a 777-query batch on the
-// 1M x 1024 SQ8 tree took about 400 us there and set the kernel's time. Here the CTA's warps first
-// share out the 32-vector blocks of its queries' heavy visits (HeavyList), and the replay reads the
-// values; a visit that finds no room in the list or in sp.hv runs its warmup in the warp.
-// A vector can only be merged when its full distance is below the bound at all d dims, at most
-// that of the heap top after the Start: those vectors are marked in the visit's bitmap, and a
-// visit without any changes nothing.
-struct HeavyList {
-    uint32_t n;
-    uint32_t warp[kHeavyList], visit[kHeavyList];
-    uint32_t base[kHeavyList];  // first column / 32 in sp.hv
-    uint32_t end[kHeavyList];   // 32-vector blocks of the list up to and with this visit
-    uint32_t thr0[kScanWarps];  // bound at all d dims of each warp's heap top after the Start
-};
+// then a long survivor path for most of them. These values do not depend on the query's heap: row
+// s < ncp of a vector's column in hv is its running distance at warmup checkpoint s, row ncp + b the
+// sum of horizontal block b, and hv_full their sum over all dims. One query in eight has such a visit
+// (1M x 1024 SQ8 tree) but the few with three of them set the time when their own CTA computed them
+// (a walk ends after 10 us on average, the last after 77), so every 32-vector block of every
+// heavy visit is split into units -- its vertical chain, and a few horizontal blocks each -- that all
+// warps of the grid share. Replay of 777 queries 79 -> 48 us, of 10,000 137 -> 103, F32 2,000 queries
+// on 200,000 x 768 225 -> 150, 300 exhaustive ones 170 -> 117.
+// Units are claimed from a counter, so each is run by a warp that is on the GPU, and a walk that needs
+// the values (heavy_ready) waits for units that are running; it gives up after a bounded number of
+// polls and then runs its warmups itself.
+// hv_full adds the units in any order: exact for U8; F32 readers allow for it (may_stay_below).
+template <bool U8>
+__device__ __forceinline__ void heavy_unit(const ScanParams& sp, uint32_t cb, uint32_t part) {
+    const DevLevel& lv = sp.l1;
+    const uint32_t lane = threadIdx.x & 31, nhb = lv.n_hblocks;
+    const uint32_t e = sp.hv_blk[2 * cb], v = sp.hv_blk[2 * cb + 1] * 32 + lane;
+    if (e == 0xFFFFFFFFu) return;
+    const DevCluster c = lv.clusters[__ldg(sp.q_order + e)];
+    if (v < c.n) {
+        const uint32_t* qw = sp.qwords + (size_t)(e / sp.q_order_stride) * sp.nwords;
+        uint32_t* out = sp.hv + ((size_t)cb << 5) + lane;
+        uint32_t sum = 0;
+        if (part == 0) {
+            const uint32_t* col = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off) + v;
+            const uint32_t groups = Raw<U8>::word(lv.dv);
+            constexpr int NL = U8 ? 16 : 32;  // words in flight
+            uint32_t s = 0, next = sp.cp1;
+            for (uint32_t g0 = 0; g0 < groups; g0 += NL) {
+                uint32_t x[NL];
+#pragma unroll
+                for (int t = 0; t < NL; ++t) x[t] = g0 + t < groups ? __ldg(col + (size_t)(g0 + t) * c.n_pad) : 0u;
+#pragma unroll
+                for (int t = 0; t < NL; ++t) {
+                    if (g0 + t < groups) {
+                        sum = Raw<U8>::step(__ldg(qw + g0 + t), x[t], sum);
+                        if ((g0 + t + 1) * (U8 ? 4 : 1) >= next) {  // checkpoints: multiples of 16 dims, then d_v
+                            out[(size_t)s * sp.hv_cap] = sum;
+                            ++s;
+                            next += c_scan_fetch[s < kNumFetchSizes ? s : kNumFetchSizes - 1];
+                            if (next > lv.dv) next = lv.dv;
+                        }
+                    }
+                }
+            }
+        } else {
+            const uint32_t b0 = (part - 1) * kHeavyBlocks<U8>;
+            out += (size_t)(sp.hv_ncp + b0) * sp.hv_cap;
+            constexpr int NB = (int)kHeavyBlocks<U8>;
+            if constexpr (U8) {
+                uint4 x[NB][4];
+#pragma unroll
+                for (int k = 0; k < NB; ++k)
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+                        x[k][t] = b0 + k < nhb ? __ldg(hblock_row<U8>(sp, c, b0 + k, v) + t) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    if (b0 + k < nhb) {
+                        const uint4* qh = reinterpret_cast<const uint4*>(qw + Raw<U8>::hword(lv, b0 + k));
+                        uint32_t h = 0;
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) h = sq16(__ldg(qh + t), x[k][t], h);
+                        out[(size_t)k * sp.hv_cap] = h;
+                        sum += h;
+                    }
+                }
+            } else {
+                for (uint32_t k = 0; k < NB && b0 + k < nhb; ++k) {
+                    const uint32_t h = hblock_sum<U8>(qw + Raw<U8>::hword(lv, b0 + k), hblock_row<U8>(sp, c, b0 + k, v));
+                    out[(size_t)k * sp.hv_cap] = h;
+                    sum = Raw<U8>::add(sum, h);
+                }
+            }
+        }
+        uint32_t* full = sp.hv_full + ((size_t)cb << 5) + lane;
+        if constexpr (U8) atomicAdd(full, sum);
+        else atomicAdd(reinterpret_cast<float*>(full), __uint_as_float(sum));
+    }
+}
+
+// Runs claimed units until none is left; returns their number.
+template <bool U8>
+__device__ __forceinline__ uint32_t heavy_units(const ScanParams& sp) {
+    const uint32_t cap = sp.hv_cap / 32, got = sp.hv_alloc[0];
+    const uint32_t blocks = got < cap ? got : cap;
+    const uint32_t parts = 1 + (sp.l1.n_hblocks + kHeavyBlocks<U8> - 1) / kHeavyBlocks<U8>;
+    const uint32_t total = blocks * parts;
+    const uint32_t chunk = total > 8192u ? 4u : 1u;  // fewer claims where the units are many
+    for (;;) {
+        uint32_t u = 0;
+        if (total && (threadIdx.x & 31) == 0) u = atomicAdd(sp.hv_next, chunk);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u >= total) return total;
+        const uint32_t end = u + chunk < total ? u + chunk : total;
+        for (uint32_t x = u; x < end; ++x) heavy_unit<U8>(sp, x % blocks, x / blocks);
+        __threadfence();  // every lane's values before the warp's count
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) atomicAdd(sp.hv_done, end - u);
+    }
+}
+
+// Whether all `total` units are done, after a bounded wait.
+__device__ __forceinline__ bool heavy_ready(const ScanParams& sp, uint32_t total) {
+    uint32_t done = 0;
+    for (uint32_t i = 0; i < kHeavyPolls; ++i) {
+        done = *reinterpret_cast<volatile uint32_t*>(sp.hv_done);
+        if (done >= total) break;
+        __nanosleep(100);
+    }
+    __threadfence();
+    return __all_sync(0xffffffffu, done >= total);
+}
 
 template <bool U8>
 __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kernel(const __grid_constant__ ScanParams sp) {
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ HeavyList HL;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // warps past r_qpc own no query (no shared-memory region either) and only share the heavy visits
-    const uint32_t q = blockIdx.x * sp.r_qpc + warp;
-    const uint32_t fi = warp < sp.r_qpc && q < sp.nq ? sp.first_i[q] : kOffPath;
+    // Queries that start in the same cluster visit the same ones next: they run at the same time, in
+    // neighbouring CTAs, and find those clusters in L2.
+    // warps past r_qpc own no query (no shared-memory region either) and only run heavy units
+    const uint32_t units = heavy_units<U8>(sp);
+    uint32_t q = warp < sp.r_qpc ? blockIdx.x + warp * gridDim.x : 0xFFFFFFFFu;
+    if (sp.by_start) q = q < sp.nq && q < __ldg(sp.n_by_start) ? __ldg(sp.by_start + q) : 0xFFFFFFFFu;
+    const uint32_t fi = q < sp.nq ? sp.first_i[q] : kOffPath;
     const DevLevel& lv = sp.l1;
     uint8_t* base = smem + (size_t)warp * sp.r_warp_bytes;
     ReplayWarp R;
@@ -847,58 +905,14 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
     const uint32_t cnt = fi == kOffPath ? 0u : __ldg(sp.q_order_count + q);
     float top = 0.0f;
     uint32_t slot = 0;
-    if (threadIdx.x == 0) HL.n = 0;
-    __syncthreads();
-    if (fi != kOffPath) {
-        for (uint32_t w = lane; w < sp.nwords; w += 32) R.qw[w] = __ldg(sp.qwords + (size_t)q * sp.nwords + w);
-        for (uint32_t j = lane; j < kq; j += 32) {
-            R.hd[j] = __ldg(sp.heap_d + (size_t)q * sp.k + j);
-            R.hid[j] = __ldg(sp.heap_id + (size_t)q * sp.k + j);
-        }
-        __syncwarp();
-        warp_heap_top(R.hd, kq, top, slot);
-        if (lane == 0) HL.thr0[warp] = Raw<U8>::thr(top, lv.d, lv, sp.ratios);
-        for (uint32_t i = fi + 1 + lane; i < cnt; i += 32) {
-            if (!(__ldg(vis + i) & kHeavyBit) || HL.n >= kHeavyList) continue;
-            // columns are handed out in units of 32; none is asked for once they are used up, so the
-            // counter stays far from its range
-            if (__ldcg(sp.hv_alloc) >= sp.hv_cap / 32) continue;
-            const uint32_t nb = (lv.clusters[__ldg(ord + i)].n + 31) >> 5;
-            const uint32_t col = atomicAdd(sp.hv_alloc, nb);
-            if (col + nb > sp.hv_cap / 32) continue;
-            const uint32_t at = atomicAdd(&HL.n, 1u);
-            if (at >= kHeavyList) continue;
-            HL.warp[at] = warp;
-            HL.visit[at] = i;
-            HL.base[at] = col;
-            HL.end[at] = nb;
-        }
+    if (fi == kOffPath) return;  // whole warp; there is no block-wide barrier
+    for (uint32_t w = lane; w < sp.nwords; w += 32) R.qw[w] = __ldg(sp.qwords + (size_t)q * sp.nwords + w);
+    for (uint32_t j = lane; j < kq; j += 32) {
+        R.hd[j] = __ldg(sp.heap_d + (size_t)q * sp.k + j);
+        R.hid[j] = __ldg(sp.heap_id + (size_t)q * sp.k + j);
     }
-    __syncthreads();
-    const uint32_t n_heavy = HL.n < kHeavyList ? HL.n : kHeavyList;
-    if (n_heavy) {  // block-uniform
-        if (threadIdx.x == 0)
-            for (uint32_t j = 1; j < n_heavy; ++j) HL.end[j] += HL.end[j - 1];
-        __syncthreads();
-        uint32_t j = 0;
-        for (uint32_t b = warp; b < HL.end[n_heavy - 1]; b += kScanWarps) {
-            while (HL.end[j] <= b) ++j;
-            const uint32_t blk = b - (j ? HL.end[j - 1] : 0u);
-            const uint32_t hw = HL.warp[j];
-            const uint32_t hq = blockIdx.x * sp.r_qpc + hw;
-            const DevCluster c = lv.clusters[__ldg(sp.q_order + (size_t)hq * stride + HL.visit[j])];
-            const uint32_t v = blk * 32 + lane;
-            uint32_t full = 0xFFFFFFFFu;
-            if (v < c.n)
-                full = heavy_column<U8>(sp, c, reinterpret_cast<const uint32_t*>(smem + (size_t)hw * sp.r_warp_bytes), v,
-                                    sp.hv + ((size_t)(HL.base[j] + blk) << 5) + lane);
-            // statistics count the blocks of vectors that end up pruned too
-            const unsigned may = __ballot_sync(0xffffffffu, v < c.n && (sp.stats || may_stay_below<U8>(full, HL.thr0[hw], lv.d)));
-            if (lane == 0) sp.bm[((size_t)hq * stride + HL.visit[j]) * sp.bm_words + blk] = may;
-        }
-        __syncthreads();
-    }
-    if (fi == kOffPath) return;  // whole warp; no block-wide barrier follows
+    __syncwarp();
+    warp_heap_top(R.hd, kq, top, slot);
     uint32_t* scratch = sp.start_dist + (size_t)__ldg(sp.start_row + (size_t)q * sp.start_visits) * sp.start_stride;
     const uint32_t S = sp.r_surv_cap;
     unsigned long long b_warm = 0, b_h = 0, b_v = 0, merged = 0;
@@ -911,21 +925,21 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
     auto merge = [&](const DevCluster& c, bool alive, uint32_t v, uint32_t raw) {
         const uint32_t idv = alive ? __ldg(reinterpret_cast<const uint32_t*>(sp.arena + c.ids_off) + v) : 0u;
         const float dd = Raw<U8>::reported(raw, lv);
-        unsigned bal = __ballot_sync(0xffffffffu, alive);
-        merged += __popc(bal);
+        merged += __popc(__ballot_sync(0xffffffffu, alive));
+        // the top only falls: a vector that is not below it once never is
+        unsigned bal = __ballot_sync(0xffffffffu, alive && dd < top);
         while (bal) {
             const int l = __ffs(bal) - 1;
-            bal &= bal - 1;
             const float ddl = __shfl_sync(0xffffffffu, dd, l);
             const uint32_t idl = __shfl_sync(0xffffffffu, idv, l);
-            if (ddl < top) {
-                if (lane == 0) {
-                    R.hd[slot] = ddl;
-                    R.hid[slot] = idl;
-                }
-                __syncwarp();
-                warp_heap_top(R.hd, kq, top, slot);
+            if (lane == 0) {
+                R.hd[slot] = ddl;
+                R.hid[slot] = idl;
             }
+            __syncwarp();
+            warp_heap_top(R.hd, kq, top, slot);
+            bal &= bal - 1;
+            bal &= __ballot_sync(0xffffffffu, dd < top);
         }
     };
 
@@ -934,43 +948,77 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
         if (alive) alive = scan_follow<U8>(sp, c, R.qw, v, cur, tp, raw, b_h, b_v);
         merge(c, alive, v, raw);
     };
-    // A heavy visit on its values computed ahead, hv pointing at its first vector's column.
-    // bmh: its mergeable vectors.
-    auto heavy_visit = [&](const DevCluster& c, const uint32_t* hv, const uint32_t* bmh) {
+    // A heavy visit on its values computed ahead; col: its first vector's column. A vector can only be
+    // merged when its full distance is below the bound at all d dims: a visit without any changes
+    // nothing. Its reads are batched, eight blocks' full distances and four steps of four blocks.
+    auto heavy_visit = [&](const DevCluster& c, size_t col) {
         const uint32_t n = c.n, W = (n + 31) >> 5;
-        uint32_t any = 0;
-        for (uint32_t w = lane; w < W; w += 32) any |= bmh[w];
-        if (!__any_sync(0xffffffffu, any != 0)) return;
-        const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
+        const uint32_t* hv = sp.hv + col;
+        const uint32_t* full = sp.hv_full + col;
         const float tp = top;  // the bound's heap top, fixed for the whole cluster
-        uint32_t cur = 0, step = 0, n_pruned = 0;
-        while (n_pruned < needed && cur < lv.dv) {  // Warmup (searcher.hpp:374-435)
-            uint32_t last = cur + c_scan_fetch[step < kNumFetchSizes ? step : kNumFetchSizes - 1];
-            if (last > lv.dv) last = lv.dv;
-            const uint32_t thr = Raw<U8>::thr(tp, last, lv, sp.ratios);
-            const uint32_t* row = hv + (size_t)step * sp.hv_cap;
-            uint32_t cntp = 0;
-            for (uint32_t v0 = 0; v0 < n; v0 += 256) {
-                uint32_t x[8];
+        const uint32_t thr_d = Raw<U8>::thr(tp, lv.d, lv, sp.ratios);
+        uint32_t any = 0;
+        for (uint32_t w0 = 0; w0 < W; w0 += 8) {
+            uint32_t x[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const uint32_t v = v0 + 32 * u + lane;
-                    x[u] = v < n ? row[v] : 0u;
-                }
+            for (int u = 0; u < 8; ++u) x[u] = (w0 + u) * 32 + lane < n ? __ldcg(full + (w0 + u) * 32 + lane) : 0u;
 #pragma unroll
-                for (int u = 0; u < 8; ++u) cntp += (v0 + 32 * u + lane < n && Raw<U8>::reached(x[u], thr)) ? 1u : 0u;
+            for (int u = 0; u < 8; ++u) {
+                // statistics count the blocks of vectors that end up pruned too
+                const unsigned may = __ballot_sync(0xffffffffu, (w0 + u) * 32 + lane < n &&
+                                                                    (sp.stats || may_stay_below<U8>(x[u], thr_d, lv.d)));
+                any |= may;
+                if (lane == 0 && w0 + u < W) R.sbits[w0 + u] = may;
             }
-            n_pruned = __reduce_add_sync(0xffffffffu, cntp);
-            if (cur == 0) n_surv += n - n_pruned;
-            else b_warm += (unsigned long long)n * (last - cur) * Raw<U8>::kElem;
-            cur = last;
-            ++step;
+        }
+        if (!any) return;
+        __syncwarp();
+        const uint32_t* bmh = R.sbits;
+        const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
+        uint32_t cur = 0, step = 0, n_pruned = 0;
+        while (n_pruned < needed && cur < lv.dv) {  // Warmup (searcher.hpp:374-435), four steps at a time
+            uint32_t last[4], thr[4], cnt[4];
+            uint32_t at = cur;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                at += c_scan_fetch[step + g < (uint32_t)kNumFetchSizes ? step + g : kNumFetchSizes - 1];
+                if (at > lv.dv) at = lv.dv;
+                last[g] = at;
+                thr[g] = Raw<U8>::thr(tp, at, lv, sp.ratios);
+                cnt[g] = 0;
+            }
+            const uint32_t* row = hv + (size_t)step * sp.hv_cap;
+            for (uint32_t v0 = 0; v0 < n; v0 += 128) {
+                uint32_t x[4][4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const uint32_t v = v0 + 32 * u + lane;
+                        x[g][u] = v < n && step + g < sp.hv_ncp ? __ldcg(row + (size_t)g * sp.hv_cap + v) : 0u;
+                    }
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        cnt[g] += (v0 + 32 * u + lane < n && Raw<U8>::reached(x[g][u], thr[g])) ? 1u : 0u;
+            }
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                if (n_pruned < needed && cur < lv.dv) {
+                    n_pruned = __reduce_add_sync(0xffffffffu, cnt[g]);
+                    if (cur == 0) n_surv += n - n_pruned;
+                    else b_warm += (unsigned long long)n * (last[g] - cur) * Raw<U8>::kElem;
+                    cur = last[g];
+                    ++step;
+                }
+            }
         }
         if (step == 1) ++n_fast;
         else ++n_full;
         // Prune (searcher.hpp:437-540) and merge of the mergeable vectors, 32 at a time in position
-        // order; their horizontal sums are loaded kHeavyBlocks at a time, ahead of their tests
-        constexpr int kHeavyBlocks = 6;
+        // order; their horizontal sums are loaded six at a time, ahead of their tests
+        constexpr int HB = 6;
         const uint32_t thr = Raw<U8>::thr(tp, cur, lv, sp.ratios);
         const uint32_t* erow = hv + (size_t)(step - 1) * sp.hv_cap;
         const uint32_t* brow = hv + (size_t)sp.hv_ncp * sp.hv_cap;
@@ -979,16 +1027,16 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
             for (uint32_t j0 = 0; j0 < total; j0 += 32) {
                 bool alive = j0 + lane < total;
                 const uint32_t v = alive ? w0 * 32 + R.cand[j0 + lane] : 0u;
-                uint32_t raw = alive ? erow[v] : 0u;
+                uint32_t raw = alive ? __ldcg(erow + v) : 0u;
                 alive = alive && Raw<U8>::below(raw, thr);
                 uint32_t cv = cur;
-                for (uint32_t b0 = 0; b0 < lv.n_hblocks && __any_sync(0xffffffffu, alive); b0 += kHeavyBlocks) {
-                    uint32_t x[kHeavyBlocks];
+                for (uint32_t b0 = 0; b0 < lv.n_hblocks && __any_sync(0xffffffffu, alive); b0 += HB) {
+                    uint32_t x[HB];
 #pragma unroll
-                    for (int u = 0; u < kHeavyBlocks; ++u)
-                        x[u] = (alive && b0 + u < lv.n_hblocks) ? brow[(size_t)(b0 + u) * sp.hv_cap + v] : 0u;
+                    for (int u = 0; u < HB; ++u)
+                        x[u] = (alive && b0 + u < lv.n_hblocks) ? __ldcg(brow + (size_t)(b0 + u) * sp.hv_cap + v) : 0u;
 #pragma unroll
-                    for (int u = 0; u < kHeavyBlocks; ++u) {
+                    for (int u = 0; u < HB; ++u) {
                         if (alive && b0 + u < lv.n_hblocks) {
                             raw = Raw<U8>::add(raw, x[u]);
                             b_h += kHDim * Raw<U8>::kElem;
@@ -1008,10 +1056,16 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
     // vectors reach the bound): only the others are walked. On the 1M x 1024 SQ8 tree a query has
     // one or two of them in 31 visits, and walking all of them was a chain of 31 record and bitmap
     // round trips.
+    uint32_t info_next = 0;
+    {
+        const uint32_t il = ((fi + 1) & ~31u) + lane;
+        if (il > fi && il < cnt) info_next = __ldg(vis + il);
+    }
     for (uint32_t i0 = (fi + 1) & ~31u; i0 < cnt; i0 += 32) {
       const uint32_t il = i0 + lane;
       const bool in = il > fi && il < cnt;
-      uint32_t info_l = in ? __ldg(vis + il) : 0u;
+      const uint32_t info_l = info_next;
+      info_next = il + 32 < cnt ? __ldg(vis + il + 32) : 0u;  // in flight during these visits
       if (sp.stats && in) {
           const uint32_t n = lv.clusters[__ldg(ord + il)].n;
           visits_l += n ? 1u : 0u;
@@ -1022,15 +1076,9 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
         const uint32_t src = __ffs(todo) - 1, i = i0 + src;
         const uint32_t info = __shfl_sync(0xffffffffu, info_l, src);
         const DevCluster c = lv.clusters[__ldg(ord + i)];
-        if (info & kHeavyBit) {
-            uint32_t at = 0xFFFFFFFFu;
-            for (uint32_t j = lane; j < n_heavy; j += 32)
-                if (HL.warp[j] == warp && HL.visit[j] == i) at = j;
-            at = __reduce_min_sync(0xffffffffu, at);
-            if (at != 0xFFFFFFFFu) {
-                heavy_visit(c, sp.hv + ((size_t)HL.base[at] << 5), sp.bm + ((size_t)q * stride + i) * sp.bm_words);
-                continue;
-            }
+        if ((info & kHeavyBit) && (info & ~kHeavyBit) && heavy_ready(sp, units)) {
+            heavy_visit(c, (size_t)((info & ~kHeavyBit) - 1) << 5);
+            continue;
         }
         const uint32_t n = c.n;
         const uint32_t* vert = reinterpret_cast<const uint32_t*>(sp.arena + c.vert_off);
@@ -1226,8 +1274,8 @@ template <bool U8>
 static cudaError_t launch_scan_t(const ScanParams& sp, cudaStream_t st, const cudaEvent_t* ev) {
     cudaError_t e = cudaMemsetAsync(sp.vl_count, 0, sizeof(uint32_t) * sp.l1.nclusters, st);
     if (e != cudaSuccess) return e;
-    // left_n, n_items and hv_alloc are consecutive
-    if ((e = cudaMemsetAsync(sp.left_n, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    // left_n, n_items, hv_alloc, hv_next, hv_done and hv_full are consecutive
+    if ((e = cudaMemsetAsync(sp.left_n, 0, (5 + (size_t)sp.hv_cap) * sizeof(uint32_t), st)) != cudaSuccess) return e;
     const uint32_t ctas = (sp.nq + sp.p_qpc - 1) / sp.p_qpc;
     scan_prep_kernel<U8><<<ctas, sp.p_qpc * 32, 0, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kPlanThreads) start_plan_kernel(const __grid_c
         sp.cl_items[c] = L ? ((L + iq - 1) / iq) * ((nv + iv - 1) / iv) : 0u;
     }
     __syncthreads();
-    cta_exclusive_scan(sp.cl_off, n1, warp_tot);
+    const uint32_t total_rows = cta_exclusive_scan(sp.cl_off, n1, warp_tot);
     const uint32_t total_items = cta_exclusive_scan(sp.cl_items, n1, warp_tot);
     if (sp.nq * sp.visits <= kPlanRows)
         for (uint32_t e = threadIdx.x; e < sp.nq * sp.visits; e += kPlanThreads) start_row(sp, e);
@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(kPlanThreads) start_plan_kernel(const __grid_c
     }
     if (threadIdx.x == 0) {
         sp.n_items[0] = total_items;
+        sp.n_rows[0] = total_rows;
         sp.queue[0] = 0;
     }
 }
