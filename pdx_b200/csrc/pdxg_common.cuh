@@ -184,6 +184,8 @@ struct StartParams {
     uint32_t* qwords;             // U8: [nq x nwords] quantized queries, packed as the scan packs them
     uint32_t* qsq;                // U8: [nq] their |q|^2
     uint32_t* cl_count;           // [n1] Starts per cluster (zeroed before)
+    uint32_t* zero;               // [n_zero] counters of the scan that follows, zeroed by the count kernel
+    uint32_t n_zero;              // (a memset each cost 3 to 4 us of a 165 us search)
     uint32_t* cl_off;             // [n1] first row of each cluster
     uint32_t* cl_items;           // [n1] first work item of each cluster
     uint32_t* first_cl;           // [nq x visits] non-empty visited clusters that fill the heap (~0u: none)
@@ -234,7 +236,7 @@ struct ScanParams {
     float* heap_d;                // [nq x k] the Start's pushes, in push order
     uint32_t* heap_id;
     uint32_t* left;               // [nq] queries left to the per-query scan kernel
-    uint32_t* left_n;             // [1] (zeroed before; n_items, hv_alloc, hv_next, hv_done, hv_full follow)
+    uint32_t* left_n;             // [1] (zeroed before, like the other counters: StartParams::zero)
     uint32_t* vl_count;           // [n1] visits per cluster (zeroed before)
     uint32_t* vl;                 // [n1 x nq] visits of each cluster: q * q_order_stride + i
     uint32_t* items;              // [2 x item bound] (cluster, first list entry of a chunk)

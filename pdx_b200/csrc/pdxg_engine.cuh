@@ -134,17 +134,14 @@ struct Workspace {
     float* d_qlo = nullptr;
     uint64_t qhi_cap = 0, qlo_cap = 0;
     int* d_gemm_err = nullptr;
-    // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq + 5
-    // + hv_cap]: first_i | lim | left | left_n, n_items, hv_alloc, hv_next, hv_done | hv_full), Start heaps, per-cluster visit lists and
-    // counters, work items, candidate bitmaps
+    // cluster-major scan (pdxg_scan.cu): packed query words, per-query state ([3 x nq]: first_i | lim |
+    // left), Start heaps, per-cluster visit lists, work items, candidate bitmaps
     uint32_t* d_sc_qw = nullptr;
     uint64_t sc_qw_cap = 0;
     uint32_t* d_sc_q = nullptr;
     uint64_t sc_q_cap = 0;
     uint32_t* d_sc_heap = nullptr;
     uint64_t sc_heap_cap = 0;
-    uint32_t* d_sc_cl = nullptr;
-    uint64_t sc_cl_cap = 0;
     uint32_t* d_sc_vl = nullptr;
     uint64_t sc_vl_cap = 0;
     uint32_t* d_sc_items = nullptr;
@@ -154,6 +151,10 @@ struct Workspace {
     // visit classes, values of heavy visits
     uint32_t* d_sc_vi = nullptr;
     uint64_t sc_vi_cap = 0;
+    // counters of the scan, zeroed by the batched Start: left_n, n_items, hv_alloc, hv_next, hv_done,
+    // search queue, - , - | vl_count [n1] | hv_full [hv_cap]
+    uint32_t* d_zero = nullptr;
+    uint64_t zero_cap = 0;
     uint32_t* d_sc_hv = nullptr;
     uint64_t sc_hv_cap = 0;
     uint32_t* d_sc_hb = nullptr;
@@ -209,6 +210,7 @@ struct Launch {
     const uint32_t* start_full_at = nullptr;  // batched Start: where each query's heap is full
     const uint32_t* start_by_cluster = nullptr;  // batched Start: its queries grouped by cluster, their
     const uint32_t* start_n_rows = nullptr;      // number (one Start per query only)
+    bool queue_zeroed = false;  // p.queue is one of the counters the batched Start zeroes
     uint32_t start_launches = 0;  // kernels of the batched Start
     uint32_t probe_launches = 0;  // kernels of the reduced-precision probe (rotation included)
 };

@@ -237,7 +237,7 @@ void free_workspace(Workspace& w) {
                     w.d_st_cl, w.d_st_q, w.d_st_items, w.d_st_dist, w.d_pq_b16, w.d_pq_r16, w.d_pq_r8,
                     w.d_pq_r8s, w.d_pq_scores, w.d_pr_keys, w.d_pr_list,
                     w.d_req, w.d_foff, w.d_rows, w.d_rows64, w.d_qhi, w.d_qlo, w.d_gemm_err, w.d_sc_qw, w.d_sc_q,
-                    w.d_sc_heap, w.d_sc_cl, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
+                    w.d_sc_heap, w.d_zero, w.d_sc_vl, w.d_sc_items, w.d_sc_bm,
                     w.d_sc_vi, w.d_sc_hv, w.d_sc_hb};
     for (void* q : ptrs) cudaFree(q);
     if (w.h_io) cudaFreeHost(w.h_io);
@@ -1103,6 +1103,17 @@ uint32_t start_visits(const HostLevel& lv, uint32_t k) {
 constexpr uint32_t kHeavyPerQuery = 128;          // cluster-major scan: see run_scan_cluster_major
 constexpr uint64_t kHeavyMaxValues = 64ull << 20;  // 256 MB
 
+// Columns for the values of heavy visits: kHeavyPerQuery vectors a query on average (16-70 were
+// measured); visits past them run their warmup in the replay.
+uint32_t heavy_columns(const DevLevel& lv, uint32_t nq, uint32_t& ncp) {
+    uint32_t cps[kMaxCheckpoints];
+    ncp = warmup_checkpoints(lv.dv, cps, kMaxCheckpoints);
+    if (ncp > (uint32_t)kMaxCheckpoints) return 0;
+    const uint64_t rows = (uint64_t)ncp + lv.n_hblocks;
+    const uint64_t cap = std::min<uint64_t>(std::max<uint64_t>((uint64_t)nq * kHeavyPerQuery, 32768), 1u << 20);
+    return (uint32_t)std::min<uint64_t>(cap, kHeavyMaxValues / rows) / 32 * 32;
+}
+
 int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st) {
     L.p.start_row = nullptr;
     if (!L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return PDXG_OK;
@@ -1124,7 +1135,12 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     if (ix->u8 && (rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
     if ((rc = dev_grow(w.d_st_items, w.st_items_cap, 2 * items))) return rc;
     if ((rc = dev_grow(w.d_st_dist, w.st_dist_cap, ne * stride))) return rc;
+    uint32_t ncp = 0;
+    const uint64_t n_zero = 8ull + n1 + heavy_columns(L.p.l1, nq, ncp);
+    if ((rc = dev_grow(w.d_zero, w.zero_cap, n_zero))) return rc;
     StartParams sp{};
+    sp.zero = w.d_zero;
+    sp.n_zero = (uint32_t)n_zero;
     sp.arena = ix->arena;
     sp.l1 = L.p.l1;
     sp.queries = qp;
@@ -1154,6 +1170,8 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     sp.dist = w.d_st_dist;
     sp.stride = stride;
     PDXG_CUDA(launch_start_batched(sp, occ * ix->num_sms, st));
+    L.p.queue = w.d_zero + 5;
+    L.queue_zeroed = true;
     L.p.start_row = sp.row_of;
     L.p.start_first = sp.first_cl;
     L.p.start_dist = sp.dist;
@@ -1196,21 +1214,14 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     if ((uint64_t)sp.r_warp_bytes * scan_queries_per_cta() + 2048 > ix->max_smem) return PDXG_OK;
     const uint64_t items = scan_item_bound(nq, stride, n1, std::max(lv.max_n, 1u));
     if (items > 0x7FFFFFFFull) return PDXG_OK;
-    // values of heavy visits: columns for kHeavyPerQuery vectors a query on average (16-70 were
-    // measured); visits past them are left to the replay
-    uint32_t cps[kMaxCheckpoints];
-    sp.hv_ncp = warmup_checkpoints(lv.dv, cps, kMaxCheckpoints);
+    sp.hv_cap = heavy_columns(lv, nq, sp.hv_ncp);
     const uint64_t hv_rows = (uint64_t)sp.hv_ncp + lv.n_hblocks;
-    sp.hv_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((uint64_t)nq * kHeavyPerQuery, 32768), 1u << 20);
-    sp.hv_cap = (uint32_t)std::min<uint64_t>(sp.hv_cap, kHeavyMaxValues / hv_rows) / 32 * 32;
-    if (sp.hv_ncp > (uint32_t)kMaxCheckpoints) sp.hv_cap = 0;
     int rc;
     if ((rc = dev_grow(w.d_sc_hv, w.sc_hv_cap, hv_rows * sp.hv_cap))) return rc;
     if ((rc = dev_grow(w.d_sc_vi, w.sc_vi_cap, (uint64_t)nq * stride))) return rc;
-    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq + 5 + sp.hv_cap))) return rc;
+    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq))) return rc;
     if ((rc = dev_grow(w.d_sc_hb, w.sc_hb_cap, std::max<uint64_t>(sp.hv_cap / 16, 1)))) return rc;
     if ((rc = dev_grow(w.d_sc_heap, w.sc_heap_cap, 2ull * nq * k))) return rc;
-    if ((rc = dev_grow(w.d_sc_cl, w.sc_cl_cap, (uint64_t)n1))) return rc;
     if ((rc = dev_grow(w.d_sc_vl, w.sc_vl_cap, (uint64_t)n1 * nq))) return rc;
     if ((rc = dev_grow(w.d_sc_items, w.sc_items_cap, 2 * items))) return rc;
     if ((rc = dev_grow(w.d_sc_bm, w.sc_bm_cap, (uint64_t)nq * stride * bm_words))) return rc;
@@ -1240,20 +1251,20 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.first_i = w.d_sc_q;
     sp.lim = reinterpret_cast<int32_t*>(w.d_sc_q + nq);
     sp.left = w.d_sc_q + 2ull * nq;
-    sp.left_n = w.d_sc_q + 3ull * nq;
-    sp.n_items = w.d_sc_q + 3ull * nq + 1;
-    sp.hv_alloc = w.d_sc_q + 3ull * nq + 2;
+    sp.left_n = w.d_zero;
+    sp.n_items = w.d_zero + 1;
+    sp.hv_alloc = w.d_zero + 2;
     sp.item_bound = (uint32_t)items;
     sp.hv = w.d_sc_hv;
-    sp.hv_next = w.d_sc_q + 3ull * nq + 3;
-    sp.hv_done = w.d_sc_q + 3ull * nq + 4;
-    sp.hv_full = w.d_sc_q + 3ull * nq + 5;
+    sp.hv_next = w.d_zero + 3;
+    sp.hv_done = w.d_zero + 4;
+    sp.hv_full = w.d_zero + 8 + n1;
     sp.hv_blk = w.d_sc_hb;
     sp.vinfo = w.d_sc_vi;
     sp.bm_tile = scan_bitmap_smem(bm_words) ? 1u : 0u;
     sp.heap_d = reinterpret_cast<float*>(w.d_sc_heap);
     sp.heap_id = w.d_sc_heap + (uint64_t)nq * k;
-    sp.vl_count = w.d_sc_cl;
+    sp.vl_count = w.d_zero + 8;
     sp.vl = w.d_sc_vl;
     sp.items = w.d_sc_items;
     sp.bm = w.d_sc_bm;
@@ -1359,7 +1370,7 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
     launches += L.scan_launches;
     ix->last_launches = launches;
     if ((rc = widen_search(ix, nq, L.p.q_list ? n_filtered : nq, L))) return rc;
-    PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
+    if (!L.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
     PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     if (timed) {
         PDXG_CUDA(cudaEventRecord(ix->tev[4], st));
@@ -1575,7 +1586,7 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
     launches += L.scan_launches;
     ix->last_launches = launches;
     ix->last_order_stride = L.p.q_order && !probe_ahead ? k1 : 0;
-    PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
+    if (!L.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
     PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, sizeof(uint32_t) * nq * k, cudaMemcpyDeviceToHost, st));
     PDXG_CUDA(cudaMemcpyAsync(dists, w.d_dists, sizeof(float) * nq * k, cudaMemcpyDeviceToHost, st));
@@ -2453,7 +2464,7 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
     }
     if ((rc = run_scan_cluster_major(ix, w, nq, L, st))) return rc;
     if ((rc = widen_search(ix, nq, L.p.q_list ? n_filtered : nq, L))) return rc;
-    PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
+    if (!L.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
     PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     return PDXG_OK;
 }

@@ -364,7 +364,7 @@ __device__ __forceinline__ uint32_t start_push(const Key& key, uint32_t n, uint3
 }
 
 template <bool U8>
-__global__ void __launch_bounds__(kScanWarps * 32) scan_prep_kernel(const __grid_constant__ ScanParams sp) {
+__global__ void __launch_bounds__(kScanWarps * 32, 3) scan_prep_kernel(const __grid_constant__ ScanParams sp) {
     __shared__ uint64_t list_all[kScanWarps][kSelectList];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t q = blockIdx.x * sp.p_qpc + warp;
@@ -1272,10 +1272,7 @@ uint32_t scan_queries_per_cta() { return kScanWarps; }
 
 template <bool U8>
 static cudaError_t launch_scan_t(const ScanParams& sp, cudaStream_t st, const cudaEvent_t* ev) {
-    cudaError_t e = cudaMemsetAsync(sp.vl_count, 0, sizeof(uint32_t) * sp.l1.nclusters, st);
-    if (e != cudaSuccess) return e;
-    // left_n, n_items, hv_alloc, hv_next, hv_done and hv_full are consecutive
-    if ((e = cudaMemsetAsync(sp.left_n, 0, (5 + (size_t)sp.hv_cap) * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    cudaError_t e;
     const uint32_t ctas = (sp.nq + sp.p_qpc - 1) / sp.p_qpc;
     scan_prep_kernel<U8><<<ctas, sp.p_qpc * 32, 0, st>>>(sp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -37,6 +37,7 @@ constexpr int kCountThreads = 256;
 // Warp per query: lane 0 walks the first visits, all lanes quantize (U8).
 __global__ void __launch_bounds__(kCountThreads) start_count_kernel(const __grid_constant__ StartParams sp) {
     const uint32_t q = (blockIdx.x * kCountThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    for (uint32_t i = blockIdx.x * kCountThreads + threadIdx.x; i < sp.n_zero; i += gridDim.x * kCountThreads) sp.zero[i] = 0;
     if (q >= sp.nq) return;
     if (sp.l1.is_u8) {
         const float* qf = sp.queries + (size_t)q * sp.l1.d;
