@@ -345,12 +345,14 @@ __global__ void __launch_bounds__(kPartialsThreads, 2) meso_partials_kernel(cons
 }
 
 // -------------------------------------------------------------------------------- replay
-// Bound by the latency of one warp's chain of visits, merge by merge. So the heap is kept in
-// registers once it is full (HR per lane: k <= 32 HR; HR = 0 keeps it in shared memory), a visit's
-// cluster record, ids and partials are requested a visit ahead, four warmup steps and four
-// horizontal blocks are read together, and a candidate that a merge has ruled out costs nothing:
-// 292 us for 10,000 queries (16 of 32 meso clusters of 31 vectors each, k 32) and 81 us for 777,
-// against 344 and 94 with the heap in shared memory and each of these read at its use.
+// Bound by the latency of one warp's chain of visits and the instructions on it. So the heap is kept
+// in registers once it is full (HR per lane: k <= 32 HR; HR = 0 keeps it in shared memory), a visit's
+// cluster record, ids and partials are requested a visit ahead, the bounds of all checkpoints and
+// blocks are computed once per visit, one a lane, four warmup steps and four horizontal blocks are
+// read together and tested without branches, and a candidate that a merge has ruled out costs
+// nothing. 235 us for 10,000 queries (16 of 32 meso clusters of 31 vectors each, k 32) and 61 us for
+// 777; 292 and 81 with a bound computed per test and the Starts' order sorted, 344 and 94 with the
+// heap in shared memory and everything read at its use.
 
 // The full heap: slot j's distance bits and id in lane j % 32, register j / 32.
 template <int HR>
@@ -485,6 +487,7 @@ __global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__
         return lane < c.n ? __ldg(reinterpret_cast<const uint32_t*>(tp.arena + c.ids_off) + lane) : 0u;
     };
 
+    const uint32_t cp_lane = lane < ncp ? tp.cp[lane] : 0u;  // at most 32 checkpoints
     uint32_t hsize = 0, slot = 0;
     float top = 0.0f;
     TopHeap<HR> heap;
@@ -519,21 +522,31 @@ __global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__
             // Start (searcher.hpp:217-281): full distances, push the best k - |heap| in the
             // order LevelOps::push_smallest uses (below the m-th key by position, then ties)
             bytes += (unsigned long long)n * d * 4u;
-            const uint32_t N = next_pow2(n);
-            for (uint32_t v = lane; v < N; v += 32) {
-                if (v < n) {
-                    float a = pre[(size_t)(ncp - 1) * stride + v];
-                    for (uint32_t b = 0; b < nb; ++b) a = __fadd_rn(a, pre[(size_t)(ncp + b) * stride + v]);
-                    dist[v] = a;
-                    sortbuf[v] = ((uint64_t)__float_as_uint(a) << 32) | v;
-                } else {
-                    sortbuf[v] = ~0ull;
-                }
+            uint32_t lo = 0xFFFFFFFFu, hi = 0;
+            for (uint32_t v = lane; v < n; v += 32) {
+                float a = pre[(size_t)(ncp - 1) * stride + v];
+#pragma unroll 4
+                for (uint32_t b = 0; b < nb; ++b) a = __fadd_rn(a, pre[(size_t)(ncp + b) * stride + v]);
+                dist[v] = a;
+                const uint32_t key = __float_as_uint(a);
+                lo = key < lo ? key : lo;
+                hi = key > hi ? key : hi;
             }
             __syncwarp();
-            warp_sort_u64(sortbuf, N);
             const uint32_t mm = (k - hsize) < n ? (k - hsize) : n;
-            const uint32_t kth = (uint32_t)(sortbuf[mm - 1] >> 32);
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            uint32_t kth = hi;  // all of them
+            if (mm < n) {  // the smallest key with at least mm keys not above it
+                while (lo < hi) {
+                    const uint32_t mid = lo + (hi - lo) / 2;
+                    uint32_t c = 0;
+                    for (uint32_t v = lane; v < n; v += 32) c += __float_as_uint(dist[v]) <= mid ? 1u : 0u;
+                    if (__reduce_add_sync(0xffffffffu, c) >= mm) hi = mid;
+                    else lo = mid + 1;
+                }
+                kth = lo;
+            }
             uint32_t cntp = 0;
             for (int pass = 0; pass < 2; ++pass) {
                 for (uint32_t b0 = 0; b0 < n; b0 += 32) {
@@ -557,19 +570,23 @@ __global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__
             }
             if (rn < m_top) id0n = first_ids(cn);
         } else {
-            // Warmup (searcher.hpp:374-435): vertical checkpoints until >= ceil(0.8 n) fail the bound
+            // Warmup (searcher.hpp:374-435): vertical checkpoints until >= ceil(0.8 n) fail the bound,
+            // lane s holding the bound of checkpoint s
             const uint32_t needed = (uint32_t)ceilf(__fmul_rn(kSelectivity, (float)n));
+            const float thr_cp = lane < ncp ? thr_at(cp_lane, top) : 0.0f;
             uint32_t step = 0;
             for (uint32_t s0 = 0, n_pruned = 0; n_pruned < needed && s0 < ncp; s0 += 4) {
                 uint32_t cnt[4] = {0, 0, 0, 0};
-                for (uint32_t c0 = 0; c0 < n; c0 += 32) {
-                    const uint32_t v = c0 + lane;
+                float thr[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) thr[u] = __shfl_sync(0xffffffffu, thr_cp, s0 + u);
+                for (uint32_t v = lane; v - lane < n; v += 32) {
+                    const float* col = pre + s0 * stride + v;
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const bool on = v < n && s0 + u < ncp;
-                        const float x = on ? pre[(size_t)(s0 + u) * stride + v] : 0.0f;
-                        const float thr = s0 + u < ncp ? thr_at(tp.cp[s0 + u], top) : 0.0f;
-                        cnt[u] += __popc(__ballot_sync(0xffffffffu, on && x >= thr));
+                        const float x = on ? col[u * stride] : 0.0f;
+                        cnt[u] += __popc(__ballot_sync(0xffffffffu, on && x >= thr[u]));
                     }
                 }
 #pragma unroll
@@ -579,7 +596,7 @@ __global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__
                         step = s0 + u + 1;
                     }
             }
-            const uint32_t cur = tp.cp[step - 1];
+            const uint32_t cur = __shfl_sync(0xffffffffu, cp_lane, step - 1);
             bytes += (unsigned long long)n * cur * 4u;
             if (rn < m_top) id0n = first_ids(cn);
             // Prune (searcher.hpp:437-540) and MergeIntoHeap (searcher.hpp:542-566). The bound's heap
@@ -588,6 +605,8 @@ __global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__
             // lane follows its own vectors, and the survivors of every step are the same, in the
             // same order, as with the step-by-step compaction.
             const float tc = top;
+            // lane b holds the bound after horizontal block b (blocks past 32 read it)
+            const float thr_hb = lane < nb ? thr_at(cur + kHDim * (lane + 1), tc) : 0.0f;
             const float* erow = pre + (size_t)(step - 1) * stride;
             const float* vert = reinterpret_cast<const float*>(tp.arena + c.vert_off);
             uint32_t lane_bytes = 0;
@@ -597,20 +616,26 @@ __global__ void __launch_bounds__(128) top_replay_kernel(const __grid_constant__
                 float dd = in ? erow[v] : 0.0f;
                 uint32_t cv = cur;
                 bool alive = in && dd < thr_at(cv, tc);
+                // four blocks at a time without branches: sums past a lane's failing test are not used
+                const float* hrow = pre + ncp * stride + (in ? v : 0u);
                 for (uint32_t b0 = 0; b0 < nb && __any_sync(0xffffffffu, alive); b0 += 4) {
-                    float x[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) x[u] = in && b0 + u < nb ? pre[(size_t)(ncp + b0 + u) * stride + v] : 0.0f;
+                    float x[4], thr[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        if (alive && b0 + u < nb) {
-                            lane_bytes += kHDim * 4u;
+                        x[u] = b0 + u < nb ? hrow[(b0 + u) * stride] : 0.0f;
+                        thr[u] = __shfl_sync(0xffffffffu, thr_hb, (b0 + u) & 31);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (b0 + u < nb) {  // uniform
+                            if (b0 + u >= 32) thr[u] = thr_at(cur + kHDim * (b0 + u + 1), tc);
+                            if (tp.stats) lane_bytes += alive ? kHDim * 4u : 0u;
                             dd = __fadd_rn(dd, x[u]);
-                            cv += kHDim;
-                            alive = dd < thr_at(cv, tc);
+                            alive = alive && dd < thr[u];
                         }
                     }
                 }
+                if (alive) cv = cur + kHDim * nb;
                 uint32_t cur_v = cur;
                 while (alive && cur_v < dv) {
                     const uint32_t last = (cur_v + kHDim < dv) ? cur_v + kHDim : dv;
