@@ -260,10 +260,10 @@ uint64_t pdxg_noalloc_scratch_bytes(void);
  * every mode. */
 int pdxg_set_top_level_mode(pdxg_index* index, uint32_t mode);
 
-/* Engine tuning, U8 tree indexes: the Start of PDXearch (searcher.hpp:217-281) on each query's
- * first visited cluster. 0 = batched when the batch has at least 32 queries and the L1 visit
- * orders come from a separate top level: queries are grouped by first cluster and the exact
- * distances computed once per cluster and group, ahead of the scan; 1 = inside each query's
+/* Engine tuning: the Starts of PDXearch (searcher.hpp:217-281) on the clusters that fill each
+ * query's heap. 0 = batched when the batch has at least 32 queries and the L1 visit orders are
+ * computed ahead of the scan: queries are grouped by cluster and the exact distances (up to
+ * four clusters a query) computed once per cluster and group; 1 = inside each query's
  * scan CTA. Results are identical in both modes. No counterpart in the reference. */
 int pdxg_set_start_mode(pdxg_index* index, uint32_t mode);
 
@@ -332,11 +332,11 @@ int pdxg_filter_release(pdxg_index* index, int32_t filter_id);
 int pdxg_set_rotation_mode(pdxg_index* index, uint32_t mode);
 int pdxg_rotation_uses_tensor_cores(const pdxg_index* index);
 
-/* Engine tuning, U8 indexes: how the scan (Warmup / Prune / MergeIntoHeap of PDXearch,
+/* Engine tuning: how the scan (Warmup / Prune / MergeIntoHeap of PDXearch,
  * searcher.hpp:374-566) runs after a batched Start. 0 = cluster-major when it fits (default):
  * each cluster's first warmup step is computed once for all the queries that visit it, bounded
  * by each query's heap top after its Start, and a warp per query replays PDXearch on those
- * results (queries with a filter, or a Start that leaves the heap short of k, take the per-query
+ * results (queries with a filter, or batched Starts that leave the heap short of k, take the per-query
  * kernel); 1 = the per-query kernel for every query. Results are identical in both modes. No
  * counterpart in the reference. */
 int pdxg_set_scan_mode(pdxg_index* index, uint32_t mode);

@@ -604,7 +604,7 @@ int plan_search(pdxg_index* ix, uint32_t nq, uint32_t k, uint32_t n_order, bool 
                                            " B) exceeds the device limit; cluster, k or nprobe too large");
     L.u8 = ix->u8;
     int threads = (int)ix->threads;
-    if (threads == 0) threads = 128;  // measured fastest on B200 (IVF2 SQ8 1M x 1024)
+    if (threads == 0) threads = 128;  // many queries; few take more (widen_search)
     return set_search_threads(ix, nq, threads, L);
 }
 
