@@ -1354,6 +1354,8 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
     } else if (ix->tree && !d_order) {
         if (any_plain) {
             rc = run_top_level(ix, w, qp, nq, L, st, 0, timed);
+            // a batch with filters runs the top level in the scan kernel where a form of its own does not fit
+            if (rc == PDXG_ERR_CAPACITY && any_filter) rc = PDXG_OK;
             if (rc) return rc;
             launches += L.top_launches;
         }
