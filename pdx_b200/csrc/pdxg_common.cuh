@@ -90,8 +90,8 @@ struct SearchParams {
     const uint32_t* q_order_count;  // [nq]
     uint32_t q_order_stride;
     uint32_t q_order_filtered;      // 1: the filtered queries have a row too (exact probe ahead)
-    // batched Start (pdxg_start.cu): exact U8 distances to every vector of each query's first
-    // visited cluster, computed ahead with reuse across queries
+    // batched Start (pdxg_start.cu): exact distances to every vector of the clusters that fill each
+    // query's heap (up to start_visits of them), computed ahead with reuse across queries
     const int32_t* start_row;       // optional [nq x start_visits]: row in start_dist, -1 = none
     const uint32_t* start_first;    // [nq x start_visits] the cluster of that row
     const uint32_t* start_dist;     // [rows x start_stride]
