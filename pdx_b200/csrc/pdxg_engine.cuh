@@ -210,8 +210,6 @@ struct Launch {
     const uint32_t* start_full_at = nullptr;  // batched Start: where each query's heap is full
     const uint32_t* start_by_cluster = nullptr;  // batched Start: its queries grouped by cluster, their
     const uint32_t* start_n_rows = nullptr;      // number (one Start per query only)
-    uint32_t np_min = 0;       // clusters that every query of the batch visits, of those there are
-    bool start_fills = false;  // batched Start: it fills the heap of every query without a filter
     bool queue_zeroed = false;  // p.queue is one of the counters the batched Start zeroes
     uint32_t start_launches = 0;  // kernels of the batched Start
     uint32_t probe_launches = 0;  // kernels of the reduced-precision probe (rotation included)

@@ -566,7 +566,6 @@ int plan_search(pdxg_index* ix, uint32_t nq, uint32_t k, uint32_t n_order, bool 
     if (np_flat_max != 0xFFFFFFFFu) np_flat = np_flat_max;
     if (top_max != 0xFFFFFFFFu) top = top_max;
     p.nprobe = np_flat;
-    L.np_min = np_flat;
     p.top_nprobe = top;
     p.n_order = n_order;
     const uint32_t d = ix->d;
@@ -614,13 +613,26 @@ int plan_search(pdxg_index* ix, uint32_t nq, uint32_t k, uint32_t n_order, bool 
 // visits' latency counts, not the throughput of many CTAs. 16 filtered queries, 32 clusters of 1,000
 // vectors each: 337 us with 128 threads and every slot of a cluster masked and selected from, 235 us
 // with 512 on the selected slots alone; 255 of a serving batch 1356 and 1040 us (256 threads).
-// After the cluster-major scan only the device knows the plain queries that four Starts could not
-// fill. They are none when start_fills, else as many as the batch has: 5,000 queries, k 100, 200
-// clusters of 20 vectors x 64 dims, all left, take 1.08 ms with 128 threads and 3.44 with 512.
+// After the cluster-major scan only the device knows the plain queries that the batched Starts did
+// not fill. Such a query met a cluster smaller than k first and second, so the share of such clusters
+// squared estimates theirs; indexes whose k-means left some clusters of one vector (9 to 32 % below k
+// on the benchmark's) have none, and one of 200 clusters of 20 vectors x 64 dims with k 100 leaves all:
+// 5,000 queries take 1.08 ms there with 128 threads and 3.44 with 512.
 int widen_search(pdxg_index* ix, uint32_t nq, uint32_t n_filtered, Launch& L) {
-    const uint32_t n = L.p.q_list && L.start_fills ? n_filtered : nq;
-    if (ix->threads != 0 || n > 2u * (uint32_t)ix->num_sms) return PDXG_OK;
-    const int threads = n <= (uint32_t)ix->num_sms ? 512 : 256;
+    const uint32_t few = 2u * (uint32_t)ix->num_sms;
+    if (ix->threads != 0) return PDXG_OK;
+    double n = nq;
+    if (L.p.q_list) {
+        uint32_t clusters = 0, small = 0;
+        for (uint32_t x : ix->l1.n) {
+            clusters += x != 0;
+            small += x != 0 && x < L.p.k;
+        }
+        const double share = (double)small / std::max(clusters, 1u);
+        n = n_filtered + nq * share * share;
+    }
+    if (n > few) return PDXG_OK;
+    const int threads = n <= (double)ix->num_sms ? 512 : 256;
     if (search_occupancy(L.u8, threads, L.p.smem_total) <= 0) return PDXG_OK;
     return set_search_threads(ix, nq, threads, L);
 }
@@ -1093,19 +1105,17 @@ constexpr uint32_t kStartMinQueries = 32;
 constexpr uint32_t kStartMaxVisits = 4;
 
 // Starts a query needs to fill a heap of k, at most kStartMaxVisits: the smallest clusters' turn.
-// `fills`: that many Starts fill the heap of every query that visits as many clusters.
-uint32_t start_visits(const HostLevel& lv, uint32_t k, bool& fills) {
+uint32_t start_visits(const HostLevel& lv, uint32_t k) {
     std::vector<uint32_t> n;
     for (uint32_t x : lv.n)
-        if (x) n.push_back(x);
-    const uint32_t m = (uint32_t)std::min<size_t>(n.size(), kStartMaxVisits);
+        if (x && x < k) n.push_back(x);
+    if (n.empty()) return 1;
+    const size_t m = std::min<size_t>(n.size(), kStartMaxVisits - 1);
     std::partial_sort(n.begin(), n.begin() + m, n.end());
     uint64_t have = 0;
-    fills = true;
-    for (uint32_t s = 0; s < m; ++s)
-        if ((have += n[s]) >= k) return s + 1;
-    fills = false;
-    return std::max(m, 1u);
+    uint32_t s = 0;
+    while (s < m && have < k) have += n[s++];
+    return have < k ? s + 1 : s;
 }
 constexpr uint32_t kHeavyPerQuery = 128;          // cluster-major scan: see run_scan_cluster_major
 constexpr uint64_t kHeavyMaxValues = 64ull << 20;  // 256 MB
@@ -1126,9 +1136,7 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     if (!L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return PDXG_OK;
     const uint32_t n1 = L.p.l1.nclusters;
     const uint32_t stride = (std::max(L.p.l1.max_n, 1u) + 3) & ~3u;
-    bool fills;
-    const uint32_t need = start_visits(ix->l1, L.p.k, fills);
-    uint32_t visits = need;
+    uint32_t visits = start_visits(ix->l1, L.p.k);
     while (visits > 1 && (uint64_t)nq * visits * stride * 4 > (4ull << 30)) --visits;
     const uint64_t ne = (uint64_t)nq * visits;
     const uint64_t items = start_item_bound(ix->u8, (uint32_t)ne, n1, std::max(L.p.l1.max_n, 1u));
@@ -1189,7 +1197,6 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     L.start_full_at = sp.full_at;
     L.start_by_cluster = visits == 1 ? sp.sorted_q : nullptr;
     L.start_n_rows = sp.n_rows;
-    L.start_fills = fills && visits == need && need <= L.np_min;
     L.start_launches = ne > 1024 ? 4 : 3;
     return PDXG_OK;
 }
@@ -2347,7 +2354,7 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
     // resolve every query's parameters as PDXearch / PDXTreeIndex::Search would
     const uint32_t n1 = (uint32_t)ix->l1.fc.size();
     const uint32_t n0 = (uint32_t)ix->l0.fc.size();
-    uint32_t np_max = 1, np_min = n1, top_max = 0, nf = 0;
+    uint32_t np_max = 1, top_max = 0, nf = 0;
     uint64_t nrows = 0;
     bool any_filter = false, any_plain = false;
     for (uint32_t q = 0; q < nq; ++q) {
@@ -2393,7 +2400,6 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
         h_req[nq + q] = npf;
         h_req[2 * nq + q] = top;
         np_max = std::max(np_max, npf);
-        np_min = std::min(np_min, npf);
         top_max = std::max(top_max, top);
         if (r.filter_id >= 0) {
             h_req[3 * nq + q] = (uint32_t)(-2 - r.filter_id);
@@ -2445,7 +2451,6 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
     Launch L;
     const bool probe_ahead = !gemm_probe && !ix->tree && probe_exact_ok(ix);
     if ((rc = plan_search(ix, nq, k_max, 0, any_filter, L, np_max, top_max, probe_ahead, st))) return rc;
-    L.np_min = np_min;
     L.p.queries = qp;
     L.p.q_k = w.d_req;
     L.p.q_nprobe = w.d_req + nq;
