@@ -874,7 +874,6 @@ struct LevelOps {
             s.top_slot = 0;
         }
         __syncthreads();
-        uint32_t pre = 0;  // Starts computed ahead that were used
         for (uint32_t ci = 0; ci < nvisit; ++ci) {
             const uint32_t cidx = order[ci];
             const DevCluster c = lv.clusters[cidx];
@@ -888,12 +887,17 @@ struct LevelOps {
             if (s.hsize < k) {
                 long long t0 = 0;
                 if (p.stats && threadIdx.x == 0) t0 = clock64();
-                if (fsel)
+                if (fsel) {
                     filtered_start(c, k, passing);
-                else if (pre < pre_n && cidx == __ldg(pre_cluster + pre))
-                    start_pre(c, k, __ldg(pre_row + pre++));
-                else
-                    start(c, k);
+                } else {
+                    // the list is walked for each Start: as a position kept along the visits it cost the
+                    // filtered queries of the 256-thread U8 form registers (255 of them 1.51 -> 1.72 ms)
+                    int32_t row = -1;
+                    for (uint32_t i = 0; i < pre_n; ++i)
+                        if (__ldg(pre_cluster + i) == cidx) row = __ldg(pre_row + i);
+                    if (row >= 0) start_pre(c, k, row);
+                    else start(c, k);
+                }
                 if (p.stats && threadIdx.x == 0 && !top_level)
                     s.cycles[1] += (unsigned long long)(clock64() - t0);
                 continue;
