@@ -11,6 +11,7 @@
 #include <mutex>
 #include <string>
 #include <unordered_set>
+#include <utility>
 #include <vector>
 
 #include "../../include/pdx_b200.h"
@@ -55,6 +56,29 @@ struct HostLevel {
     std::vector<float> centroids;
     uint32_t max_n = 0, sel_words = 0, n_vwords = 0, qw_hoff = 0, n_hblocks = 0;
     uint64_t total_vectors = 0;
+    std::vector<uint32_t> by_size;  // n in ascending order
+    // n[c] = size, with by_size kept in order
+    void resize_cluster(size_t c, uint32_t size) {
+        const uint32_t old = n[c];
+        n[c] = size;
+        if (size > old) {
+            const auto end = std::lower_bound(by_size.begin(), by_size.end(), size);
+            const auto at = std::upper_bound(by_size.begin(), end, old) - 1;
+            std::copy(at + 1, end, at);
+            *(end - 1) = size;
+        } else if (size < old) {
+            const auto at = std::lower_bound(by_size.begin(), by_size.end(), old);
+            const auto to = std::upper_bound(by_size.begin(), at, size);
+            std::copy_backward(to, at, at + 1);
+            *to = size;
+        }
+    }
+    // clusters with at least one and fewer than `size` vectors: by_size[first, second)
+    std::pair<size_t, size_t> smaller(uint32_t size) const {
+        const auto a = std::upper_bound(by_size.begin(), by_size.end(), 0u);
+        const auto b = std::lower_bound(a, by_size.end(), size);
+        return {(size_t)(a - by_size.begin()), (size_t)(b - by_size.begin())};
+    }
 };
 
 struct Workspace {

@@ -192,6 +192,8 @@ uint64_t plan_level(HostLevel& lv, uint64_t off) {
     }
     lv.ids_start[ncl] = lv.total_vectors;
     lv.sel_words = sel;
+    lv.by_size = lv.n;
+    std::sort(lv.by_size.begin(), lv.by_size.end());
     return align_up(off, 256);
 }
 
@@ -623,12 +625,8 @@ int widen_search(pdxg_index* ix, uint32_t nq, uint32_t n_filtered, Launch& L) {
     if (ix->threads != 0) return PDXG_OK;
     double n = nq;
     if (L.p.q_list) {
-        uint32_t clusters = 0, small = 0;
-        for (uint32_t x : ix->l1.n) {
-            clusters += x != 0;
-            small += x != 0 && x < L.p.k;
-        }
-        const double share = (double)small / std::max(clusters, 1u);
+        const auto [a, b] = ix->l1.smaller(L.p.k);
+        const double share = a == b ? 0.0 : (double)(b - a) / (double)(ix->l1.by_size.size() - a);
         n = n_filtered + nq * share * share;
     }
     if (n > few) return PDXG_OK;
@@ -1104,17 +1102,13 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
 constexpr uint32_t kStartMinQueries = 32;
 constexpr uint32_t kStartMaxVisits = 4;
 
-// Starts a query needs to fill a heap of k, at most kStartMaxVisits: the smallest clusters' turn.
+// Starts a query needs to fill a heap of k, at most kStartMaxVisits: the smallest clusters' turn. (The
+// sizes are kept in order with the index: collecting them took 40 us of every search on 40,000 clusters.)
 uint32_t start_visits(const HostLevel& lv, uint32_t k) {
-    std::vector<uint32_t> n;
-    for (uint32_t x : lv.n)
-        if (x && x < k) n.push_back(x);
-    if (n.empty()) return 1;
-    const size_t m = std::min<size_t>(n.size(), kStartMaxVisits - 1);
-    std::partial_sort(n.begin(), n.begin() + m, n.end());
+    const auto [a, b] = lv.smaller(k);
     uint64_t have = 0;
     uint32_t s = 0;
-    while (s < m && have < k) have += n[s++];
+    while (s < kStartMaxVisits - 1 && a + s < b && have < k) have += lv.by_size[a + s++];
     return have < k ? s + 1 : s;
 }
 constexpr uint32_t kHeavyPerQuery = 128;          // cluster-major scan: see run_scan_cluster_major

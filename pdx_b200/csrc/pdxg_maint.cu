@@ -141,7 +141,7 @@ void mark_cluster(pdxg_index* ix, uint32_t c) {
     DevCluster& m = ix->l1.meta[c];
     m.n = K.used;
     m.live = K.num_embeddings;
-    ix->l1.n[c] = K.used;
+    ix->l1.resize_cluster(c, K.used);
     ix->l1.max_n = std::max(ix->l1.max_n, K.used);
     M.records_dirty = M.dirty = true;
 }
