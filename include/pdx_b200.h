@@ -191,10 +191,11 @@ int pdxg_prepare_queries(pdxg_index* index, const float* queries, uint32_t nq, f
 int pdxg_get_stats(pdxg_index* index, uint64_t out[12]);
 
 /* Counters of the cluster-major scan in the last search launched with PDXG_COLLECT_STATS
- * (synchronizes the index's stream): out[0] candidates tested (vectors below the first warmup
- * checkpoint's bound at the heap top after the Start), out[1] of those below the bound at the
- * heap top of their visit, out[2] visits whose warmup stopped after its first step, out[3]
- * visits that ran the whole warmup. No counterpart in the reference; diagnostics of
+ * (synchronizes the index's stream): out[0] candidates (vectors below the first warmup
+ * checkpoint's bound at the heap top after the Start; F32 levels: that may be below it, within the
+ * error of the TF32 products that find them), out[1] of those below the bound at the heap top of
+ * their visit, out[2] visits whose warmup stopped after its first step, out[3] visits that ran the
+ * whole warmup. No counterpart in the reference; diagnostics of
  * pdxg_set_scan_mode 0. */
 int pdxg_get_scan_stats(pdxg_index* index, uint64_t out[4]);
 

@@ -633,6 +633,7 @@ __global__ void __launch_bounds__(kBitmapThreads) scan_bitmap_kernel(const __gri
         if (threadIdx.x < nqc) {
             const uint32_t cnt = qcnt[threadIdx.x];
             uint32_t info = cnt;
+            if (sp.stats) add_stat(sp, 12, cnt);
             if (sp.cp1 < lv.dv && n - cnt < needed) {
                 // columns are handed out in units of 32; none is asked for once they are used up, so
                 // the counter stays far from its range
@@ -916,7 +917,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
     uint32_t* scratch = sp.start_dist + (size_t)__ldg(sp.start_row + (size_t)q * sp.start_visits) * sp.start_stride;
     const uint32_t S = sp.r_surv_cap;
     unsigned long long b_warm = 0, b_h = 0, b_v = 0, merged = 0;
-    unsigned long long n_cand = 0, n_surv = 0, n_fast = 0, n_full = 0;
+    unsigned long long n_surv = 0, n_fast = 0, n_full = 0;
     unsigned long long b_warm_l = 0;  // per lane: the first step of every visit
     uint32_t visits_l = 0, fast_l = 0;
 
@@ -1094,7 +1095,6 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
             const uint32_t w = w0 + lane;
             const uint32_t word = w < W ? __ldg(bmp + w) : 0u;
             const uint32_t total = scan_bits_to_offsets(word, lane, R.cand);
-            n_cand += total;
             constexpr int CP = kCandPerLane<U8>;
             constexpr int GW = U8 ? 4 : (int)kScanDims;  // words of the first step at most
             for (uint32_t j0 = 0; j0 < total; j0 += 32 * CP) {
@@ -1188,6 +1188,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
             }
             n_pruned = __reduce_add_sync(0xffffffffu, cntp);
             if (cur > 0) b_warm += (unsigned long long)n * (last - cur) * Raw<U8>::kElem;
+            else if (!light) n_surv += n - n_pruned;
             cur = last;
             ++step;
         }
@@ -1248,7 +1249,6 @@ __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kerne
             add_stat(sp, 3 + kSurvivorV, vv);
             add_stat(sp, 1, visits);
             add_stat(sp, 2, merged);
-            add_stat(sp, 12, n_cand);
             add_stat(sp, 13, n_surv);
             add_stat(sp, 14, n_fast);
             add_stat(sp, 15, n_full);
