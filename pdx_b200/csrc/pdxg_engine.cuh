@@ -273,10 +273,6 @@ int rotate_tf32x3(pdxg_index* ix, const float* q, uint32_t nq, bool norm, float*
                   float* out, cudaStream_t st);
 int run_top_level(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st,
                   uint32_t q_offset = 0, bool timed = false);
-// The cluster-major scan for the queries it can take (U8 level after a batched Start, visit
-// orders ahead, no tombstones); sets L.p.q_list to the rest, for the per-query kernel.
-int run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq, Launch& L, cudaStream_t st,
-                           bool timed = false);
 int check_index(const pdxg_index* ix);
 // Selection bitmap + passing counts of one row-id list in the device bitmap layout.
 void build_filter(const pdxg_index* ix, const uint64_t* rows, uint64_t n, uint32_t* sel, uint32_t* pass);

@@ -45,6 +45,7 @@ cudaError_t launch_probe_exact(const ProbeParams& pp, cudaStream_t st);
 int start_dist_occupancy(bool u8, size_t smem);
 size_t start_dist_smem(const DevLevel& lv);
 uint64_t start_item_bound(bool u8, uint32_t nq, uint32_t n1, uint32_t max_n);
+uint64_t start_max_starts(bool u8, uint32_t max_n);
 }  // namespace pdxg
 
 using namespace pdxg;
@@ -1096,9 +1097,6 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
     return PDXG_OK;
 }
 
-// Batched Start (pdxg_start.cu) for levels whose visit orders are known before the scan
-// (tree indexes with a separate top level). Sets L.p.start_* when it ran; a batch outside its
-// limits leaves them unset and the scan runs Start itself.
 constexpr uint32_t kStartMinQueries = 32;
 constexpr uint32_t kStartMaxVisits = 4;
 
@@ -1111,34 +1109,90 @@ uint32_t start_visits(const HostLevel& lv, uint32_t k) {
     while (s < kStartMaxVisits - 1 && a + s < b && have < k) have += lv.by_size[a + s++];
     return have < k ? s + 1 : s;
 }
-constexpr uint32_t kHeavyPerQuery = 128;          // cluster-major scan: see run_scan_cluster_major
-constexpr uint64_t kHeavyMaxValues = 64ull << 20;  // 256 MB
 
-// Columns for the values of heavy visits: kHeavyPerQuery vectors a query on average (16-70 were
-// measured); visits past them run their warmup in the replay.
-uint32_t heavy_columns(const DevLevel& lv, uint32_t nq, uint32_t& ncp) {
+// Columns (one vector each) for the values of heavy visits in the cluster-major scan: kHeavyPerQuery
+// vectors a query on average (16-70 were measured), within 256 MB; visits past them run their warmup
+// in the replay.
+constexpr uint32_t kHeavyPerQuery = 128, kHeavyPerQueryMin = 16;
+constexpr uint64_t kHeavyMaxValues = 64ull << 20;
+
+uint64_t heavy_columns_max(const DevLevel& lv, uint32_t& ncp) {
     uint32_t cps[kMaxCheckpoints];
     ncp = warmup_checkpoints(lv.dv, cps, kMaxCheckpoints);
-    if (ncp > (uint32_t)kMaxCheckpoints) return 0;
-    const uint64_t rows = (uint64_t)ncp + lv.n_hblocks;
-    const uint64_t cap = std::min<uint64_t>(std::max<uint64_t>((uint64_t)nq * kHeavyPerQuery, 32768), 1u << 20);
-    return (uint32_t)std::min<uint64_t>(cap, kHeavyMaxValues / rows) / 32 * 32;
+    return ncp > (uint32_t)kMaxCheckpoints ? 0 : kHeavyMaxValues / ((uint64_t)ncp + lv.n_hblocks);
 }
 
-int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, Launch& L, cudaStream_t st) {
-    L.p.start_row = nullptr;
-    if (!L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return PDXG_OK;
+uint32_t heavy_columns(const DevLevel& lv, uint32_t nq, uint32_t& ncp) {
+    const uint64_t cap = std::max<uint64_t>((uint64_t)nq * kHeavyPerQuery, 32768);
+    return (uint32_t)std::min<uint64_t>(cap, heavy_columns_max(lv, ncp)) / 32 * 32;
+}
+
+// Shared memory of a replay warp (pdxg_scan.cu), in ScanParams' fields.
+uint64_t replay_warp_bytes(const DevLevel& lv, uint32_t k, ScanParams& sp) {
+    sp.nwords = lv.is_u8 ? lv.qw_hoff + lv.n_hblocks * 16 : lv.d;
+    sp.bm_words = (std::max(lv.max_n, 1u) + 31) / 32;
+    sp.r_heap_cap = (k + 3) & ~3u;
+    sp.r_area_bytes = (uint32_t)align_up(std::max<uint64_t>(2048, 8ull * next_pow2(k)), 16);
+    // a first warmup step that ends the warmup keeps at most n - ceil(0.8 n) survivors
+    sp.r_surv_cap = (std::max(lv.max_n, 1u) / 5 + 33 + 31) / 32 * 32;
+    return align_up((uint64_t)sp.nwords * 4, 16) + 8ull * sp.r_heap_cap + sp.r_area_bytes +
+           align_up((uint64_t)sp.bm_words * 4, 16) + 8ull * sp.r_surv_cap;
+}
+
+// How a batch goes through the batched Start and the scan: in slices of `rows` queries, one after the
+// other, so that none of their arrays exceeds kSliceBytes and no counter its range. Queries of one
+// slice share a cluster's reads, so slices are as large as that allows: at 1 GB instead of 8, 10,000
+// queries on 1,000 clusters with 4,000-vector bitmaps took 14.1 ms instead of 8.1. A batch past a
+// limit left the route before: 20,000 of those queries took 63 ms in the per-query kernel (16.2 in two
+// slices), 140,000 F32 queries with four Starts each 8.7 (5.9).
+constexpr uint64_t kSliceBytes = 8ull << 30;
+
+struct Slices {
+    uint32_t rows;        // a multiple of 32, or the whole batch
+    uint32_t visits = 0;  // batched Starts of a query (0: none, the per-query kernel runs Start itself)
+    bool scan = false;    // cluster-major
+};
+
+Slices plan_slices(const pdxg_index* ix, const Launch& L, uint32_t nq) {
+    Slices s{nq};
+    // the visit orders are known before the scan (tree indexes with a separate top level, probes ahead)
+    if (!L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return s;
+    const DevLevel& lv = L.p.l1;
+    const uint32_t n1 = lv.nclusters, k = L.p.k, max_n = std::max(lv.max_n, 1u), k1 = L.p.q_order_stride;
+    const size_t smem = start_dist_smem(lv);
+    if (smem + 1024 > ix->max_smem || start_dist_occupancy(ix->u8, smem) <= 0) return s;
+    const uint64_t starts = std::min<uint64_t>(start_max_starts(ix->u8, max_n), kSliceBytes / (4ull * ((max_n + 3) & ~3u)));
+    uint32_t visits = start_visits(ix->l1, k);
+    while (visits > 1 && starts / visits < kStartMinQueries) --visits;
+    uint64_t rows = std::min<uint64_t>(starts / visits, 1u << 20);
+    if (rows < kStartMinQueries || start_item_bound(ix->u8, (uint32_t)(rows * visits), n1, max_n) > 0xFFFFFFFFull) return s;
+    s.visits = visits;
+    ScanParams sp{};
+    if (ix->scan_mode == 0 && !L.p.order && !lv.tomb && k1 > 0 &&
+        replay_warp_bytes(lv, k, sp) * scan_queries_per_cta() + 2048 <= ix->max_smem) {
+        uint32_t ncp;
+        const uint64_t heavy = std::max<uint64_t>(heavy_columns_max(lv, ncp) / kHeavyPerQueryMin, 4096);
+        const uint64_t m = std::min<uint64_t>({kSliceBytes / (4ull * k1 * sp.bm_words), kSliceBytes / (4ull * n1),
+                                     kSliceBytes / (8ull * k), heavy});
+        if (m >= kStartMinQueries) {
+            s.scan = true;
+            rows = std::min(rows, m);
+        }
+    }
+    if (rows < nq) {
+        const uint64_t most = rows / 32 * 32, n = (nq + most - 1) / most;
+        s.rows = (uint32_t)std::min(most, ((nq + n - 1) / n + 31) / 32 * 32);
+    }
+    return s;
+}
+
+// Batched Start (pdxg_start.cu) of nq queries, `visits` each; sets L.p.start_*.
+int run_start_batched(pdxg_index* ix, Workspace& w, uint32_t nq, uint32_t visits, Launch& L, cudaStream_t st) {
     const uint32_t n1 = L.p.l1.nclusters;
     const uint32_t stride = (std::max(L.p.l1.max_n, 1u) + 3) & ~3u;
-    uint32_t visits = start_visits(ix->l1, L.p.k);
-    while (visits > 1 && (uint64_t)nq * visits * stride * 4 > (4ull << 30)) --visits;
     const uint64_t ne = (uint64_t)nq * visits;
     const uint64_t items = start_item_bound(ix->u8, (uint32_t)ne, n1, std::max(L.p.l1.max_n, 1u));
-    if (items == 0 || (uint64_t)nq * stride * 4 > (4ull << 30) || items > 0xFFFFFFFFull || nq > (1u << 20)) return PDXG_OK;
-    const size_t smem = start_dist_smem(L.p.l1);
-    if (smem + 1024 > ix->max_smem) return PDXG_OK;
-    const int occ = start_dist_occupancy(ix->u8, smem);
-    if (occ <= 0) return PDXG_OK;
+    const int occ = start_dist_occupancy(ix->u8, start_dist_smem(L.p.l1));
     int rc;
     if ((rc = dev_grow(w.d_st_cl, w.st_cl_cap, (uint64_t)3 * n1))) return rc;
     if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + 2ull * nq + 3))) return rc;
@@ -1154,7 +1208,7 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     sp.n_zero = (uint32_t)n_zero;
     sp.arena = ix->arena;
     sp.l1 = L.p.l1;
-    sp.queries = qp;
+    sp.queries = L.p.queries;
     sp.nq = nq;
     sp.q_order = L.p.q_order;
     sp.q_order_count = L.p.q_order_count;
@@ -1195,36 +1249,19 @@ int run_start_batched(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq
     return PDXG_OK;
 }
 
-}  // namespace
-
-int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq, Launch& L, cudaStream_t st,
-                                       bool timed) {
-    L.p.q_list = nullptr;
-    L.p.q_list_n = nullptr;
-    L.scan_launches = 0;
-    ix->tev_scan = false;
-    if (ix->scan_mode != 0 || !L.p.start_row || !L.p.q_order || L.p.order || L.p.l1.tomb) return PDXG_OK;
+// The cluster-major scan of nq queries after their batched Starts; sets L.p.q_list to those it leaves
+// to the per-query kernel (with a filter, or a heap that the Starts did not fill).
+int run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq, Launch& L, cudaStream_t st, bool timed) {
     const DevLevel& lv = L.p.l1;
     const uint32_t n1 = lv.nclusters, stride = L.p.q_order_stride, k = L.p.k;
-    const uint32_t nwords = L.u8 ? lv.qw_hoff + lv.n_hblocks * 16 : lv.d;
-    const uint32_t bm_words = (std::max(lv.max_n, 1u) + 31) / 32;
-    if ((uint64_t)nq * stride >= 0xFFFFFFFFull || (uint64_t)n1 * nq > (256ull << 20) || stride == 0 ||
-        (uint64_t)nq * stride * bm_words > (2ull << 30))  // 8 GB of bitmaps
-        return PDXG_OK;
     ScanParams sp{};
-    sp.r_heap_cap = (k + 3) & ~3u;
-    sp.r_area_bytes = (uint32_t)align_up(std::max<uint64_t>(2048, 8ull * next_pow2(k)), 16);
-    // a first warmup step that ends the warmup keeps at most n - ceil(0.8 n) survivors
-    sp.r_surv_cap = (std::max(lv.max_n, 1u) / 5 + 33 + 31) / 32 * 32;
-    sp.r_warp_bytes = (uint32_t)(align_up((uint64_t)nwords * 4, 16) + 8ull * sp.r_heap_cap + sp.r_area_bytes +
-                                 align_up((uint64_t)bm_words * 4, 16) + 8ull * sp.r_surv_cap);
+    sp.r_warp_bytes = (uint32_t)replay_warp_bytes(lv, k, sp);
+    const uint32_t bm_words = sp.bm_words;
     sp.p_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + ix->num_sms - 1) / ix->num_sms);
     // a replay CTA of 8 warps takes as few queries as still fill the GPU at 2 CTAs per SM: all its
     // warps share the heavy visits
     sp.r_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + 2 * ix->num_sms - 1) / (2 * ix->num_sms));
-    if ((uint64_t)sp.r_warp_bytes * scan_queries_per_cta() + 2048 > ix->max_smem) return PDXG_OK;
     const uint64_t items = scan_item_bound(nq, stride, n1, std::max(lv.max_n, 1u));
-    if (items > 0x7FFFFFFFull) return PDXG_OK;
     sp.hv_cap = heavy_columns(lv, nq, sp.hv_ncp);
     const uint64_t hv_rows = (uint64_t)sp.hv_ncp + lv.n_hblocks;
     int rc;
@@ -1257,7 +1294,6 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.start_stride = L.p.start_stride;
     sp.cp1 = std::min(16u, lv.dv);
     sp.g1 = L.u8 ? (sp.cp1 + 3) / 4 : sp.cp1;
-    sp.nwords = nwords;
     sp.qwords = L.u8 ? w.d_sc_qw : reinterpret_cast<const uint32_t*>(L.p.queries);
     sp.first_i = w.d_sc_q;
     sp.lim = reinterpret_cast<int32_t*>(w.d_sc_q + nq);
@@ -1279,7 +1315,6 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     sp.vl = w.d_sc_vl;
     sp.items = w.d_sc_items;
     sp.bm = w.d_sc_bm;
-    sp.bm_words = bm_words;
     sp.out_ids = L.p.out_ids;
     sp.out_dists = L.p.out_dists;
     sp.out_counts = L.p.out_counts;
@@ -1292,7 +1327,49 @@ int pdxg::host::run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq
     return PDXG_OK;
 }
 
-namespace {
+// Launch parameters of the queries from q0 on.
+Launch slice_of(const Launch& L, uint32_t q0, uint32_t nq) {
+    Launch S = L;
+    SearchParams& p = S.p;
+    p.nq = nq;
+    p.queries += (size_t)q0 * p.l1.d;
+    p.out_ids += (size_t)q0 * p.k;
+    p.out_dists += (size_t)q0 * p.k;
+    p.out_counts += q0;
+    if (p.filter_of) p.filter_of += q0;
+    if (p.q_k) p.q_k += q0;
+    if (p.q_nprobe) p.q_nprobe += q0;
+    if (p.q_top) p.q_top += q0;
+    if (p.q_order) {
+        p.q_order += (size_t)q0 * p.q_order_stride;
+        p.q_order_count += q0;
+    }
+    S.grid = (int)std::min<uint32_t>((uint32_t)S.grid, nq);
+    return S;
+}
+
+// Everything after the visit orders: batched Start, cluster-major scan and the per-query kernel for the
+// queries that those leave. Adds the kernels to `launches`.
+int run_scan(pdxg_index* ix, Workspace& w, uint32_t nq, uint32_t n_filtered, const Launch& L, cudaStream_t st,
+             uint32_t& launches, bool timed = false) {
+    const Slices sl = n_filtered < nq ? plan_slices(ix, L, nq) : Slices{nq};
+    const bool whole = sl.rows >= nq;  // kernel times within the scan are those of one slice
+    ix->tev_scan = false;
+    if (timed && !whole) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
+    int rc;
+    for (uint32_t q0 = 0; q0 < nq; q0 += sl.rows) {
+        const uint32_t m = std::min(sl.rows, nq - q0);
+        Launch S = slice_of(L, q0, m);
+        if (sl.visits && m >= kStartMinQueries && (rc = run_start_batched(ix, w, m, sl.visits, S, st))) return rc;
+        if (timed && whole) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
+        if (sl.scan && S.p.start_row && (rc = run_scan_cluster_major(ix, w, m, S, st, timed && whole))) return rc;
+        if ((rc = widen_search(ix, m, std::min(n_filtered, m), S))) return rc;
+        if (!S.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
+        PDXG_CUDA(launch_search(S.p, S.u8, S.threads, S.grid, st));
+        launches += S.start_launches + S.scan_launches + 1;
+    }
+    return PDXG_OK;
+}
 
 // Core device-side search: queries/ids/dists/counts are device pointers. d_filtered: the
 // n_filtered queries with a filter.
@@ -1319,7 +1396,7 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
     // the reduced-precision probe rotates the queries itself (BF16 GEMM)
     const bool gemm_probe = ix->probe_mode != 0 && !d_order && probe_gemm_ok(ix);
     ix->tev_prep = !(flags & PDXG_QUERY_TRANSFORMED) && !gemm_probe;
-    uint32_t launches = 1;  // the scan
+    uint32_t launches = 0;
     if (!(flags & PDXG_QUERY_TRANSFORMED) && !gemm_probe) {
         if ((rc = prepare_dev(ix, w, q, nq, w.d_rq, st))) return rc;
         qp = w.d_rq;
@@ -1376,15 +1453,8 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
         L.p.q_order && !any_filter && (!probe_ahead || nq >= kProbeAheadMinQueries) ? L.p.q_order_stride : 0;
     // the batched Start belongs to the scan's time
     if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[2], st));
-    if (any_plain && (rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
-    launches += L.start_launches;
-    if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
-    if ((rc = run_scan_cluster_major(ix, w, nq, L, st, timed))) return rc;
-    launches += L.scan_launches;
+    if ((rc = run_scan(ix, w, nq, n_filtered, L, st, launches, timed))) return rc;
     ix->last_launches = launches;
-    if ((rc = widen_search(ix, nq, n_filtered, L))) return rc;
-    if (!L.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
-    PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
     if (timed) {
         PDXG_CUDA(cudaEventRecord(ix->tev[4], st));
         ix->tev_ready = true;
@@ -1561,7 +1631,7 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
         if ((rc = dev_grow(w.d_l1_order, w.l1_order_cap, (uint64_t)nq * k1))) return rc;
         if ((rc = dev_grow(w.d_l1_count, w.l1_count_cap, nq))) return rc;
     }
-    uint32_t launches = 1;
+    uint32_t launches = 0;
     bool orders = top;
     for (uint32_t c = 0; c < nch; ++c) {
         const uint32_t off = chunk_off(c), n = chunk_len(c);
@@ -1593,15 +1663,9 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
         if ((rc = run_probe_exact(ix, w, L.p.queries, nq, L, st))) return rc;
         launches += L.probe_launches;
     }
-    if ((rc = run_start_batched(ix, w, L.p.queries, nq, L, st))) return rc;
-    launches += L.start_launches;
-    if ((rc = run_scan_cluster_major(ix, w, nq, L, st))) return rc;
-    launches += L.scan_launches;
-    ix->last_launches = launches;
     ix->last_order_stride = L.p.q_order && !probe_ahead ? k1 : 0;
-    if ((rc = widen_search(ix, nq, 0, L))) return rc;
-    if (!L.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
-    PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
+    if ((rc = run_scan(ix, w, nq, 0, L, st, launches))) return rc;
+    ix->last_launches = launches;
     PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, sizeof(uint32_t) * nq * k, cudaMemcpyDeviceToHost, st));
     PDXG_CUDA(cudaMemcpyAsync(dists, w.d_dists, sizeof(float) * nq * k, cudaMemcpyDeviceToHost, st));
     PDXG_CUDA(cudaMemcpyAsync(counts, w.d_counts, sizeof(uint32_t) * nq, cudaMemcpyDeviceToHost, st));
@@ -2462,25 +2526,16 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
     L.p.queue = w.d_queue;
     if (gemm_probe) {
         if ((rc = run_probe_gemm(ix, w, queries, nq, (flags & PDXG_QUERY_TRANSFORMED) != 0, L, st))) return rc;
-        qp = L.p.queries;
-        if ((rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
     } else if (ix->tree) {
-        if (any_plain) {
-            if ((rc = run_top_level(ix, w, qp, nq, L, st))) return rc;
-            if ((rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
-        }
+        if (any_plain && (rc = run_top_level(ix, w, qp, nq, L, st))) return rc;
         if (any_filter && (L.p.q_order || !any_plain) && probe_exact_ok(ix) &&
             (rc = run_probe_exact(ix, w, qp, nq, L, st, w.d_req + 4 * (uint64_t)nq, n_filtered)))
             return rc;
     } else if (probe_ahead) {
         if ((rc = run_probe_exact(ix, w, qp, nq, L, st))) return rc;
-        if (any_plain && (rc = run_start_batched(ix, w, qp, nq, L, st))) return rc;
     }
-    if ((rc = run_scan_cluster_major(ix, w, nq, L, st))) return rc;
-    if ((rc = widen_search(ix, nq, n_filtered, L))) return rc;
-    if (!L.queue_zeroed) PDXG_CUDA(cudaMemsetAsync(w.d_queue, 0, sizeof(uint32_t), st));
-    PDXG_CUDA(launch_search(L.p, L.u8, L.threads, L.grid, st));
-    return PDXG_OK;
+    uint32_t launches = 0;
+    return run_scan(ix, w, nq, n_filtered, L, st, launches);
 }
 
 int pdxg_filter_register(pdxg_index* ix, const uint64_t* row_ids, uint64_t n, int32_t* filter_id) {

@@ -510,12 +510,16 @@ int start_dist_occupancy(bool u8, size_t smem) {
     return blocks;
 }
 
-// Work items of nq Starts at most; 0 when the items' 16-bit chunk numbers cannot hold them.
-uint64_t start_item_bound(bool u8, uint32_t nq, uint32_t n1, uint32_t max_n) {
+// Starts of one launch at most: an item numbers its query and vector chunks in 16 bits each.
+uint64_t start_max_starts(bool u8, uint32_t max_n) {
+    const uint32_t iv = u8 ? kStartV : kStartVF;
+    return ((uint64_t)max_n + iv - 1) / iv > 65536 ? 0 : 65536ull * (u8 ? kStartQ : kStartQF);
+}
+
+// Work items of `starts` Starts at most.
+uint64_t start_item_bound(bool u8, uint32_t starts, uint32_t n1, uint32_t max_n) {
     const uint32_t iq = u8 ? kStartQ : kStartQF, iv = u8 ? kStartV : kStartVF;
-    const uint64_t nqc = ((uint64_t)nq + iq - 1) / iq, nvc = ((uint64_t)max_n + iv - 1) / iv;
-    if (nqc > 65536 || nvc > 65536) return 0;
-    return (nqc + n1) * nvc;
+    return (((uint64_t)starts + iq - 1) / iq + n1) * (((uint64_t)max_n + iv - 1) / iv);
 }
 
 }  // namespace pdxg
