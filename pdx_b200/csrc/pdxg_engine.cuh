@@ -81,6 +81,8 @@ struct HostLevel {
     }
 };
 
+constexpr uint64_t kSliceBytes = 8ull << 30;  // see plan_slices (pdxg_index.cu)
+
 struct Workspace {
     uint32_t q_cap = 0, k_cap = 0;
     float* d_q = nullptr;
@@ -183,6 +185,10 @@ struct Workspace {
     uint64_t sc_hv_cap = 0;
     uint32_t* d_sc_hb = nullptr;
     uint64_t sc_hb_cap = 0;
+    // bytes that one array of a slice of the scan may take: kSliceBytes, less where the device had no
+    // memory for that (free_at: its free memory then, with the scan's arrays given back)
+    uint64_t room = kSliceBytes;
+    uint64_t free_at = 0;
 };
 
 // Mutable state of a tree index once Append / Delete have been used (PDXTreeIndex,
@@ -244,16 +250,23 @@ struct Launch {
 extern std::atomic<uint64_t> g_alloc_gen;
 
 template <class T>
-int dev_grow(T*& ptr, uint64_t& cap, uint64_t need) {
-    if (need <= cap && ptr) return PDXG_OK;
+cudaError_t dev_try_grow(T*& ptr, uint64_t& cap, uint64_t need) {
+    if (need <= cap && ptr) return cudaSuccess;
     g_alloc_gen.fetch_add(1);
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
     const uint64_t n = std::max<uint64_t>(need, 1);
-    PDXG_CUDA(cudaMalloc(&ptr, n * sizeof(T)));
-    cap = n;
-    return PDXG_OK;
+    const cudaError_t e = cudaMalloc(&ptr, n * sizeof(T));
+    if (e == cudaSuccess) cap = n;
+    else ptr = nullptr;
+    return e;
+}
+
+template <class T>
+int dev_grow(T*& ptr, uint64_t& cap, uint64_t need) {
+    const cudaError_t e = dev_try_grow(ptr, cap, need);
+    return e == cudaSuccess ? PDXG_OK : fail(PDXG_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
 }
 
 // Search plumbing (pdxg_index.cu).

@@ -1049,6 +1049,55 @@ int run_probe_gemm(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq, bo
     return PDXG_OK;
 }
 
+// Every array of the scan's slices as (pointer, capacity).
+template <class F>
+void scan_arrays(Workspace& w, F f) {
+    f(w.d_st_cl, w.st_cl_cap);
+    f(w.d_st_q, w.st_q_cap);
+    f(w.d_st_items, w.st_items_cap);
+    f(w.d_st_dist, w.st_dist_cap);
+    f(w.d_zero, w.zero_cap);
+    f(w.d_sc_qw, w.sc_qw_cap);
+    f(w.d_sc_q, w.sc_q_cap);
+    f(w.d_sc_heap, w.sc_heap_cap);
+    f(w.d_sc_vl, w.sc_vl_cap);
+    f(w.d_sc_items, w.sc_items_cap);
+    f(w.d_sc_bm, w.sc_bm_cap);
+    f(w.d_sc_vi, w.sc_vi_cap);
+    f(w.d_sc_hv, w.sc_hv_cap);
+    f(w.d_sc_hb, w.sc_hb_cap);
+}
+
+// Free device memory, counting what the scan's arrays hold.
+int scan_memory(Workspace& w, uint64_t& bytes) {
+    size_t mem_free = 0, mem_all = 0;
+    PDXG_CUDA(cudaMemGetInfo(&mem_free, &mem_all));
+    bytes = mem_free;
+    scan_arrays(w, [&](auto*& ptr, uint64_t& cap) { bytes += cap * sizeof(*ptr); });
+    return PDXG_OK;
+}
+
+// After an allocation failed: half the room for an array, and at most an eighth of what there is. The
+// workspace keeps that bound, so that a later call (a graph's capture) allocates nothing it did not,
+// until the device has twice the memory (restore_room).
+int shrink_room(Workspace& w) {
+    cudaGetLastError();  // not sticky
+    if (int rc = scan_memory(w, w.free_at)) return rc;
+    w.room = std::min(w.room / 2, w.free_at / 8);
+    return PDXG_OK;
+}
+
+int restore_room(Workspace& w, cudaStream_t st) {
+    if (w.room == kSliceBytes) return PDXG_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PDXG_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return PDXG_OK;
+    uint64_t bytes;
+    if (int rc = scan_memory(w, bytes)) return rc;
+    if (bytes / 2 >= w.free_at) w.room = kSliceBytes;
+    return PDXG_OK;
+}
+
 // Exact probe ahead of the scan (centroid_dist_kernel, probe_pick_kernel): the order of the scan
 // kernel's own probe; lets the scan keep per-vector arrays only, and shares every centroid read
 // among 32 queries. Few queries gain too: 16 filtered queries x 1,000 centroids x 1024 dims spent 580 us
@@ -1071,8 +1120,15 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
     if ((rc = dev_grow(w.d_l1_order, w.l1_order_cap, (uint64_t)nq * k1))) return rc;
     if ((rc = dev_grow(w.d_l1_count, w.l1_count_cap, nq))) return rc;
     ProbeParams pp{};
-    pp.keys_rows = (uint32_t)std::min<uint64_t>(rows, std::max<uint64_t>(kProbeKeysMax / n1, 32));
-    if ((rc = dev_grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)pp.keys_rows * n1))) return rc;
+    if ((rc = restore_room(w, st))) return rc;
+    for (cudaError_t e;;) {
+        pp.keys_rows = (uint32_t)std::min<uint64_t>(rows, std::max<uint64_t>(std::min(kProbeKeysMax, w.room / 4) / n1, 32));
+        e = dev_try_grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)pp.keys_rows * n1);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation || pp.keys_rows <= 32)
+            return fail(PDXG_ERR_CUDA, std::string("probe distances: ") + cudaGetErrorString(e));
+        if ((rc = shrink_room(w))) return rc;
+    }
     pp.keys = w.d_pr_keys;
     pp.q_list = d_list;
     pp.queries = qp;
@@ -1116,15 +1172,16 @@ uint32_t start_visits(const HostLevel& lv, uint32_t k) {
 constexpr uint32_t kHeavyPerQuery = 128, kHeavyPerQueryMin = 16;
 constexpr uint64_t kHeavyMaxValues = 64ull << 20;
 
-uint64_t heavy_columns_max(const DevLevel& lv, uint32_t& ncp) {
+uint64_t heavy_columns_max(const DevLevel& lv, uint64_t room, uint32_t& ncp) {
     uint32_t cps[kMaxCheckpoints];
     ncp = warmup_checkpoints(lv.dv, cps, kMaxCheckpoints);
-    return ncp > (uint32_t)kMaxCheckpoints ? 0 : kHeavyMaxValues / ((uint64_t)ncp + lv.n_hblocks);
+    const uint64_t values = std::min(kHeavyMaxValues, room / 64);
+    return ncp > (uint32_t)kMaxCheckpoints ? 0 : values / ((uint64_t)ncp + lv.n_hblocks);
 }
 
-uint32_t heavy_columns(const DevLevel& lv, uint32_t nq, uint32_t& ncp) {
+uint32_t heavy_columns(const DevLevel& lv, uint32_t nq, uint64_t room, uint32_t& ncp) {
     const uint64_t cap = std::max<uint64_t>((uint64_t)nq * kHeavyPerQuery, 32768);
-    return (uint32_t)std::min<uint64_t>(cap, heavy_columns_max(lv, ncp)) / 32 * 32;
+    return (uint32_t)std::min<uint64_t>(cap, heavy_columns_max(lv, room, ncp)) / 32 * 32;
 }
 
 // Shared memory of a replay warp (pdxg_scan.cu), in ScanParams' fields.
@@ -1145,15 +1202,16 @@ uint64_t replay_warp_bytes(const DevLevel& lv, uint32_t k, ScanParams& sp) {
 // queries on 1,000 clusters with 4,000-vector bitmaps took 14.1 ms instead of 8.1. A batch past a
 // limit left the route before: 20,000 of those queries took 63 ms in the per-query kernel (16.2 in two
 // slices), 140,000 F32 queries with four Starts each 8.7 (5.9).
-constexpr uint64_t kSliceBytes = 8ull << 30;
-
+//
+// The per-query kernel needs none of these arrays. So a device without memory for them gets smaller
+// slices (`room`, see reserve_slices), down to none at all.
 struct Slices {
     uint32_t rows;        // a multiple of 32, or the whole batch
     uint32_t visits = 0;  // batched Starts of a query (0: none, the per-query kernel runs Start itself)
     bool scan = false;    // cluster-major
 };
 
-Slices plan_slices(const pdxg_index* ix, const Launch& L, uint32_t nq) {
+Slices plan_slices(const pdxg_index* ix, const Launch& L, uint32_t nq, uint64_t room) {
     Slices s{nq};
     // the visit orders are known before the scan (tree indexes with a separate top level, probes ahead)
     if (!L.p.q_order || ix->start_mode == 1 || nq < kStartMinQueries) return s;
@@ -1161,7 +1219,7 @@ Slices plan_slices(const pdxg_index* ix, const Launch& L, uint32_t nq) {
     const uint32_t n1 = lv.nclusters, k = L.p.k, max_n = std::max(lv.max_n, 1u), k1 = L.p.q_order_stride;
     const size_t smem = start_dist_smem(lv);
     if (smem + 1024 > ix->max_smem || start_dist_occupancy(ix->u8, smem) <= 0) return s;
-    const uint64_t starts = std::min<uint64_t>(start_max_starts(ix->u8, max_n), kSliceBytes / (4ull * ((max_n + 3) & ~3u)));
+    const uint64_t starts = std::min<uint64_t>(start_max_starts(ix->u8, max_n), room / (4ull * ((max_n + 3) & ~3u)));
     uint32_t visits = start_visits(ix->l1, k);
     while (visits > 1 && starts / visits < kStartMinQueries) --visits;
     uint64_t rows = std::min<uint64_t>(starts / visits, 1u << 20);
@@ -1171,9 +1229,9 @@ Slices plan_slices(const pdxg_index* ix, const Launch& L, uint32_t nq) {
     if (ix->scan_mode == 0 && !L.p.order && !lv.tomb && k1 > 0 &&
         replay_warp_bytes(lv, k, sp) * scan_queries_per_cta() + 2048 <= ix->max_smem) {
         uint32_t ncp;
-        const uint64_t heavy = std::max<uint64_t>(heavy_columns_max(lv, ncp) / kHeavyPerQueryMin, 4096);
-        const uint64_t m = std::min<uint64_t>({kSliceBytes / (4ull * k1 * sp.bm_words), kSliceBytes / (4ull * n1),
-                                     kSliceBytes / (8ull * k), heavy});
+        const uint64_t heavy = std::max<uint64_t>(heavy_columns_max(lv, room, ncp) / kHeavyPerQueryMin, 4096);
+        const uint64_t m = std::min<uint64_t>({room / (4ull * k1 * sp.bm_words), room / (4ull * n1),
+                                     room / (8ull * k), heavy});
         if (m >= kStartMinQueries) {
             s.scan = true;
             rows = std::min(rows, m);
@@ -1186,26 +1244,69 @@ Slices plan_slices(const pdxg_index* ix, const Launch& L, uint32_t nq) {
     return s;
 }
 
+// The arrays of a slice as (pointer, capacity, elements) through `f`, until it fails.
+template <class F>
+cudaError_t slice_arrays(const pdxg_index* ix, Workspace& w, const Launch& L, const Slices& sl, F f) {
+    cudaError_t e = cudaSuccess;
+    auto array = [&](auto*& ptr, uint64_t& cap, uint64_t n) {
+        if (e == cudaSuccess) e = f(ptr, cap, n);
+    };
+    const DevLevel& lv = L.p.l1;
+    const uint64_t n1 = lv.nclusters, max_n = std::max(lv.max_n, 1u), nq = sl.rows, ne = nq * sl.visits;
+    uint32_t ncp = 0;
+    const uint64_t hv_cap = heavy_columns(lv, sl.rows, w.room, ncp);
+    if (!sl.visits) return e;
+    array(w.d_st_cl, w.st_cl_cap, 3 * n1);
+    array(w.d_st_q, w.st_q_cap, 4 * ne + 2 * nq + 3);
+    if (ix->u8) array(w.d_sc_qw, w.sc_qw_cap, nq * (lv.qw_hoff + lv.n_hblocks * 16ull));
+    array(w.d_st_items, w.st_items_cap, 2 * start_item_bound(ix->u8, (uint32_t)ne, (uint32_t)n1, (uint32_t)max_n));
+    array(w.d_st_dist, w.st_dist_cap, ne * ((max_n + 3) / 4 * 4));
+    array(w.d_zero, w.zero_cap, 8 + n1 + hv_cap);
+    if (!sl.scan) return e;
+    const uint64_t visits = nq * L.p.q_order_stride;
+    array(w.d_sc_hv, w.sc_hv_cap, (ncp + lv.n_hblocks) * hv_cap);
+    array(w.d_sc_hb, w.sc_hb_cap, std::max<uint64_t>(hv_cap / 16, 1));
+    array(w.d_sc_vi, w.sc_vi_cap, visits);
+    array(w.d_sc_q, w.sc_q_cap, 3 * nq);
+    array(w.d_sc_heap, w.sc_heap_cap, 2 * nq * L.p.k);
+    array(w.d_sc_vl, w.sc_vl_cap, n1 * nq);
+    array(w.d_sc_items, w.sc_items_cap, 2 * scan_item_bound(sl.rows, L.p.q_order_stride, (uint32_t)n1, (uint32_t)max_n));
+    array(w.d_sc_bm, w.sc_bm_cap, visits * ((max_n + 31) / 32));
+    return e;
+}
+
+// Plans the slices of a batch and allocates their arrays. Without the memory for them the arrays are
+// given back and smaller slices planned.
+int reserve_slices(pdxg_index* ix, Workspace& w, const Launch& L, uint32_t nq, Slices& sl, cudaStream_t st) {
+    if (int rc = restore_room(w, st)) return rc;
+    for (;;) {
+        sl = plan_slices(ix, L, nq, w.room);
+        const cudaError_t e = slice_arrays(ix, w, L, sl, [](auto*& ptr, uint64_t& cap, uint64_t n) {
+            return dev_try_grow(ptr, cap, n);
+        });
+        if (e == cudaSuccess) return PDXG_OK;
+        if (e != cudaErrorMemoryAllocation) return fail(PDXG_ERR_CUDA, std::string("scan arrays: ") + cudaGetErrorString(e));
+        g_alloc_gen.fetch_add(1);
+        scan_arrays(w, [](auto*& ptr, uint64_t& cap) {
+            cudaFree(ptr);
+            ptr = nullptr;
+            cap = 0;
+        });
+        if (int rc = shrink_room(w)) return rc;
+    }
+}
+
 // Batched Start (pdxg_start.cu) of nq queries, `visits` each; sets L.p.start_*.
 int run_start_batched(pdxg_index* ix, Workspace& w, uint32_t nq, uint32_t visits, Launch& L, cudaStream_t st) {
     const uint32_t n1 = L.p.l1.nclusters;
     const uint32_t stride = (std::max(L.p.l1.max_n, 1u) + 3) & ~3u;
     const uint64_t ne = (uint64_t)nq * visits;
-    const uint64_t items = start_item_bound(ix->u8, (uint32_t)ne, n1, std::max(L.p.l1.max_n, 1u));
     const int occ = start_dist_occupancy(ix->u8, start_dist_smem(L.p.l1));
-    int rc;
-    if ((rc = dev_grow(w.d_st_cl, w.st_cl_cap, (uint64_t)3 * n1))) return rc;
-    if ((rc = dev_grow(w.d_st_q, w.st_q_cap, 4 * ne + 2ull * nq + 3))) return rc;
     const uint32_t nwords = L.p.l1.qw_hoff + L.p.l1.n_hblocks * 16;
-    if (ix->u8 && (rc = dev_grow(w.d_sc_qw, w.sc_qw_cap, (uint64_t)nq * nwords))) return rc;
-    if ((rc = dev_grow(w.d_st_items, w.st_items_cap, 2 * items))) return rc;
-    if ((rc = dev_grow(w.d_st_dist, w.st_dist_cap, ne * stride))) return rc;
     uint32_t ncp = 0;
-    const uint64_t n_zero = 8ull + n1 + heavy_columns(L.p.l1, nq, ncp);
-    if ((rc = dev_grow(w.d_zero, w.zero_cap, n_zero))) return rc;
     StartParams sp{};
     sp.zero = w.d_zero;
-    sp.n_zero = (uint32_t)n_zero;
+    sp.n_zero = 8 + n1 + heavy_columns(L.p.l1, nq, w.room, ncp);
     sp.arena = ix->arena;
     sp.l1 = L.p.l1;
     sp.queries = L.p.queries;
@@ -1262,17 +1363,7 @@ int run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq, Launch& L,
     // warps share the heavy visits
     sp.r_qpc = std::min<uint32_t>(scan_queries_per_cta(), (nq + 2 * ix->num_sms - 1) / (2 * ix->num_sms));
     const uint64_t items = scan_item_bound(nq, stride, n1, std::max(lv.max_n, 1u));
-    sp.hv_cap = heavy_columns(lv, nq, sp.hv_ncp);
-    const uint64_t hv_rows = (uint64_t)sp.hv_ncp + lv.n_hblocks;
-    int rc;
-    if ((rc = dev_grow(w.d_sc_hv, w.sc_hv_cap, hv_rows * sp.hv_cap))) return rc;
-    if ((rc = dev_grow(w.d_sc_vi, w.sc_vi_cap, (uint64_t)nq * stride))) return rc;
-    if ((rc = dev_grow(w.d_sc_q, w.sc_q_cap, 3ull * nq))) return rc;
-    if ((rc = dev_grow(w.d_sc_hb, w.sc_hb_cap, std::max<uint64_t>(sp.hv_cap / 16, 1)))) return rc;
-    if ((rc = dev_grow(w.d_sc_heap, w.sc_heap_cap, 2ull * nq * k))) return rc;
-    if ((rc = dev_grow(w.d_sc_vl, w.sc_vl_cap, (uint64_t)n1 * nq))) return rc;
-    if ((rc = dev_grow(w.d_sc_items, w.sc_items_cap, 2 * items))) return rc;
-    if ((rc = dev_grow(w.d_sc_bm, w.sc_bm_cap, (uint64_t)nq * stride * bm_words))) return rc;
+    sp.hv_cap = heavy_columns(lv, nq, w.room, sp.hv_ncp);
     sp.arena = L.p.arena;
     sp.l1 = lv;
     sp.ratios = L.p.ratios;
@@ -1352,11 +1443,12 @@ Launch slice_of(const Launch& L, uint32_t q0, uint32_t nq) {
 // queries that those leave. Adds the kernels to `launches`.
 int run_scan(pdxg_index* ix, Workspace& w, uint32_t nq, uint32_t n_filtered, const Launch& L, cudaStream_t st,
              uint32_t& launches, bool timed = false) {
-    const Slices sl = n_filtered < nq ? plan_slices(ix, L, nq) : Slices{nq};
+    int rc;
+    Slices sl{nq};
+    if (n_filtered < nq && (rc = reserve_slices(ix, w, L, nq, sl, st))) return rc;
     const bool whole = sl.rows >= nq;  // kernel times within the scan are those of one slice
     ix->tev_scan = false;
     if (timed && !whole) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
-    int rc;
     for (uint32_t q0 = 0; q0 < nq; q0 += sl.rows) {
         const uint32_t m = std::min(sl.rows, nq - q0);
         Launch S = slice_of(L, q0, m);
@@ -1567,11 +1659,17 @@ struct FilterLists {
 int build_filters_device(pdxg_index* ix, Workspace& w, const FilterLists& fl, cudaStream_t st) {
     if (int rc = flush_maintenance(ix, st)) return rc;  // the device row maps
     const uint32_t nf = (uint32_t)fl.foff.size() - 1, words = ix->l1.sel_words, n1 = (uint32_t)ix->l1.fc.size();
-    constexpr unsigned long long kChunk = 32ull << 20;
+    unsigned long long chunk = 32ull << 20;
     const unsigned long long first = fl.foff[0], last = fl.foff[nf];
     int rc;
     if ((rc = dev_grow(w.d_foff, w.foff_cap, (uint64_t)nf + 1))) return rc;
-    if ((rc = dev_grow(w.d_rows64, w.rows64_cap, std::max<uint64_t>(std::min(last - first, kChunk), 1)))) return rc;
+    // smaller pieces where the device has no memory for that
+    while (chunk > 4096 && dev_try_grow(w.d_rows64, w.rows64_cap, std::max<uint64_t>(std::min(last - first, chunk), 1)) ==
+                               cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        chunk /= 8;
+    }
+    if ((rc = dev_grow(w.d_rows64, w.rows64_cap, std::max<uint64_t>(std::min(last - first, chunk), 1)))) return rc;
     if ((rc = dev_grow(w.d_sel, w.sel_cap, (uint64_t)nf * words))) return rc;
     if ((rc = dev_grow(w.d_pass, w.pass_cap, (uint64_t)nf * n1))) return rc;
     PDXG_CUDA(cudaMemcpyAsync(w.d_foff, fl.foff.data(), (size_t)(nf + 1) * 8, cudaMemcpyHostToDevice, st));
@@ -1579,8 +1677,8 @@ int build_filters_device(pdxg_index* ix, Workspace& w, const FilterLists& fl, cu
     PDXG_CUDA(cudaMemsetAsync(w.d_pass, 0, (size_t)nf * n1 * 4, st));
     unsigned long long max_len = 0;
     for (uint32_t f = 0; f < nf; ++f) max_len = std::max(max_len, fl.foff[f + 1] - fl.foff[f]);
-    for (unsigned long long r0 = first; r0 < last; r0 += kChunk) {
-        const unsigned long long r1 = std::min(last, r0 + kChunk);
+    for (unsigned long long r0 = first; r0 < last; r0 += chunk) {
+        const unsigned long long r1 = std::min(last, r0 + chunk);
         PDXG_CUDA(cudaMemcpyAsync(w.d_rows64, fl.rows + r0, (size_t)(r1 - r0) * 8, cudaMemcpyHostToDevice, st));
         for (uint32_t f0 = 0; f0 < nf; f0 += 65535) {
             const uint32_t m = std::min(nf - f0, 65535u);

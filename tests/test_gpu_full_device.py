@@ -1,0 +1,56 @@
+"""Searches on a device whose memory is nearly used up: the arrays of the batched Start, the scan and the
+centroid probe shrink to what there is (pdxg_index.cu), results stay the same, the batch can still be
+captured, and with the memory free again the next search takes its whole batch at once."""
+import numpy as np
+import pytest
+
+from pdx_b200 import compiled
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("itype", ["pdx_f32", "pdx_u8"])
+def test_arrays_shrink_to_the_free_memory(itype):
+    import torch
+    n, d, nq, k = 20_000, 16, 60_000, 10
+    rng = np.random.default_rng(5)
+    ix = compiled.PDXIndex(itype, d, seed=11, num_clusters=10, normalize=False)
+    ix.build_index(rng.standard_normal((n, d)).astype(np.float32))
+    ix.set_nprobe(0)
+    q = torch.from_numpy(ix.prepare_queries(rng.standard_normal((nq, d)).astype(np.float32))).cuda()
+    ids = torch.empty(nq, k, dtype=torch.int32, device="cuda")
+    dist = torch.empty(nq, k, device="cuda")
+    cnt = torch.empty(nq, dtype=torch.int32, device="cuda")
+
+    def run(index, m=nq, graph=False):
+        args = (q.data_ptr(), m, k, ids.data_ptr(), dist.data_ptr(), cnt.data_ptr())
+        if graph:
+            index.capture(*args, transformed=True).launch(0)
+        else:
+            index.search_device(*args, transformed=True)
+        torch.cuda.synchronize()
+        return [x.cpu().numpy().copy() for x in (ids, dist, cnt)]
+
+    run(ix, 3000)  # the kernels of every route are loaded
+    ix.set_scan_mode(1)
+    ix.set_start_mode(1)
+    expect = run(ix)  # the per-query route: its buffers are there from now on
+    ix.set_scan_mode(0)
+    ix.set_start_mode(0)
+    torch.cuda.empty_cache()
+    filler = []
+    for keep in (8 << 30, 160 << 20):
+        size = torch.cuda.mem_get_info()[0] - keep
+        if size > 0:
+            filler.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+    try:
+        for graph in (False, True):
+            for a, b in zip(run(ix, graph=graph), expect):
+                np.testing.assert_array_equal(a, b)
+            sliced = ix.last_launch_count()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    for a, b in zip(run(ix), expect):
+        np.testing.assert_array_equal(a, b)
+    assert ix.last_launch_count() < sliced
