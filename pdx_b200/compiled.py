@@ -403,7 +403,8 @@ class PDXIndex:
         _check(library().pdxg_set_start_mode(self._handle().ptr, int(mode)))
 
     def autotune(self, queries_ptr: int, nq: int, knn: int, transformed: bool = False) -> dict:
-        """Times the engine's forms on this batch of device queries and keeps the fastest."""
+        """Times the engine's forms on this batch of device queries and keeps the fastest. The threads per
+        query stay automatic (128 for a batch) where the batch takes the cluster-major scan."""
         out = np.zeros(3, np.uint32)
         _check(library().pdxg_autotune(self._handle().ptr, C.c_void_p(queries_ptr), nq, knn,
                                        PDXG_QUERY_TRANSFORMED if transformed else 0, out.ctypes.data))

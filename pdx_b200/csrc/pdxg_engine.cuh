@@ -361,6 +361,7 @@ struct pdxg_index {
     // (after the meso probe, after the partials)
     cudaEvent_t tev[10] = {};
     bool tev_ready = false, tev_top = false, tev_prep = false, tev_scan = false, tev_tiled = false;
+    bool last_cluster_major = false;  // the last search of this index took the cluster-major scan
     uint32_t last_launches = 0;  // engine kernels launched by the last search_device_impl
     uint32_t last_order_stride = 0;  // row stride of the visit orders of the last search (0: none)
     pdxg::host::Workspace ws;

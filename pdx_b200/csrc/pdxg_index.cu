@@ -1446,6 +1446,7 @@ int run_scan(pdxg_index* ix, Workspace& w, uint32_t nq, uint32_t n_filtered, con
     int rc;
     Slices sl{nq};
     if (n_filtered < nq && (rc = reserve_slices(ix, w, L, nq, sl, st))) return rc;
+    ix->last_cluster_major = sl.scan;
     const bool whole = sl.rows >= nq;  // kernel times within the scan are those of one slice
     ix->tev_scan = false;
     if (timed && !whole) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
@@ -2117,18 +2118,20 @@ int pdxg_autotune(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k,
     if (rc == PDXG_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
         rc = fail(PDXG_ERR_CUDA, "cannot create events");
     const uint32_t old_threads = ix->threads, old_top = ix->top_mode, old_start = ix->start_mode;
-    const uint32_t threads_c[3] = {64, 128, 256};
+    const uint32_t threads_c[4] = {0, 64, 128, 256};
     const uint32_t tops_c[2] = {3, 2};
     const uint32_t starts_c[2] = {0, 1};
     const uint32_t ntop = ix->tree ? 2 : 1, nstart = (ix->tree && ix->u8) ? 2 : 1;
     float best = 1e30f;
     uint32_t bt = old_threads, btop = old_top, bstart = old_start;
-    for (uint32_t a = 0; a < 3 && rc == PDXG_OK; ++a)
-        for (uint32_t b = 0; b < ntop && rc == PDXG_OK; ++b)
-            for (uint32_t c = 0; c < nstart && rc == PDXG_OK; ++c) {
+    for (uint32_t b = 0; b < ntop && rc == PDXG_OK; ++b)
+        for (uint32_t c = 0; c < nstart && rc == PDXG_OK; ++c) {
+            ix->top_mode = ix->tree ? tops_c[b] : old_top;
+            ix->start_mode = starts_c[c];
+            // the automatic width first; it stays where the batch takes the cluster-major scan, which has
+            // no threads per query (a fixed one would also hold for later filtered and single searches)
+            for (uint32_t a = 0; a < 4 && rc == PDXG_OK && !(a == 1 && ix->last_cluster_major); ++a) {
                 ix->threads = threads_c[a];
-                ix->top_mode = ix->tree ? tops_c[b] : old_top;
-                ix->start_mode = starts_c[c];
                 float t_min = 1e30f;
                 for (int rep = 0; rep < 4 && rc == PDXG_OK; ++rep) {
                     if (cudaEventRecord(e0, ix->stream) != cudaSuccess) rc = fail(PDXG_ERR_CUDA, "event");
@@ -2142,18 +2145,19 @@ int pdxg_autotune(pdxg_index* ix, const float* queries, uint32_t nq, uint32_t k,
                     if (rc == PDXG_OK && rep > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
                         t_min = std::min(t_min, ms);  // the first run of a form warms it up
                 }
-                if (rc == PDXG_OK && t_min < best) {
+                if (rc == PDXG_OK && t_min < best && (threads_c[a] != 0 || ix->last_cluster_major)) {
                     best = t_min;
                     bt = ix->threads;
                     btop = ix->top_mode;
                     bstart = ix->start_mode;
                 }
             }
+        }
     if (rc == PDXG_OK) rc = check_gemm_error(ix->ws);
     ix->threads = rc == PDXG_OK ? bt : old_threads;
     ix->top_mode = rc == PDXG_OK ? btop : old_top;
     ix->start_mode = rc == PDXG_OK ? bstart : old_start;
-    choice[0] = ix->threads;
+    choice[0] = ix->threads ? ix->threads : 128;  // what the automatic width is for a batch
     choice[1] = ix->top_mode;
     choice[2] = ix->start_mode;
     if (e0) cudaEventDestroy(e0);
