@@ -14,9 +14,11 @@ rotation, top-level (meso) search and the pruned PDX scan of 32 clusters per que
                own batch against their own replica of the index: weak scaling).
 * e2e       -- the same through the C ABI's host-buffer entry point (pdxg_search): pinned host
                queries in, host results out, copies inside the timed region.
-* roofline  -- the search kernel alone: algorithmic bytes (index bytes the PDXearch algorithm
-               reads, counted in-kernel) / its average event-timed duration, against the
-               measured HBM copy bandwidth.
+* roofline  -- the part of the step that streams the index from HBM, the batched Start: the bytes
+               it cannot do without (every cluster that some query starts in read once, the
+               distances written once) / its average event-timed duration, against the measured
+               HBM copy bandwidth. A step without a batched Start reports the per-query scan with
+               the bytes it reads per query.
 * cpu_baseline -- the reference's own search code (oracle/_ref, compiled from its headers) on
                this host's cores over a bounded sample of the same queries.
 `--impl reference` times that reference CPU search as the benchmark's reference arm.
@@ -299,6 +301,30 @@ def unique_bytes(ix, nq, nprobe, elem):
             "first_checkpoint_rows": int(size[later].sum()) * cp1 * elem,
             "clusters_started": int(first.sum()), "clusters_visited_later": int(later.sum()),
             "visits": visits}
+
+
+def roofline(stats, unique, kernels_ms, d, elem, peak, peak_src):
+    """Roofline entry of one batch: last_stats(), unique_bytes() (None without visit orders) and
+    kernel_times() in ms. Bytes that many queries read from one cluster count once where one kernel
+    reads the cluster for all of them (the batched Start); the scan after it reads the first rows of
+    clusters that L2 holds, so its per-query bytes are no HBM traffic and make no fraction of it."""
+    bp = stats["bytes_by_phase"]
+    batched = kernels_ms["start"] > 0.0 and unique is not None
+    if batched:
+        kernel, ms = "batched Start (start_count, start_plan, start_rows, start_dist)", kernels_ms["start"]
+        total = unique["start_rows"] + bp["start"] // (d * elem) * 4
+    else:
+        kernel, ms = "search_kernel", kernels_ms["search_kernel"]
+        total = sum(bp[p] for p in ("start", "warmup", "survivor_horizontal", "survivor_vertical", "probe"))
+    achieved = total / (ms / 1e3) / 1e9
+    out = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+           "frac": round(achieved / peak, 4), "kernel": kernel, "kernel_ms": round(ms, 3),
+           "algorithmic_bytes_per_launch": total, "peak_source": peak_src}
+    if batched:
+        out["per_query_bytes"] = {"start": bp["start"], "scan": bp["warmup"] + bp["survivor_horizontal"] +
+                                  bp["survivor_vertical"]}
+        out["unique_bytes"] = unique
+    return out
 
 
 def recall_at(ids, counts, gt, k):
@@ -590,13 +616,13 @@ def main():
     total_ms = max_over_ranks(sum(step_ms), device)
     value = whole_job_qps(nq, args.steps, world, total_ms)
 
-    # ---- roofline of the search kernel alone (prepared queries, same batch)
+    # ---- roofline (prepared queries, same batch)
     prepared = torch.from_numpy(ix.prepare_queries(Qh)).to(device)
     ix.search_device(prepared.data_ptr(), nq, k, ids_dev.data_ptr(), dist_dev.data_ptr(),
                      cnt_dev.data_ptr(), stream=sp, transformed=True, stats=True)
     stats = ix.last_stats()
     scan_stats = ix.last_scan_stats()
-    # the scan kernel alone: events the engine records around its own launches on `stream`
+    # the stages alone: events the engine records around its own launches on `stream`
     times = []
     for i in range(args.steps):
         ix.search_device(q_dev.data_ptr(), nq, k, ids_dev.data_ptr(), dist_dev.data_ptr(),
@@ -605,28 +631,19 @@ def main():
         flush.zero_()
     torch.cuda.synchronize()
     kernels_ms = {key: round(statistics.mean(t[key] for t in times), 4) for key in times[0]}
-    kern_ms = statistics.mean(t["search_kernel"] for t in times)
-    start_ms = statistics.mean(t["start"] for t in times)
-    top_ms = statistics.mean(t["top_level"] for t in times)
-    prep_ms = statistics.mean(t["prepare"] for t in times)
-    bp = stats["bytes_by_phase"]
-    batched_start = start_ms > 0.0
-    # index bytes the scan kernel itself reads per the algorithm: warmup rows, survivor rows,
-    # centroids of an in-kernel probe, and for each query's first cluster either its full
-    # vectors (Start in the kernel) or the 4-byte distances the batched Start wrote for it
-    start_reads = (bp["start"] // d) * 4 if batched_start else bp["start"]
-    scan_bytes = bp["warmup"] + bp["survivor_horizontal"] + bp["survivor_vertical"] + bp["probe"] + start_reads
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(peaks_path):
         peak = float(json.load(open(peaks_path))["hbm_gbs"])
         peak_src = "measured"
     else:
         peak, peak_src = 6650.0, "fallback"
-    achieved = scan_bytes / (kern_ms / 1e3) / 1e9
-    traffic = None
+    try:
+        unique = unique_bytes(ix, nq, cfg["nprobe"] or ix.get_num_clusters(), 1 if "u8" in cfg["itype"] else 4)
+    except ValueError:  # the orders were computed inside the scan
+        unique = None
+    roof = roofline(stats, unique, kernels_ms, d, 1 if "u8" in cfg["itype"] else 4, peak, peak_src)
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(tpath):
-        traffic = json.load(open(tpath)).get(args.config)
+    roof["traffic"] = json.load(open(tpath)).get(args.config) if os.path.exists(tpath) else None
 
     # ---- probe-set error against the FP64 nearest L1 centroids (probe modes 1 and 2)
     probe = None
@@ -726,17 +743,7 @@ def main():
                 "autotuned": tuned if tuned else "off",
                 "step_launch": "CUDA graph" if graph is not None else "direct",
             },
-            "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                         "frac": round(achieved / peak, 4), "traffic": traffic,
-                         "kernel": "search_kernel", "kernel_ms": round(kern_ms, 3),
-                         "algorithmic_bytes_per_launch": scan_bytes, "peak_source": peak_src,
-                         "other_kernels_ms": {("precision probe (rotation + scores + select)" if probe_mode
-                                               else "tree top level"): round(top_ms, 3),
-                                              "batched start": round(start_ms, 3),
-                                              "query preparation": round(prep_ms, 3)},
-                         "batched_start_replaces_bytes": bp["start"] if batched_start else 0,
-                         "top_level_bytes_l2_resident": bp["top_level"],
-                         "clusters_visited": stats["clusters_visited"],
+            "roofline": {**roof, "clusters_visited": stats["clusters_visited"],
                          "kernels_ms": kernels_ms,
                          "scan_counters": scan_stats,
                          "bytes_by_phase": stats["bytes_by_phase"],
