@@ -460,6 +460,14 @@ def main():
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     cfg = dict(CONFIGS[args.config])
+    if args.impl == "reference":
+        from oracle.oracle import Reference
+        if not Reference.available(reference_lib_flavour()):
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable":
+                                  "oracle/_ref is not built: the reference's sources were not present at build time"}),
+                      flush=True)
+            return
     if args.nprobe is not None:
         cfg["nprobe"] = args.nprobe
     if args.nq is not None:
