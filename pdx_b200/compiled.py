@@ -399,7 +399,7 @@ class PDXIndex:
         _check(library().pdxg_set_top_level_mode(self._handle().ptr, int(mode)))
 
     def set_start_mode(self, mode: int) -> None:
-        """U8 tree indexes: 0 batched first-cluster Start when it fits, 1 inside the scan."""
+        """0 batched Starts ahead of the scan when they fit (32 queries or more), 1 inside the scan."""
         _check(library().pdxg_set_start_mode(self._handle().ptr, int(mode)))
 
     def autotune(self, queries_ptr: int, nq: int, knn: int, transformed: bool = False) -> dict:
@@ -443,7 +443,7 @@ class PDXIndex:
         _check(library().pdxg_set_threads_per_query(self._handle().ptr, int(threads)))
 
     def set_scan_mode(self, mode: int) -> None:
-        """U8 scan after a batched Start: 0 cluster-major (default), 1 the per-query kernel only."""
+        """Scan after a batched Start: 0 cluster-major (default), 1 the per-query kernel only."""
         _check(library().pdxg_set_scan_mode(self._handle().ptr, int(mode)))
 
     def register_filter(self, row_ids: np.ndarray) -> int:

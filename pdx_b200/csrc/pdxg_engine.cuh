@@ -332,9 +332,9 @@ struct pdxg_index {
     uint32_t threads = 0;
     uint32_t top_mode = 0;  // tree top level: 0 auto, 1 inside the search CTA, 2 own launch of
                             // per-query CTAs, 3 tiled (probe, partials, replay)
-    uint32_t start_mode = 0;  // U8 first-cluster Start: 0 batched when it fits, 1 in the scan
-    uint32_t scan_mode = 0;   // U8 scan after a batched Start: 0 cluster-major when it fits,
-                              // 1 the per-query kernel only
+    uint32_t start_mode = 0;  // Start: 0 batched when it fits, 1 in the scan
+    uint32_t scan_mode = 0;   // scan after a batched Start: 0 cluster-major when it fits, 1 the
+                              // per-query kernel only
     // centroid probe: 0 the reference's (exact FP32 probe / tree top-level search), 1 BF16
     // tensor-core rotation and centroid scores + widened list + FP32 rescore, 2 the same with
     // FP8-E4M3 centroid scores. Operands are built on first use.
@@ -353,12 +353,10 @@ struct pdxg_index {
     cudaStream_t copy_stream = nullptr;  // host-buffer search: query upload of later chunks
     cudaEvent_t chunk_ev[8] = {};
     cudaStream_t stats_stream = nullptr;
-    // PDXG_TIME_KERNELS marks: start, after preparation, after top level / probe, after the
-    // batched Start, end
     // PDXG_TIME_KERNELS: [0..4] stage boundaries (start, after query preparation, after the top
     // level, after the batched Start, after the scan); [5..7] inside the cluster-major scan (after
     // its planning kernels, after the bitmaps, after the replay); [8..9] inside the tiled top level
-    // (after the meso probe, after the partials)
+    // (after the meso probe, after the partials). A batch in slices counts as scan from the Start on.
     cudaEvent_t tev[10] = {};
     bool tev_ready = false, tev_top = false, tev_prep = false, tev_scan = false, tev_tiled = false;
     bool last_cluster_major = false;  // the last search of this index took the cluster-major scan

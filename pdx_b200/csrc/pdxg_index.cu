@@ -1411,7 +1411,7 @@ int run_scan_cluster_major(pdxg_index* ix, Workspace& w, uint32_t nq, Launch& L,
     sp.out_counts = L.p.out_counts;
     sp.stats = L.p.stats;
     PDXG_CUDA(launch_scan(sp, st, timed ? ix->tev + 5 : nullptr));
-    ix->tev_scan = timed;
+    if (timed) ix->tev_scan = true;
     L.p.q_list = sp.left;
     L.p.q_list_n = sp.left_n;
     L.scan_launches = 3;
@@ -1440,15 +1440,18 @@ Launch slice_of(const Launch& L, uint32_t q0, uint32_t nq) {
 }
 
 // Everything after the visit orders: batched Start, cluster-major scan and the per-query kernel for the
-// queries that those leave. Adds the kernels to `launches`.
+// queries that those leave. Adds the kernels to `launches`. `one` (a search of the index itself, not of a
+// context): the index's records of that search are kept, and its times with `timed`.
 int run_scan(pdxg_index* ix, Workspace& w, uint32_t nq, uint32_t n_filtered, const Launch& L, cudaStream_t st,
-             uint32_t& launches, bool timed = false) {
+             uint32_t& launches, bool one, bool timed = false) {
     int rc;
     Slices sl{nq};
     if (n_filtered < nq && (rc = reserve_slices(ix, w, L, nq, sl, st))) return rc;
-    ix->last_cluster_major = sl.scan;
     const bool whole = sl.rows >= nq;  // kernel times within the scan are those of one slice
-    ix->tev_scan = false;
+    if (one) {
+        ix->last_cluster_major = sl.scan;
+        ix->tev_scan = false;
+    }
     if (timed && !whole) PDXG_CUDA(cudaEventRecord(ix->tev[3], st));
     for (uint32_t q0 = 0; q0 < nq; q0 += sl.rows) {
         const uint32_t m = std::min(sl.rows, nq - q0);
@@ -1546,7 +1549,7 @@ int search_device_impl(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq
         L.p.q_order && !any_filter && (!probe_ahead || nq >= kProbeAheadMinQueries) ? L.p.q_order_stride : 0;
     // the batched Start belongs to the scan's time
     if (timed) PDXG_CUDA(cudaEventRecord(ix->tev[2], st));
-    if ((rc = run_scan(ix, w, nq, n_filtered, L, st, launches, timed))) return rc;
+    if ((rc = run_scan(ix, w, nq, n_filtered, L, st, launches, true, timed))) return rc;
     ix->last_launches = launches;
     if (timed) {
         PDXG_CUDA(cudaEventRecord(ix->tev[4], st));
@@ -1763,7 +1766,7 @@ int search_host_pipelined(pdxg_index* ix, const float* queries, uint32_t nq, uin
         launches += L.probe_launches;
     }
     ix->last_order_stride = L.p.q_order && !probe_ahead ? k1 : 0;
-    if ((rc = run_scan(ix, w, nq, 0, L, st, launches))) return rc;
+    if ((rc = run_scan(ix, w, nq, 0, L, st, launches, true))) return rc;
     ix->last_launches = launches;
     PDXG_CUDA(cudaMemcpyAsync(ids, w.d_ids, sizeof(uint32_t) * nq * k, cudaMemcpyDeviceToHost, st));
     PDXG_CUDA(cudaMemcpyAsync(dists, w.d_dists, sizeof(float) * nq * k, cudaMemcpyDeviceToHost, st));
@@ -2637,7 +2640,7 @@ int pdxg_search_requests(pdxg_context* ctx, const float* queries, uint32_t nq,
         if ((rc = run_probe_exact(ix, w, qp, nq, L, st))) return rc;
     }
     uint32_t launches = 0;
-    return run_scan(ix, w, nq, n_filtered, L, st, launches);
+    return run_scan(ix, w, nq, n_filtered, L, st, launches, false);
 }
 
 int pdxg_filter_register(pdxg_index* ix, const uint64_t* row_ids, uint64_t n, int32_t* filter_id) {

@@ -54,7 +54,6 @@ constexpr uint32_t kHeavyBit = 0x80000000u;  // visit class: 0 empty, candidates
                                              // kHeavyBit | 1 + its first column / 32 in hv (0: no
                                              // room) a heavy one
 constexpr uint32_t kHeavyPolls = 1u << 20;  // bound of the wait for the heavy values
-template <bool U8>
 constexpr uint32_t kHeavyBlocks = 2;  // horizontal blocks of a heavy work unit
 constexpr uint32_t kBitmapTileMax = 64 * 1024;  // bytes of a work item's bitmaps in shared memory
 
@@ -809,9 +808,9 @@ __device__ __forceinline__ void heavy_unit(const ScanParams& sp, uint32_t cb, ui
                 }
             }
         } else {
-            const uint32_t b0 = (part - 1) * kHeavyBlocks<U8>;
+            const uint32_t b0 = (part - 1) * kHeavyBlocks;
             out += (size_t)(sp.hv_ncp + b0) * sp.hv_cap;
-            constexpr int NB = (int)kHeavyBlocks<U8>;
+            constexpr int NB = (int)kHeavyBlocks;
             if constexpr (U8) {
                 uint4 x[NB][4];
 #pragma unroll
@@ -849,9 +848,13 @@ template <bool U8>
 __device__ __forceinline__ uint32_t heavy_units(const ScanParams& sp) {
     const uint32_t cap = sp.hv_cap / 32, got = sp.hv_alloc[0];
     const uint32_t blocks = got < cap ? got : cap;
-    const uint32_t parts = 1 + (sp.l1.n_hblocks + kHeavyBlocks<U8> - 1) / kHeavyBlocks<U8>;
+    const uint32_t parts = 1 + (sp.l1.n_hblocks + kHeavyBlocks - 1) / kHeavyBlocks;
     const uint32_t total = blocks * parts;
-    const uint32_t chunk = total > 8192u ? 4u : 1u;  // fewer claims where the units are many
+    // units of a claim: a grid has up to 3,552 warps, so with a few units for each of them a claim of
+    // four leaves warps idle, and with many the counter's atomics queue. Replay with claims of 1 and of 4:
+    // 10,000 queries on the 1M x 1024 SQ8 tree 133 and 108 us, 300 exhaustive F32 ones 119 and 166,
+    // 1,000 F32 ones on 316 clusters 37 and 53.
+    const uint32_t chunk = total > 8192u ? 4u : 1u;
     for (;;) {
         uint32_t u = 0;
         if (total && (threadIdx.x & 31) == 0) u = atomicAdd(sp.hv_next, chunk);
@@ -881,8 +884,9 @@ template <bool U8>
 __global__ void __launch_bounds__(kScanWarps * 32, U8 ? 3 : 2) scan_replay_kernel(const __grid_constant__ ScanParams sp) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // Queries that start in the same cluster visit the same ones next: they run at the same time, in
-    // neighbouring CTAs, and find those clusters in L2.
+    // Queries that start in the same cluster visit the same ones next: with one Start a query they run at
+    // the same time, in neighbouring CTAs. (Batches with several Starts a query run in their order; no
+    // difference was measured on indexes whose clusters L2 holds.)
     // warps past r_qpc own no query (no shared-memory region either) and only run heavy units
     const uint32_t units = heavy_units<U8>(sp);
     uint32_t q = warp < sp.r_qpc ? blockIdx.x + warp * gridDim.x : 0xFFFFFFFFu;
