@@ -751,6 +751,55 @@ uint32_t warmup_checkpoints(uint32_t dv, uint32_t* cp, uint32_t cap) {
     return n;
 }
 
+// Every array of the scan's slices as (pointer, capacity).
+template <class F>
+void scan_arrays(Workspace& w, F f) {
+    f(w.d_st_cl, w.st_cl_cap);
+    f(w.d_st_q, w.st_q_cap);
+    f(w.d_st_items, w.st_items_cap);
+    f(w.d_st_dist, w.st_dist_cap);
+    f(w.d_zero, w.zero_cap);
+    f(w.d_sc_qw, w.sc_qw_cap);
+    f(w.d_sc_q, w.sc_q_cap);
+    f(w.d_sc_heap, w.sc_heap_cap);
+    f(w.d_sc_vl, w.sc_vl_cap);
+    f(w.d_sc_items, w.sc_items_cap);
+    f(w.d_sc_bm, w.sc_bm_cap);
+    f(w.d_sc_vi, w.sc_vi_cap);
+    f(w.d_sc_hv, w.sc_hv_cap);
+    f(w.d_sc_hb, w.sc_hb_cap);
+}
+
+// Free device memory, counting what the scan's arrays hold.
+int scan_memory(Workspace& w, uint64_t& bytes) {
+    size_t mem_free = 0, mem_all = 0;
+    PDXG_CUDA(cudaMemGetInfo(&mem_free, &mem_all));
+    bytes = mem_free;
+    scan_arrays(w, [&](auto*& ptr, uint64_t& cap) { bytes += cap * sizeof(*ptr); });
+    return PDXG_OK;
+}
+
+// After an allocation failed: half the room for an array, and at most an eighth of what there is. The
+// workspace keeps that bound, so that a later call (a graph's capture) allocates nothing it did not,
+// until the device has twice the memory (restore_room).
+int shrink_room(Workspace& w) {
+    cudaGetLastError();  // not sticky
+    if (int rc = scan_memory(w, w.free_at)) return rc;
+    w.room = std::min(w.room / 2, w.free_at / 8);
+    return PDXG_OK;
+}
+
+int restore_room(Workspace& w, cudaStream_t st) {
+    if (w.room == kSliceBytes) return PDXG_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PDXG_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return PDXG_OK;
+    uint64_t bytes;
+    if (int rc = scan_memory(w, bytes)) return rc;
+    if (bytes / 2 >= w.free_at) w.room = kSliceBytes;
+    return PDXG_OK;
+}
+
 // Tiled top level (pdxg_toplevel.cu). Returns PDXG_OK with L.p.q_order set when it ran,
 // PDXG_OK with L.p.q_order unset when this index or batch does not fit its limits (the caller
 // then uses the per-query form), or an error.
@@ -773,7 +822,8 @@ int run_top_level_tiled(pdxg_index* ix, Workspace& w, const float* qp, uint32_t 
     for (uint32_t i = 0; i < std::min(top, nL0); ++i) per_query += (uint64_t)strides[i] * tp.nvals;
     if (per_query >= (1ull << 31)) return PDXG_OK;
     const uint64_t vals_bytes = (uint64_t)nq * per_query * 4;
-    if (vals_bytes + (uint64_t)nL0 * nq * 4 > (8ull << 30)) return PDXG_OK;
+    if (int rc = restore_room(w, st)) return rc;
+    if (vals_bytes + (uint64_t)nL0 * nq * 4 > w.room) return PDXG_OK;
     const uint32_t max_n0 = std::max(l0.max_n, 1u);
     if (max_n0 > (1u << 20)) return PDXG_OK;
     tp.probe_q = 16;
@@ -794,15 +844,21 @@ int run_top_level_tiled(pdxg_index* ix, Workspace& w, const float* qp, uint32_t 
     if (ratio_bytes + (uint64_t)warps * wb + 1024 > ix->max_smem) return PDXG_OK;
     tp.r_warp_bytes = (uint32_t)wb;
 
+    cudaError_t e = cudaSuccess;
+    auto grow = [&](auto*& ptr, uint64_t& cap, uint64_t n) {
+        if (e == cudaSuccess) e = dev_try_grow(ptr, cap, n);
+    };
+    grow(w.d_top_order, w.top_order_cap, (uint64_t)nq * top);
+    grow(w.d_top_off, w.top_off_cap, (uint64_t)nq * top);
+    grow(w.d_top_lists, w.top_lists_cap, (uint64_t)nL0 * nq);
+    grow(w.d_top_count, w.top_count_cap, (uint64_t)nL0 + nq);
+    grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)nq * nL0);
+    grow(w.d_top_vals, w.top_vals_cap, std::max<uint64_t>((uint64_t)nq * per_query, 4));
+    if (e == cudaErrorMemoryAllocation) return shrink_room(w);  // the per-query form needs none of them
+    if (e != cudaSuccess) return fail(PDXG_ERR_CUDA, std::string("top-level arrays: ") + cudaGetErrorString(e));
     int rc;
-    if ((rc = dev_grow(w.d_top_order, w.top_order_cap, (uint64_t)nq * top))) return rc;
-    if ((rc = dev_grow(w.d_top_off, w.top_off_cap, (uint64_t)nq * top))) return rc;
-    if ((rc = dev_grow(w.d_top_lists, w.top_lists_cap, (uint64_t)nL0 * nq))) return rc;
-    if ((rc = dev_grow(w.d_top_count, w.top_count_cap, (uint64_t)nL0 + nq))) return rc;
-    if ((rc = dev_grow(w.d_top_vals, w.top_vals_cap, std::max<uint64_t>((uint64_t)nq * per_query, 4)))) return rc;
     if ((rc = dev_grow(w.d_l1_order, w.l1_order_cap, (uint64_t)(q_offset + nq) * k1))) return rc;
     if ((rc = dev_grow(w.d_l1_count, w.l1_count_cap, q_offset + nq))) return rc;
-    if ((rc = dev_grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)nq * nL0))) return rc;
     tp.probe_keys = w.d_pr_keys;
     tp.arena = ix->arena;
     tp.l0 = l0;
@@ -1046,55 +1102,6 @@ int run_probe_gemm(pdxg_index* ix, Workspace& w, const float* q, uint32_t nq, bo
     L.p.q_order = w.d_l1_order;
     L.p.q_order_count = w.d_l1_count;
     L.p.q_order_stride = k1;
-    return PDXG_OK;
-}
-
-// Every array of the scan's slices as (pointer, capacity).
-template <class F>
-void scan_arrays(Workspace& w, F f) {
-    f(w.d_st_cl, w.st_cl_cap);
-    f(w.d_st_q, w.st_q_cap);
-    f(w.d_st_items, w.st_items_cap);
-    f(w.d_st_dist, w.st_dist_cap);
-    f(w.d_zero, w.zero_cap);
-    f(w.d_sc_qw, w.sc_qw_cap);
-    f(w.d_sc_q, w.sc_q_cap);
-    f(w.d_sc_heap, w.sc_heap_cap);
-    f(w.d_sc_vl, w.sc_vl_cap);
-    f(w.d_sc_items, w.sc_items_cap);
-    f(w.d_sc_bm, w.sc_bm_cap);
-    f(w.d_sc_vi, w.sc_vi_cap);
-    f(w.d_sc_hv, w.sc_hv_cap);
-    f(w.d_sc_hb, w.sc_hb_cap);
-}
-
-// Free device memory, counting what the scan's arrays hold.
-int scan_memory(Workspace& w, uint64_t& bytes) {
-    size_t mem_free = 0, mem_all = 0;
-    PDXG_CUDA(cudaMemGetInfo(&mem_free, &mem_all));
-    bytes = mem_free;
-    scan_arrays(w, [&](auto*& ptr, uint64_t& cap) { bytes += cap * sizeof(*ptr); });
-    return PDXG_OK;
-}
-
-// After an allocation failed: half the room for an array, and at most an eighth of what there is. The
-// workspace keeps that bound, so that a later call (a graph's capture) allocates nothing it did not,
-// until the device has twice the memory (restore_room).
-int shrink_room(Workspace& w) {
-    cudaGetLastError();  // not sticky
-    if (int rc = scan_memory(w, w.free_at)) return rc;
-    w.room = std::min(w.room / 2, w.free_at / 8);
-    return PDXG_OK;
-}
-
-int restore_room(Workspace& w, cudaStream_t st) {
-    if (w.room == kSliceBytes) return PDXG_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    PDXG_CUDA(cudaStreamIsCapturing(st, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return PDXG_OK;
-    uint64_t bytes;
-    if (int rc = scan_memory(w, bytes)) return rc;
-    if (bytes / 2 >= w.free_at) w.room = kSliceBytes;
     return PDXG_OK;
 }
 

@@ -1,6 +1,7 @@
 """Searches on a device whose memory is nearly used up: the arrays of the batched Start, the scan and the
-centroid probe shrink to what there is (pdxg_index.cu), results stay the same, the batch can still be
-captured, and with the memory free again the next search takes its whole batch at once."""
+centroid probe shrink to what there is, and a tree's top level takes the form without partials
+(pdxg_index.cu). Results stay the same, the batch can still be captured, and with the memory free again
+the next search takes its whole batch at once."""
 import numpy as np
 import pytest
 
@@ -9,14 +10,16 @@ from pdx_b200 import compiled
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("itype", ["pdx_f32", "pdx_u8"])
-def test_arrays_shrink_to_the_free_memory(itype):
+@pytest.mark.parametrize("itype,d,nlist,nprobe", [("pdx_f32", 16, 10, 0), ("pdx_u8", 16, 10, 0),
+                                                  ("pdx_tree_f32", 128, 1000, 64)])  # 0.9 GB of partials
+def test_arrays_shrink_to_the_free_memory(itype, d, nlist, nprobe):
     import torch
-    n, d, nq, k = 20_000, 16, 60_000, 10
+    n, nq, k = 20_000, 60_000, 10
     rng = np.random.default_rng(5)
-    ix = compiled.PDXIndex(itype, d, seed=11, num_clusters=10, normalize=False)
+    ix = compiled.PDXIndex(itype, d, seed=11, num_clusters=nlist, num_meso_clusters=32 if "tree" in itype else 0,
+                           normalize=False)
     ix.build_index(rng.standard_normal((n, d)).astype(np.float32))
-    ix.set_nprobe(0)
+    ix.set_nprobe(nprobe)
     q = torch.from_numpy(ix.prepare_queries(rng.standard_normal((nq, d)).astype(np.float32))).cuda()
     ids = torch.empty(nq, k, dtype=torch.int32, device="cuda")
     dist = torch.empty(nq, k, device="cuda")
@@ -34,9 +37,11 @@ def test_arrays_shrink_to_the_free_memory(itype):
     run(ix, 3000)  # the kernels of every route are loaded
     ix.set_scan_mode(1)
     ix.set_start_mode(1)
+    ix.set_top_level_mode(2)
     expect = run(ix)  # the per-query route: its buffers are there from now on
     ix.set_scan_mode(0)
     ix.set_start_mode(0)
+    ix.set_top_level_mode(0)
     torch.cuda.empty_cache()
     filler = []
     for keep in (8 << 30, 160 << 20):
