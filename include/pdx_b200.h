@@ -280,7 +280,8 @@ int pdxg_set_start_mode(pdxg_index* index, uint32_t mode);
 int pdxg_set_probe_mode(pdxg_index* index, uint32_t mode);
 
 /* The L1 visit orders of the last pdxg_search_device call, when it computed them ahead of the
- * scan (tree top level in its own launch, or probe modes 1 and 2): orders[i * stride + j] for
+ * scan (tree top level in its own launch, the exact probe of a flat index for 32 queries or more, or
+ * probe modes 1 and 2): orders[i * stride + j] for
  * j < counts[i]. Waits for the device. No counterpart in the reference. */
 int pdxg_last_visit_orders(pdxg_index* index, uint32_t nq, uint32_t stride, uint32_t* orders, uint32_t* counts);
 

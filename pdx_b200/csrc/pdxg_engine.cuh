@@ -28,8 +28,10 @@ int fail(int code, const std::string& msg);
 #define PDXG_CUDA(x)                                                                      \
     do {                                                                                  \
         cudaError_t e_ = (x);                                                             \
-        if (e_ != cudaSuccess)                                                            \
+        if (e_ != cudaSuccess) {                                                          \
+            cudaGetLastError(); /* reported here, not by the next launch */               \
             return fail(PDXG_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
+        }                                                                                 \
     } while (0)
 
 inline uint32_t next_pow2(uint32_t x) {
@@ -265,8 +267,8 @@ cudaError_t dev_try_grow(T*& ptr, uint64_t& cap, uint64_t need) {
 
 template <class T>
 int dev_grow(T*& ptr, uint64_t& cap, uint64_t need) {
-    const cudaError_t e = dev_try_grow(ptr, cap, need);
-    return e == cudaSuccess ? PDXG_OK : fail(PDXG_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    PDXG_CUDA(dev_try_grow(ptr, cap, need));
+    return PDXG_OK;
 }
 
 // Search plumbing (pdxg_index.cu).

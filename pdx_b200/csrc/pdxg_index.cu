@@ -855,7 +855,7 @@ int run_top_level_tiled(pdxg_index* ix, Workspace& w, const float* qp, uint32_t 
     grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)nq * nL0);
     grow(w.d_top_vals, w.top_vals_cap, std::max<uint64_t>((uint64_t)nq * per_query, 4));
     if (e == cudaErrorMemoryAllocation) return shrink_room(w);  // the per-query form needs none of them
-    if (e != cudaSuccess) return fail(PDXG_ERR_CUDA, std::string("top-level arrays: ") + cudaGetErrorString(e));
+    PDXG_CUDA(e);
     int rc;
     if ((rc = dev_grow(w.d_l1_order, w.l1_order_cap, (uint64_t)(q_offset + nq) * k1))) return rc;
     if ((rc = dev_grow(w.d_l1_count, w.l1_count_cap, q_offset + nq))) return rc;
@@ -1132,8 +1132,7 @@ int run_probe_exact(pdxg_index* ix, Workspace& w, const float* qp, uint32_t nq, 
         pp.keys_rows = (uint32_t)std::min<uint64_t>(rows, std::max<uint64_t>(std::min(kProbeKeysMax, w.room / 4) / n1, 32));
         e = dev_try_grow(w.d_pr_keys, w.pr_keys_cap, (uint64_t)pp.keys_rows * n1);
         if (e == cudaSuccess) break;
-        if (e != cudaErrorMemoryAllocation || pp.keys_rows <= 32)
-            return fail(PDXG_ERR_CUDA, std::string("probe distances: ") + cudaGetErrorString(e));
+        if (e != cudaErrorMemoryAllocation || pp.keys_rows <= 32) PDXG_CUDA(e);
         if ((rc = shrink_room(w))) return rc;
     }
     pp.keys = w.d_pr_keys;
@@ -1292,7 +1291,7 @@ int reserve_slices(pdxg_index* ix, Workspace& w, const Launch& L, uint32_t nq, S
             return dev_try_grow(ptr, cap, n);
         });
         if (e == cudaSuccess) return PDXG_OK;
-        if (e != cudaErrorMemoryAllocation) return fail(PDXG_ERR_CUDA, std::string("scan arrays: ") + cudaGetErrorString(e));
+        if (e != cudaErrorMemoryAllocation) PDXG_CUDA(e);
         g_alloc_gen.fetch_add(1);
         scan_arrays(w, [](auto*& ptr, uint64_t& cap) {
             cudaFree(ptr);

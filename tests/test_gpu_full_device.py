@@ -59,3 +59,29 @@ def test_arrays_shrink_to_the_free_memory(itype, d, nlist, nprobe):
     for a, b in zip(run(ix), expect):
         np.testing.assert_array_equal(a, b)
     assert ix.last_launch_count() < sliced
+
+
+def test_a_search_after_a_refused_one():
+    """A batch whose results have no room is refused; the next search does not report that again."""
+    import torch
+    n, d = 2_000, 16
+    rng = np.random.default_rng(6)
+    ix = compiled.PDXIndex("pdx_f32", d, seed=11, num_clusters=10, normalize=False)
+    ix.build_index(rng.standard_normal((n, d)).astype(np.float32))
+    ix.set_nprobe(0)
+    q = rng.standard_normal((200_000, d)).astype(np.float32)
+    expect = ix.search_batch(q[:64], 10)
+    torch.cuda.empty_cache()
+    filler = []
+    for keep in (8 << 30, 160 << 20):
+        size = torch.cuda.mem_get_info()[0] - keep
+        if size > 0:
+            filler.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+    try:
+        with pytest.raises(RuntimeError):
+            ix.search_batch(q, 300)  # 480 MB of results
+        for a, b in zip(ix.search_batch(q[:64], 10), expect):
+            np.testing.assert_array_equal(a, b)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
