@@ -1,7 +1,7 @@
 """Host time of a search on an index of 40,000 clusters: the number of batched Starts and the width of
 the per-query scan look the cluster sizes up instead of collecting them for every search. k 40 (every
 cluster is smaller) took 1.5 to 2 times the host time of k 1 (none is); both now enqueue the same
-kernels in the same time. Medians of 60 calls, the best of three. Results with k 40 equal the per-query route's, also
+kernels in the same time. The best of 180 calls each. Results with k 40 equal the per-query route's, also
 after Append and Delete changed sizes."""
 import time
 
@@ -34,7 +34,7 @@ def test_host_time_does_not_grow_with_the_clusters_below_k():
                              stream=stream.cuda_stream)
             times.append(time.perf_counter() - t)
             torch.cuda.synchronize()
-        return float(np.median(times)), (ids.cpu().numpy(), dist.cpu().numpy(), cnt.cpu().numpy())
+        return min(times), (ids.cpu().numpy(), dist.cpu().numpy(), cnt.cpu().numpy())
 
     run(1)
     few = min(run(1)[0] for _ in range(3))
